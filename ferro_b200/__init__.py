@@ -1,7 +1,8 @@
 """ferro_b200 - B200-native batched token sampler behind the interface of ferro's ``Sampler``.
 
 The product is the C-ABI shared library built from ``ferro_b200/csrc`` (hand-written sm_100a CUDA kernels plus
-a C++ host shim; no PyTorch inside).  This module is a thin ctypes binding used by the tests and the benchmark:
+a C++ host shim; no PyTorch inside).  This module is a thin binding used by the tests and the benchmark; the calls of a
+decode loop go through a small native module (``csrc/fsb_python.cpp``), the rest through ctypes:
 
 * :class:`Engine`   - one sampler engine on one CUDA device (``fsb_create``), batched calls;
 * :class:`Sampler`  - the reference's class shape: ``Sampler(params).sample(logits, n_vocab, history)``
@@ -14,6 +15,7 @@ There is no CPU fallback: if the library is missing it is built with nvcc, and w
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 import numpy as np
@@ -68,6 +70,7 @@ class _Counters(C.Structure):
 
 
 _lib = None
+_native = None   # the native half of the binding, loaded with the library
 
 
 def library_path() -> str:
@@ -76,7 +79,7 @@ def library_path() -> str:
 
 def load_library(build_if_missing: bool = True):
     """Load (building first if needed) the C-ABI library.  Never falls back to anything else."""
-    global _lib
+    global _lib, _native
     if _lib is not None:
         return _lib
     if build_if_missing:
@@ -84,6 +87,9 @@ def load_library(build_if_missing: bool = True):
     if not os.path.exists(_build.LIB_PATH):
         raise FileNotFoundError(f"{_build.LIB_PATH} is missing: build it with `python -m ferro_b200._build`")
     L = C.CDLL(_build.LIB_PATH)
+    spec = importlib.util.spec_from_file_location("_fsb_native", _build.EXT_PATH)
+    _native = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(_native)
     vp, i32, i64, u32, u64 = C.c_void_p, C.c_int, C.c_int64, C.c_uint, C.c_uint64
     L.fsb_create.argtypes = [i32, i32, i32, i64, C.POINTER(vp)]
     L.fsb_destroy.argtypes = [vp]
@@ -161,7 +167,7 @@ def _flatten_hist(hists):
     return flat, off
 
 
-def _logits_pointer(logits, n_rows, n_vocab, flags):
+def _logits_pointer(logits, n_vocab, flags):
     """Accepts a numpy array (host), an int device pointer, or any object with ``data_ptr()`` (device tensor)."""
     if isinstance(logits, np.ndarray):
         if logits.dtype != np.float32:
@@ -170,10 +176,10 @@ def _logits_pointer(logits, n_rows, n_vocab, flags):
             logits = logits.reshape(1, -1)
         if logits.strides[-1] != 4 or logits.strides[0] % 4:
             raise ValueError("logits rows must be contiguous")
-        return logits.ctypes.data, logits.strides[0] // 4, flags | LOGITS_ON_HOST, logits
+        return logits.__array_interface__["data"][0], logits.strides[0] // 4, flags | LOGITS_ON_HOST, logits
     if hasattr(logits, "data_ptr"):
         ld = logits.stride(0) if logits.dim() == 2 else n_vocab
-        return int(logits.data_ptr()), int(ld), flags & ~LOGITS_ON_HOST, logits
+        return logits.data_ptr(), ld, flags & ~LOGITS_ON_HOST, logits
     raise TypeError("logits: numpy array or device tensor expected")
 
 
@@ -182,12 +188,15 @@ class Batch:
 
     def __init__(self, engine: "Engine", ptr, n_rows: int):
         self.engine, self._ptr, self.n_rows = engine, ptr, n_rows
+        self._pv = ptr.value or 0   # the same handle as an integer, for the native calls
 
     def redraw(self):
-        self.engine._check(self.engine.lib.fsb_batch_redraw(self.engine._h, self._ptr))
+        self.engine._check(_native.batch_redraw(self.engine._hv, self._pv))
 
     def launch(self, logits_dev_ptr: int):
-        self.engine._check(self.engine.lib.fsb_batch_launch(self.engine._h, self._ptr, C.c_void_p(int(logits_dev_ptr))))
+        rc = _native.batch_launch(self.engine._hv, self._pv, logits_dev_ptr)
+        if rc:
+            self.engine._check(rc)
 
     def shard_launch(self, logits_shard_dev_ptr: int, lists_out_dev_ptr: int, counts_out_dev_ptr: int):
         """Vocabulary-sharded first half: this device's best k candidates per row (``fsb_batch_shard_launch``)."""
@@ -206,13 +215,13 @@ class Batch:
 
     def shard_launch_packed(self, logits_shard_dev_ptr: int, packed_out_dev_ptr: int, stride_words: int):
         """``fsb_batch_shard_launch_packed``: per row [count, candidates ...] in `stride_words` 64-bit words."""
-        self.engine._check(self.engine.lib.fsb_batch_shard_launch_packed(self.engine._h, self._ptr, C.c_void_p(int(logits_shard_dev_ptr)),
-                                                                         C.c_void_p(int(packed_out_dev_ptr)), int(stride_words)))
+        self.engine._check(_native.batch_shard_launch_packed(self.engine._hv, self._pv, int(logits_shard_dev_ptr), int(packed_out_dev_ptr),
+                                                             int(stride_words)))
 
     def merge_launch_packed(self, packed_dev_ptr: int, stride_words: int, n_lists: int, row_begin: int, n_rows: int):
         """``fsb_batch_merge_launch_packed``: finish rows [row_begin, row_begin + n_rows) from [n_lists][n_rows][stride_words]."""
-        self.engine._check(self.engine.lib.fsb_batch_merge_launch_packed(self.engine._h, self._ptr, C.c_void_p(int(packed_dev_ptr)), int(stride_words),
-                                                                         int(n_lists), int(row_begin), int(n_rows)))
+        self.engine._check(_native.batch_merge_launch_packed(self.engine._hv, self._pv, int(packed_dev_ptr), int(stride_words), int(n_lists),
+                                                             int(row_begin), int(n_rows)))
 
     @property
     def tokens_device_ptr(self) -> int:
@@ -221,7 +230,7 @@ class Batch:
 
     def check(self):
         """Waits for the batch's launches and raises if the device reported an error."""
-        self.engine._check(self.engine.lib.fsb_batch_check(self.engine._h, self._ptr))
+        self.engine._check(_native.batch_check(self.engine._hv, self._pv))
 
     def tokens(self) -> np.ndarray:
         out = np.zeros(self.n_rows, dtype=np.int32)
@@ -235,7 +244,7 @@ class Batch:
     def free(self):
         if self._ptr:
             self.engine.lib.fsb_batch_free(self.engine._h, self._ptr)
-            self._ptr = None
+            self._ptr, self._pv = None, 0
 
 
 class Engine:
@@ -248,6 +257,7 @@ class Engine:
         if rc != 0:
             raise SamplerError(rc, "fsb_create failed (a CUDA device of compute capability 10.x is required; there is no CPU path)")
         self._h = h
+        self._hv = h.value   # the same handle as an integer, for the native calls
         self.max_rows, self.max_vocab = max_rows, max_vocab
 
     # -- plumbing
@@ -258,7 +268,7 @@ class Engine:
     def close(self):
         if getattr(self, "_h", None):
             self.lib.fsb_destroy(self._h)
-            self._h = None
+            self._h, self._hv = None, 0
 
     def __del__(self):
         try:
@@ -290,15 +300,15 @@ class Engine:
     # -- streams
     def open_stream(self, params) -> int:
         p = np.ascontiguousarray(np.asarray(params, dtype=PARAMS_DTYPE).reshape(-1)[:1])
-        sid = C.c_int(-1)
-        self._check(self.lib.fsb_stream_open(self._h, p.ctypes.data, C.byref(sid)))
-        return sid.value
+        rc, sid = _native.open_stream(self._hv, p.view(np.uint8))
+        self._check(rc)
+        return sid
 
     def open_streams(self, params) -> np.ndarray:
         return np.array([self.open_stream(params[i:i + 1]) for i in range(len(params))], dtype=np.int32)
 
     def close_stream(self, sid: int):
-        self._check(self.lib.fsb_stream_close(self._h, int(sid)))
+        self._check(_native.close_stream(self._hv, int(sid)))
 
     def stream_params(self, sid: int) -> np.ndarray:
         p = np.zeros(1, dtype=PARAMS_DTYPE)
@@ -315,60 +325,30 @@ class Engine:
 
     # -- sampling
     def sample_batch(self, stream_ids, logits, histories, n_vocab: int | None = None, flags: int = 0) -> np.ndarray:
-        sids = np.ascontiguousarray(stream_ids, dtype=np.int32)
-        n_rows = len(sids)
         if n_vocab is None:
             n_vocab = int(logits.shape[-1])
-        ptr, ld, flags, keep = _logits_pointer(logits, n_rows, n_vocab, flags)
-        flat, off = _flatten_hist(histories)
-        tokens = np.zeros(n_rows, dtype=np.int32)
-        self._check(self.lib.fsb_sample_batch(self._h, n_rows, sids.ctypes.data, C.c_void_p(ptr), ld, n_vocab, flat.ctypes.data,
-                                              off.ctypes.data, tokens.ctypes.data, flags))
-        return tokens
+        ptr, ld, flags, keep = _logits_pointer(logits, n_vocab, flags)
+        out = _native.sample_batch(self._hv, stream_ids, ptr, ld, n_vocab, histories, flags)
+        if type(out) is int:
+            self._check(out)
+        return out
 
     def verify_windows(self, stream_ids, rows, logits, histories, n_vocab: int | None = None, max_accept=None, flags: int = 0):
         """rows: per stream [last token, draft_1, ...].  Returns (tokens[list of arrays], acc, confirmed)."""
-        sids = np.ascontiguousarray(stream_ids, dtype=np.int32)
-        n_streams = len(sids)
-        row_off = np.zeros(n_streams + 1, dtype=np.int32)
-        for i, r in enumerate(rows):
-            row_off[i + 1] = row_off[i] + len(r)
-        rows_flat = np.concatenate([np.asarray(r, dtype=np.int32) for r in rows]).astype(np.int32)
-        n_rows = int(row_off[-1])
+        return self._verify(stream_ids, rows, logits, histories, n_vocab, max_accept, flags)
+
+    def _verify(self, stream_ids, rows, logits, histories, n_vocab, max_accept, flags):
         if n_vocab is None:
             n_vocab = int(logits.shape[-1])
-        ptr, ld, flags, keep = _logits_pointer(logits, n_rows, n_vocab, flags)
-        flat, off = _flatten_hist(histories)
-        tokens = np.zeros(n_rows, dtype=np.int32)
-        acc = np.zeros(n_streams, dtype=np.int32)
-        conf = np.zeros(n_streams, dtype=np.int32)
-        ma = np.ascontiguousarray(max_accept, dtype=np.int32) if max_accept is not None else None
-        self._check(self.lib.fsb_verify_windows(self._h, n_streams, sids.ctypes.data, row_off.ctypes.data, rows_flat.ctypes.data,
-                                                C.c_void_p(ptr), ld, n_vocab, flat.ctypes.data, off.ctypes.data,
-                                                ma.ctypes.data if ma is not None else None, tokens.ctypes.data, acc.ctypes.data,
-                                                conf.ctypes.data, flags))
-        return [tokens[row_off[i]:row_off[i + 1]] for i in range(n_streams)], acc, conf
+        ptr, ld, flags, keep = _logits_pointer(logits, n_vocab, flags)
+        out = _native.verify_windows(self._hv, stream_ids, rows, ptr, ld, n_vocab, histories, max_accept, flags)
+        if type(out) is int:
+            self._check(out)
+        return out
 
     def verify_windows_resident(self, stream_ids, rows, logits, n_vocab: int | None = None, max_accept=None, flags: int = 0):
         """``verify_windows`` with the streams' resident histories; with APPEND_SAMPLED the accepted tokens are appended."""
-        sids = np.ascontiguousarray(stream_ids, dtype=np.int32)
-        n_streams = len(sids)
-        row_off = np.zeros(n_streams + 1, dtype=np.int32)
-        for i, r in enumerate(rows):
-            row_off[i + 1] = row_off[i] + len(r)
-        rows_flat = np.concatenate([np.asarray(r, dtype=np.int32) for r in rows]).astype(np.int32)
-        n_rows = int(row_off[-1])
-        if n_vocab is None:
-            n_vocab = int(logits.shape[-1])
-        ptr, ld, flags, keep = _logits_pointer(logits, n_rows, n_vocab, flags)
-        tokens = np.zeros(n_rows, dtype=np.int32)
-        acc = np.zeros(n_streams, dtype=np.int32)
-        conf = np.zeros(n_streams, dtype=np.int32)
-        ma = np.ascontiguousarray(max_accept, dtype=np.int32) if max_accept is not None else None
-        self._check(self.lib.fsb_verify_windows_resident(self._h, n_streams, sids.ctypes.data, row_off.ctypes.data, rows_flat.ctypes.data,
-                                                         C.c_void_p(ptr), ld, n_vocab, ma.ctypes.data if ma is not None else None,
-                                                         tokens.ctypes.data, acc.ctypes.data, conf.ctypes.data, flags))
-        return [tokens[row_off[i]:row_off[i + 1]] for i in range(n_streams)], acc, conf
+        return self._verify(stream_ids, rows, logits, None, n_vocab, max_accept, flags)
 
     def last_kept(self, row: int, cap: int = MAX_CANDIDATE_K):
         ids = np.zeros(cap, dtype=np.int32)
@@ -380,25 +360,17 @@ class Engine:
 
     # ---- device-resident histories (fsb_stream_history_*, fsb_sample_batch_resident)
     def history_set(self, stream_id: int, ids):
-        a = np.ascontiguousarray(ids, dtype=np.int32)
-        self._check(self.lib.fsb_stream_history_set(self._h, int(stream_id), a.ctypes.data, len(a)))
+        self._check(_native.history_set(self._hv, int(stream_id), ids))
 
     def history_append(self, stream_id: int, ids):
-        a = np.ascontiguousarray(np.atleast_1d(ids), dtype=np.int32)
-        self._check(self.lib.fsb_stream_history_append(self._h, int(stream_id), a.ctypes.data, len(a)))
+        self._check(_native.history_append(self._hv, int(stream_id), ids))
 
     def lookup_drafts(self, stream_ids, kmax, min_n, eos: int):
         """Prompt-lookup drafts of resident histories (``fsb_lookup_drafts_resident``): a list of int32 arrays."""
-        sids = np.ascontiguousarray(stream_ids, dtype=np.int32)
-        n = len(sids)
-        km = np.ascontiguousarray(np.broadcast_to(np.asarray(kmax, dtype=np.int32), (n,)))
-        mn = np.ascontiguousarray(np.broadcast_to(np.asarray(min_n, dtype=np.int32), (n,)))
-        stride = max(int(km.max()) if n else 1, 1)
-        out = np.zeros((n, stride), dtype=np.int32)
-        cnt = np.zeros(n, dtype=np.int32)
-        self._check(self.lib.fsb_lookup_drafts_resident(self._h, n, sids.ctypes.data, km.ctypes.data, mn.ctypes.data, int(eos), out.ctypes.data,
-                                                        stride, cnt.ctypes.data))
-        return [out[i, : cnt[i]].copy() for i in range(n)]
+        out = _native.lookup_drafts(self._hv, stream_ids, kmax, min_n, int(eos))
+        if type(out) is int:
+            self._check(out)
+        return out
 
     def history_len(self, stream_id: int) -> int:
         n = C.c_int64(0)
@@ -408,7 +380,6 @@ class Engine:
     def sample_batch_resident(self, stream_ids, logits, n_vocab: int | None = None, ld: int | None = None, flags: int = 0) -> np.ndarray:
         """``fsb_sample_batch`` with every row's history taken from its stream's resident history.  `logits` is a
         host float32 array (FSB_LOGITS_ON_HOST is added) or an int device pointer (then n_vocab is required)."""
-        sids = np.ascontiguousarray(stream_ids, dtype=np.int32)
         if isinstance(logits, np.ndarray):
             assert logits.dtype == np.float32 and logits.ndim == 2 and logits.flags.c_contiguous
             n_vocab = logits.shape[1] if n_vocab is None else n_vocab
@@ -416,8 +387,9 @@ class Engine:
             ptr, flags = logits.ctypes.data, flags | LOGITS_ON_HOST
         else:
             ptr, ld = int(logits), (n_vocab if ld is None else ld)
-        out = np.zeros(len(sids), dtype=np.int32)
-        self._check(self.lib.fsb_sample_batch_resident(self._h, len(sids), sids.ctypes.data, C.c_void_p(ptr), ld, n_vocab, out.ctypes.data, flags))
+        out = _native.sample_batch_resident(self._hv, stream_ids, ptr, ld, n_vocab, flags)
+        if type(out) is int:
+            self._check(out)
         return out
 
     def prepare_batch(self, stream_ids, histories, n_vocab: int, ld: int | None = None, flags: int = 0) -> Batch:
@@ -465,8 +437,7 @@ class Sampler:
         self._sid = self.engine.open_stream(params)
 
     def sample(self, logits: np.ndarray, n_vocab: int, history) -> int:
-        row = logits.reshape(1, -1)[:, :n_vocab] if logits.shape[-1] != n_vocab else logits.reshape(1, -1)
-        tok = self.engine.sample_batch([self._sid], row, [np.asarray(history, dtype=np.int32)], n_vocab=n_vocab, flags=WRITE_BACK)
+        tok = self.engine.sample_batch([self._sid], logits.reshape(1, -1), [history], n_vocab=n_vocab, flags=WRITE_BACK)
         return int(tok[0])
 
     def params(self) -> np.ndarray:

@@ -136,3 +136,16 @@ int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows,
                            int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream);
 
 }  // namespace fsb
+
+// fsb_sample_batch and fsb_verify_windows with one history array per row / stream instead of a packed one; for the
+// Python binding (fsb_python.cpp), whose callers hold one array per slot.
+struct fsb_handle;
+extern "C" {
+__attribute__((visibility("default"))) int fsb_sample_batch_lists(fsb_handle* h, int n_rows, const int* stream_ids, const float* logits, int64_t ld,
+                                                                  int n_vocab, const int32_t* const* hist_lists, const int64_t* hist_lens,
+                                                                  int32_t* tokens_out, unsigned flags);
+__attribute__((visibility("default"))) int fsb_verify_windows_lists(fsb_handle* h, int n_streams, const int* stream_ids, const int* row_off,
+                                                                    const int32_t* rows_flat, const float* logits, int64_t ld, int n_vocab,
+                                                                    const int32_t* const* hist_lists, const int64_t* hist_lens, const int* max_accept,
+                                                                    int32_t* tokens_out, int* acc_out, int* confirmed_out, unsigned flags);
+}

@@ -149,6 +149,18 @@ int fail(fsb_handle* h, int code, const char* fmt, ...) {
 
 bool is_greedy(const ferro_sampler_params& p) { return p.temperature <= 0.0f || p.top_k == 1; }   // src/sampler.cpp:19
 
+// Where a call's explicit histories lie: packed behind one another with offsets, or one array per stream (a scheduler
+// keeps one growing vector per slot: only the windows are read, and nothing has to be packed first).
+struct HistSource {
+    const int32_t* flat;
+    const int64_t* off;
+    const int32_t* const* lists;
+    const int64_t* lens;
+    bool ok() const { return off != nullptr || (lists != nullptr && lens != nullptr); }
+    int64_t len(int i) const { return off ? off[i + 1] - off[i] : lens[i]; }
+    const int32_t* data(int i) const { return off ? (flat ? flat + off[i] : nullptr) : lists[i]; }
+};
+
 // penalty window [b, len) of src/sampler.cpp:11-14; returns len when the window is empty or the penalty is off
 int64_t window_begin(const ferro_sampler_params& p, int64_t len) {
     if (p.repetition_penalty == 1.0f || p.repeat_last_n == 0 || len <= 0) return len;
@@ -440,20 +452,19 @@ void rollback_draws(fsb_handle* h, const fsb_batch* b) {
 }
 
 // Stages rows "stream_ids[i] samples row i with history i" into batch b.  Consumes engine outputs.
-int stage_rows(fsb_handle* h, fsb_batch* b, int n_rows, const int* stream_ids, int64_t ld, int n_vocab, const int32_t* hist_flat,
-               const int64_t* hist_off, unsigned flags) {
+int stage_rows(fsb_handle* h, fsb_batch* b, int n_rows, const int* stream_ids, int64_t ld, int n_vocab, const HistSource& hist, unsigned flags) {
     int rc = check_common(h, n_rows, ld, n_vocab, b);
     if (rc) return rc;
     if (!stream_ids) return fail(h, FSB_ERR_INVALID, "stream_ids is null");
-    if (!hist_off) return fail(h, FSB_ERR_INVALID, "hist_off is null");
+    if (!hist.ok()) return fail(h, FSB_ERR_INVALID, "hist_off is null");
     // first pass: validate and size the staged windows, without touching any engine
     int64_t need = 0;
     for (int i = 0; i < n_rows; ++i) {
         Stream* s = get_stream(h, stream_ids[i]);
         if (!s) return fail(h, FSB_ERR_STREAM_ID, "row %d: unknown stream id %d", i, stream_ids[i]);
-        const int64_t len = hist_off[i + 1] - hist_off[i];
+        const int64_t len = hist.len(i);
         if (len < 0) return fail(h, FSB_ERR_INVALID, "row %d: hist_off is not ascending", i);
-        if (len > 0 && !hist_flat) return fail(h, FSB_ERR_INVALID, "hist_flat is null");
+        if (len > 0 && !hist.data(i)) return fail(h, FSB_ERR_INVALID, "hist_flat is null");
         need += len - window_begin(s->p, len);
     }
     if (need > b->cap_hist) return fail(h, FSB_ERR_CAPACITY, "%lld penalty-window ids exceed the capacity of %lld", (long long)need,
@@ -470,9 +481,9 @@ int stage_rows(fsb_handle* h, fsb_batch* b, int n_rows, const int* stream_ids, i
     int64_t pos = 0;
     for (int i = 0; i < n_rows; ++i) {
         Stream* s = get_stream(h, stream_ids[i]);
-        const int64_t len = hist_off[i + 1] - hist_off[i];
+        const int64_t len = hist.len(i);
         const int64_t wb = window_begin(s->p, len), wl = len - wb;
-        if (wl > 0) std::memcpy(hs + pos, hist_flat + hist_off[i] + wb, sizeof(int32_t) * (size_t)wl);
+        if (wl > 0) std::memcpy(hs + pos, hist.data(i) + wb, sizeof(int32_t) * (size_t)wl);
         uint64_t word = 0;
         if (!is_greedy(s->p)) {   // exactly one engine output per stochastic call, none per greedy call
             word = s->rng();
@@ -784,13 +795,13 @@ int fsb_stream_state_set(fsb_handle* h, int stream_id, uint64_t seed, uint64_t d
     return FSB_OK;
 }
 
-int fsb_sample_batch(fsb_handle* h, int n_rows, const int* stream_ids, const float* logits, int64_t ld, int n_vocab,
-                     const int32_t* hist_flat, const int64_t* hist_off, int32_t* tokens_out, unsigned flags) {
+static int sample_batch_impl(fsb_handle* h, int n_rows, const int* stream_ids, const float* logits, int64_t ld, int n_vocab, const HistSource& hist,
+                             int32_t* tokens_out, unsigned flags) {
     if (!h) return FSB_ERR_INVALID;
     if (!logits || !tokens_out) return fail(h, FSB_ERR_INVALID, "null logits or tokens_out");
     cudaSetDevice(h->device);
     fsb_batch* b = h->own;
-    int rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, hist_flat, hist_off, flags);
+    int rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, hist, flags);
     if (rc) return rc;
     rc = run_staged(h, b, logits, flags, false, tokens_out);
     if (rc) return rc;
@@ -802,6 +813,15 @@ int fsb_sample_batch(fsb_handle* h, int n_rows, const int* stream_ids, const flo
     }
     count_rows(h, b);
     return FSB_OK;
+}
+
+int fsb_sample_batch(fsb_handle* h, int n_rows, const int* stream_ids, const float* logits, int64_t ld, int n_vocab,
+                     const int32_t* hist_flat, const int64_t* hist_off, int32_t* tokens_out, unsigned flags) {
+    return sample_batch_impl(h, n_rows, stream_ids, logits, ld, n_vocab, HistSource{hist_flat, hist_off, nullptr, nullptr}, tokens_out, flags);
+}
+int fsb_sample_batch_lists(fsb_handle* h, int n_rows, const int* stream_ids, const float* logits, int64_t ld, int n_vocab,
+                           const int32_t* const* hist_lists, const int64_t* hist_lens, int32_t* tokens_out, unsigned flags) {
+    return sample_batch_impl(h, n_rows, stream_ids, logits, ld, n_vocab, HistSource{nullptr, nullptr, hist_lists, hist_lens}, tokens_out, flags);
 }
 
 int fsb_stream_history_set(fsb_handle* h, int stream_id, const int32_t* ids, int64_t n) {
@@ -944,12 +964,12 @@ int fsb_sample_batch_resident(fsb_handle* h, int n_rows, const int* stream_ids, 
     return FSB_OK;
 }
 
-// The two window calls share everything but where a stream's history comes from: `hist_flat` / `hist_off` (host
-// memory, staged with the call) or, when hist_off is null, the streams' resident histories.
+// The window calls share everything but where a stream's history comes from: `hist` (host memory, staged with the
+// call) or, when it is null, the streams' resident histories.
 static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_ids, const int* row_off, const int32_t* rows_flat,
-                               const float* logits, int64_t ld, int n_vocab, const int32_t* hist_flat, const int64_t* hist_off,
+                               const float* logits, int64_t ld, int n_vocab, const HistSource* hist,
                                const int* max_accept, int32_t* tokens_out, int* acc_out, int* confirmed_out, unsigned flags) {
-    const bool resident = hist_off == nullptr;
+    const bool resident = hist == nullptr;
     if (!stream_ids || !row_off || !rows_flat || !logits || !tokens_out || !acc_out) return fail(h, FSB_ERR_INVALID, "null argument");
     if (n_streams <= 0) return fail(h, FSB_ERR_INVALID, "n_streams must be positive");
     if (flags & FSB_WRITE_BACK) return fail(h, FSB_ERR_INVALID, "write-back is not defined for verification windows");
@@ -969,11 +989,11 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
         if (s->seen == h->call_no) return fail(h, FSB_ERR_INVALID, "stream id %d appears twice", stream_ids[i]);
         s->seen = h->call_no;
         const int m = row_off[i + 1] - row_off[i];
-        const int64_t len = resident ? (int64_t)s->hist.size() : hist_off[i + 1] - hist_off[i];
+        const int64_t len = resident ? (int64_t)s->hist.size() : hist->len(i);
         if (m <= 0 || len < 0) return fail(h, FSB_ERR_INVALID, "stream %d: empty window or bad history offsets", i);
         if (resident && (flags & FSB_APPEND_SAMPLED) && m - 1 > fsb::kWindowTableInts - 6)
             return fail(h, FSB_ERR_CAPACITY, "stream %d: a resident window with FSB_APPEND_SAMPLED holds at most %d drafts", i, fsb::kWindowTableInts - 6);
-        if (!resident && len > 0 && !hist_flat) return fail(h, FSB_ERR_INVALID, "hist_flat is null");
+        if (!resident && len > 0 && !hist->data(i)) return fail(h, FSB_ERR_INVALID, "hist_flat is null");
         need += resident ? 0 : (len - window_begin(s->p, len)) + (m - 1);
     }
     if (need > b->cap_hist) return fail(h, FSB_ERR_CAPACITY, "%lld penalty-window ids exceed the capacity of %lld", (long long)need,
@@ -1002,7 +1022,7 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
     for (int i = 0; i < n_streams; ++i) {
         Stream* s = get_stream(h, stream_ids[i]);
         const int r0 = row_off[i], m = row_off[i + 1] - r0;
-        const int64_t len = resident ? (int64_t)s->hist.size() : hist_off[i + 1] - hist_off[i];
+        const int64_t len = resident ? (int64_t)s->hist.size() : hist->len(i);
         const bool pen_on = !(s->p.repetition_penalty == 1.0f || s->p.repeat_last_n == 0);
         // row r samples with history_i followed by draft_1..draft_r; the windows of successive rows only move
         // forward, so one copy [b_0 .. len + m - 1) serves the whole stream: staged here, or the stream's pool region
@@ -1011,7 +1031,7 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
         if (resident) {
             base = s->pool_off + b0;
         } else if (pen_on) {
-            if (len > b0) std::memcpy(hs + pos, hist_flat + hist_off[i] + b0, sizeof(int32_t) * (size_t)(len - b0));
+            if (len > b0) std::memcpy(hs + pos, hist->data(i) + b0, sizeof(int32_t) * (size_t)(len - b0));
             pos += len - b0;
             for (int r = 1; r < m; ++r) hs[pos++] = rows_flat[r0 + r];
         }
@@ -1105,16 +1125,26 @@ int fsb_verify_windows(fsb_handle* h, int n_streams, const int* stream_ids, cons
                        const int* max_accept, int32_t* tokens_out, int* acc_out, int* confirmed_out, unsigned flags) {
     if (!h) return FSB_ERR_INVALID;
     if (!hist_off) return fail(h, FSB_ERR_INVALID, "null argument");
-    return verify_windows_impl(h, n_streams, stream_ids, row_off, rows_flat, logits, ld, n_vocab, hist_flat, hist_off, max_accept, tokens_out, acc_out,
-                               confirmed_out, flags);
+    const HistSource hist{hist_flat, hist_off, nullptr, nullptr};
+    return verify_windows_impl(h, n_streams, stream_ids, row_off, rows_flat, logits, ld, n_vocab, &hist, max_accept, tokens_out, acc_out, confirmed_out,
+                               flags);
+}
+int fsb_verify_windows_lists(fsb_handle* h, int n_streams, const int* stream_ids, const int* row_off, const int32_t* rows_flat,
+                             const float* logits, int64_t ld, int n_vocab, const int32_t* const* hist_lists, const int64_t* hist_lens,
+                             const int* max_accept, int32_t* tokens_out, int* acc_out, int* confirmed_out, unsigned flags) {
+    if (!h) return FSB_ERR_INVALID;
+    const HistSource hist{nullptr, nullptr, hist_lists, hist_lens};
+    if (!hist.ok()) return fail(h, FSB_ERR_INVALID, "null argument");
+    return verify_windows_impl(h, n_streams, stream_ids, row_off, rows_flat, logits, ld, n_vocab, &hist, max_accept, tokens_out, acc_out, confirmed_out,
+                               flags);
 }
 
 int fsb_verify_windows_resident(fsb_handle* h, int n_streams, const int* stream_ids, const int* row_off, const int32_t* rows_flat,
                                 const float* logits, int64_t ld, int n_vocab, const int* max_accept, int32_t* tokens_out, int* acc_out,
                                 int* confirmed_out, unsigned flags) {
     if (!h) return FSB_ERR_INVALID;
-    return verify_windows_impl(h, n_streams, stream_ids, row_off, rows_flat, logits, ld, n_vocab, nullptr, nullptr, max_accept, tokens_out, acc_out,
-                               confirmed_out, flags);
+    return verify_windows_impl(h, n_streams, stream_ids, row_off, rows_flat, logits, ld, n_vocab, nullptr, max_accept, tokens_out, acc_out, confirmed_out,
+                               flags);
 }
 
 int fsb_last_kept(fsb_handle* h, int row, int cap, int32_t* ids, double* probs, int* n_keep) {
@@ -1141,7 +1171,7 @@ int fsb_batch_prepare(fsb_handle* h, int n_rows, const int* stream_ids, int64_t 
     fsb_batch* b = nullptr;
     int rc = alloc_batch(h, n_rows, hist_off[n_rows] - hist_off[0], 0, &b);
     if (rc) return rc;
-    rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, hist_flat, hist_off, flags);
+    rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, HistSource{hist_flat, hist_off, nullptr, nullptr}, flags);
     if (rc == FSB_OK) {
         rc = upload_batch(h, b);
         if (rc == FSB_OK && cudaStreamSynchronize(h->stream) != cudaSuccess) rc = fail(h, FSB_ERR_CUDA, "upload failed");
