@@ -1,11 +1,10 @@
-// fsb_device.cuh - device-side building blocks of the static-plan streaming kernel (sm_100a).
+// fsb_device.cuh - device-side building blocks of the sampling kernels (sm_100a).
 //
 //  * order-preserving 64-bit candidate keys ("composites"): (logit descending, token id ascending) becomes plain
 //    unsigned descending order, with -0.0f and +0.0f mapped to the same key - the order of the reference's
 //    comparator `a.first > b.first || (a.first == b.first && a.second < b.second)` (src/sampler.cpp:31,34);
-//  * mbarrier + 1-D bulk asynchronous copy (global -> this CTA's shared memory) wrappers; streaming 16-byte
-//    loads and the programmatic-dependent-launch controls;
-//  * a CTA-wide selection of the k largest composites by bisection with counting barriers;
+//  * thread-block cluster and programmatic-launch primitives;
+//  * a CTA-wide ordering of the k largest composites of a list;
 //  * the per-row epilogue: softmax in fp64 with the reference's sequential sums, min-p, top-p and the draw
 //    (src/sampler.cpp:37-49).
 #pragma once
@@ -46,56 +45,23 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-// A float t with: key(x) >= (L >> 32)  =>  x >= t.  L may have its low bits cleared, which can name a NaN pattern.
-__device__ __forceinline__ float comp_floor_value(u64 L) {
-    const float t = comp_value(L);
-    return (t != t) ? -__int_as_float(0x7f800000) : t;
-}
+// Asynchronous 16-byte copies global -> shared memory; a thread waits for its own, by groups.
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// ---------------------------------------------------------------------------------------------- mbarrier / bulk copy
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void mbar_init(u64* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(u64* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// 1-D bulk copy global -> shared memory of this CTA; both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, u64* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-// One poll of a barrier phase, with a suspend-time hint (the hardware may park the thread until the phase completes).
-__device__ __forceinline__ bool mbar_try_wait(u64* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void mbar_arrive(u64* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // ---------------------------------------------------------------------------------------------- launch order
 // Programmatic dependent launch: let the next launch in the stream begin as resources free up, and wait for the
 // previous launch to be complete (and its memory visible) before touching anything it wrote.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Thread-block clusters (pairs of CTAs that share a row): rank in the cluster, the address of a shared-memory
-// location in another CTA of the cluster, stores to it, and the cluster's barrier (arrive releases this thread's
-// stores to the cluster, wait acquires the others').
-__device__ __forceinline__ unsigned cluster_cta_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
+// Thread-block clusters (the CTAs that share a row): the address of a shared-memory location in another CTA of the
+// cluster, stores to it, and the cluster's barrier (arrive releases this thread's stores to the cluster, wait acquires
+// the others').
 __device__ __forceinline__ unsigned cluster_map_shared(unsigned local_addr, unsigned rank) {
     unsigned a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
@@ -106,15 +72,6 @@ __device__ __forceinline__ void cluster_store_u32(unsigned addr, unsigned v) { a
 __device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// Ticket counter shared by the CTAs of a row: the add releases this thread's earlier writes - and those of the
-// CTA's other threads that a barrier ordered before it - to the whole device, and acquires what earlier ticket
-// holders released.
-__device__ __forceinline__ unsigned ticket_add_acq_rel(unsigned* p, unsigned v) {
-    unsigned old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
-
 __device__ __forceinline__ u64 global_timer_ns() {
     u64 t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -124,47 +81,23 @@ __device__ __forceinline__ u64 global_timer_ns() {
 // ---------------------------------------------------------------------------------------------- shared control block
 constexpr int kNumWarps = kThreads / 32;
 
-// Barrier of the kThreads consumer threads of a CTA (named barrier 1).  The streaming kernel has one more warp,
-// the copy producer, which never takes part in it; kernels with only kThreads threads use it like __syncthreads().
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
-
-// What the streaming kernel knows about the segment it is working on (written once per segment by one thread).
-struct SegCtx {
-    const float* row;   // the row's logits
-    float pen;          // repetition penalty of the row
-    float cap;          // softcap, 0 = off
-    int has_pen;
-    int id_base;        // token id of column 0
-    int seg_lo;         // first column of the segment (= column of bit 0 of the bitmap)
-    int seg_hi;         // one past its last column
-    int n_vocab;
-    int vec_ok;         // rows start on 16-byte boundaries
-    int k;              // the row's candidate count
-    int final_in_mem;   // write-back mode: the row in global memory already holds the transformed logits
-};
-
 struct SharedCtl {
-    u64 full[kStages];                // "tile landed": completed by the copy (or by the producer for tiny tails)
-    u64 empty[kStages];               // "tile consumed": every consumer warp hands the ring slot back
-    u64 red[2 * kNumWarps];           // cross-warp reduction scratch
-    double dsum;
-    alignas(16) float wbound[kNumWarps];   // per-warp admission bounds (see the streaming kernel); read with 16-byte loads
-    int wcount[kNumWarps];            // lengths of a row's ordered candidate lists while they are merged
-    int sum[3];                       // rotating counters of the selection steps
+    alignas(16) unsigned keys[kNumWarps][64];              // each warp's maxima while their ranks are counted; digit counts of the exact selection
+    alignas(16) unsigned top[kNumWarps];      // per-warp bounds (keys)
+    u64 red[2 * kNumWarps];                   // cross-warp reduction scratch
+    double part[kNumWarps];                   // partial sums of the epilogue
+    int sum[3];                               // rotating counters of the selection steps
+    int list_n;                               // cells the streaming kernel has listed (those past the list's capacity counted too)
+    int kept_n;                               // candidates picked from them
     int out_cnt;
-    int base, last;
-    int imax, imin1, imin2;
-    int need_compact;                 // a lane's queue is nearly full: the CTA must re-select
-    int abort;                        // a copy did not land in time
-    u64 ev_bound;                     // composite bound of the latest re-selection (0: nothing was dropped)
-    int rank[kMaxK];                  // ranks of the entries while a list is ordered
-    int recv_n[8];                    // clustered CTAs: candidates CTA r of the row's cluster has put into part r - 1 of the receive buffer (entry r)
-    SegCtx seg;
+    int recv_n[8];                            // clusters: candidates that segment r of the row has sent
+    u64 sel_prefix;
+    int sel_need, sel_in_bin;
 };
 
 // ---------------------------------------------------------------------------------------------- top-k selection
 // Smallest and largest of the composites the threads hold (each thread passes the extremes of its own; threads
-// with nothing pass ~0 and 0).  All threads of the CTA must call.
+// with nothing pass ~0 and 0).  All kThreads threads of the CTA must call.
 __device__ __forceinline__ void cta_minmax(u64& mn, u64& mx, SharedCtl* ctl) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -176,7 +109,7 @@ __device__ __forceinline__ void cta_minmax(u64& mn, u64& mx, SharedCtl* ctl) {
         ctl->red[warp] = mn;
         ctl->red[kNumWarps + warp] = mx;
     }
-    consumer_sync();
+    __syncthreads();
     mn = ctl->red[0];
     mx = ctl->red[kNumWarps];
 #pragma unroll
@@ -184,7 +117,7 @@ __device__ __forceinline__ void cta_minmax(u64& mn, u64& mx, SharedCtl* ctl) {
         mn = min(mn, ctl->red[w]);
         mx = max(mx, ctl->red[kNumWarps + w]);
     }
-    consumer_sync();   // the scratch may be written again
+    __syncthreads();   // the scratch may be written again
 }
 
 // Bound L of the k largest among n > k distinct composites held by the threads of the CTA: exactly k composites
@@ -198,7 +131,7 @@ __device__ __forceinline__ u64 bisect_bound(int k, u64 mn, u64 mx, SharedCtl* ct
     const int hb = 63 - __clzll((long long)(mx ^ mn));
     u64 pfx = (hb == 63) ? 0ull : (mx & (~0ull << (hb + 1)));
     if (tid == 0) ctl->sum[0] = 0;
-    consumer_sync();
+    __syncthreads();
     int step = 0;
 #pragma unroll 1
     for (int b = hb; b >= 0; --b, ++step) {
@@ -206,7 +139,7 @@ __device__ __forceinline__ u64 bisect_bound(int k, u64 mn, u64 mx, SharedCtl* ct
         const int wsum = __reduce_add_sync(0xffffffffu, count_ge(trial));
         if ((tid & 31) == 0 && wsum) atomicAdd(&ctl->sum[step % 3], wsum);
         if (tid == 0) ctl->sum[(step + 1) % 3] = 0;   // last read two barriers ago
-        consumer_sync();
+        __syncthreads();
         const int total = ctl->sum[step % 3];
         if (total >= k) pfx = trial;
         if (total == k) break;
@@ -234,7 +167,7 @@ static __device__ __noinline__ int select_list_topk(u64* list, int n, int k, u64
         return c;
     });
     if (tid == 0) ctl->out_cnt = 0;
-    consumer_sync();
+    __syncthreads();
 #pragma unroll 1
     for (int i = tid; i < n; i += kThreads) {
         const u64 c = list[i];
@@ -243,11 +176,41 @@ static __device__ __noinline__ int select_list_topk(u64* list, int n, int k, u64
             if (p < k) tmp[p] = c;
         }
     }
-    consumer_sync();
+    __syncthreads();
 #pragma unroll 1
     for (int i = tid; i < k; i += kThreads) list[i] = tmp[i];
-    consumer_sync();
+    __syncthreads();
     return k;
+}
+
+// Ranks the composites buf[0..n) (distinct but for zeros, which rank last; shared memory, 16-byte aligned, room for
+// seven more entries) by counting, and calls emit(rank, composite) once for each that ranks below k.  Four lanes count
+// for an entry, each a quarter of the list, two entries per 16-byte broadcast read and no dependency between the reads
+// (the quarters are interleaved: no bank conflicts); no atomics, one barrier.  64 entries take one round; the work grows
+// with n^2, so lists of more than kRankCap entries are first cut down to k by bisection (`tmp`: scratch for k composites).
+// All kThreads threads must call, after a barrier that made buf visible.
+constexpr int kRankCap = 512;
+template <class Emit>
+__device__ __forceinline__ void rank_emit(u64* buf, int n, int k, u64* tmp, SharedCtl* ctl, Emit emit) {
+    const int tid = threadIdx.x;
+    if (n > kRankCap) n = select_list_topk(buf, n, k, tmp, ctl);
+    const int n8 = (n + 7) & ~7;
+    if (tid < n8 - n) buf[n + tid] = 0ull;   // padding: 0 is below every composite
+    __syncthreads();
+    const int part = tid & 3;
+    for (int e0 = 0; e0 < n; e0 += kThreads / 4) {
+        const int e = e0 + (tid >> 2);
+        const u64 c = e < n ? buf[e] : 0ull;
+        int larger = 0;
+#pragma unroll 4
+        for (int j = 2 * part; j < n8; j += 8) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(buf + j);
+            larger += (v.x > c ? 1 : 0) + (v.y > c ? 1 : 0);
+        }
+        larger += __shfl_xor_sync(0xffffffffu, larger, 1);
+        larger += __shfl_xor_sync(0xffffffffu, larger, 2);
+        if (part == 0 && c != 0ull && larger < k) emit(larger, c);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------- row epilogue
@@ -255,15 +218,16 @@ static __device__ __noinline__ int select_list_topk(u64* list, int n, int k, u64
 struct RowTail {
     u64 rng_word;
     float temperature, top_p, min_p;
-    int k;
     int flags;
     int out_index;
+    long long append_at;    // resident histories: where the token goes in the id pool (used with kRowAppend)
 };
 
 struct TailOut {
     int32_t* tokens;
     int32_t* tokens_host;   // mirror of the tokens in mapped host memory, or null
     unsigned* status_host;  // takes a non-zero word whenever a status bit is set, or null
+    int32_t* pool;          // id pool of the resident histories
     int32_t* kept_ids;
     double* kept_pr;
     int32_t* kept_n;
@@ -272,43 +236,6 @@ struct TailOut {
     int shard_stride;
     unsigned* status;
 };
-
-// Orders the k largest of buf[0..n) (distinct composites in shared memory; fewer if n < k) into out[0..kk),
-// descending, and returns kk = min(n, k).  Long lists are first cut down to k by bisection.  What is left (at most
-// kMaxK entries) is ranked by counting: entry e is looked after by kThreads / n threads, each of which counts the
-// larger entries in its part of the list - two per 16-byte broadcast read, no dependency between the reads - and
-// the parts are added up with one shared-memory atomic each.  buf (16-byte aligned, room for one entry of padding)
-// is overwritten; `out` has room for kMaxK composites and must not overlap buf; the ranks live in ctl->rank.  All
-// consumer threads must call, after a barrier that made buf visible; out is visible to all on return.
-static __device__ __forceinline__ int topk_sorted(u64* buf, int n, int k, u64* out, SharedCtl* ctl) {
-    const int tid = threadIdx.x;
-    if (n > kMaxK) n = select_list_topk(buf, n, k, out, ctl);
-    if (n <= 0) return 0;
-    const int parts = kThreads / n;                    // >= 2 threads per entry
-    const int part = tid / n, e = tid - part * n;
-    if (tid < kMaxK) ctl->rank[tid] = 0;
-    if (tid == 0 && (n & 1)) buf[n] = 0ull;            // padding: 0 is below every composite
-    consumer_sync();
-    if (part < parts) {
-        const u64 c = buf[e];
-        const int per = (((n + parts - 1) / parts) + 1) & ~1;   // entries per part, even: parts start on 16-byte boundaries
-        const int j0 = part * per, j1 = min(n, j0 + per);
-        int larger = 0;
-#pragma unroll 4
-        for (int j = j0; j < j1; j += 2) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(buf + j);
-            larger += (v.x > c ? 1 : 0) + (v.y > c ? 1 : 0);
-        }
-        if (larger) atomicAdd(&ctl->rank[e], larger);
-    }
-    consumer_sync();
-    if (tid < n) {
-        const int r = ctl->rank[tid];
-        if (r < k) out[r] = buf[tid];
-    }
-    consumer_sync();
-    return n < k ? n : k;
-}
 
 // A status bit for the host: the device word collects the bits, the host mirror (if any) just becomes non-zero.
 __device__ __forceinline__ void report_status(unsigned* status, unsigned* status_host, unsigned bit) {
@@ -323,24 +250,19 @@ __device__ __forceinline__ void put_token(int32_t* tokens, int32_t* tokens_host,
 
 // srt[0..kk) holds the row's candidates in order (largest first).  Either hands them out (vocabulary-sharded mode)
 // or finishes the row: softmax over the candidates in fp64, sequential sums in candidate order, min-p, top-p,
-// draw.  `work` is scratch for 2 * kMaxK doubles that does not overlap srt.  All consumer threads must call it with
-// the same arguments.
+// draw.  `work` is scratch for 2 * kMaxK doubles that does not overlap srt.  All threads must call it with the same
+// arguments; it is the last thing they do (no barrier at the end).
+// Exponentials, their sum (pairwise, like a tree) and the probabilities are one thread's work each.  The cumulative
+// probabilities follow the reference's order of additions exactly, since a cut may fall on a tie: one warp runs the chain
+// of dependent adds (15 cycles each), all lanes alike over broadcast reads, and stops soon after top-p is reached; the
+// cuts and the draw are warp votes.
 static __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     double* e = work;
     double* P = work + kMaxK;
-    if (kk <= 0) {   // nothing but NaNs in the row
-        if (tid == 0) {
-            report_status(o.status, o.status_host, kStatusEmptyRow);
-            if (o.shard_out && o.shard_n) o.shard_n[r.out_index] = 0;
-            else if (o.shard_out) o.shard_out[(size_t)r.out_index * o.shard_stride] = 0ull;
-            else put_token(o.tokens, o.tokens_host, r.out_index, 0);
-            if (o.kept_n) o.kept_n[r.out_index] = 0;
-        }
-        return;
-    }
     if (o.shard_out) {
         u64* list = o.shard_out + (size_t)r.out_index * o.shard_stride;
+        if (kk <= 0 && tid == 0) report_status(o.status, o.status_host, kStatusEmptyRow);
         if (o.shard_n) {
             if (tid < kk) list[tid] = srt[tid];
             if (tid == 0) o.shard_n[r.out_index] = kk;
@@ -350,74 +272,84 @@ static __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, cons
         }
         return;
     }
-    if (r.flags & kRowGreedy) {   // first index of the maximum (src/sampler.cpp:19-23)
-        if (tid == 0) {
-            put_token(o.tokens, o.tokens_host, r.out_index, comp_id(srt[0]));
-            if (o.kept_n) o.kept_n[r.out_index] = 0;
+    int token = 0, keep = 0;
+    if (kk > 0 && !(r.flags & kRowGreedy)) {
+        // pr[i] = exp((double)(x_i - x_0) / T)   (fp32 subtraction, fp64 division, src/sampler.cpp:40)
+        double x = 0.0;
+        if (tid < kk) x = exp(__ddiv_rn((double)__fsub_rn(comp_value(srt[tid]), comp_value(srt[0])), (double)r.temperature));
+        double s = x;
+        if ((tid & ~31) < kk) {
+#pragma unroll
+            for (int d = 16; d; d >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, d));
+            if (lane == 0) ctl->part[tid >> 5] = s;
         }
-        return;
-    }
-    // pr[i] = exp((double)(x_i - x_0) / T)   (fp32 subtraction, fp64 division, src/sampler.cpp:40)
-    const float mx = comp_value(srt[0]);
-    if (tid < kk) e[tid] = exp(__ddiv_rn((double)__fsub_rn(comp_value(srt[tid]), mx), (double)r.temperature));
-    consumer_sync();
-    // The reference adds in candidate order, one after the other: one thread runs the chain (the loads do not depend
-    // on it, so they run ahead).  (Letting that thread also find the min-p and top-p cuts and the draw while it walks
-    // the sums - no atomics, two barriers fewer - was measured 0.3 us slower: the compares lengthen the chain.)  The cumulative sums P[i] = pr[0] + ... + pr[i] serve the top-p walk, `tot` and the
-    // draw walk alike: the reference adds the same numbers in the same order in all three.
-    if (tid == 0) {
-        double s = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < kk; ++i) s = __dadd_rn(s, e[i]);
-        ctl->dsum = s;
-        ctl->imax = 0;
-        ctl->imin1 = 0x7fffffff;
-        ctl->imin2 = 0x7fffffff;
-    }
-    consumer_sync();
-    if (tid < kk) e[tid] = __ddiv_rn(e[tid], ctl->dsum);
-    consumer_sync();
-    if (tid == 0) {
+        __syncthreads();
+        s = ctl->part[0];
+        for (int w = 1; 32 * w < kk; ++w) s = __dadd_rn(s, ctl->part[w]);
+        // probabilities; min-p keeps those not below pr[0] * min_p (they do not increase, pr[0] is 1 / sum)
+        const double p = __ddiv_rn(x, s);
+        if (tid < kk) e[tid] = p;
+        const bool cut = r.min_p > 0.0f && p < __dmul_rn(__ddiv_rn(1.0, s), (double)r.min_p);
+        keep = __syncthreads_count(tid < kk && !cut);
+        if (tid >= 32) return;
+        // cumulative sums P[i] = pr[0] + ... + pr[i]; top-p keeps the shortest prefix whose sum reaches top_p, the crossing
+        // candidate included
+        const double top_p = r.top_p < 1.0f ? (double)r.top_p : 2.0;
         double c = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < kk; ++i) {
-            c = __dadd_rn(c, e[i]);
-            P[i] = c;
+        int i = 0;
+        while (i < keep) {
+            double v[16];
+            const int n = min(16, keep - i);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = q < n ? e[i + q] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                c = __dadd_rn(c, v[q]);
+                if (lane == q) P[i + q] = c;
+            }
+            i += n;
+            if (c >= top_p) break;
         }
+        __syncwarp();
+        if (r.top_p < 1.0f) {
+            for (int b = 0; b < i; b += 32) {
+                const unsigned m = __ballot_sync(0xffffffffu, b + lane < i && P[b + lane] >= top_p);
+                if (m) {
+                    keep = min(keep, b + __ffs(m));
+                    break;
+                }
+            }
+        }
+        const double tot = P[keep - 1];
+        // one engine output -> U[0,1) as libstdc++ does it, then r = u * tot + 0.0
+        double u = __dmul_rn(__ull2double_rn(r.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
+        if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
+        const double rr = __dadd_rn(__dmul_rn(u, tot), 0.0);
+        int pick = keep - 1;
+        for (int b = 0; b < keep; b += 32) {
+            const unsigned m = __ballot_sync(0xffffffffu, b + lane < keep && rr <= P[b + lane]);
+            if (m) {
+                pick = b + __ffs(m) - 1;
+                break;
+            }
+        }
+        token = comp_id(srt[pick]);
+    } else {
+        if (tid >= 32) return;
+        if (kk > 0) token = comp_id(srt[0]);   // greedy: first index of the maximum (src/sampler.cpp:19-23)
     }
-    consumer_sync();
-    const double pr = tid < kk ? e[tid] : 0.0;
-    if (r.min_p > 0.0f && tid < kk) {   // keep = 1 + last index whose probability is not below pr[0] * min_p
-        const double thr = __dmul_rn(e[0], (double)r.min_p);
-        if (!(pr < thr)) atomicMax(&ctl->imax, tid);
-    }
-    consumer_sync();
-    int keep = kk;
-    if (r.min_p > 0.0f) keep = ctl->imax + 1;
-    if (r.top_p < 1.0f) {   // shortest prefix whose cumulative probability reaches top_p, crossing element included
-        if (tid < keep && P[tid] >= (double)r.top_p) atomicMin(&ctl->imin1, tid);
-        consumer_sync();
-        const int i1 = ctl->imin1;
-        if (i1 != 0x7fffffff && i1 + 1 < keep) keep = i1 + 1;
-    }
-    const double tot = P[keep - 1];
-    // one engine output -> U[0,1) as libstdc++ does it, then r = u * tot + 0.0
-    double u = __dmul_rn(__ull2double_rn(r.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
-    if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
-    const double rr = __dadd_rn(__dmul_rn(u, tot), 0.0);
-    if (tid < keep && rr <= P[tid]) atomicMin(&ctl->imin2, tid);
-    consumer_sync();
-    const int i2 = ctl->imin2;
-    const int pick = (i2 != 0x7fffffff) ? i2 : keep - 1;
-    if (tid == 0) put_token(o.tokens, o.tokens_host, r.out_index, comp_id(srt[pick]));
     if (o.kept_n) {
-        if (tid < keep) {
-            o.kept_ids[(size_t)r.out_index * kMaxK + tid] = comp_id(srt[tid]);
-            o.kept_pr[(size_t)r.out_index * kMaxK + tid] = e[tid];
+        for (int i = lane; i < keep; i += 32) {
+            o.kept_ids[(size_t)r.out_index * kMaxK + i] = comp_id(srt[i]);
+            o.kept_pr[(size_t)r.out_index * kMaxK + i] = e[i];
         }
-        if (tid == 0) o.kept_n[r.out_index] = keep;
+        if (lane == 0) o.kept_n[r.out_index] = keep;
     }
-    consumer_sync();
+    if (lane == 0) {
+        if (kk <= 0) report_status(o.status, o.status_host, kStatusEmptyRow);   // nothing but NaNs in the row
+        if (r.flags & kRowAppend) o.pool[r.append_at] = token;
+        put_token(o.tokens, o.tokens_host, r.out_index, token);
+    }
 }
 
 }  // namespace fsb

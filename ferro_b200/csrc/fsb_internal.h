@@ -5,24 +5,14 @@
 
 namespace fsb {
 
-// ---- compile-time geometry of the streaming kernel ---------------------------------------------------------
-constexpr int kThreads = 512;                 // consumer threads per CTA (16 warps); the streaming kernel adds one producer warp
-constexpr int kTile = 8192;                   // fp32 logits per CTA tile (32 KiB, one bulk copy; 512 logits per warp)
-constexpr int kStages = 4;                    // tiles in flight per CTA
+// ---- compile-time geometry -----------------------------------------------------------------------------------
+constexpr int kThreads = 256;                 // threads per CTA (8 warps) of the streaming kernel and of the list merge
 constexpr int kMaxK = 256;                    // largest k of the candidate path (== FSB_MAX_CANDIDATE_K)
-constexpr int kLaneQueue = 16;                // cells (4-byte entries) a lane can note before it must drop stale ones
-constexpr int kFlatCells = 960;               // cells (float4 + token id) gathered for one selection round
-constexpr int kCellBytes = 20;
-constexpr int kMergeCap = kFlatCells * kCellBytes / 8;   // 2400: candidates one row may gather from all its segments
-                                                          // (the gathered cells' memory seen as a list of composites)
-constexpr int kBitmapSpan = 262144;           // columns one penalty bitmap covers (one segment never spans more)
-constexpr int kBitmapWords = kBitmapSpan / 32;
-constexpr int kMaxTilesPerCta = kBitmapSpan / kTile;
+constexpr int kMergeCap = 2400;               // candidates of one row that the list merge can gather
 
 // status word bits written by kernels (0 = fine)
 enum : uint32_t {
-    kStatusCopyTimeout = 1u,     // a bulk copy did not land within the wait limit
-    kStatusMergeOverflow = 4u,   // a row has more segments than its scratch has room for (the planner prevents it)
+    kStatusMergeOverflow = 4u,   // the candidate lists of a row hold more than the merge has room for
     kStatusEmptyRow = 8u         // a row produced no candidate (all logits NaN)
 };
 
@@ -59,8 +49,7 @@ struct StreamArgs {
     const float* logits;       // base of the [rows][ld] matrix
     const RowDesc* rows;       // n_rows descriptors (only rows of the candidate path)
     const int32_t* hist;       // packed penalty-window ids
-    uint64_t* scratch;         // [n_rows][kMergeCap]: per segment of a row k ordered candidates, the counts at the end
-    uint32_t* ticket;          // [n_rows] segments that have finished (self-resetting)
+    int32_t* pool;             // id pool of the resident histories (rows with kRowAppend store their token there)
     int32_t* tokens;           // output tokens, indexed by RowDesc::out_index
     uint32_t* status;          // one word, OR of kStatus* bits
     // optional mirror in mapped host memory (device addresses of pinned host words; null = off): tokens are stored
@@ -77,34 +66,25 @@ struct StreamArgs {
     int32_t* shard_n;          // [rows] their number; null: a list starts with a header word that holds it
     int32_t shard_stride;      // 64-bit words per row of shard_out
     uint64_t* trace;           // optional [grid][8] timestamps (diagnostics), null = off
-    int64_t row_ld;            // >= 0: row r starts at r * row_ld (no descriptor read before the first copy)
+    int64_t row_ld;            // >= 0: row r starts at r * row_ld (no descriptor read before the first load)
     int32_t n_rows;
     int32_t n_vocab;
-    int32_t tiles_per_row;
-    int32_t tiles_per_cta;
-    int32_t total_tiles;
-    int32_t bulk_ok;           // rows start on 16-byte boundaries: tiles can come by bulk async copy
+    int32_t nseg;              // CTAs per row (1..8), a thread-block cluster when more than one
+    int32_t kmax;              // largest k of the rows
+    int32_t penalised;         // some row has a penalty window
     int32_t write_back;        // store penalised values into the caller's rows
     int32_t vocab_offset;      // token id of column 0
     float softcap;             // 0 = off
-    int32_t overlap;           // launch with programmatic stream serialization (see fsb_set_launch_overlap)
-    int32_t all_greedy;        // every row of the launch is greedy: the variant of the kernel that keeps one best logit per lane
-                               // instead of queues of candidates
-    int32_t pair;              // 0, or c = 2, 4, 8: every row is exactly c aligned CTAs (c r .. c r + c - 1), launched as a cluster
-                               // whose CTAs hand their candidates to the first one through shared memory instead of the row's scratch
+    int32_t overlap;           // see fsb_set_launch_overlap
 };
 
-// The launch plan: the flat list of tiles is dealt to the CTAs in equal contiguous ranges of tiles_per_cta tiles.
-struct Plan {
-    int tiles_per_row = 0, tiles_per_cta = 0, total_tiles = 0, grid = 0;
-};
-// `slots` = CTAs that run at once.
-Plan make_plan(int n_rows, int n_vocab, int kmax, int slots);
+// CTAs per row for a launch of n_rows rows on a device of `sms` multiprocessors.
+int plan_segments(int n_rows, int n_vocab, int sms);
 
-size_t stream_kernel_smem_bytes();
 // All return a cudaError_t as int (0 = success).
-int prepare_device_kernels(int* ctas_per_sm);
-int launch_stream_kernel(const StreamArgs& a, int grid, void* stream);
+int prepare_device_kernels();
+// host_rows: the descriptors in host memory (sent with the launch when they are few), or null.
+int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* stream);
 
 // One stream of a prompt-lookup drafting call: where its history lies in the id pool and what to look for.
 struct LookupDesc {
@@ -120,7 +100,6 @@ constexpr int kDraftStride = 68;              // int32 words per stream of a dra
 // Defined in fsb_support.cu.
 int prepare_support_kernels();
 int launch_lookup_drafts(const int32_t* pool, const LookupDesc* desc, int n_streams, int32_t* out, int stride, void* stream);
-int launch_append_tokens(const RowDesc* rows, int n_rows, const int32_t* tokens, int32_t* pool, void* stream);
 int launch_merge_lists(const void* lists, const int32_t* list_n, int n_lists, int list_stride, int n_rows, const RowDesc* rows, int32_t* tokens,
                        int32_t* kept_ids, double* kept_pr, int32_t* kept_n, uint32_t* status, void* stream);
 int launch_write_drafts(const RowDesc* rows, int n_rows, int32_t* pool, void* stream);
@@ -131,7 +110,7 @@ int launch_gather_patched(const float* logits, const RowDesc* rows, int n_rows, 
 // Defined in fsb_fullrow.cu.
 size_t full_row_smem_bytes(int n_vocab);
 int prepare_full_row_kernel(int max_vocab);
-int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int32_t* tokens, int32_t* tokens_host,
+int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
                            int32_t* kept_ids, double* kept_pr, int32_t* kept_n, int record, uint32_t* status, uint32_t* status_host, int n_vocab,
                            int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream);
 

@@ -51,8 +51,8 @@ struct fsb_batch {
     int64_t cap_hist = 0;
     int n_cand = 0, n_full = 0;   // rows of the candidate kernel / of the full-row kernel
     int kmax = 1;
-    bool all_greedy = false;      // every row of the streaming kernel is greedy
-    fsb::Plan plan;               // how the candidate rows are dealt to the CTAs of the streaming kernel
+    int nseg = 1;                 // CTAs per row of the streaming kernel
+    bool penalised = false;       // some row of the streaming kernel has a penalty window
     int64_t hist_ids = 0;         // window ids staged with the batch
     int64_t gather_ids = 0;       // window values a write-back for a host caller brings back
     int64_t table_ints = 0;       // int32 words of the per-stream table of a resident verification call, staged behind the window ids
@@ -89,8 +89,7 @@ struct fsb_handle {
     int device = 0;
     int max_rows = 0, max_vocab = 0;
     int64_t max_hist = 0;
-    int sm_count = 0, ctas_per_sm = 0;
-    int pair_ok = 1;                   // clusters of CTAs can be launched on this device
+    int sm_count = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaStream_t side = nullptr;       // the full-vocabulary kernel of a mixed batch runs here, beside the streaming kernel
@@ -103,8 +102,6 @@ struct fsb_handle {
     std::vector<Stream> streams;
     std::vector<int> free_ids;
     // device scratch shared by all batches of this handle
-    uint64_t* d_scratch = nullptr;     // [max_rows][kMergeCap] candidates the segments of a row publish
-    uint32_t* d_counters = nullptr;    // [max_rows] tickets: all zero between launches
     int32_t* d_kept_ids = nullptr;
     double* d_kept_pr = nullptr;
     int32_t* d_kept_n = nullptr;
@@ -123,8 +120,6 @@ struct fsb_handle {
     std::vector<std::vector<int64_t>> pool_free;   // freed regions by size class
     fsb_counters_t counters{};
     std::string err;
-
-    size_t counter_words() const { return (size_t)max_rows; }
 };
 
 namespace {
@@ -247,26 +242,25 @@ int finalize_batch(fsb_handle* h, fsb_batch* b) {
     int n_cand = 0, kmax = 1;
     fsb::RowDesc* dst = b->h_rows();
     auto on_chip = [](const fsb::RowDesc& d) { return d.k <= fsb::kMaxK && d.k_global <= fsb::kMaxK; };
-    bool all_greedy = true;
+    b->penalised = false;
     for (const auto& d : b->descs)
         if (on_chip(d)) {
             dst[n_cand++] = d;
             kmax = std::max(kmax, d.k);
-            all_greedy = all_greedy && (d.flags & fsb::kRowGreedy) != 0;
+            b->penalised = b->penalised || (d.flags & fsb::kRowPenalty) != 0;
         }
-    b->all_greedy = all_greedy && n_cand > 0;
     int n_full = 0;
     for (const auto& d : b->descs)
         if (!on_chip(d)) dst[n_cand + n_full++] = d;
     b->n_cand = n_cand;
     b->n_full = n_full;
     b->kmax = kmax;
-    b->plan = fsb::make_plan(std::max(n_cand, 1), b->n_vocab, kmax, std::max(1, h->sm_count * std::max(1, h->ctas_per_sm)));
+    b->nseg = fsb::plan_segments(std::max(n_cand, 1), b->n_vocab, std::max(1, h->sm_count));
     return FSB_OK;
 }
 
 // Sends what the kernels need to know about the batch.  `lone_launch`: the sampling kernels are the only readers of the
-// descriptors (nothing is appended, gathered or drafted on the device afterwards).  Then, if only descriptors are to be
+// descriptors (nothing is gathered or drafted on the device around them).  Then, if only descriptors are to be
 // sent, the batch is one wave of CTAs and long enough to hide a read across PCIe behind its first tiles (measured on
 // B200: 64 x 262144 gains 6 us per call, 8 x 65536 nothing, one row loses 2 us), nothing is copied at all: the kernels
 // read the descriptors from the pinned host block.
@@ -304,7 +298,7 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
             FSB_CUDA(h, cudaStreamWaitEvent(h->side, h->ev_fork, 0));
             where = h->side;
         }
-        const int e = fsb::launch_full_row_kernel(logits_dev, b->d_rows() + b->n_cand, b->n_full, hist, b->d_tokens, tokens_host,
+        const int e = fsb::launch_full_row_kernel(logits_dev, b->d_rows() + b->n_cand, b->n_full, hist, h->d_pool, b->d_tokens, tokens_host,
                                                   h->d_kept_ids, h->d_kept_pr, h->d_kept_n, keep_kept ? 1 : 0, b->d_status(), status_host, b->n_vocab, h->vocab_offset,
                                                   (b->flags & FSB_WRITE_BACK) ? 1 : 0, h->softcap, h->d_trace ? h->d_trace + 4096 * 8 : nullptr, where);
         if (e != 0) return fail(h, FSB_ERR_CUDA, "full-row kernel launch: %s", cudaGetErrorString((cudaError_t)e));
@@ -316,8 +310,7 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.logits = logits_dev;
         a.rows = b->d_rows();
         a.hist = hist;
-        a.scratch = h->d_scratch;
-        a.ticket = h->d_counters;
+        a.pool = h->d_pool;
         a.tokens = b->d_tokens;
         a.status = b->d_status();
         a.tokens_host = tokens_host;
@@ -332,21 +325,14 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.row_ld = (b->n_full == 0) ? b->ld : -1;   // descriptors are in row order when every row takes this kernel
         a.n_rows = b->n_cand;
         a.n_vocab = b->n_vocab;
-        a.tiles_per_row = b->plan.tiles_per_row;
-        a.tiles_per_cta = b->plan.tiles_per_cta;
-        a.total_tiles = b->n_cand * b->plan.tiles_per_row;
-        a.bulk_ok = ((reinterpret_cast<uintptr_t>(logits_dev) & 15u) == 0 && (b->ld & 3) == 0) ? 1 : 0;
+        a.nseg = b->nseg;
+        a.kmax = b->kmax;
+        a.penalised = b->penalised ? 1 : 0;
         a.write_back = (b->flags & FSB_WRITE_BACK) ? 1 : 0;
         a.vocab_offset = h->vocab_offset;
         a.softcap = h->softcap;
         a.overlap = h->launch_overlap;
-        a.all_greedy = b->all_greedy ? 1 : 0;
-        const int grid = (a.total_tiles + a.tiles_per_cta - 1) / a.tiles_per_cta;
-        // rows of exactly 2, 4 or 8 aligned segments: the CTAs of a row run as a cluster and exchange candidates on chip
-        a.pair = 0;
-        for (int c = 2; c <= 8; c *= 2)   // receive buffer: (c - 1) lists of kmax entries in 512
-            if (h->pair_ok && a.tiles_per_row == c * a.tiles_per_cta && grid == c * a.n_rows && (c - 1) * b->kmax <= 512) a.pair = c;
-        const int e = fsb::launch_stream_kernel(a, grid, h->stream);
+        const int e = fsb::launch_stream_kernel(a, b->h_rows(), h->stream);
         if (e != 0) return fail(h, FSB_ERR_CUDA, "stream kernel launch: %s", cudaGetErrorString((cudaError_t)e));
         h->counters.kernel_launches++;
     }
@@ -368,11 +354,10 @@ int fetch_tokens(fsb_handle* h, fsb_batch* b, int32_t* tokens_out, int64_t patch
         if (cudaMemcpy(&word, b->d_status(), sizeof word, cudaMemcpyDeviceToHost) == cudaSuccess && word != 0u) st = word;
     }
     if (st != 0u) {
-        // put the self-resetting counters and the status word back into their idle state
-        cudaMemsetAsync(h->d_counters, 0, sizeof(uint32_t) * h->counter_words(), h->stream);
+        // put the status word back into its idle state
         cudaMemsetAsync(b->d_status(), 0, sizeof(uint32_t), h->stream);
         cudaStreamSynchronize(h->stream);
-        return fail(h, FSB_ERR_DEVICE, "kernel status 0x%x (1 wait timeout, 4 merge overflow, 8 row without a finite logit)", st);
+        return fail(h, FSB_ERR_DEVICE, "kernel status 0x%x (4 merge overflow, 8 row without a finite logit)", st);
     }
     if (tokens_out) std::memcpy(tokens_out, b->h_tokens, sizeof(int32_t) * (size_t)b->n_rows);
     return FSB_OK;
@@ -540,14 +525,13 @@ void scatter_patched(const fsb_handle* h, const fsb_batch* b, float* logits_host
     }
 }
 
-// The common tail of the synchronous calls: upload, (stage host logits), launch, (append), fetch, (write back to host).
+// The common tail of the synchronous calls: upload, (stage host logits), launch, fetch, (write back to host).
 // `window_streams` > 0: a resident verification call - the drafts go into the id pool before the launch, and the last
 // accepted token of every stream after it (see verify_windows_impl).
-int run_staged(fsb_handle* h, fsb_batch* b, const float* logits, unsigned flags, bool append, int32_t* tokens_out, int window_streams = 0,
-               bool window_append = false) {
+int run_staged(fsb_handle* h, fsb_batch* b, const float* logits, unsigned flags, int32_t* tokens_out, int window_streams = 0, bool window_append = false) {
     const bool on_host = (flags & FSB_LOGITS_ON_HOST) != 0;
     const bool host_wb = on_host && (flags & FSB_WRITE_BACK) && b->gather_ids > 0;
-    int rc = upload_batch(h, b, !append && window_streams == 0 && !host_wb);
+    int rc = upload_batch(h, b, window_streams == 0 && !host_wb);
     const float* dev = logits;
     if (rc == FSB_OK && on_host) rc = stage_host_logits(h, logits, b->n_rows, b->ld, b->n_vocab, &dev);
     if (rc == FSB_OK && window_streams > 0) {
@@ -562,11 +546,6 @@ int run_staged(fsb_handle* h, fsb_batch* b, const float* logits, unsigned flags,
         else h->counters.kernel_launches++;
     }
     if (rc == FSB_OK && host_wb) rc = launch_gather(h, b, dev);
-    if (rc == FSB_OK && append) {
-        const int e = fsb::launch_append_tokens(b->d_rows(), b->n_rows, b->d_tokens, h->d_pool, h->stream);
-        if (e != 0) rc = fail(h, FSB_ERR_CUDA, "append kernel launch: %s", cudaGetErrorString((cudaError_t)e));
-        else h->counters.kernel_launches++;
-    }
     if (rc == FSB_OK) rc = fetch_tokens(h, b, tokens_out, host_wb ? b->gather_ids : 0);
     if (rc) rollback_draws(h, b);
     return rc;
@@ -629,7 +608,7 @@ int fsb_create(int device, int max_rows, int max_vocab, int64_t max_hist_ids, fs
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return bail(FSB_ERR_CUDA);
     if (prop.major < 10) return bail(FSB_ERR_NO_DEVICE);   // kernels are built for sm_100a only
     h->sm_count = prop.multiProcessorCount;
-    if (fsb::prepare_device_kernels(&h->ctas_per_sm) != 0 || h->ctas_per_sm <= 0) return bail(FSB_ERR_CUDA);
+    if (fsb::prepare_device_kernels() != 0) return bail(FSB_ERR_CUDA);
     if (fsb::prepare_support_kernels() != 0) return bail(FSB_ERR_CUDA);
     if (fsb::prepare_full_row_kernel(max_vocab) != 0) return bail(FSB_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(FSB_ERR_CUDA);
@@ -641,10 +620,7 @@ int fsb_create(int device, int max_rows, int max_vocab, int64_t max_hist_ids, fs
     // Everything a call may need is allocated here, so that no call allocates: the rows' scratch, the counters, the
     // kept-set record, the id pool and the staging area of host logits.
     h->logits_stage_elems = (size_t)max_rows * (size_t)max_vocab;
-    if (cudaMalloc(reinterpret_cast<void**>(&h->d_scratch), sizeof(uint64_t) * (size_t)max_rows * fsb::kMergeCap) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&h->d_counters), sizeof(uint32_t) * h->counter_words()) != cudaSuccess ||
-        cudaMemset(h->d_counters, 0, sizeof(uint32_t) * h->counter_words()) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&h->d_kept_ids), sizeof(int32_t) * (size_t)max_rows * fsb::kMaxK) != cudaSuccess ||
+    if (cudaMalloc(reinterpret_cast<void**>(&h->d_kept_ids), sizeof(int32_t) * (size_t)max_rows * fsb::kMaxK) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&h->d_kept_pr), sizeof(double) * (size_t)max_rows * fsb::kMaxK) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&h->d_kept_n), sizeof(int32_t) * (size_t)max_rows) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&h->d_pool), sizeof(int32_t) * (size_t)std::max<int64_t>(max_hist_ids, 1)) != cudaSuccess ||
@@ -667,8 +643,6 @@ int fsb_destroy(fsb_handle* h) {
         free_batch_buffers(h->own);
         delete h->own;
     }
-    if (h->d_scratch) cudaFree(h->d_scratch);
-    if (h->d_counters) cudaFree(h->d_counters);
     if (h->d_kept_ids) cudaFree(h->d_kept_ids);
     if (h->d_kept_pr) cudaFree(h->d_kept_pr);
     if (h->d_kept_n) cudaFree(h->d_kept_n);
@@ -803,7 +777,7 @@ static int sample_batch_impl(fsb_handle* h, int n_rows, const int* stream_ids, c
     fsb_batch* b = h->own;
     int rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, hist, flags);
     if (rc) return rc;
-    rc = run_staged(h, b, logits, flags, false, tokens_out);
+    rc = run_staged(h, b, logits, flags, tokens_out);
     if (rc) return rc;
     if ((flags & FSB_LOGITS_ON_HOST) && (flags & FSB_WRITE_BACK)) {
         for (int i = 0; i < n_rows; ++i) {
@@ -947,7 +921,7 @@ int fsb_sample_batch_resident(fsb_handle* h, int n_rows, const int* stream_ids, 
         rollback_draws(h, b);
         return rc;
     }
-    rc = run_staged(h, b, logits, flags & ~FSB_APPEND_SAMPLED, append, tokens_out);
+    rc = run_staged(h, b, logits, flags & ~FSB_APPEND_SAMPLED, tokens_out);
     if (rc) return rc;
     for (int i = 0; i < n_rows; ++i) {
         Stream* s = get_stream(h, stream_ids[i]);
@@ -1080,7 +1054,7 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
     }
     rc = finalize_batch(h, b);
     if (rc) return rc;
-    rc = run_staged(h, b, logits, flags & ~FSB_APPEND_SAMPLED, false, nullptr, resident ? n_streams : 0, win_append);   // no engine was advanced: nothing to roll back
+    rc = run_staged(h, b, logits, flags & ~FSB_APPEND_SAMPLED, nullptr, resident ? n_streams : 0, win_append);   // no engine was advanced: nothing to roll back
     if (rc) return rc;
     // accept loop of src/server.cpp:626-636 on the sampled tokens
     for (int i = 0; i < n_streams; ++i) {

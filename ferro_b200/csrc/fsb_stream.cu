@@ -1,1084 +1,729 @@
-// fsb_stream.cu - the static-plan streaming candidate kernel of the B200 batched token sampler (sm_100a).
+// fsb_stream.cu - the streaming candidate kernel of the B200 batched token sampler (sm_100a).
 //
 // One launch samples every row of a batch whose effective k is at most kMaxK (greedy rows are k = 1):
 //   repetition penalty (src/sampler.cpp:11-18) -> greedy argmax (:19-23) or top-k candidates (:25-35)
 //   -> fp64 softmax (:37-41) -> min-p (:43) -> top-p (:44) -> seeded draw (:45-49).
 // (reference paths are relative to the paragontasx/ferro project root)
-// How it works is described above SegCtx below.
 #include <cuda_runtime.h>
 
 #include "../../include/ferro_sampler_b200.h"
 #include <algorithm>
+#include <cfloat>
+#include <cstring>
 
 #include "fsb_device.cuh"
 
 namespace fsb {
 namespace {
 
-constexpr int kWarps = kThreads / 32;
-constexpr int kWTile = kTile / kWarps;          // 512 logits: a warp's part of a CTA tile
-constexpr int kBlockThreads = kThreads + 32;    // consumers + the producer warp
-constexpr int kMaxJ = (kFlatCells + kMaxK + kThreads - 1) / kThreads;   // cells one thread may hold in a re-selection
+// How it works.
+// A row is cut into 1 to 8 equal segments, one CTA each; the CTAs of a row are a thread-block cluster.  A CTA reads its
+// segment once, in chunks of four 16-byte cells per thread.  Every thread copies its own cells to shared memory
+// asynchronously (cp.async), two chunks ahead, and reads back only what it copied itself: no barrier between copy and
+// look, 32 KB per CTA in flight, four CTAs per SM.
+// The look works on raw logits and leaves the penalised ones out.  A thread keeps two running maxima (of different cells);
+// from all threads' maxima the CTA derives a bound that at least k logits of the segment reach (cta_bound), at chunks 0, 1,
+// 3, 7, 15, ...  A cell whose maximum reaches the bound is listed in shared memory, data and all: about 100 in each of these
+// intervals for k = 64.  Should the list overflow, the segment is gone through once more with the final bound.
+// At the end the listed cells are taken apart: the logits that reach the final bound are the segment's candidates, and
+// with them the penalised logits of the window that do so once penalised, each id once.  The softcap is applied here too,
+// to candidates only: it is monotone up to the rounding of tanhf, and a margin under the bound covers that.
+// The candidates are ordered; a row of several segments sends each segment's k best to its first CTA through distributed
+// shared memory, which picks the k best of all and finishes the row.
+// What bounds it: the stream (HBM) for large batches, for small ones a chain of about ten dependent steps.  A step's
+// latency is its instruction count: a warp alone issues a dependent instruction every four to five cycles, so the code
+// after the stream counts over broadcast reads instead of sorting and branches little.
+// The exact path (exact_select) makes no assumption: a radix selection over the transformed segment that reads it again
+// (from L2) per digit.  It runs when hundreds of equal logits reach the final bound.
+// Nobody waits for another CTA but at the cluster's two barriers.
 
-constexpr size_t kSmemStage = (size_t)kStages * kTile * sizeof(float);
-constexpr size_t kSmemQueue = (size_t)kLaneQueue * kThreads * sizeof(unsigned);   // the lanes' queues of noted cells
-constexpr size_t kSmemCells = (size_t)kFlatCells * kCellBytes;                     // gathered cells; a list of composites otherwise
-constexpr size_t kSmemKept = (size_t)kMaxK * kCellBytes;                           // cells that survived a re-selection; selection scratch
-constexpr size_t kSmemBitmap = (size_t)kBitmapWords * sizeof(unsigned);
-constexpr int kRecvCap = 512;                                // clustered CTAs: the other CTAs' ordered candidates arrive here,
-constexpr size_t kSmemRecv = (size_t)kRecvCap * sizeof(u64);   // (cluster size - 1) parts of k entries
-static_assert(kRecvCap >= kMaxK, "a pair can always exchange");
-constexpr size_t kSmemTotal = kSmemStage + kSmemQueue + kSmemCells + kSmemKept + kSmemBitmap + kSmemRecv + sizeof(SharedCtl);
-static_assert(kSmemTotal <= 227 * 1024, "one CTA per SM");
-static_assert(kSmemCells >= (size_t)kMergeCap * sizeof(u64), "the element list lives in the gathered cells' memory");
-static_assert(kMergeCap >= 4 * kMaxK, "the logits of kMaxK surviving cells must fit into the element list");
-static_assert(kMergeCap >= 2 * kMaxK, "the epilogue's arrays live in the list's memory");
-static_assert(kSmemKept >= (size_t)kMaxK * sizeof(u64), "the ordered candidates live in the survivors' memory");
-static_assert(kWTile == 512, "a lane owns four float4 of a warp tile");
-static_assert(kMaxTilesPerCta <= 32, "a location is seven bits: the tile number above two bits (bit 7 is free)");
-static_assert(kFlatCells >= kThreads, "a capped gather round takes at least one cell per thread");
-static_assert(kLaneQueue % 4 == 0 && kLaneQueue >= 8, "lanes look at four cells per tile");
+constexpr int kWarps = kNumWarps;
+constexpr int kCells = 4;                               // cells of a thread per chunk
+constexpr int kChunkCells = kCells * kThreads;
+constexpr int kStages = 2;
+constexpr int kCellCap = 512;                           // cells a CTA can list
+constexpr int kPickCap = kRankCap;                      // candidates of a segment
+constexpr int kSendCap = 256;                           // candidates a segment sends to the row's first CTA
+constexpr int kMergeList = 8 * kSendCap;                // candidates of all segments
+constexpr size_t kRingBytes = (size_t)kStages * kChunkCells * sizeof(float4);
+static_assert((kPickCap + 8 + kMaxK + kMergeList + 8) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
+static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merge list's memory");
 
-constexpr long long kCopyWaitCycles = 2000000000ll;   // about 1 s: a bulk copy that has not landed by then is reported, not awaited
+constexpr int kSelectSmemMax = 200 * 1024;
+__host__ __device__ constexpr size_t recv_entries(int nseg) { return nseg > 1 ? (size_t)nseg * kSendCap : 0; }
 
-// How the streaming kernel works.
-// The [rows][n_vocab] matrix is cut into CTA tiles of kTile logits; the flat list of tiles is dealt to the CTAs in
-// equal contiguous ranges, and the part of a row that one CTA owns is a "segment".  One extra warp, the producer,
-// brings the CTA tiles into a ring of kStages shared-memory slots, one 1-D bulk copy per tile, so every logit is
-// read from HBM exactly once; the sixteen consumer warps each own one sixteenth (a warp tile of kWTile logits) of
-// every tile, wait for it to land, look at it and hand the slot back - they meet at the ring, never at a barrier.
-// Lane l owns float4 number l + 32 * q (q = 0..3) of a warp tile: a "cell" of four consecutive logits.  While
-// streaming a lane does not look at single logits: it takes the maximum of each cell, and where that reaches the
-// admission bound it notes the cell (one predicated 4-byte store of its truncated maximum and its location into a
-// queue only this lane writes).  At the end of a segment the noted cells the bound has not overtaken are read again
-// (from L2, as a rule), their logits that reach the final bound are ordered, and the segment's k best are the row's
-// candidates - or, when a row has several segments, go to the first CTA of the row's cluster through shared memory,
-// or to the row's scratch area, where the CTA that draws the row's last ticket merges them.  Nobody spins on
-// another CTA; waits for this CTA's own copies are bounded.
+// dynamic shared memory: ring, listed cells (data, numbers), control block, receive buffer, bitmap of the penalised columns
+// of the segment (its first word: the up to three columns before the cells)
+size_t select_smem_bytes(int nseg, int seg_cols) {
+    return kRingBytes + kCellCap * (sizeof(float4) + sizeof(int)) + sizeof(SharedCtl) + recv_entries(nseg) * sizeof(u64) +
+           (seg_cols > 0 ? (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0);
+}
 
-// The shared memory of a CTA.  The gathered cells' memory doubles as a list of composites (elements, merging),
-// the survivors' memory as the ordered candidates of the epilogue.
-struct Smem {
-    float* stage;       // [kStages][kTile] ring of CTA tiles
-    unsigned* queue;    // [kLaneQueue][kThreads] cells noted by each lane: truncated maximum | location
-    float4* cells;      // [kFlatCells] gathered cells ...
-    int* ids;           // [kFlatCells] ... and their first token ids
-    float4* kcells;     // [kMaxK] survivors of re-selections
-    int* kids;          // [kMaxK]
-    u64* list;          // = cells
-    u64* sorted;        // = kcells
-    unsigned* bitmap;
-    u64* recv;          // [kRecvCap] receive buffer of the first CTA of a cluster
-    SharedCtl* ctl;
+struct Segment {
+    const float* row;          // the row's logits
+    unsigned* bitmap;          // penalised columns (bit 0 = column bit0), valid when has_pen
+    const int32_t* hist;       // the penalty window
+    int hist_len;
+    int lo, hi;                // columns
+    int bit0;
+    int id_base;               // token id of column 0
+    bool has_pen;
+    float pen, cap;
 };
-__device__ __forceinline__ Smem smem_view() {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    Smem m;
-    unsigned char* p = smem_raw;
-    m.stage = reinterpret_cast<float*>(p);
-    p += kSmemStage;
-    m.queue = reinterpret_cast<unsigned*>(p);
-    p += kSmemQueue;
-    m.cells = reinterpret_cast<float4*>(p);
-    m.ids = reinterpret_cast<int*>(p + (size_t)kFlatCells * sizeof(float4));
-    m.list = reinterpret_cast<u64*>(p);
-    p += kSmemCells;
-    m.kcells = reinterpret_cast<float4*>(p);
-    m.kids = reinterpret_cast<int*>(p + (size_t)kMaxK * sizeof(float4));
-    m.sorted = reinterpret_cast<u64*>(p);
-    p += kSmemKept;
-    m.bitmap = reinterpret_cast<unsigned*>(p);
-    p += kSmemBitmap;
-    m.recv = reinterpret_cast<u64*>(p);
-    m.ctl = reinterpret_cast<SharedCtl*>(p + kSmemRecv);
-    return m;
+
+__device__ __forceinline__ float penalise(float x, float pen) { return x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen); }   // src/sampler.cpp:17
+__device__ __noinline__ float softcap_call(float x, float cap) { return __fmul_rn(cap, tanhf(__fdiv_rn(x, cap))); }          // src/model_gemma4.cpp:521
+__device__ __forceinline__ bool penalised(const Segment& s, int c) { return s.has_pen && ((s.bitmap[(c - s.bit0) >> 5] >> ((c - s.bit0) & 31)) & 1u); }
+
+// Logit of column c as the sampler sees it.
+__device__ __forceinline__ float transform(float x, int c, const Segment& s) {
+    if (s.cap != 0.0f) x = softcap_call(x, s.cap);
+    if (penalised(s, c)) x = penalise(x, s.pen);
+    return x;
 }
 
-// Final-logit softcap over a warp tile, in place (src/model_gemma4.cpp:521).  Only the softcap build calls it.
-__device__ __noinline__ void softcap_tile(float* st, int len, float cap, float* wb) {
-    for (int e = threadIdx.x & 31; e < len; e += 32) {
-        const float y = __fmul_rn(cap, tanhf(__fdiv_rn(st[e], cap)));
-        st[e] = y;
-        if (wb) wb[e] = y;
-    }
-    __syncwarp();
-}
-
-// Repetition penalty on the penalised columns of a warp tile, in place in shared memory (src/sampler.cpp:17).
-// The tile's bits of the segment bitmap are one word per 32 columns; each of the first lanes owns one word and
-// patches the columns whose bits are set.  A bit is set once however often an id occurs in the window.
-// (Patching the lanes' registers after the look's loads instead - four bitmap reads per lane and tile - was measured
-// slower: the loop is bound by instruction issue, and this way most lanes do nothing.)
-__device__ __forceinline__ void patch_tile(float* st, int len, int col0, int seg_lo, float pen, const unsigned* bitmap, float* wb_row) {
-    const int lane = threadIdx.x & 31;
-    const int nw = (len + 31) >> 5;
-    unsigned w = (lane < nw) ? bitmap[((col0 - seg_lo) >> 5) + lane] : 0u;
-    if (__ballot_sync(0xffffffffu, w != 0u) == 0u) return;
-    while (w) {
-        const int off = 32 * lane + __ffs(w) - 1;
-        w &= w - 1u;
-        const float x = st[off];
-        const float y = x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen);
-        st[off] = y;
-        if (wb_row) wb_row[col0 + off] = y;
-    }
-    __syncwarp();
-}
-
-// The r-th largest (r = 1..32) of the 32 lane values of a warp: a bitonic sort across the lanes.
-__device__ __forceinline__ unsigned warp_rth_largest(unsigned v, int r) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const unsigned o = __shfl_xor_sync(0xffffffffu, v, j);
-            const bool up = (lane & k) == 0;   // k == 32: every lane, the final order is ascending
-            const bool low = (lane & j) == 0;
-            v = (up == low) ? min(v, o) : max(v, o);
+// A bound that at least k logits of the segment reach, from the threads' maxima (each a logit of its own; two per
+// thread, of different cells).  Minus infinity - and what is no number - never reaches a bound.  All threads get the same
+// value; contains two barriers.  `listed`: the number of cells listed so far, the same in every thread.
+//  k <= 64: the r-th largest thread maximum of every warp, r = ceil(k / warps), minimum over the warps: 1.3 k to 2 k logits
+//    reach it.  r warp reductions take the largest out one after the other (equal ones together: the bound is lower then).
+//    (The k-th largest of all threads' maxima, found by counting, lets fewer through but cost more than it saved.)
+//  otherwise: the same over the 64 maxima of every warp, ranked by counting; keys give up their low bits to be distinct,
+//    which lowers the bound by less than 2^-16 of its value.
+__device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, SharedCtl* ctl, int& listed) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned m = ~0u;
+    if (k <= 64) {
+        unsigned key = float_key(fmaxf(run_a, run_b)), top = __reduce_max_sync(0xffffffffu, key);
+        for (int r = (k - 1) / kWarps; r > 0; --r) {
+            if (key == top) key = 0u;
+            top = __reduce_max_sync(0xffffffffu, key);
         }
+        if (lane == 0) ctl->top[warp] = top;
+    } else {
+        const int r = (k + kWarps - 1) / kWarps;
+        const unsigned ka = (float_key(run_a) & ~127u) | (unsigned)lane, kb = (float_key(run_b) & ~127u) | (unsigned)(lane + 32);
+        ctl->keys[warp][lane] = ka;
+        ctl->keys[warp][lane + 32] = kb;
+        __syncwarp();
+        int rank_a = 0, rank_b = 0;
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+            const uint4 v = *reinterpret_cast<const uint4*>(&ctl->keys[warp][4 * i]);
+            rank_a += (v.x > ka ? 1 : 0) + (v.y > ka ? 1 : 0) + (v.z > ka ? 1 : 0) + (v.w > ka ? 1 : 0);
+            rank_b += (v.x > kb ? 1 : 0) + (v.y > kb ? 1 : 0) + (v.z > kb ? 1 : 0) + (v.w > kb ? 1 : 0);
+        }
+        if (rank_a == r - 1) ctl->top[warp] = ka & ~127u;
+        if (rank_b == r - 1) ctl->top[warp] = kb & ~127u;
     }
-    return __shfl_sync(0xffffffffu, v, 32 - r);
-}
-
-// A bound that at least r = min(32, ceil(k / warps)) logits of this warp's stream reach: the r-th largest of the
-// lanes' running maxima (each is a logit of its own).
-__device__ __forceinline__ float warp_bound(float run_max, int k) {
-    const int r = min(32, (k + kWarps - 1) / kWarps);
-    const unsigned key = warp_rth_largest(float_key(run_max), r);
-    return key_float(key);
-}
-
-// Admission bound of the CTA: at least k logits of the segment reach the smallest of the warps' bounds (eight
-// warps, at least ceil(k / 8) logits each, or 32 * 8 >= kMaxK), so no logit below it is among the segment's k
-// best.  Each warp posts its value; values only grow, so a reader may use another warp's older value without a
-// barrier.
-__device__ __forceinline__ float min_warp_bounds(SharedCtl* ctl) {
-    float m = __int_as_float(0x7f800000);
+    __syncthreads();
+    listed = ctl->list_n;
 #pragma unroll
     for (int w = 0; w < kWarps; w += 4) {
-        float4 v;   // volatile: re-read on every call
-        asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_u32(&ctl->wbound[w])));
-        m = fminf(m, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
+        const uint4 v = *reinterpret_cast<const uint4*>(&ctl->top[w]);
+        m = min(m, min(min(v.x, v.y), min(v.z, v.w)));
     }
-    return m;
+    __syncthreads();   // nobody lists another cell before everybody has read the length
+    return fmaxf(key_float(m), -FLT_MAX);   // (also for the patterns just below minus infinity's key, which are no numbers)
 }
-// Diagnostics: slot 0 takes the global timer (ns) once, the others the SM cycle counter (cheap to read).
+
+// The softcap y(x) = cap * tanhf(x / cap) is monotone up to rounding: the division, tanhf (2 ulp) and the product are
+// together off by less than cap * 2^-22.  For a raw bound `thr`: `seen` is a value that every logit x >= thr reaches
+// after the softcap, `admit` a raw value below which no logit reaches `seen` - the raw bound moved down until the
+// softcap's value is a margin of cap * 2^-20 below `seen` (lane j tries 2^j times a small step).
+__device__ __forceinline__ void softcap_bounds(float thr, float cap, float& admit, float& seen) {
+    if (thr <= -FLT_MAX) {
+        admit = -FLT_MAX;
+        seen = -__int_as_float(0x7f800000);
+        return;
+    }
+    const float t0 = fminf(thr, 1e38f), margin = cap * 9.5367431640625e-7f;
+    seen = softcap_call(t0, cap) - margin;
+    const float t = t0 - ldexpf((fabsf(t0) + cap) * 9.5367431640625e-7f, threadIdx.x & 31);
+    const unsigned ok = __ballot_sync(0xffffffffu, softcap_call(t, cap) <= seen - margin);
+    admit = ok ? __shfl_sync(0xffffffffu, t, __ffs(ok) - 1) : -FLT_MAX;
+    admit = fmaxf(admit, -FLT_MAX);
+}
+
+// Keeps the listed cells that reach `admit`.  All threads call, after a barrier.
+__device__ __noinline__ void prune_cells(float4* cells, int* nums, SharedCtl* ctl, float admit) {
+    constexpr int kPer = kCellCap / kThreads;
+    const int n = min(ctl->list_n, kCellCap);
+    float4 x[kPer];
+    int num[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int p = threadIdx.x + i * kThreads;
+        num[i] = -1;
+        if (p < n) {
+            x[i] = cells[p];
+            num[i] = nums[p];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ctl->list_n = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+        if (num[i] >= 0 && fmaxf(fmaxf(x[i].x, x[i].y), fmaxf(x[i].z, x[i].w)) >= admit) {
+            const int p = atomicAdd(&ctl->list_n, 1);
+            cells[p] = x[i];
+            nums[p] = num[i];
+        }
+    __syncthreads();
+}
+
+// The penalty window's bits: set them all (again: picking the penalised candidates clears them).  All threads call.
+__device__ __forceinline__ void set_bits(const Segment& s, int first_id) {
+    for (int i = threadIdx.x; i < s.hist_len; i += kThreads) {
+        const int c = (i == threadIdx.x ? first_id : s.hist[i]) - s.id_base;
+        if (c >= s.lo && c < s.hi) atomicOr(&s.bitmap[(c - s.bit0) >> 5], 1u << ((c - s.bit0) & 31));
+    }
+}
+// Whether this thread is the first to come for column c: an id counts once however often it occurs in the window.
+__device__ __forceinline__ bool claim(const Segment& s, int c) {
+    const unsigned bit = 1u << ((c - s.bit0) & 31);
+    return (atomicAnd(&s.bitmap[(c - s.bit0) >> 5], ~bit) & bit) != 0u;
+}
+
+// Exact selection of the min(k, candidates) largest composites of the transformed segment into list (unordered);
+// returns their number.  MSB-first over 8-bit digits of the composites: count the digits of the composites that match
+// the prefix, walk the counts from the top, go on in the digit in which the k-th lies; stops early when a digit is
+// taken whole.  Every digit reads the segment again.  All threads call, after a barrier.
+__device__ __noinline__ int exact_select(const Segment& s, int k, u64* list, SharedCtl* ctl) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    unsigned* bins = &ctl->keys[0][0];
+    static_assert(kNumWarps * 64 >= 256, "one counter per digit");
+    if (s.has_pen) set_bits(s, tid < s.hist_len ? s.hist[tid] : 0);
+    u64 prefix = 0ull, mask = 0ull;
+    int need = k;
+    const int rounds = (s.hi - s.lo + kThreads - 1) / kThreads;
+    for (int shift = 56; shift >= 0; shift -= 8) {
+        if (tid < 256) bins[tid] = 0u;
+        __syncthreads();
+        for (int i = 0; i < rounds; ++i) {
+            const int c = s.lo + i * kThreads + tid;
+            unsigned digit = 256u;
+            if (c < s.hi) {
+                const float x = transform(__ldcg(s.row + c), c, s);
+                const u64 m = make_comp(x, c + s.id_base);
+                if (x == x && (m & mask) == prefix) digit = (unsigned)(m >> shift) & 255u;
+            }
+            const unsigned peers = __match_any_sync(0xffffffffu, digit);   // equal logits would meet in one counter
+            if (digit < 256u && lane == __ffs(peers) - 1) atomicAdd(&bins[digit], (unsigned)__popc(peers));
+        }
+        __syncthreads();
+        if (tid < 32) {   // lane l owns digits 255 - 8 l .. 248 - 8 l
+            int mine = 0;
+#pragma unroll
+            for (int d = 0; d < 8; ++d) mine += (int)bins[255 - 8 * lane - d];
+            int inc = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            const int total = __shfl_sync(0xffffffffu, inc, 31);
+            int above = inc - mine;
+            if (total < need) {   // first digit only: fewer than k candidates, all are taken
+                if (lane == 0) ctl->sel_in_bin = -1;
+            } else if (above < need && inc >= need) {
+                for (int d = 0; d < 8; ++d) {
+                    const int in = (int)bins[255 - 8 * lane - d];
+                    if (above + in >= need) {
+                        ctl->sel_prefix = prefix | ((u64)(255 - 8 * lane - d) << shift);
+                        ctl->sel_need = need - above;
+                        ctl->sel_in_bin = in;
+                        break;
+                    }
+                    above += in;
+                }
+            }
+        }
+        __syncthreads();
+        const int in_bin = ctl->sel_in_bin;
+        if (in_bin < 0) {
+            prefix = 0ull;
+            break;
+        }
+        prefix = ctl->sel_prefix;
+        need = ctl->sel_need;
+        mask |= 255ull << shift;
+        if (in_bin == need) break;
+    }
+    __syncthreads();
+    if (tid == 0) ctl->kept_n = 0;
+    __syncthreads();
+    for (int i = 0; i < rounds; ++i) {
+        const int c = s.lo + i * kThreads + tid;
+        if (c >= s.hi) continue;
+        const float x = transform(__ldcg(s.row + c), c, s);
+        const u64 m = make_comp(x, c + s.id_base);
+        if (x == x && m >= prefix) list[atomicAdd(&ctl->kept_n, 1)] = m;   // at most k
+    }
+    __syncthreads();
+    return ctl->kept_n;
+}
+
+// A segment with fewer than k logits above minus infinity (masked vocabularies): its first columns that hold minus
+// infinity are candidates too.  Appends up to k - n of them to the list; returns the new length.  All threads call.
+__device__ __noinline__ int append_masked(const Segment& s, int n, int k, u64* list, SharedCtl* ctl) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    if (s.has_pen) set_bits(s, tid < s.hist_len ? s.hist[tid] : 0);
+    __syncthreads();
+    for (int c0 = s.lo; c0 < s.hi && n < k; c0 += kThreads) {
+        const int c = c0 + tid;
+        const bool hit = c < s.hi && transform(__ldcg(s.row + c), c, s) == -__int_as_float(0x7f800000);
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) ctl->keys[0][warp] = (unsigned)__popc(m);
+        __syncthreads();
+        int before = n, total = 0;
+        for (int w = 0; w < kWarps; ++w) {
+            if (w < warp) before += (int)ctl->keys[0][w];
+            total += (int)ctl->keys[0][w];
+        }
+        before += __popc(m & ((1u << lane) - 1u));
+        if (hit && before < k) list[before] = make_comp(-__int_as_float(0x7f800000), c + s.id_base);
+        n = min(k, n + total);
+        __syncthreads();
+    }
+    return n;
+}
+
+// Write-back: the transformed logits go to the caller's row.  Nothing reads the raw row after this.
+__device__ __noinline__ void write_back(const Segment& s) {
+    float* row = const_cast<float*>(s.row);
+    __syncthreads();
+    if (s.has_pen) set_bits(s, threadIdx.x < s.hist_len ? s.hist[threadIdx.x] : 0);
+    __syncthreads();
+    if (s.cap != 0.0f) {
+        for (int c = s.lo + threadIdx.x; c < s.hi; c += kThreads) row[c] = transform(__ldcg(row + c), c, s);
+        return;
+    }
+    for (int i = threadIdx.x; i < s.hist_len; i += kThreads) {
+        const int c = s.hist[i] - s.id_base;
+        if (c >= s.lo && c < s.hi && claim(s, c)) row[c] = penalise(__ldcg(row + c), s.pen);
+    }
+}
+
 __device__ __forceinline__ void trace_mark(const StreamArgs& a, int slot) {
-    if (a.trace && threadIdx.x == 0) {
+    if (a.trace && threadIdx.x == 0 && blockIdx.x < 4096u) {
         a.trace[(size_t)blockIdx.x * 8 + slot] = slot == 0 ? global_timer_ns() : (u64)clock64();
         if (slot == 0) a.trace[(size_t)blockIdx.x * 8 + 7] = (u64)clock64();
     }
 }
 
-// Composite of a cell: (largest of its four logits, first token id).  A logit of the k best of a set of cells
-// always lies in one of the k cells with the largest composites.
-__device__ __forceinline__ u64 cell_comp(float4 x, int id0) { return make_comp(fmaxf(max3(x.x, x.y, x.z), x.w), id0); }
-
-// A queue entry: the cell's maximum with its low eight bits cleared (rounded toward zero) | the cell's location,
-// (tile of the segment << 2) | q.  For any a >= b, entry_value of a's entry >= truncated(b): testing entries
-// against a truncated bound never drops a cell whose maximum reaches the bound.
-__device__ __forceinline__ unsigned make_entry(float mx, unsigned loc) { return (__float_as_uint(mx) & 0xFFFFFF00u) | loc; }
-__device__ __forceinline__ float entry_value(unsigned e) { return __uint_as_float(e & 0xFFFFFF00u); }
-__device__ __forceinline__ float truncated(float x) { return __uint_as_float(__float_as_uint(x) & 0xFFFFFF00u); }
-
-// Notes a cell in this lane's queue if its maximum reaches the bound: a compare, the entry, one predicated store and
-// one predicated increment - no branch.  `q_base` is the shared-memory address of the lane's entry 0; entries of
-// one lane are kThreads * 4 bytes apart.
-__device__ __forceinline__ void note_cell_if(float mx, float thr, unsigned loc, unsigned q_base, int& qn) {
-    const unsigned entry = make_entry(mx, loc);
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .u32 a;\n\t"
-        "setp.ge.f32 p, %2, %3;\n\t"
-        "mad.lo.u32 a, %0, %5, %1;\n\t"
-        "@p st.shared.u32 [a], %4;\n\t"
-        "@p add.s32 %0, %0, 1;\n\t}"
-        : "+r"(qn)
-        : "r"(q_base), "f"(mx), "f"(thr), "r"(entry), "n"(kThreads * 4)
-        : "memory");
+__device__ __forceinline__ unsigned lanes_below() {
+    unsigned m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
 }
-
-// Drops the entries of this lane's queue whose cell maximum cannot reach `thr` any more; returns the new length.
-__device__ __forceinline__ int drop_stale(unsigned* myq, int qn, float thr) {
-    const float t = truncated(thr);
-    int w = 0;
-    for (int i = 0; i < qn; ++i) {
-        const unsigned e = myq[i * kThreads];
-        if (entry_value(e) >= t) myq[(w++) * kThreads] = e;
-    }
-    return w;
-}
-
-// Column of the cell a queue entry of this thread names.
-__device__ __forceinline__ int loc_column(unsigned loc, const SegCtx& sc) {
-    loc &= 0xFFu;
-    return sc.seg_lo + (int)(loc >> 2) * kTile + (int)(threadIdx.x >> 5) * kWTile + 4 * ((int)(threadIdx.x & 31) + 32 * (int)(loc & 3u));
-}
-
-// The cell at column `col` of the row, as loaded (no transformation).  Columns past the end of the row are NaN.
-__device__ __forceinline__ float4 load_cell(const SegCtx& sc, int col) {
-    if (sc.vec_ok && col + 4 <= sc.n_vocab) return __ldcg(reinterpret_cast<const float4*>(sc.row + col));
-    const float qnan = __int_as_float(0x7fc00000);
-    float4 t;
-    t.x = (col < sc.n_vocab) ? __ldcg(sc.row + col) : qnan;
-    t.y = (col + 1 < sc.n_vocab) ? __ldcg(sc.row + col + 1) : qnan;
-    t.z = (col + 2 < sc.n_vocab) ? __ldcg(sc.row + col + 2) : qnan;
-    t.w = (col + 3 < sc.n_vocab) ? __ldcg(sc.row + col + 3) : qnan;
-    return t;
-}
-
-// Softcap, then penalty, as the streaming pass applied them to the cell at column `col`.
-template <bool SOFTCAP>
-__device__ __forceinline__ float4 transform_cell(float4 t, const SegCtx& sc, const unsigned* bitmap, int col) {
-    if (sc.final_in_mem) return t;
-    if (SOFTCAP) {
-        t.x = __fmul_rn(sc.cap, tanhf(__fdiv_rn(t.x, sc.cap)));
-        t.y = __fmul_rn(sc.cap, tanhf(__fdiv_rn(t.y, sc.cap)));
-        t.z = __fmul_rn(sc.cap, tanhf(__fdiv_rn(t.z, sc.cap)));
-        t.w = __fmul_rn(sc.cap, tanhf(__fdiv_rn(t.w, sc.cap)));
-    }
-    if (sc.has_pen) {
-        const int b = col - sc.seg_lo;   // a multiple of four: the four bits lie in one word
-        const unsigned bits = (bitmap[b >> 5] >> (b & 31)) & 0xFu;
-        if (bits) {
-            if (bits & 1u) t.x = t.x > 0.0f ? __fdiv_rn(t.x, sc.pen) : __fmul_rn(t.x, sc.pen);
-            if (bits & 2u) t.y = t.y > 0.0f ? __fdiv_rn(t.y, sc.pen) : __fmul_rn(t.y, sc.pen);
-            if (bits & 4u) t.z = t.z > 0.0f ? __fdiv_rn(t.z, sc.pen) : __fmul_rn(t.z, sc.pen);
-            if (bits & 8u) t.w = t.w > 0.0f ? __fdiv_rn(t.w, sc.pen) : __fmul_rn(t.w, sc.pen);
-        }
-    }
-    return t;
-}
-
-// Exclusive prefix sum of one int per consumer thread over the CTA (thread order) and the total.  Contains two
-// barriers; uses ctl->red.
-struct ScanResult {
-    int before;
-    int total;
-};
-__device__ __forceinline__ ScanResult cta_scan(int v, SharedCtl* ctl) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    if (lane == 31) reinterpret_cast<int*>(ctl->red)[warp] = inc;
-    consumer_sync();
-    int before = inc - v, total = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-        const int s = reinterpret_cast<int*>(ctl->red)[w];
-        if (w < warp) before += s;
-        total += s;
-    }
-    consumer_sync();   // the scratch may be written again
-    return ScanResult{before, total};
-}
-
-// Re-selection over the nq gathered cells (flat arrays) and the nkept survivors: the k cells with the largest
-// composites become the survivors' list.  Returns their number and the composite bound they passed (0: nothing was
-// dropped).  All consumer threads must call, after a barrier that made the gathered cells visible.
-struct SelectResult {
-    int count;
-    u64 bound;
-};
-__device__ __noinline__ SelectResult select_cells(int nq, int nkept, int k) {
-    const Smem cs = smem_view();
-    SharedCtl* ctl = cs.ctl;
-    const int tid = threadIdx.x;
-    const int n = nq + nkept;
-    float4 cx[kMaxJ];
-    int cid[kMaxJ];
-    u64 cc[kMaxJ];
-#pragma unroll
-    for (int j = 0; j < kMaxJ; ++j) {
-        const int f = tid + j * kThreads;
-        cc[j] = 0ull;
-        cid[j] = 0;
-        cx[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (f < n) {
-            cx[j] = f < nq ? cs.cells[f] : cs.kcells[f - nq];
-            cid[j] = f < nq ? cs.ids[f] : cs.kids[f - nq];
-            cc[j] = cell_comp(cx[j], cid[j]);
-        }
-    }
-    consumer_sync();   // every cell is in registers: the survivors' memory may be rewritten
-    u64 L = 0ull;
-    if (n > k) {
-        u64 mn = ~0ull, mx = 0ull;
-#pragma unroll
-        for (int j = 0; j < kMaxJ; ++j) {
-            if (cc[j] != 0ull) {
-                mn = min(mn, cc[j]);
-                mx = max(mx, cc[j]);
-            }
-        }
-        cta_minmax(mn, mx, ctl);
-        L = bisect_bound(k, mn, mx, ctl, [&](u64 t) {
-            int c = 0;
-#pragma unroll
-            for (int j = 0; j < kMaxJ; ++j) c += cc[j] >= t ? 1 : 0;   // empty slots hold 0, t is never 0
-            return c;
-        });
-    }
-    if (tid == 0) ctl->out_cnt = 0;
-    consumer_sync();
-#pragma unroll
-    for (int j = 0; j < kMaxJ; ++j) {
-        if (cc[j] != 0ull && cc[j] >= L) {
-            const int p = atomicAdd(&ctl->out_cnt, 1);
-            if (p < kMaxK) {
-                cs.kcells[p] = cx[j];
-                cs.kids[p] = cid[j];
-            }
-        }
-    }
-    consumer_sync();
-    return SelectResult{min(ctl->out_cnt, kMaxK), L};
-}
-
-// The re-selection proper (rare): every lane drops the noted cells the bound has overtaken, the rest are read again
-// and the CTA keeps the k best cells.  All consumer threads call it, after the barrier of the rendez-vous.
-template <bool SOFTCAP>
-__device__ __noinline__ int compact_cells(int qn, int nkept, float thr_f) {
-    const Smem m = smem_view();
-    SharedCtl* ctl = m.ctl;
-    const SegCtx& sc = ctl->seg;
-    const int k = sc.k;
-    const int tid = threadIdx.x;
-    u64 bound = 0ull;
-    // every lane first drops what the bound has overtaken; then gather rounds: everything at once if it fits, else
-    // three cells per thread and round
-    qn = drop_stale(m.queue + tid, qn, fmaxf(thr_f, min_warp_bounds(ctl)));
-    int cap = kLaneQueue;
-    if (cta_scan(qn, ctl).total > kFlatCells) cap = kFlatCells / kThreads;
-    for (;;) {
-        const int cnt = min(qn, cap);
-        const ScanResult sr = cta_scan(cnt, ctl);
-        if (sr.total == 0) break;
-        for (int i0 = 0; i0 < cnt; i0 += 4) {   // four loads in flight
-            float4 c[4];
-            int col[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                col[u] = -1;
-                if (i0 + u < cnt) {
-                    col[u] = loc_column(m.queue[(size_t)(qn - 1 - i0 - u) * kThreads + tid], sc);
-                    c[u] = load_cell(sc, col[u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (col[u] >= 0) {
-                    m.cells[sr.before + i0 + u] = transform_cell<SOFTCAP>(c[u], sc, m.bitmap, col[u]);
-                    m.ids[sr.before + i0 + u] = col[u] + sc.id_base;
-                }
-            }
-        }
-        qn -= cnt;
-        consumer_sync();
-        const SelectResult r = select_cells(sr.total, nkept, k);
-        nkept = r.count;
-        bound = max(bound, r.bound);
-    }
-    if (tid == 0) {
-        ctl->need_compact = 0;
-        ctl->ev_bound = bound;
-    }
-    consumer_sync();
-    return 1 | (nkept << 1);
-}
-
-// One rendez-vous of all consumer warps of the CTA.  A warp comes here because it saw a request for a re-selection
-// (a lane's queue is nearly full), or because it has finished its part of the segment.  Every warp posts its
-// bound and the number of cells its lanes hold.  If a re-selection was asked for, the queued cells are read again
-// and the CTA keeps the k best cells (they become the survivors' list, all queues become empty), and `happened`
-// is set; otherwise every warp had finished and the posted values describe the whole segment.  Warps depend on
-// nothing but their own copies while streaming and look out for requests at every tile and in every wait, so
-// every warp gets here in bounded time.
-// Returns (happened) | (survivors << 1); the composite bound of a re-selection is left in ctl->ev_bound and the
-// warps' bounds in ctl->wbound.
-__device__ __forceinline__ int event_happened(int ev) { return ev & 1; }
-__device__ __forceinline__ int event_nkept(int ev) { return (ev >> 1) & 1023; }
-template <bool SOFTCAP>
-__device__ __forceinline__ int cta_event(int qn, int nkept, float run_max, float thr_f) {
-    const Smem m = smem_view();
-    SharedCtl* ctl = m.ctl;
-    const SegCtx& sc = ctl->seg;
-    const int k = sc.k;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float wb = warp_bound(run_max, k);
-    if (lane == 0) *reinterpret_cast<volatile float*>(&ctl->wbound[warp]) = wb;
-    if (tid == 0) ctl->out_cnt = 0;
-    consumer_sync();
-    if (*reinterpret_cast<volatile int*>(&ctl->need_compact) == 0) return nkept << 1;
-    return compact_cells<SOFTCAP>(qn, nkept, thr_f);
-}
-
-// Appends to the element list the logits of up to N cells of this thread that reach `thr` (NaNs and columns past
-// the end of the row take no part).  A warp reserves its part of the list with one atomic.  All lanes of the warp
-// must call; ncell = 0 contributes nothing.  Entries past the list's capacity are counted but not written.
+// Room in a list for every value of the warp that reaches `bound`: one shared-memory atomic per warp (lanes of a warp
+// that add to one word are served one after the other, 8 cycles each).  hit[i]: the lanes whose i-th value does; entries go
+// in order of i, then of lanes.  All lanes call.
 template <int N>
-__device__ __forceinline__ void append_elements(const float4 (&c)[N], const int (&id0)[N], int ncell, float thr, int id_end, u64* list,
-                                                SharedCtl* ctl) {
-    static_assert(N <= 8, "one mask bit per logit");
-    const int lane = threadIdx.x & 31;
-    unsigned mask = 0u;
+__device__ __forceinline__ int warp_reserve(const float (&v)[N], float bound, unsigned (&hit)[N], int* counter) {
+    int total = 0;
 #pragma unroll
-    for (int u = 0; u < N; ++u) {
-        if (u < ncell) {
-            const float xs[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (xs[e] >= thr && id0[u] + e < id_end) mask |= 1u << (4 * u + e);
-        }
+    for (int i = 0; i < N; ++i) {
+        hit[i] = __ballot_sync(0xffffffffu, v[i] >= bound);
+        total += __popc(hit[i]);
     }
-    const int mine = __popc(mask);
-    int inc = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    const int wtotal = __shfl_sync(0xffffffffu, inc, 31);
-    if (wtotal == 0) return;
-    int base = 0;
-    if (lane == 31) base = atomicAdd(&ctl->out_cnt, wtotal);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    int p = base + inc - mine;
-#pragma unroll
-    for (int u = 0; u < N; ++u) {
-        const float xs[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (mask & (1u << (4 * u + e))) {
-                if (p < kMergeCap) list[p] = make_comp(xs[e], id0[u] + e);
-                ++p;
-            }
-    }
+    int p = 0;
+    if ((threadIdx.x & 31) == 0 && total) p = atomicAdd(counter, total);
+    return __shfl_sync(0xffffffffu, p, 0);
 }
+__device__ __forceinline__ float cell_max(const float4& x) { return fmaxf(max3(x.x, x.y, x.z), x.w); }
 
-// The producer: one lane brings the CTA tiles in, one 1-D bulk copy per tile (large copies: the copy engine's cost
-// is per request), into a ring of kStages slots.  A slot is refilled once all consumer warps have handed it back.
-__device__ __forceinline__ void producer_loop(const StreamArgs& a, float* stage, SharedCtl* ctl, int t_begin, int nt) {
-    if ((threadIdx.x & 31) != 0) return;
-    const int T = a.tiles_per_row, V = a.n_vocab;
-    int irow = t_begin / T, ij = t_begin - irow * T;
-    long long t_last = clock64();
-    int i = 0;
-    while (i < nt) {
-        const int slot = i % kStages;
-        // the first kStages tiles find their slots free; later ones wait for the consumers' hand-back
-        if (i >= kStages && !mbar_try_wait(&ctl->empty[slot], (unsigned)((i / kStages - 1) & 1))) {
-            if (clock64() - t_last > kCopyWaitCycles) {   // the consumers never came back: report and stop
-                report_status(a.status, a.status_host, kStatusCopyTimeout);
-                return;
-            }
-            continue;
-        }
-        const int col0 = ij * kTile;
-        const int len = min(kTile, V - col0);   // >= 1
-        const float* src = a.logits + (a.row_ld >= 0 ? (int64_t)irow * a.row_ld : a.rows[irow].logits_off) + col0;
-        float* dst = stage + (size_t)slot * kTile;
-        const unsigned bytes = (unsigned)(len & ~3) * 4u;
-        for (int e = len & ~3; e < len; ++e) dst[e] = src[e];   // ragged tail by plain loads
-        if (bytes) {
-            fence_proxy_async_smem();   // generic-proxy accesses to this slot (the consumers' patches) precede the async write
-            mbar_expect_tx(&ctl->full[slot], bytes);
-            bulk_g2s(dst, src, bytes, &ctl->full[slot]);
-        } else {
-            mbar_arrive(&ctl->full[slot]);
-        }
-        t_last = clock64();
-        ++i;
-        if (++ij == T) {
-            ij = 0;
-            ++irow;
-        }
-    }
-}
+// A launch's arguments: with NDESC > 0 the row descriptors come with them (a batch of few rows needs no copy to the
+// device before the launch, and no CTA waits for a read of global memory before it knows its row).
+template <int NDESC>
+struct SelectArgs {
+    StreamArgs a;
+    RowDesc rows[NDESC > 0 ? NDESC : 1];
+};
 
-// The end of a segment.  All consumer threads call it once they have looked at their last tile of the segment:
-// re-selections that were still asked for, the rendez-vous of the finished warps, the element list, the segment's
-// k best logits in order, and - in the CTA that draws the row's last ticket - the merge and the row's epilogue.
-// With GREEDY (a launch whose rows are all greedy: a verification step, the static entry point) the streaming loop has
-// kept no queues: every lane brings the best logit it saw as a composite (`lane_best`, 0 = none), the CTA takes the
-// largest, and that one candidate goes through the same merge and epilogue as an ordered list of length one.
-template <bool SOFTCAP, bool GREEDY>
-__device__ __forceinline__ void segment_end(const StreamArgs& a, int row, int qn, int nkept, float thr_f, float run_max, bool mark, u64 lane_best) {
-    const Smem m = smem_view();
-    SharedCtl* ctl = m.ctl;
-    const SegCtx& sc = ctl->seg;
+template <int NDESC>
+__global__ void __launch_bounds__(kThreads, 4) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
+    const StreamArgs& a = args.a;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    float4* ring = reinterpret_cast<float4*>(smem_raw);
+    u64* picked = reinterpret_cast<u64*>(smem_raw);   // after the stream: candidates, the row's candidates in order, merge list
+    u64* out = picked + kPickCap + 8;
+    u64* list = out + kMaxK;
+    float4* listed = reinterpret_cast<float4*>(smem_raw + kRingBytes);
+    int* listed_num = reinterpret_cast<int*>(listed + kCellCap);
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(listed_num + kCellCap);
+    u64* recv = reinterpret_cast<u64*>(ctl + 1);
     const int tid = threadIdx.x;
-    const int T = a.tiles_per_row, V = a.n_vocab, Q = a.tiles_per_cta;
-    const RowDesc d = a.rows[row];
-    unsigned* myq = m.queue + tid;
-    const TailOut tout{a.tokens, a.tokens_host, a.status_host, a.kept_ids, a.kept_pr, a.kept_n, reinterpret_cast<u64*>(a.shard_out), a.shard_n, a.shard_stride, a.status};
-    float thr_final;
-    int n_el = 0;
-    int kk = 0;
-    if (GREEDY) {
-        u64 mn = lane_best ? lane_best : ~0ull, mx = lane_best;
-        cta_minmax(mn, mx, ctl);
-        if (mx == 0ull && !SOFTCAP) {
-            // No lane saw anything above minus infinity.  A segment of nothing but -inf (and NaN) still has an argmax in
-            // the reference - its first -inf - so look for one in memory (the penalty leaves -inf as it is).
-            u64 mine = 0ull;
-            for (int c = sc.seg_lo + tid; c < sc.seg_hi; c += kThreads) {
-                const float x = __ldcg(sc.row + c);
-                if (x == -__int_as_float(0x7f800000)) mine = max(mine, make_comp(x, c + sc.id_base));
-            }
-            mn = mine ? mine : ~0ull;
-            mx = mine;
-            cta_minmax(mn, mx, ctl);
-        }
-        if (mark) trace_mark(a, 4);
-        if (tid == 0) m.sorted[0] = mx;
-        consumer_sync();
-        kk = mx != 0ull ? 1 : 0;
-        n_el = kk;
-    }
-    for (; !GREEDY;) {
-        for (;;) {   // re-selections that were still asked for, then the rendez-vous of the finished warps
-            const int ev = cta_event<SOFTCAP>(qn, nkept, run_max, thr_f);
-            if (!event_happened(ev)) break;
-            qn = 0;
-            nkept = event_nkept(ev);
-        }
-        thr_final = fmaxf(thr_f, min_warp_bounds(ctl));
-        if (mark) trace_mark(a, 4);
-        // ---- the logits of the noted cells that reach the final bound become the element list
-        const int id_end = V + sc.id_base;
-        if (nkept > 0) {
-            float4 c[1];
-            int id0[1];
-            c[0] = m.kcells[min(tid, nkept - 1)];
-            id0[0] = m.kids[min(tid, nkept - 1)];
-            append_elements<1>(c, id0, tid < nkept ? 1 : 0, thr_final, id_end, m.list, ctl);
-        }
-        qn = drop_stale(myq, qn, thr_final);   // most noted cells have been overtaken by the bound
-        // a thread reads up to four of its cells per round (lanes rarely hold more that the bound has not overtaken)
-        const int rounds = (__reduce_max_sync(0xffffffffu, qn) + 3) >> 2;
-#pragma unroll 1
-        for (int rd = 0; rd < rounds; ++rd) {
-            float4 c[4];
-            int id0[4];
-            const int n = max(0, min(4, qn - 4 * rd));
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                id0[u] = 0;
-                c[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (u < n) {
-                    id0[u] = loc_column(myq[(4 * rd + u) * kThreads], sc);
-                    c[u] = load_cell(sc, id0[u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (u < n) {
-                    c[u] = transform_cell<SOFTCAP>(c[u], sc, m.bitmap, id0[u]);
-                    id0[u] += sc.id_base;
-                }
-            }
-            append_elements<4>(c, id0, n, thr_final, id_end, m.list, ctl);
-        }
-        consumer_sync();
-        n_el = ctl->out_cnt;
-        if (n_el <= kMergeCap) break;
-        // more logits reach the bound than the list can take (many equal values): keep the k best cells first
-        consumer_sync();
-        *reinterpret_cast<volatile int*>(&ctl->need_compact) = 1;
-    }
-    if (mark) trace_mark(a, 2);
-    if (mark && a.trace && tid == 0) a.trace[(size_t)blockIdx.x * 8 + 3] = (u64)n_el;
-    if (a.overlap == 1) pdl_wait_prior();   // from here on this launch writes what the previous launch in the stream may still be using
-    // the segment's k best logits (or all, if fewer), in order
-    const int first_cta = (row * T) / Q, last_cta = (row * T + T - 1) / Q;
-    const int nseg = last_cta - first_cta + 1;
-    bool merge_here = true;
-    if (!GREEDY) kk = topk_sorted(m.list, n_el, d.k, m.sorted, ctl);
-    if (a.pair) {
-        // The row's CTAs are a cluster: CTA r > 0 puts its ordered candidates into part r - 1 of CTA 0's receive
-        // buffer, all arrive at the cluster's barrier (the only phase of it in this kernel: the producer warps arrived
-        // when they finished), and CTA 0 merges.  No global memory, no ticket.
-        const unsigned rank = cluster_cta_rank();
-        if (rank != 0u) {
-            const unsigned remote = cluster_map_shared(smem_u32(m.recv + (rank - 1u) * (unsigned)d.k), 0u);
-            for (int i = tid; i < kk; i += kThreads) cluster_store_u64(remote + 8u * (unsigned)i, m.sorted[i]);
-            if (tid == 0) cluster_store_u32(cluster_map_shared(smem_u32(&ctl->recv_n[rank]), 0u), (unsigned)kk);
-        }
-        __syncwarp();
-        cluster_arrive_release();
-        merge_here = rank == 0u;
-        if (merge_here) {
-            cluster_wait_acquire();
-            if (a.pair == 2) {
-                // two lists: the rank of an entry is its place in its own list plus the number of entries of the other above it
-                const int n1 = min(*reinterpret_cast<volatile int*>(&ctl->recv_n[1]), d.k);
-                for (int e = tid; e < kk + n1; e += kThreads) {
-                    const bool mine = e < kk;
-                    const int i1 = mine ? e : e - kk;
-                    const u64 c = mine ? m.sorted[i1] : m.recv[i1];
-                    const u64* run = mine ? m.recv : m.sorted;
-                    int lo = 0, hi = mine ? n1 : kk;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (run[mid] > c) lo = mid + 1;
-                        else hi = mid;
-                    }
-                    if (i1 + lo < d.k) m.list[i1 + lo] = c;
-                }
-                consumer_sync();
-                kk = min(kk + n1, d.k);
-            } else {
-                // several lists: the same, summed over all the other lists
-                const int nl = a.pair;
-                if (tid == 0) ctl->recv_n[0] = kk;
-                consumer_sync();
-                int total = 0;
-                for (int s2 = 0; s2 < nl; ++s2) total += min(*reinterpret_cast<volatile int*>(&ctl->recv_n[s2]), d.k);
-                for (int e = tid; e < nl * d.k; e += kThreads) {
-                    const int s1 = e / d.k, i1 = e - s1 * d.k;
-                    if (i1 >= min(ctl->recv_n[s1], d.k)) continue;
-                    const u64 c = s1 == 0 ? m.sorted[i1] : m.recv[(s1 - 1) * d.k + i1];
-                    int rk = i1;
-                    for (int s2 = 0; s2 < nl; ++s2) {
-                        if (s2 == s1) continue;
-                        const u64* run = s2 == 0 ? m.sorted : m.recv + (s2 - 1) * d.k;   // descending: count its entries above c
-                        int lo = 0, hi = min(ctl->recv_n[s2], d.k);
-                        while (lo < hi) {
-                            const int mid = (lo + hi) >> 1;
-                            if (run[mid] > c) lo = mid + 1;
-                            else hi = mid;
-                        }
-                        rk += lo;
-                    }
-                    if (rk < d.k) m.list[rk] = c;
-                }
-                consumer_sync();
-                kk = min(total, d.k);
-            }
-            for (int i = tid; i < kk; i += kThreads) m.sorted[i] = m.list[i];
-            consumer_sync();
-        }
-    } else if (nseg > 1) {
-        // A row with several segments: segment s publishes its ordered candidates in its own part of the row's
-        // scratch (entries [s * k, s * k + count), the count in entry kMergeCap - 1 - s), then draws a ticket; the
-        // CTA that draws the row's last ticket merges.  The planner keeps nseg * (k + 1) within kMergeCap.
-        const int seg = (int)blockIdx.x - first_cta;
-        u64* dst = reinterpret_cast<u64*>(a.scratch) + (size_t)row * kMergeCap;
-        if ((seg + 1) * d.k + nseg <= kMergeCap) {
-            for (int i = tid; i < kk; i += kThreads) dst[seg * d.k + i] = m.sorted[i];
-            if (tid == 0) dst[kMergeCap - 1 - seg] = (u64)kk;
-        } else if (tid == 0) {
-            report_status(a.status, a.status_host, kStatusMergeOverflow);
-        }
-        consumer_sync();   // orders the CTA's stores before the ticket, whose release publishes them to the device
-        if (tid == 0) ctl->last = (ticket_add_acq_rel(&a.ticket[row], 1u) == (unsigned)(nseg - 1)) ? 1 : 0;
-        consumer_sync();
-        merge_here = ctl->last != 0;
-        if (merge_here) {   // all segments of the row have published (L2 reads, never L1)
-            if (tid == 0) a.ticket[row] = 0u;   // ready for the next launch
-            if (nseg <= kNumWarps) {
-                // few ordered lists: the rank of an entry is its place in its own list plus, for every other list,
-                // the number of entries above it (binary search); the lists keep their places in shared memory
-                // (counts and entries are read in one go; entries past a list's count are stale and ignored below)
-                const int span = nseg * d.k;
-                if (tid < nseg) ctl->wcount[tid] = min((int)__ldcg(dst + kMergeCap - 1 - tid), d.k);
-                for (int e = tid; e < span; e += kThreads) m.list[e] = __ldcg(dst + e);
-                consumer_sync();
-                int total = 0;
-                for (int s2 = 0; s2 < nseg; ++s2) total += ctl->wcount[s2];
-                for (int e = tid; e < span; e += kThreads) {
-                    const int s1 = e / d.k, i1 = e - s1 * d.k;
-                    if (i1 >= ctl->wcount[s1]) continue;
-                    const u64 c = m.list[e];
-                    int rank = i1;
-                    for (int s2 = 0; s2 < nseg; ++s2) {
-                        if (s2 == s1) continue;
-                        const u64* run = m.list + s2 * d.k;   // descending: count its entries above c
-                        int lo = 0, hi = ctl->wcount[s2];
-                        while (lo < hi) {
-                            const int mid = (lo + hi) >> 1;
-                            if (run[mid] > c) lo = mid + 1;
-                            else hi = mid;
-                        }
-                        rank += lo;
-                    }
-                    if (rank < d.k) m.sorted[rank] = c;
-                }
-                kk = min(total, d.k);
-                consumer_sync();
-            } else {   // many short lists: gather them into one list and order that
-                int total = 0;
-                for (int s2 = 0; s2 < nseg; ++s2) {
-                    const int n2 = min((int)__ldcg(dst + kMergeCap - 1 - s2), d.k);
-                    for (int i = tid; i < n2; i += kThreads) m.list[total + i] = __ldcg(dst + s2 * d.k + i);
-                    total += n2;
-                }
-                consumer_sync();
-                kk = topk_sorted(m.list, total, d.k, m.sorted, ctl);
-            }
-        }
-    }
-    if (mark) trace_mark(a, 5);
-    if (merge_here) {
-        const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.k, d.flags, d.out_index};
-        row_epilogue(m.sorted, kk, rt, reinterpret_cast<double*>(m.list), ctl, tout);
-    }
-    consumer_sync();
-    if (mark) trace_mark(a, 6);
-}
-
-template <bool SOFTCAP, bool GREEDY>
-__global__ void __launch_bounds__(kBlockThreads, 1) stream_select_kernel(const __grid_constant__ StreamArgs a) {
-    const Smem m = smem_view();
-    SharedCtl* ctl = m.ctl;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int T = a.tiles_per_row, V = a.n_vocab;
-    const int t_begin = blockIdx.x * a.tiles_per_cta;
-    const int t_end = min(t_begin + a.tiles_per_cta, a.total_tiles);
-    const int nt = t_end - t_begin;
-    // With launch overlap on, the next launch in the stream may start as soon as this one leaves room; like this one
-    // it waits for its predecessor before it writes anything (segment_end), so only the reading of logits overlaps -
-    // or, in mode 2, before it does anything at all, so only its placement on the SMs does.
     pdl_launch_dependents();
-    if (nt <= 0) return;
     trace_mark(a, 0);
-    if (a.write_back || a.overlap == 2) pdl_wait_prior();   // this launch stores into the logits while it streams, or was asked to wait
+    // Mode 1 waits only before its first write (unless it stores into the logits); otherwise only the launch's latency -
+    // placing the CTAs on the SMs - overlaps the end of the launch before it.
+    if (a.write_back || a.overlap != 1) pdl_wait_prior();
 
-    if (tid == 0) {   // one thread initialises every barrier, then makes the initialisation visible to the copy engine
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(&ctl->full[s], 1u);                  // the producer's arrive (+ the copy's bytes)
-            mbar_init(&ctl->empty[s], (unsigned)kWarps);   // one arrive per consumer warp
+    const int nseg = a.nseg;
+    const int row = nseg == 1 ? (int)blockIdx.x : (int)blockIdx.x / nseg;
+    const int seg = (int)blockIdx.x - row * nseg;
+    const RowDesc& dp = NDESC > 0 ? args.rows[row] : a.rows[row];
+    const float* row_ptr = a.logits + (a.row_ld >= 0 ? (int64_t)row * a.row_ld : dp.logits_off);
+
+    // The row's whole 16-byte cells, cut into nseg runs.  Up to three logits before the first cell belong to the first
+    // segment, up to three after the last cell to the last one: rows may start anywhere.
+    const int V = a.n_vocab;
+    const int head = min(V, (int)((0u - ((unsigned)reinterpret_cast<uintptr_t>(row_ptr) >> 2)) & 3u));
+    const int n_cells = (V - head) >> 2;
+    const int per = (n_cells + nseg - 1) / nseg;
+    const int c_lo = min(seg * per, n_cells), c_hi = min(c_lo + per, n_cells);
+    const float4* cells = reinterpret_cast<const float4*>(row_ptr + head);
+    const float qnan = __int_as_float(0x7fc00000), ninf = -__int_as_float(0x7f800000);
+    const unsigned slot0 = smem_u32(ring + tid);
+    // chunk c of this thread: cells j, j + kThreads, ... go to stage c % kStages
+    auto fetch = [&](int c) {
+        const int j = c_lo + c * kChunkCells + tid;
+        const unsigned dst = slot0 + (unsigned)((c % kStages) * kChunkCells) * (unsigned)sizeof(float4);
+#pragma unroll
+        for (int u = 0; u < kCells; ++u)
+            if (j + u * kThreads < c_hi) cp_async16(dst + (unsigned)(u * kThreads * sizeof(float4)), cells + j + u * kThreads);
+        cp_async_commit();
+    };
+    for (int c = 0; c < kStages; ++c) fetch(c);
+    float edge = qnan;   // one of the logits outside the whole cells
+    int edge_col = -1;
+    if (seg == 0 && tid < head) edge_col = tid;
+    if (seg == nseg - 1 && tid >= 4 && tid < 4 + V - head - 4 * n_cells) edge_col = head + 4 * n_cells + tid - 4;
+    if (edge_col >= 0) edge = __ldcg(row_ptr + edge_col);
+
+    Segment s;
+    s.row = row_ptr;
+    s.bitmap = reinterpret_cast<unsigned*>(recv + recv_entries(nseg));
+    s.lo = seg == 0 ? 0 : head + 4 * c_lo;
+    s.hi = seg == nseg - 1 ? V : head + 4 * c_hi;
+    s.bit0 = head + 4 * c_lo - 32;
+    s.id_base = a.vocab_offset;
+    s.has_pen = (dp.flags & kRowPenalty) != 0;
+    s.pen = dp.penalty;
+    s.cap = a.softcap;
+    s.hist = nullptr;
+    s.hist_len = 0;
+    const int k = dp.k;
+    int pen_col = -1;        // the first window id of this thread, if it is a column of the segment, and its logit
+    float pen_raw = qnan;
+    if (tid == 0) {
+        ctl->list_n = 0;
+        ctl->kept_n = 0;
+    }
+    if (nseg > 1) cluster_arrive_release();   // (waited for before the first store to another CTA's shared memory)
+    if (s.has_pen) {
+        s.hist = a.hist + dp.hist_begin;
+        s.hist_len = dp.hist_len;
+        const int first_id = tid < s.hist_len ? s.hist[tid] : -1;
+        for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += kThreads) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        set_bits(s, first_id);
+        const int c = first_id - s.id_base;
+        if (tid < s.hist_len && c >= s.lo && c < s.hi) {
+            pen_col = c;
+            pen_raw = __ldcg(row_ptr + c);
         }
-        ctl->abort = 0;
-        ctl->need_compact = 0;
-        fence_mbar_init();
     }
-    __syncthreads();   // the only barrier the producer warp takes part in
-    if (warp == kWarps) {
-        if (a.bulk_ok) producer_loop(a, m.stage, ctl, t_begin, nt);
-        __syncwarp();
-        if (a.pair) cluster_arrive_release();   // every thread of the cluster arrives exactly once (see segment_end)
-        return;
-    }
+    __syncthreads();
+    if (edge_col >= 0 && penalised(s, edge_col)) edge = qnan;   // penalised logits are looked at on their own
     trace_mark(a, 1);
 
-    // ------------------------------------------------------------------------------------------ consumers
-    // The loop over a segment's tiles contains no call: everything rare (re-selections, the end of the segment)
-    // happens outside it, so that the loop's state stays in registers.
-    const float ninf = -__int_as_float(0x7f800000);
-    unsigned* myq = m.queue + tid;   // entry i of this lane's queue is myq[i * kThreads]
-    const unsigned q_base = smem_u32(myq);
-    float* const st_warp = m.stage + warp * kWTile;
-    int it = 0;                            // tiles of this CTA looked at so far (the position in the ring)
-    for (int tile = t_begin; tile < t_end;) {
-        // ---- a new segment starts (all consumer warps are here together: kernel start or after a segment end)
-        const int row = tile / T, j0 = tile - row * T;
-        const int seg_nt = min(t_end - tile, T - j0);
-        const int seg_lo = j0 * kTile;
-        const int seg_hi = min(V, (j0 + seg_nt) * kTile);
-        const RowDesc d = a.rows[row];
-        const float* row_ptr = a.logits + d.logits_off;
-        float* wb_row = a.write_back ? const_cast<float*>(row_ptr) : nullptr;
-        const float pen = d.penalty;
-        const int row_k = d.k;
-        const bool has_pen = (d.flags & kRowPenalty) != 0;
-        if (tid == 0) {   // what the rendez-vous code needs to know about the segment
-            SegCtx& sc = ctl->seg;
-            sc.row = row_ptr;
-            sc.pen = pen;
-            sc.cap = a.softcap;
-            sc.has_pen = has_pen ? 1 : 0;
-            sc.id_base = a.vocab_offset;
-            sc.seg_lo = seg_lo;
-            sc.seg_hi = seg_hi;
-            sc.n_vocab = V;
-            sc.vec_ok = a.bulk_ok;
-            sc.k = row_k;
-            sc.final_in_mem = a.write_back;
+    // ---- the stream
+    float run_a = ninf, run_b = ninf, thr = -FLT_MAX, admit = -FLT_MAX, seen = ninf;
+    bool fresh = false;   // the bound takes in everything seen so far
+    bool lost = false;    // a list was too short
+    bool again = false;   // the second time through: the bound is final
+    int n = 0;
+again_from_the_start:
+    for (int c = 0, j0 = c_lo + tid;; ++c, j0 += kChunkCells) {
+        const int left = c_hi - (j0 - tid);   // cells of the segment from this chunk on
+        cp_async_wait<kStages - 1>();
+        const float4* st = ring + (c % kStages) * kChunkCells + tid;
+        float4 x[kCells];
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) x[u] = st[u * kThreads];
+        if (left < kChunkCells) {
+#pragma unroll
+            for (int u = 0; u < kCells; ++u)
+                if (tid + u * kThreads >= left) x[u] = make_float4(ninf, ninf, ninf, ninf);
         }
-        if (has_pen) {   // bitmap of the penalised columns of this segment
-            const int words = (seg_hi - seg_lo + 31) >> 5;
-            for (int i = tid; i < words; i += kThreads) m.bitmap[i] = 0u;
-            consumer_sync();
-            const int32_t* h = a.hist + d.hist_begin;
-            for (int i = tid; i < d.hist_len; i += kThreads) {
-                const int c = h[i] - a.vocab_offset;
-                if (c >= seg_lo && c < seg_hi) atomicOr(&m.bitmap[(c - seg_lo) >> 5], 1u << ((c - seg_lo) & 31));
-            }
-        }
-        consumer_sync();
-
-        float thr_f = ninf, run_max = ninf;
-        // GREEDY: the lane's best logit so far - the cell it sits in, that cell's first column, the cell's maximum
-        float4 best_cell = make_float4(0.f, 0.f, 0.f, 0.f);
-        float best = ninf;
-        int best_col = -1;
-        u64 thr_comp = 0ull;
-        int qn = 0;       // cells in this lane's queue
-        int nkept = 0;    // cells in the survivors' list (the same value in every thread)
-        int s = 0;        // tiles of the segment this warp has looked at
-        int col0 = seg_lo + warp * kWTile;   // first column of this warp's part of tile s
-
-        for (;;) {
-            int reason = 0;   // why the loop over the tiles was left: 0 = segment done, 1 = a queue of this warp is nearly full,
-                              // 2 = another warp asked for a re-selection while this one was waiting for a copy
-            unsigned slot = (unsigned)it % kStages, par = ((unsigned)it / kStages) & 1u;   // ring slot of tile `it` and its phase
-            for (; s < seg_nt; ++s, ++it, col0 += kTile, slot = (slot + 1u) % kStages, par ^= (slot == 0u ? 1u : 0u)) {
-                if (!GREEDY && __any_sync(0xffffffffu, qn > kLaneQueue - 4)) {
-                    reason = 1;
-                    break;
-                }
-                float* st = st_warp + slot * kTile;              // this warp's part of the CTA tile
-                const int len = min(kWTile, V - col0);            // may be <= 0 in a row's last tile
-                if (a.bulk_ok) {
-                    // ---- wait for the CTA tile's copy.  A warp that has to wait also answers re-selection requests of
-                    // other warps: a requester sits at the barrier of cta_event, and the ring only moves when every warp does.
-                    bool landed = mbar_try_wait(&ctl->full[slot], par);
-                    if (!landed) {
-                        const long long lim = ctl->abort ? 2000ll : kCopyWaitCycles;
-                        const long long t0 = clock64();
-                        for (;;) {
-                            if (mbar_try_wait(&ctl->full[slot], par)) {
-                                landed = true;
-                                break;
-                            }
-                            if (__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&ctl->need_compact) != 0)) break;
-                            if (clock64() - t0 > lim) {   // the copy never landed: report, carry on with what is there
-                                ctl->abort = 1;
-                                report_status(a.status, a.status_host, kStatusCopyTimeout);
-                                landed = true;
-                                break;
-                            }
-                        }
-                        if (!landed) {
-                            reason = 2;
-                            break;
-                        }
-                    }
-                } else if (len > 0) {   // rows not on 16-byte boundaries: the warp loads its tile itself
-                    const float* src = row_ptr + col0;
-                    for (int e = lane; e < len; e += 32) st[e] = src[e];
-                    __syncwarp();
-                }
-                if (SOFTCAP) {
-                    if (len > 0) softcap_tile(st, len, a.softcap, wb_row ? wb_row + col0 : nullptr);
-                }
-                if (has_pen && len > 0) patch_tile(st, len, col0, seg_lo, pen, m.bitmap, wb_row);
-                if (len < kWTile) {   // what lies past the end of a ragged row is made NaN: never a maximum, never reaches a bound
-                    for (int e = max(len, 0) + lane; e < kWTile; e += 32) st[e] = __int_as_float(0x7fc00000);
-                    __syncwarp();
-                }
-                // ---- look: the lane's four cells go to registers (four independent 16-byte loads)
-                const float4* st4 = reinterpret_cast<const float4*>(st);
-                const float4 x0 = st4[lane], x1 = st4[lane + 32], x2 = st4[lane + 64], x3 = st4[lane + 96];
-                const float m0 = fmaxf(max3(x0.x, x0.y, x0.z), x0.w);
-                const float m1 = fmaxf(max3(x1.x, x1.y, x1.z), x1.w);
-                const float m2 = fmaxf(max3(x2.x, x2.y, x2.z), x2.w);
-                const float m3 = fmaxf(max3(x3.x, x3.y, x3.z), x3.w);
-                run_max = fmaxf(max3(run_max, m0, m1), fmaxf(m2, m3));
-                __syncwarp();
-                if (lane == 0 && a.bulk_ok) mbar_arrive(&ctl->empty[slot]);   // the slot goes back to the producer
-                if (GREEDY) {
-                    // the lane meets its cells in ascending column order, so "strictly larger" keeps the first of equals
-                    const int c0 = col0 + 4 * lane;
-                    if (m0 > best) { best = m0; best_cell = x0; best_col = c0; }
-                    if (m1 > best) { best = m1; best_cell = x1; best_col = c0 + 128; }
-                    if (m2 > best) { best = m2; best_cell = x2; best_col = c0 + 256; }
-                    if (m3 > best) { best = m3; best_cell = x3; best_col = c0 + 384; }
-                    continue;
-                }
-
-                // ---- the admission bound: set at the segment's first tile (all warps must have posted: one barrier per
-                // segment), then refreshed without a barrier at tiles 1, 2, 4, 8, ... of the segment
-                if ((s & (s - 1)) == 0) {   // s = 0, 1, 2, 4, 8, ...
-                    const float wb = warp_bound(run_max, row_k);
-                    if (lane == 0) *reinterpret_cast<volatile float*>(&ctl->wbound[warp]) = wb;
-                    if (s == 0) consumer_sync();
-                    else __syncwarp();
-                    thr_f = fmaxf(thr_f, min_warp_bounds(ctl));
-                }
-
-                // ---- note the cells whose maximum reaches the bound (padding past the end of a row never does)
-                const unsigned loc = (unsigned)s << 2;
-                if (thr_comp == 0ull) {
-                    note_cell_if(m0, thr_f, loc, q_base, qn);
-                    note_cell_if(m1, thr_f, loc | 1u, q_base, qn);
-                    note_cell_if(m2, thr_f, loc | 2u, q_base, qn);
-                    note_cell_if(m3, thr_f, loc | 3u, q_base, qn);
-                } else {   // after a re-selection: ties at the bound are settled by token id
-                    const int id_lane = col0 + 4 * lane + a.vocab_offset;
-                    if (m0 >= thr_f && make_comp(m0, id_lane) >= thr_comp) myq[(qn++) * kThreads] = make_entry(m0, loc);
-                    if (m1 >= thr_f && make_comp(m1, id_lane + 128) >= thr_comp) myq[(qn++) * kThreads] = make_entry(m1, loc | 1u);
-                    if (m2 >= thr_f && make_comp(m2, id_lane + 256) >= thr_comp) myq[(qn++) * kThreads] = make_entry(m2, loc | 2u);
-                    if (m3 >= thr_f && make_comp(m3, id_lane + 384) >= thr_comp) myq[(qn++) * kThreads] = make_entry(m3, loc | 3u);
-                }
-            }
-            if (reason == 0) break;
-            // ---- a re-selection: the CTA keeps the k best of the cells noted so far, every queue becomes empty
-            if (reason == 1) {   // first drop what the bound has overtaken: that alone makes room, as a rule
-                qn = drop_stale(myq, qn, thr_f);
-                if (!__any_sync(0xffffffffu, qn > kLaneQueue - 4)) continue;
-                *reinterpret_cast<volatile int*>(&ctl->need_compact) = 1;
-            }
-            const int ev = cta_event<SOFTCAP>(qn, nkept, run_max, thr_f);
-            if (event_happened(ev)) {
-                qn = 0;
-                nkept = event_nkept(ev);
-                const u64 eb = ctl->ev_bound;
-                if (eb) {
-                    thr_comp = max(thr_comp, eb);
-                    thr_f = fmaxf(thr_f, comp_floor_value(eb));
+        if (s.has_pen) {   // penalised logits are left out
+            const unsigned* w = s.bitmap + ((j0 - c_lo) >> 3) + 1;
+            const int sh = 4 * ((j0 - c_lo) & 7);
+            unsigned bits[kCells];
+#pragma unroll
+            for (int u = 0; u < kCells; ++u) bits[u] = tid + u * kThreads < left ? (w[u * (kThreads / 8)] >> sh) & 15u : 0u;
+            if (bits[0] | bits[1] | bits[2] | bits[3]) {
+#pragma unroll
+                for (int u = 0; u < kCells; ++u) {
+                    if (bits[u] & 1u) x[u].x = ninf;
+                    if (bits[u] & 2u) x[u].y = ninf;
+                    if (bits[u] & 4u) x[u].z = ninf;
+                    if (bits[u] & 8u) x[u].w = ninf;
                 }
             }
         }
-        u64 lane_best = 0ull;
-        if (GREEDY && best_col >= 0) {   // the first logit of the cell that equals its maximum (-0 and +0 are equal here and in a composite)
-            const int e = best_cell.x == best ? 0 : best_cell.y == best ? 1 : best_cell.z == best ? 2 : 3;
-            lane_best = make_comp(best, best_col + e + a.vocab_offset);
+        const float m0 = cell_max(x[0]), m1 = cell_max(x[1]), m2 = cell_max(x[2]), m3 = cell_max(x[3]);
+        const float ma = fmaxf(m0, m1), mb = fmaxf(m2, m3);
+        run_a = fmaxf(run_a, ma);
+        run_b = fmaxf(run_b, mb);
+        fetch(c + kStages);   // into the stage just read
+        fresh = !again && ((c & (c + 1)) == 0 || thr <= -FLT_MAX || (k > 64 && c < 8));
+        if (fresh) {
+            thr = cta_bound(run_a, run_b, k, ctl, n);
+            admit = thr;
+            if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
+            else seen = thr > -FLT_MAX ? thr : ninf;
+            lost = lost || n > kCellCap;
+            if (n > kCellCap / 2 && !lost) prune_cells(listed, listed_num, ctl, admit);
         }
-        segment_end<SOFTCAP, GREEDY>(a, row, qn, nkept, thr_f, run_max, tile + seg_nt >= t_end, lane_best);
-        tile += seg_nt;
+        if (__any_sync(0xffffffffu, fmaxf(ma, mb) >= admit)) {
+            const float m[kCells] = {m0, m1, m2, m3};
+            unsigned hit[kCells];
+            int p = warp_reserve<kCells>(m, admit, hit, &ctl->list_n);
+#pragma unroll
+            for (int u = 0; u < kCells; ++u) {
+                const int q = p + __popc(hit[u] & lanes_below());
+                if (m[u] >= admit && q < kCellCap) {
+                    listed[q] = x[u];
+                    listed_num[q] = j0 + u * kThreads;
+                }
+                p += __popc(hit[u]);
+            }
+        }
+        if (left <= kChunkCells) break;
     }
+    cp_async_wait<0>();
+    trace_mark(a, 4);
+
+    // ---- the segment's candidates: logits that reach the final bound
+    if (fresh || again) {
+        __syncthreads();
+    } else {
+        thr = cta_bound(run_a, run_b, k, ctl, n);
+        admit = thr;
+        if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
+        else seen = thr > -FLT_MAX ? thr : ninf;
+    }
+    const bool bounded = thr > -FLT_MAX;
+    n = ctl->list_n;
+    lost = lost || n > kCellCap;
+    if (lost && bounded && !again) {   // the early bounds let too much through: the final one will not, unless many logits are equal
+        __syncthreads();
+        if (tid == 0) ctl->list_n = 0;
+        for (int c = 0; c < kStages; ++c) fetch(c);
+        lost = false;
+        again = true;
+        __syncthreads();
+        goto again_from_the_start;
+    }
+    auto pick = [&](bool hit, float y, int col) {   // all lanes of the warp
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (m == 0u) return;
+        int p = 0;
+        if ((tid & 31) == 0) p = atomicAdd(&ctl->kept_n, __popc(m));
+        p = __shfl_sync(0xffffffffu, p, 0) + __popc(m & lanes_below());
+        if (hit && p < kPickCap) picked[p] = make_comp(y, col + s.id_base);
+    };
+    if (!lost) {
+        for (int p0 = tid & ~31; p0 < n; p0 += kThreads) {
+            const int p = p0 + (tid & 31);
+            float xs[4] = {ninf, ninf, ninf, ninf};
+            int col = 0;
+            if (p < n) {
+                *reinterpret_cast<float4*>(xs) = listed[p];
+                col = head + 4 * listed_num[p];
+            }
+            if (s.cap != 0.0f) {
+#pragma unroll 1
+                for (int e = 0; e < 4; ++e) xs[e] = xs[e] >= admit ? softcap_call(xs[e], s.cap) : ninf;
+            }
+            unsigned hit[4];
+            int q = warp_reserve<4>(xs, fmaxf(seen, -FLT_MAX), hit, &ctl->kept_n);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int at = q + __popc(hit[e] & lanes_below());
+                if (xs[e] >= fmaxf(seen, -FLT_MAX) && at < kPickCap) picked[at] = make_comp(xs[e], col + e + s.id_base);
+                q += __popc(hit[e]);
+            }
+        }
+        if (tid < 32 && V != 4 * n_cells) {
+            const float y = s.cap != 0.0f ? softcap_call(edge, s.cap) : edge;
+            pick(edge >= admit && y >= seen, y, edge_col);
+        }
+        if (s.has_pen) {
+            for (int i0 = tid & ~31; i0 < s.hist_len; i0 += kThreads) {
+                const int i = i0 + (tid & 31);
+                float x = pen_raw;
+                int col = pen_col;
+                if (i != tid) {
+                    col = i < s.hist_len ? s.hist[i] - s.id_base : -1;
+                    x = col >= s.lo && col < s.hi ? __ldcg(row_ptr + col) : qnan;
+                }
+                const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
+                pick(y >= seen && y > ninf && claim(s, col), y, col);
+            }
+        }
+    }
+    __syncthreads();
+    n = ctl->kept_n;
+    lost = lost || n > kPickCap;
+    if (lost || (n < k && (bounded || s.cap != 0.0f))) n = exact_select(s, k, picked, ctl);
+    else if (n < k) n = append_masked(s, n, k, picked, ctl);
+    if (a.write_back) write_back(s);
+    trace_mark(a, 2);
+    if (a.trace && tid == 0 && blockIdx.x < 4096u) a.trace[(size_t)blockIdx.x * 8 + 3] = (u64)n;
+    if (a.overlap == 1) pdl_wait_prior();   // from here on this launch writes what the previous launch in the stream may still be using
+
+    // ---- the row: the k best of all its segments' candidates, in order
+    u64* all = picked;
+    if (nseg > 1) {
+        const int lseg = nseg == 8 ? 3 : nseg == 4 ? 2 : 1;
+        cluster_wait_acquire();   // every CTA of the row runs: the first one's shared memory may be written
+        const unsigned dst = cluster_map_shared(smem_u32(recv + seg * kSendCap), 0u);
+        if (n > kSendCap) {       // (k > 64, or many equal logits)
+            rank_emit(picked, n, k, list, ctl, [&](int rank, u64 m) { cluster_store_u64(dst + 8u * (unsigned)rank, m); });
+            n = min(n, k);
+        } else if (tid < n) {
+            cluster_store_u64(dst + 8u * (unsigned)tid, picked[tid]);
+        }
+        if (tid == 0) cluster_store_u32(cluster_map_shared(smem_u32(&ctl->recv_n[seg]), 0u), (unsigned)n);
+        __syncwarp();
+        cluster_arrive_release();
+        if (seg != 0) {
+            trace_mark(a, 6);
+            return;
+        }
+        if (tid == 0) ctl->out_cnt = 0;
+        cluster_wait_acquire();
+        // a bound that k of them reach, then those that reach it (thread t looks after every (256 / nseg)-th candidate of one segment)
+        const int q = tid & (nseg - 1), n_q = ctl->recv_n[q];
+        const u64* from = recv + q * kSendCap;
+        run_a = run_b = ninf;
+        for (int i = tid >> lseg; i < n_q; i += kThreads >> lseg) {
+            const float y = comp_value(from[i]);
+            if (i & (kThreads >> lseg)) run_b = fmaxf(run_b, y);
+            else run_a = fmaxf(run_a, y);
+        }
+        const float floor_y = cta_bound(run_a, run_b, k, ctl, n);
+        const float least = floor_y > -FLT_MAX ? floor_y : ninf;
+        int most = 0;
+        for (int g = 0; g < nseg; ++g) most = max(most, ctl->recv_n[g]);
+        for (int i = tid >> lseg; (i - (tid >> lseg)) < most; i += kThreads >> lseg) {
+            const u64 m = i < n_q ? from[i] : 0ull;
+            const bool hit = m != 0ull && comp_value(m) >= least;
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            if (hits == 0u) continue;
+            int p = 0;
+            if ((tid & 31) == 0) p = atomicAdd(&ctl->out_cnt, __popc(hits));
+            p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
+            if (hit) list[p] = m;
+        }
+        __syncthreads();
+        n = ctl->out_cnt;
+        all = list;
+    }
+    rank_emit(all, n, k, all == list ? picked : list, ctl, [&](int rank, u64 m) { out[rank] = m; });
+    __syncthreads();
+    trace_mark(a, 5);
+    const RowDesc& d = dp;
+    const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.flags, d.out_index, d.hist_begin + d.hist_len};
+    const TailOut tout{a.tokens, a.tokens_host, a.status_host, a.pool, a.kept_ids, a.kept_pr, a.kept_n, reinterpret_cast<u64*>(a.shard_out), a.shard_n, a.shard_stride, a.status};
+    row_epilogue(out, min(n, k), rt, reinterpret_cast<double*>(list), ctl, tout);
+    trace_mark(a, 6);
+}
+
+constexpr int kFewRows = 8, kArgRows = 64;   // batches of up to this many rows send their descriptors with the launch
+
+template <int NDESC>
+int launch_select(const cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows) {
+    SelectArgs<NDESC> args;
+    args.a = a;
+    if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
+    return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<NDESC>, args);
 }
 
 }  // namespace
 
-size_t stream_kernel_smem_bytes() { return kSmemTotal; }
-
-// Per-device set-up (the current device): opt in to the large dynamic shared memory; report resident CTAs per SM.
-int prepare_device_kernels(int* ctas_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(stream_select_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(stream_select_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(stream_select_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(stream_select_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
-    if (e != cudaSuccess) return (int)e;
-    int n = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stream_select_kernel<false, false>, kBlockThreads, kSmemTotal);
-    if (e != cudaSuccess) return (int)e;
-    if (ctas_per_sm) *ctas_per_sm = n;
-    return 0;
+// Per-device set-up (the current device): opt in to the large dynamic shared memory.
+int prepare_device_kernels() {
+    cudaError_t e = cudaFuncSetAttribute(stream_select_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<kFewRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<kArgRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    return (int)e;
 }
 
-int launch_stream_kernel(const StreamArgs& a, int grid, void* stream) {
+int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* stream) {
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (a.overlap) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
-    if (a.pair) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = a.overlap ? 1 : 0;
+    ++n;
+    if (a.nseg > 1) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = (unsigned)a.pair;
+        attr[n].val.clusterDim.x = (unsigned)a.nseg;
         attr[n].val.clusterDim.y = 1;
         attr[n].val.clusterDim.z = 1;
         ++n;
     }
+    const int seg_cols = a.penalised ? 4 * ((a.n_vocab / 4 + a.nseg - 1) / a.nseg) + 8 : 0;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kBlockThreads);
-    cfg.dynamicSmemBytes = kSmemTotal;
+    cfg.gridDim = dim3((unsigned)(a.n_rows * a.nseg));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = select_smem_bytes(a.nseg, seg_cols);
+    if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    if (a.all_greedy) {
-        if (a.softcap != 0.0f) return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<true, true>, a);
-        return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<false, true>, a);
-    }
-    if (a.softcap != 0.0f) return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<true, false>, a);
-    return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<false, false>, a);
+    if (host_rows && a.n_rows <= kFewRows) return launch_select<kFewRows>(cfg, a, host_rows);
+    if (host_rows && a.n_rows <= kArgRows) return launch_select<kArgRows>(cfg, a, host_rows);
+    return launch_select<0>(cfg, a, nullptr);
 }
 
-// The launch plan (host).  A row's scratch holds kMergeCap entries: k candidates and a count per segment.
-Plan make_plan(int n_rows, int n_vocab, int kmax, int slots) {
-    Plan pl;
-    const int T = (n_vocab + kTile - 1) / kTile;
-    pl.tiles_per_row = T;
-    pl.total_tiles = n_rows * T;
-    slots = std::max(1, slots);
-    const int max_seg = std::max(2, kMergeCap / (std::max(1, kmax) + 1));
-    const int q_min = (T + (max_seg - 1) - 1) / (max_seg - 1);
-    const int q_fill = (pl.total_tiles + slots - 1) / slots;   // fewest tiles per CTA that still give a single wave
-    int q = std::max(1, std::min(std::max(q_fill, q_min), kMaxTilesPerCta));
-    if (T <= kMaxTilesPerCta && n_rows >= 2 * slots) {
-        // Plenty of rows: one CTA per row, in waves.  Every CTA pays its start and its end-of-segment work once per row
-        // and no row has to be merged.  The exception is a last wave that would be nearly empty (300 rows on 148 SMs:
-        // two full waves and four CTAs): then one wave of CTAs each takes the same number of consecutive tiles, a little
-        // more than two rows' worth, and a row that straddles two CTAs is merged through its scratch.  Measured on B200:
-        // 300 x 262144 takes 101 us by rows and 87 us this way; with a last wave that is a third full or more the waves
-        // win (512 rows: 138 against 141 us), because a thin last wave streams faster than a full one.
-        const int rest = n_rows % slots;
-        q = (rest > 0 && rest * 8 < slots) ? (pl.total_tiles + slots - 1) / slots : T;
-    } else {
-        // Otherwise a row is cut into nseg = T / q aligned pieces.  Fewer tiles per CTA shorten the streaming (per 32 KiB
-        // tile about 0.4 us on a lone SM, 0.6 us when every SM streams), more pieces lengthen the merge: nothing for one
-        // piece, the on-chip exchange inside a cluster of 2, 4 or 8 CTAs, ordered lists merged through scratch up to 16, a
-        // gather-and-select beyond (measured on B200, in us).  Pick the cheapest q that divides the row and keeps
-        // the grid within one wave.
-        double best = 1e30;
-        for (int c = q; c <= std::min(T, kMaxTilesPerCta); ++c) {
-            if (T % c != 0) continue;
-            const int nseg = T / c;
-            const double busy = std::min(1.0, (double)n_rows * nseg / slots);
-            const bool on_chip = (nseg == 2 || nseg == 4 || nseg == 8) && (nseg - 1) * std::max(1, kmax) <= 512;   // a cluster per row
-            const double merge = nseg == 1 ? 0.0 : on_chip ? (nseg == 2 ? 1.4 : nseg == 4 ? 2.8 : 4.3)
-                                 : nseg <= 8 ? 2.4 + 0.25 * nseg : nseg <= 16 ? 4.4 + 0.5 * nseg : 10.0 + 0.3 * nseg;
-            const double cost = (0.4 + 0.2 * busy) * c + merge;
-            if (cost < best) {
-                best = cost;
-                q = c;
-            }
-        }
-    }
-    pl.tiles_per_cta = q;
-    pl.grid = (pl.total_tiles + q - 1) / q;
-    return pl;
+// Segments per row: up to eight, as long as there are not more CTAs than two per SM and a segment has at least two chunks.
+// Measured on B200 (1 / 2 / 4 / 8 segments, us per synchronous call): 1 x 65536 33 / 30 / 27 / 25, 32 x 131072 (four steps)
+// 176 / 153 / 130 / 124, 64 x 262144 (launch) 55 / 40 / 33 / 40, 72 x 131072 93 / 87 / 84 / 93, 136 x 65536 32 / 34 / 36 / 48,
+// 512 x 32768 73 / 91 / 106 / 160: a segment more costs every CTA its fixed steps once more.
+int plan_segments(int n_rows, int n_vocab, int sms) {
+    int nseg = 1;
+    while (nseg < 8 && (int64_t)n_rows * nseg * 2 <= 2 * sms && n_vocab / (nseg * 2) >= 8 * kChunkCells) nseg *= 2;
+    return nseg;
 }
 
 }  // namespace fsb
 
 // ---------------------------------------------------------------------------------------------- fsb_argmax_rows_static
-// Greedy tokens of device-resident rows with no allocation at all: the streaming kernel above, run with every piece
-// of device memory it needs taken from one array that is part of this library's image.
+// Greedy tokens of device-resident rows with no allocation at all: the streaming kernel above, with its row descriptors
+// and status word in one array that is part of this library's image.
 namespace fsb {
 namespace {
 
 constexpr int kStaticMaxRows = FSB_STATIC_MAX_ROWS;
-constexpr size_t kStaticRowsOff = 0;                                                       // RowDesc[kStaticMaxRows]
-constexpr size_t kStaticFillOff = kStaticRowsOff + sizeof(RowDesc) * kStaticMaxRows;       // fill[], ticket[]: zero between calls
-constexpr size_t kStaticStatusOff = kStaticFillOff + 2 * sizeof(uint32_t) * kStaticMaxRows;   // status word: zero between calls
-constexpr size_t kStaticScratchOff = 8192;                                                 // [kStaticMaxRows][kMergeCap] candidates
-constexpr size_t kStaticBytes = kStaticScratchOff + sizeof(u64) * (size_t)kMergeCap * kStaticMaxRows;
-static_assert(kStaticStatusOff + sizeof(uint32_t) <= kStaticScratchOff, "descriptors, counters and status fit below the candidates");
-
-// Zero when the library is loaded (static storage); every call starts by putting counters and status back to zero.
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
+constexpr size_t kStaticStatusOff = sizeof(RowDesc) * kStaticMaxRows;   // behind RowDesc[kStaticMaxRows]
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticStatusOff + 256];
 
 constexpr int kStaticMaxDevices = 64;
 struct StaticDevice {
     void* base = nullptr;   // device address of g_static_scratch on this device
-    int slots = 0;          // CTAs of the streaming kernel that fit on the device at once
+    int sms = 0;            // its multiprocessors
 };
 StaticDevice g_static_dev[kStaticMaxDevices];
 
 // Row descriptors of plain greedy rows (no penalty window): row r starts at r * ld, its token goes to tokens[r].
-// The kernel also clears the counters and the status word a previous call may have left set (a call that was not
-// waited for and whose kernel reported an error): stream order puts this before the streaming kernel.
-__global__ void static_greedy_rows_kernel(RowDesc* rows, int n_rows, int64_t ld, uint32_t* counters, int n_counter_words) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n_counter_words) counters[r] = 0u;
+// The kernel also clears the status word a previous call may have left set (a call that was not waited for and whose
+// kernel reported an error): stream order puts this before the streaming kernel.
+__global__ void static_greedy_rows_kernel(RowDesc* rows, int n_rows, int64_t ld, uint32_t* status) {
+    const int r = threadIdx.x;
+    if (r == 0) *status = 0u;
     if (r >= n_rows) return;
     RowDesc d{};
     d.logits_off = (int64_t)r * ld;
     d.k = 1;
+    d.k_global = 1;
     d.temperature = 0.0f;
     d.top_p = 1.0f;
     d.penalty = 1.0f;
@@ -1094,7 +739,7 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
                                       void* cuda_stream, unsigned flags) {
     using namespace fsb;
     if (!logits_dev || !tokens_dev || n_rows < 0 || n_vocab <= 0 || ld < n_vocab || (flags & ~FSB_STATIC_WAIT)) return FSB_ERR_INVALID;
-    if (n_rows > kStaticMaxRows) return FSB_ERR_CAPACITY;   // the static array holds FSB_STATIC_MAX_ROWS rows of scratch, no more
+    if (n_rows > kStaticMaxRows) return FSB_ERR_CAPACITY;   // the static array holds FSB_STATIC_MAX_ROWS descriptors, no more
     if (device < 0 || device >= kStaticMaxDevices) return FSB_ERR_NO_DEVICE;
     if (n_rows == 0) return FSB_OK;
     int prev = -1;
@@ -1102,55 +747,39 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
     if (cudaSetDevice(device) != cudaSuccess) return FSB_ERR_NO_DEVICE;
     int rc = FSB_OK;
     StaticDevice& sd = g_static_dev[device];
-    if (!sd.base) {   // first call on this device (it is current): where the array lives, how many CTAs fit
+    if (!sd.base) {   // first call on this device (it is current): where the array lives, how many SMs there are
         void* p = nullptr;
-        int per_sm = 0, sms = 0;
+        int sms = 0;
         if (cudaGetSymbolAddress(&p, g_static_scratch) != cudaSuccess || !p) rc = FSB_ERR_CUDA;
-        if (rc == FSB_OK && prepare_device_kernels(&per_sm) != 0) rc = FSB_ERR_CUDA;
+        if (rc == FSB_OK && prepare_device_kernels() != 0) rc = FSB_ERR_CUDA;
         if (rc == FSB_OK && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) rc = FSB_ERR_CUDA;
         if (rc == FSB_OK) {
-            sd.slots = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
+            sd.sms = sms > 0 ? sms : 1;
             sd.base = p;
         }
     }
     if (rc == FSB_OK) {
         unsigned char* base = static_cast<unsigned char*>(sd.base);
         cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
-        RowDesc* rows = reinterpret_cast<RowDesc*>(base + kStaticRowsOff);
-        const int n_counter_words = (int)((kStaticScratchOff - kStaticFillOff) / sizeof(uint32_t));   // fill[], ticket[], status
-        static_greedy_rows_kernel<<<(n_counter_words + 63) / 64, 64, 0, st>>>(rows, n_rows, ld, reinterpret_cast<uint32_t*>(base + kStaticFillOff), n_counter_words);
+        RowDesc* rows = reinterpret_cast<RowDesc*>(base);
+        uint32_t* status = reinterpret_cast<uint32_t*>(base + kStaticStatusOff);
+        static_greedy_rows_kernel<<<1, kStaticMaxRows, 0, st>>>(rows, n_rows, ld, status);
         if (cudaGetLastError() != cudaSuccess) rc = FSB_ERR_CUDA;
         StreamArgs a{};
         a.logits = logits_dev;
         a.rows = rows;
-        a.hist = nullptr;
-        a.scratch = reinterpret_cast<uint64_t*>(base + kStaticScratchOff);
-        a.ticket = reinterpret_cast<uint32_t*>(base + kStaticFillOff) + kStaticMaxRows;
         a.tokens = tokens_dev;
-        a.status = reinterpret_cast<uint32_t*>(base + kStaticStatusOff);
+        a.status = status;
         a.row_ld = ld;
         a.n_rows = n_rows;
         a.n_vocab = n_vocab;
-        a.tiles_per_row = (n_vocab + kTile - 1) / kTile;
-        a.total_tiles = n_rows * a.tiles_per_row;
-        int q = (a.total_tiles + sd.slots - 1) / sd.slots;   // equal contiguous ranges of tiles, one per resident CTA
-        q = q < 1 ? 1 : (q > kMaxTilesPerCta ? kMaxTilesPerCta : q);
-        a.tiles_per_cta = q;
-        a.all_greedy = 1;
-        a.bulk_ok = ((reinterpret_cast<uintptr_t>(logits_dev) & 15u) == 0 && (ld & 3) == 0) ? 1 : 0;
-        if (rc != FSB_OK) {
-        } else if (2 * ((a.tiles_per_row + q - 1) / q + 1) > kMergeCap) {   // one candidate and one count per segment
-            rc = FSB_ERR_CAPACITY;   // more segments per row than a row's scratch has entries (one candidate per segment)
-        } else if (launch_stream_kernel(a, (a.total_tiles + q - 1) / q, st) != 0) {
-            rc = FSB_ERR_CUDA;
-        } else if (flags & FSB_STATIC_WAIT) {
-            uint32_t status = 0;
-            if (cudaMemcpyAsync(&status, a.status, sizeof status, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess) {
-                rc = FSB_ERR_CUDA;
-            } else if (status != 0u) {
-                rc = FSB_ERR_DEVICE;
-            }
+        a.kmax = 1;
+        a.nseg = plan_segments(n_rows, n_vocab, sd.sms);
+        if (rc == FSB_OK && launch_stream_kernel(a, nullptr, st) != 0) rc = FSB_ERR_CUDA;
+        if (rc == FSB_OK && (flags & FSB_STATIC_WAIT)) {
+            uint32_t word = 0;
+            if (cudaMemcpyAsync(&word, status, sizeof word, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) rc = FSB_ERR_CUDA;
+            else if (word != 0u) rc = FSB_ERR_DEVICE;
         }
     }
     if (prev >= 0 && prev != device) cudaSetDevice(prev);

@@ -9,7 +9,7 @@
 namespace fsb {
 namespace {
 
-constexpr size_t kSmemMerge = (size_t)(kMergeCap + kMaxK) * sizeof(u64) + sizeof(SharedCtl);   // gathered lists, ordered candidates, control
+constexpr size_t kSmemMerge = (size_t)(kMergeCap + 8 + kMaxK) * sizeof(u64) + sizeof(SharedCtl);   // gathered lists, ordered candidates, control
 
 // Merge of per-shard candidate lists: one CTA per row gathers the row's n_lists ordered lists (already in this
 // device's memory, list g of row r at lists + (g * n_rows + r) * list_stride) and finishes the row exactly as the
@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(kThreads, 1) merge_lists_kernel(const u64* lis
                                                                  int32_t* kept_n, unsigned* status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     u64* buf = reinterpret_cast<u64*>(smem_raw);
-    u64* out = buf + kMergeCap;
+    u64* out = buf + kMergeCap + 8;
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(out + kMaxK);
     const int row = blockIdx.x, tid = threadIdx.x;
     if (row >= n_rows) return;
@@ -39,11 +39,12 @@ __global__ void __launch_bounds__(kThreads, 1) merge_lists_kernel(const u64* lis
             atomicOr(status, kStatusMergeOverflow);
         }
     }
-    consumer_sync();
-    const TailOut tout{tokens, nullptr, nullptr, kept_ids, kept_pr, kept_n, nullptr, nullptr, 0, status};
-    const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.k_global, d.flags, d.out_index};
-    const int kk = topk_sorted(buf, total, d.k_global, out, ctl);
-    row_epilogue(out, kk, rt, reinterpret_cast<double*>(buf), ctl, tout);
+    __syncthreads();
+    const TailOut tout{tokens, nullptr, nullptr, nullptr, kept_ids, kept_pr, kept_n, nullptr, nullptr, 0, status};
+    const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.flags & ~kRowAppend, d.out_index, 0};
+    rank_emit(buf, total, d.k_global, out, ctl, [&](int rank, u64 c) { out[rank] = c; });
+    __syncthreads();
+    row_epilogue(out, min(total, d.k_global), rt, reinterpret_cast<double*>(buf), ctl, tout);
 }
 
 // Write-back for callers whose logits live in host memory: after a launch with write-back on the device copy, the
@@ -58,14 +59,6 @@ __global__ void gather_patched_kernel(const float* logits, const RowDesc* rows, 
         const int c = hist[d.hist_begin + i] - vocab_offset;
         out[d.gather_off + i] = (c >= 0 && c < n_vocab) ? logits[d.logits_off + c] : 0.0f;
     }
-}
-
-// Resident histories: appends every row's new token to its stream's history on the device.  A row's window always
-// ends where its history ends, so the token goes to entry hist_begin + hist_len of the id pool.
-__global__ void append_tokens_kernel(const RowDesc* rows, int n_rows, const int32_t* tokens, int32_t* pool) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    if (rows[r].flags & kRowAppend) pool[rows[r].hist_begin + rows[r].hist_len] = tokens[rows[r].out_index];
 }
 
 // Resident verification windows.  Before the launch: draft r of a stream is the last id of row r's window, and goes
@@ -155,11 +148,6 @@ int launch_merge_lists(const void* lists, const int32_t* list_n, int n_lists, in
 int launch_gather_patched(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int n_vocab, int vocab_offset, float* out,
                           void* stream) {
     gather_patched_kernel<<<n_rows, 128, 0, static_cast<cudaStream_t>(stream)>>>(logits, rows, n_rows, hist, n_vocab, vocab_offset, out);
-    return (int)cudaGetLastError();
-}
-
-int launch_append_tokens(const RowDesc* rows, int n_rows, const int32_t* tokens, int32_t* pool, void* stream) {
-    append_tokens_kernel<<<(n_rows + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(rows, n_rows, tokens, pool);
     return (int)cudaGetLastError();
 }
 
