@@ -47,6 +47,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // Asynchronous 16-byte copies global -> shared memory; a thread waits for its own, by groups.
 __device__ __forceinline__ void cp_async16(unsigned dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async4(unsigned dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -79,16 +80,30 @@ __device__ __forceinline__ u64 global_timer_ns() {
 }
 
 // ---------------------------------------------------------------------------------------------- shared control block
-constexpr int kNumWarps = kThreads / 32;
+// A barrier of the CTA's first T threads.  BAR 0: the whole CTA; BAR 1: those that are still at work when the others have
+// left (the steps after the stream are short chains: more than eight warps would only issue the same instructions more
+// often).
+template <int T, int BAR>
+__device__ __forceinline__ void block_sync() { asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(T) : "memory"); }
+// The same, with the number of threads whose `pred` holds.
+template <int T, int BAR>
+__device__ __forceinline__ int block_sync_count(bool pred) {
+    int n;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.popc.u32 %0, %2, %3, p;\n\t}" : "=r"(n) : "r"((int)pred), "n"(BAR), "n"(T) : "memory");
+    return n;
+}
+
+constexpr int kPost = 256;   // threads that finish a row
 
 struct SharedCtl {
-    alignas(16) unsigned keys[kNumWarps][64];              // each warp's maxima while their ranks are counted; digit counts of the exact selection
-    alignas(16) unsigned top[kNumWarps];      // per-warp bounds (keys)
-    u64 red[2 * kNumWarps];                   // cross-warp reduction scratch
-    double part[kNumWarps];                   // partial sums of the epilogue
+    alignas(16) unsigned top[2][32];          // per-warp bounds (keys), double buffered
+    float edge[8];                            // the row's logits outside its whole 16-byte cells (NaN: none)
+    u64 red[2 * kPost / 32];                  // cross-warp reduction scratch
+    double part[kMaxK / 32];                  // partial sums of the epilogue
     int sum[3];                               // rotating counters of the selection steps
-    int list_n;                               // cells the streaming kernel has listed (those past the list's capacity counted too)
-    int kept_n;                               // candidates picked from them
+    int lost;                                 // a warp's list of cells was too short
+    int kept_n;                               // candidates picked from the lists
+    int pen_n;                                // penalised columns of the segment
     int out_cnt;
     int recv_n[8];                            // clusters: candidates that segment r of the row has sent
     u64 sel_prefix;
@@ -97,8 +112,9 @@ struct SharedCtl {
 
 // ---------------------------------------------------------------------------------------------- top-k selection
 // Smallest and largest of the composites the threads hold (each thread passes the extremes of its own; threads
-// with nothing pass ~0 and 0).  All kThreads threads of the CTA must call.
+// with nothing pass ~0 and 0).  All of the first kPost threads must call.
 __device__ __forceinline__ void cta_minmax(u64& mn, u64& mx, SharedCtl* ctl) {
+    constexpr int T = kPost;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -107,20 +123,20 @@ __device__ __forceinline__ void cta_minmax(u64& mn, u64& mx, SharedCtl* ctl) {
     }
     if (lane == 0) {
         ctl->red[warp] = mn;
-        ctl->red[kNumWarps + warp] = mx;
+        ctl->red[T / 32 + warp] = mx;
     }
-    __syncthreads();
+    block_sync<kPost, 1>();
     mn = ctl->red[0];
-    mx = ctl->red[kNumWarps];
+    mx = ctl->red[T / 32];
 #pragma unroll
-    for (int w = 1; w < kNumWarps; ++w) {
+    for (int w = 1; w < T / 32; ++w) {
         mn = min(mn, ctl->red[w]);
-        mx = max(mx, ctl->red[kNumWarps + w]);
+        mx = max(mx, ctl->red[T / 32 + w]);
     }
-    __syncthreads();   // the scratch may be written again
+    block_sync<kPost, 1>();   // the scratch may be written again
 }
 
-// Bound L of the k largest among n > k distinct composites held by the threads of the CTA: exactly k composites
+// Bound L of the k largest among n > k distinct composites held by the first kPost threads: exactly k composites
 // are >= L.  count_ge(t) = how many of this thread's composites are >= t.  MSB-first bisection from the highest bit
 // in which the composites differ: every step is one warp reduction, one shared-memory add per warp and one
 // barrier, and the search stops as soon as a trial bound is passed by exactly k composites.
@@ -131,7 +147,7 @@ __device__ __forceinline__ u64 bisect_bound(int k, u64 mn, u64 mx, SharedCtl* ct
     const int hb = 63 - __clzll((long long)(mx ^ mn));
     u64 pfx = (hb == 63) ? 0ull : (mx & (~0ull << (hb + 1)));
     if (tid == 0) ctl->sum[0] = 0;
-    __syncthreads();
+    block_sync<kPost, 1>();
     int step = 0;
 #pragma unroll 1
     for (int b = hb; b >= 0; --b, ++step) {
@@ -139,7 +155,7 @@ __device__ __forceinline__ u64 bisect_bound(int k, u64 mn, u64 mx, SharedCtl* ct
         const int wsum = __reduce_add_sync(0xffffffffu, count_ge(trial));
         if ((tid & 31) == 0 && wsum) atomicAdd(&ctl->sum[step % 3], wsum);
         if (tid == 0) ctl->sum[(step + 1) % 3] = 0;   // last read two barriers ago
-        __syncthreads();
+        block_sync<kPost, 1>();
         const int total = ctl->sum[step % 3];
         if (total >= k) pfx = trial;
         if (total == k) break;
@@ -148,13 +164,14 @@ __device__ __forceinline__ u64 bisect_bound(int k, u64 mn, u64 mx, SharedCtl* ct
 }
 
 // Keeps the k largest of list[0..n) (distinct composites in shared memory) in list[0..k), unordered, and returns
-// min(n, k).  `tmp` is scratch for k composites outside the list.  All threads of the CTA must call.
+// min(n, k).  `tmp` is scratch for k composites outside the list.  The first kPost threads call.
 static __device__ __noinline__ int select_list_topk(u64* list, int n, int k, u64* tmp, SharedCtl* ctl) {
+    constexpr int T = kPost;
     if (n <= k) return n;
     const int tid = threadIdx.x;
     u64 mn = ~0ull, mx = 0ull;
 #pragma unroll 1
-    for (int i = tid; i < n; i += kThreads) {
+    for (int i = tid; i < n; i += T) {
         const u64 c = list[i];
         mn = min(mn, c);
         mx = max(mx, c);
@@ -163,53 +180,92 @@ static __device__ __noinline__ int select_list_topk(u64* list, int n, int k, u64
     const u64 L = bisect_bound(k, mn, mx, ctl, [&](u64 t) {
         int c = 0;
 #pragma unroll 1
-        for (int i = tid; i < n; i += kThreads) c += list[i] >= t ? 1 : 0;
+        for (int i = tid; i < n; i += T) c += list[i] >= t ? 1 : 0;
         return c;
     });
     if (tid == 0) ctl->out_cnt = 0;
-    __syncthreads();
+    block_sync<kPost, 1>();
 #pragma unroll 1
-    for (int i = tid; i < n; i += kThreads) {
+    for (int i = tid; i < n; i += T) {
         const u64 c = list[i];
         if (c >= L) {
             const int p = atomicAdd(&ctl->out_cnt, 1);
             if (p < k) tmp[p] = c;
         }
     }
-    __syncthreads();
+    block_sync<kPost, 1>();
 #pragma unroll 1
-    for (int i = tid; i < k; i += kThreads) list[i] = tmp[i];
-    __syncthreads();
+    for (int i = tid; i < k; i += T) list[i] = tmp[i];
+    block_sync<kPost, 1>();
     return k;
 }
 
 // Ranks the composites buf[0..n) (distinct but for zeros, which rank last; shared memory, 16-byte aligned, room for
-// seven more entries) by counting, and calls emit(rank, composite) once for each that ranks below k.  Four lanes count
-// for an entry, each a quarter of the list, two entries per 16-byte broadcast read and no dependency between the reads
-// (the quarters are interleaved: no bank conflicts); no atomics, one barrier.  64 entries take one round; the work grows
-// with n^2, so lists of more than kRankCap entries are first cut down to k by bisection (`tmp`: scratch for k composites).
-// All kThreads threads must call, after a barrier that made buf visible.
-constexpr int kRankCap = 512;
+// 31 more entries) and calls emit(rank, composite) once for each that ranks below k.
+//  n <= 128: by counting.  Four lanes count for an entry, each a quarter of the list, two entries per 16-byte broadcast
+//    read and no dependency between the reads (the quarters are interleaved: no bank conflicts); no atomics, one barrier.
+//    64 entries take one round; the work grows with n^2.
+//  n <= kRankCap: in runs of 32 that the warps sort across their lanes; an entry's rank is its place in its run plus the
+//    larger entries of the other runs, by binary searches that do not depend on one another.
+//  longer lists are first cut down to k by bisection (`tmp`: scratch for k composites).
+// The first kPost threads call, after a barrier that made buf visible.
+constexpr int kRankCap = 1024;
 template <class Emit>
 __device__ __forceinline__ void rank_emit(u64* buf, int n, int k, u64* tmp, SharedCtl* ctl, Emit emit) {
+    constexpr int T = kPost;
     const int tid = threadIdx.x;
     if (n > kRankCap) n = select_list_topk(buf, n, k, tmp, ctl);
-    const int n8 = (n + 7) & ~7;
-    if (tid < n8 - n) buf[n + tid] = 0ull;   // padding: 0 is below every composite
-    __syncthreads();
-    const int part = tid & 3;
-    for (int e0 = 0; e0 < n; e0 += kThreads / 4) {
-        const int e = e0 + (tid >> 2);
-        const u64 c = e < n ? buf[e] : 0ull;
-        int larger = 0;
+    if (n <= 128) {
+        const int n8 = (n + 7) & ~7;
+        if (tid < n8 - n) buf[n + tid] = 0ull;   // padding: 0 is below every composite
+        block_sync<kPost, 1>();
+        const int part = tid & 3;
+        for (int e0 = 0; e0 < n; e0 += T / 4) {
+            const int e = e0 + (tid >> 2);
+            if (e0 + ((tid & ~31) >> 2) >= n) break;   // (whole warps)
+            const u64 c = e < n ? buf[e] : 0ull;
+            int larger = 0;
 #pragma unroll 4
-        for (int j = 2 * part; j < n8; j += 8) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(buf + j);
-            larger += (v.x > c ? 1 : 0) + (v.y > c ? 1 : 0);
+            for (int j = 2 * part; j < n8; j += 8) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(buf + j);
+                larger += (v.x > c ? 1 : 0) + (v.y > c ? 1 : 0);
+            }
+            larger += __shfl_xor_sync(0xffffffffu, larger, 1);
+            larger += __shfl_xor_sync(0xffffffffu, larger, 2);
+            if (part == 0 && c != 0ull && larger < k) emit(larger, c);
         }
-        larger += __shfl_xor_sync(0xffffffffu, larger, 1);
-        larger += __shfl_xor_sync(0xffffffffu, larger, 2);
-        if (part == 0 && c != 0ull && larger < k) emit(larger, c);
+        return;
+    }
+    const int lane = tid & 31, runs = (n + 31) >> 5;
+    for (int q = tid >> 5; q < runs; q += T / 32) {
+        u64 c = 32 * q + lane < n ? buf[32 * q + lane] : 0ull;
+#pragma unroll
+        for (int kk = 2; kk <= 32; kk <<= 1) {   // bitonic, descending
+#pragma unroll
+            for (int j = kk >> 1; j > 0; j >>= 1) {
+                const u64 o = __shfl_xor_sync(0xffffffffu, c, j);
+                const bool down = (lane & kk) == 0, low = (lane & j) == 0;
+                c = (down == low) ? max(c, o) : min(c, o);
+            }
+        }
+        buf[32 * q + lane] = c;
+    }
+    block_sync<kPost, 1>();
+    for (int e = tid; e < 32 * runs; e += T) {
+        const u64 c = buf[e];
+        if (lane >= k) continue;
+        int r = lane;
+#pragma unroll 4
+        for (int q = 0; q < runs; ++q) {
+            const u64* run = buf + 32 * q;
+            int lo = 0;   // entries of the run above c (0 .. 32)
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1)
+                if (run[lo + s - 1] > c) lo += s;
+            if (run[lo] > c) lo += 1;
+            r += q == e >> 5 ? 0 : lo;
+        }
+        if (c != 0ull && r < k) emit(r, c);
     }
 }
 
@@ -250,13 +306,13 @@ __device__ __forceinline__ void put_token(int32_t* tokens, int32_t* tokens_host,
 
 // srt[0..kk) holds the row's candidates in order (largest first).  Either hands them out (vocabulary-sharded mode)
 // or finishes the row: softmax over the candidates in fp64, sequential sums in candidate order, min-p, top-p,
-// draw.  `work` is scratch for 2 * kMaxK doubles that does not overlap srt.  All threads must call it with the same
+// draw.  `work` is scratch for 2 * kMaxK doubles that does not overlap srt.  The first kPost threads call it with the same
 // arguments; it is the last thing they do (no barrier at the end).
 // Exponentials, their sum (pairwise, like a tree) and the probabilities are one thread's work each.  The cumulative
 // probabilities follow the reference's order of additions exactly, since a cut may fall on a tie: one warp runs the chain
 // of dependent adds (15 cycles each), all lanes alike over broadcast reads, and stops soon after top-p is reached; the
 // cuts and the draw are warp votes.
-static __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
+__device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
     const int tid = threadIdx.x, lane = tid & 31;
     double* e = work;
     double* P = work + kMaxK;
@@ -283,14 +339,14 @@ static __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, cons
             for (int d = 16; d; d >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, d));
             if (lane == 0) ctl->part[tid >> 5] = s;
         }
-        __syncthreads();
+        block_sync<kPost, 1>();
         s = ctl->part[0];
         for (int w = 1; 32 * w < kk; ++w) s = __dadd_rn(s, ctl->part[w]);
         // probabilities; min-p keeps those not below pr[0] * min_p (they do not increase, pr[0] is 1 / sum)
         const double p = __ddiv_rn(x, s);
         if (tid < kk) e[tid] = p;
         const bool cut = r.min_p > 0.0f && p < __dmul_rn(__ddiv_rn(1.0, s), (double)r.min_p);
-        keep = __syncthreads_count(tid < kk && !cut);
+        keep = block_sync_count<kPost, 1>(tid < kk && !cut);
         if (tid >= 32) return;
         // cumulative sums P[i] = pr[0] + ... + pr[i]; top-p keeps the shortest prefix whose sum reaches top_p, the crossing
         // candidate included

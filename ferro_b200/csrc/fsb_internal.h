@@ -6,7 +6,6 @@
 namespace fsb {
 
 // ---- compile-time geometry -----------------------------------------------------------------------------------
-constexpr int kThreads = 256;                 // threads per CTA (8 warps) of the streaming kernel and of the list merge
 constexpr int kMaxK = 256;                    // largest k of the candidate path (== FSB_MAX_CANDIDATE_K)
 constexpr int kMergeCap = 2400;               // candidates of one row that the list merge can gather
 
@@ -70,6 +69,7 @@ struct StreamArgs {
     int32_t n_rows;
     int32_t n_vocab;
     int32_t nseg;              // CTAs per row (1..8), a thread-block cluster when more than one
+    int32_t wide;              // large CTAs (see SelectPlan)
     int32_t kmax;              // largest k of the rows
     int32_t penalised;         // some row has a penalty window
     int32_t write_back;        // store penalised values into the caller's rows
@@ -78,8 +78,13 @@ struct StreamArgs {
     int32_t overlap;           // see fsb_set_launch_overlap
 };
 
-// CTAs per row for a launch of n_rows rows on a device of `sms` multiprocessors.
-int plan_segments(int n_rows, int n_vocab, int sms);
+// How a launch of n_rows rows is laid out on a device of `sms` multiprocessors: CTAs per row, and whether they are large
+// ones (1024 threads, one per SM) or small ones (256 threads, several per SM).
+struct SelectPlan {
+    int nseg = 1;
+    bool wide = false;
+};
+SelectPlan plan_select(int n_rows, int n_vocab, int sms);
 
 // All return a cudaError_t as int (0 = success).
 int prepare_device_kernels();

@@ -51,7 +51,7 @@ struct fsb_batch {
     int64_t cap_hist = 0;
     int n_cand = 0, n_full = 0;   // rows of the candidate kernel / of the full-row kernel
     int kmax = 1;
-    int nseg = 1;                 // CTAs per row of the streaming kernel
+    fsb::SelectPlan plan;         // how the streaming kernel is laid out
     bool penalised = false;       // some row of the streaming kernel has a penalty window
     int64_t hist_ids = 0;         // window ids staged with the batch
     int64_t gather_ids = 0;       // window values a write-back for a host caller brings back
@@ -255,7 +255,7 @@ int finalize_batch(fsb_handle* h, fsb_batch* b) {
     b->n_cand = n_cand;
     b->n_full = n_full;
     b->kmax = kmax;
-    b->nseg = fsb::plan_segments(std::max(n_cand, 1), b->n_vocab, std::max(1, h->sm_count));
+    b->plan = fsb::plan_select(std::max(n_cand, 1), b->n_vocab, std::max(1, h->sm_count));
     return FSB_OK;
 }
 
@@ -325,7 +325,8 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.row_ld = (b->n_full == 0) ? b->ld : -1;   // descriptors are in row order when every row takes this kernel
         a.n_rows = b->n_cand;
         a.n_vocab = b->n_vocab;
-        a.nseg = b->nseg;
+        a.nseg = b->plan.nseg;
+        a.wide = b->plan.wide ? 1 : 0;
         a.kmax = b->kmax;
         a.penalised = b->penalised ? 1 : 0;
         a.write_back = (b->flags & FSB_WRITE_BACK) ? 1 : 0;

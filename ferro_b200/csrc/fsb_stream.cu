@@ -24,7 +24,8 @@ namespace {
 // The look works on raw logits and leaves the penalised ones out.  A thread keeps two running maxima (of different cells);
 // from all threads' maxima the CTA derives a bound that at least k logits of the segment reach (cta_bound), at chunks 0, 1,
 // 3, 7, 15, ...  A cell whose maximum reaches the bound is listed in shared memory, data and all: about 100 in each of these
-// intervals for k = 64.  Should the list overflow, the segment is gone through once more with the final bound.
+// intervals for k = 64.  Every warp has a list of its own and keeps its length in a register: votes, but no atomics and
+// nothing to wait for.  Should a list overflow, the segment is gone through once more with the final bound.
 // At the end the listed cells are taken apart: the logits that reach the final bound are the segment's candidates, and
 // with them the penalised logits of the window that do so once penalised, each id once.  The softcap is applied here too,
 // to candidates only: it is monotone up to the rounding of tanhf, and a margin under the bound covers that.
@@ -37,27 +38,32 @@ namespace {
 // (from L2) per digit.  It runs when hundreds of equal logits reach the final bound.
 // Nobody waits for another CTA but at the cluster's two barriers.
 
-constexpr int kWarps = kNumWarps;
 constexpr int kCells = 4;                               // cells of a thread per chunk
-constexpr int kChunkCells = kCells * kThreads;
 constexpr int kStages = 2;
-constexpr int kCellCap = 512;                           // cells a CTA can list
-constexpr int kPickCap = kRankCap;                      // candidates of a segment
+constexpr int kPenCap = 1024;                           // penalised columns of a segment that are looked up ahead
+constexpr int kPickCap = 1024;                          // candidates of a segment
 constexpr int kSendCap = 256;                           // candidates a segment sends to the row's first CTA
 constexpr int kMergeList = 8 * kSendCap;                // candidates of all segments
-constexpr size_t kRingBytes = (size_t)kStages * kChunkCells * sizeof(float4);
-static_assert((kPickCap + 8 + kMaxK + kMergeList + 8) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
+constexpr int kSelectSmemMax = 224 * 1024;
 static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merge list's memory");
 
-constexpr int kSelectSmemMax = 200 * 1024;
-__host__ __device__ constexpr size_t recv_entries(int nseg) { return nseg > 1 ? (size_t)nseg * kSendCap : 0; }
-
-// dynamic shared memory: ring, listed cells (data, numbers), control block, receive buffer, bitmap of the penalised columns
-// of the segment (its first word: the up to three columns before the cells)
-size_t select_smem_bytes(int nseg, int seg_cols) {
-    return kRingBytes + kCellCap * (sizeof(float4) + sizeof(int)) + sizeof(SharedCtl) + recv_entries(nseg) * sizeof(u64) +
-           (seg_cols > 0 ? (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0);
-}
+// Sizes that go with T, the threads of a CTA.
+template <int T>
+struct Geometry {
+    static constexpr int kWarps = T / 32;
+    static constexpr int kChunkCells = kCells * T;
+    static constexpr size_t kRingBytes = (size_t)kStages * kChunkCells * sizeof(float4);
+    // cells a warp can list; with k > 64
+    static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64;
+    static_assert((kPickCap + 32 + kMaxK + kMergeList + 32) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
+    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns), control block, maxima
+    // (k > 64), receive buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
+    static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
+        return kRingBytes + (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int)) +
+               (seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0) + sizeof(SharedCtl) + (kmax > 64 ? (size_t)kWarps * 64 * sizeof(unsigned) : 0) +
+               (nseg > 1 ? (size_t)nseg * kSendCap * sizeof(u64) : 0);
+    }
+};
 
 struct Segment {
     const float* row;          // the row's logits
@@ -84,46 +90,42 @@ __device__ __forceinline__ float transform(float x, int c, const Segment& s) {
 
 // A bound that at least k logits of the segment reach, from the threads' maxima (each a logit of its own; two per
 // thread, of different cells).  Minus infinity - and what is no number - never reaches a bound.  All threads get the same
-// value; contains two barriers.  `listed`: the number of cells listed so far, the same in every thread.
+// value; contains one barrier; buffers alternate, so that the next call may write while a slow warp still reads.
 //  k <= 64: the r-th largest thread maximum of every warp, r = ceil(k / warps), minimum over the warps: 1.3 k to 2 k logits
 //    reach it.  r warp reductions take the largest out one after the other (equal ones together: the bound is lower then).
 //    (The k-th largest of all threads' maxima, found by counting, lets fewer through but cost more than it saved.)
 //  otherwise: the same over the 64 maxima of every warp, ranked by counting; keys give up their low bits to be distinct,
 //    which lowers the bound by less than 2^-16 of its value.
-__device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, SharedCtl* ctl, int& listed) {
+template <int T, int BAR>
+__device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, int buf, SharedCtl* ctl, unsigned* maxima) {
+    constexpr int kWarps = T / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned m = ~0u;
     if (k <= 64) {
         unsigned key = float_key(fmaxf(run_a, run_b)), top = __reduce_max_sync(0xffffffffu, key);
         for (int r = (k - 1) / kWarps; r > 0; --r) {
             if (key == top) key = 0u;
             top = __reduce_max_sync(0xffffffffu, key);
         }
-        if (lane == 0) ctl->top[warp] = top;
+        if (lane == 0) ctl->top[buf][warp] = top;
     } else {
         const int r = (k + kWarps - 1) / kWarps;
         const unsigned ka = (float_key(run_a) & ~127u) | (unsigned)lane, kb = (float_key(run_b) & ~127u) | (unsigned)(lane + 32);
-        ctl->keys[warp][lane] = ka;
-        ctl->keys[warp][lane + 32] = kb;
+        unsigned* mine = maxima + 64 * warp;
+        mine[lane] = ka;
+        mine[lane + 32] = kb;
         __syncwarp();
         int rank_a = 0, rank_b = 0;
 #pragma unroll 4
         for (int i = 0; i < 16; ++i) {
-            const uint4 v = *reinterpret_cast<const uint4*>(&ctl->keys[warp][4 * i]);
+            const uint4 v = *reinterpret_cast<const uint4*>(mine + 4 * i);
             rank_a += (v.x > ka ? 1 : 0) + (v.y > ka ? 1 : 0) + (v.z > ka ? 1 : 0) + (v.w > ka ? 1 : 0);
             rank_b += (v.x > kb ? 1 : 0) + (v.y > kb ? 1 : 0) + (v.z > kb ? 1 : 0) + (v.w > kb ? 1 : 0);
         }
-        if (rank_a == r - 1) ctl->top[warp] = ka & ~127u;
-        if (rank_b == r - 1) ctl->top[warp] = kb & ~127u;
+        if (rank_a == r - 1) ctl->top[buf][warp] = ka & ~127u;
+        if (rank_b == r - 1) ctl->top[buf][warp] = kb & ~127u;
     }
-    __syncthreads();
-    listed = ctl->list_n;
-#pragma unroll
-    for (int w = 0; w < kWarps; w += 4) {
-        const uint4 v = *reinterpret_cast<const uint4*>(&ctl->top[w]);
-        m = min(m, min(min(v.x, v.y), min(v.z, v.w)));
-    }
-    __syncthreads();   // nobody lists another cell before everybody has read the length
+    block_sync<T, BAR>();
+    const unsigned m = __reduce_min_sync(0xffffffffu, ctl->top[buf][lane & (kWarps - 1)]);
     return fmaxf(key_float(m), -FLT_MAX);   // (also for the patterns just below minus infinity's key, which are no numbers)
 }
 
@@ -145,64 +147,46 @@ __device__ __forceinline__ void softcap_bounds(float thr, float cap, float& admi
     admit = fmaxf(admit, -FLT_MAX);
 }
 
-// Keeps the listed cells that reach `admit`.  All threads call, after a barrier.
-__device__ __noinline__ void prune_cells(float4* cells, int* nums, SharedCtl* ctl, float admit) {
-    constexpr int kPer = kCellCap / kThreads;
-    const int n = min(ctl->list_n, kCellCap);
-    float4 x[kPer];
-    int num[kPer];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        const int p = threadIdx.x + i * kThreads;
-        num[i] = -1;
-        if (p < n) {
-            x[i] = cells[p];
-            num[i] = nums[p];
+// Keeps those of a warp's n <= 128 listed cells that reach `admit`, in order; returns their number.
+__device__ __noinline__ int prune_cells(float4* cells, int* nums, int n, float admit) {
+    const int lane = threadIdx.x & 31;
+    int w = 0;
+    for (int p0 = 0; p0 < n; p0 += 32) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        int num = 0;
+        bool keep = false;
+        if (p0 + lane < n) {
+            x = cells[p0 + lane];
+            num = nums[p0 + lane];
+            keep = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)) >= admit;
         }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) ctl->list_n = 0;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kPer; ++i)
-        if (num[i] >= 0 && fmaxf(fmaxf(x[i].x, x[i].y), fmaxf(x[i].z, x[i].w)) >= admit) {
-            const int p = atomicAdd(&ctl->list_n, 1);
-            cells[p] = x[i];
-            nums[p] = num[i];
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {   // (never ahead of what is still to be read)
+            const int q = w + __popc(m & ((1u << lane) - 1u));
+            cells[q] = x;
+            nums[q] = num;
         }
-    __syncthreads();
-}
-
-// The penalty window's bits: set them all (again: picking the penalised candidates clears them).  All threads call.
-__device__ __forceinline__ void set_bits(const Segment& s, int first_id) {
-    for (int i = threadIdx.x; i < s.hist_len; i += kThreads) {
-        const int c = (i == threadIdx.x ? first_id : s.hist[i]) - s.id_base;
-        if (c >= s.lo && c < s.hi) atomicOr(&s.bitmap[(c - s.bit0) >> 5], 1u << ((c - s.bit0) & 31));
+        w += __popc(m);
+        __syncwarp();
     }
-}
-// Whether this thread is the first to come for column c: an id counts once however often it occurs in the window.
-__device__ __forceinline__ bool claim(const Segment& s, int c) {
-    const unsigned bit = 1u << ((c - s.bit0) & 31);
-    return (atomicAnd(&s.bitmap[(c - s.bit0) >> 5], ~bit) & bit) != 0u;
+    return w;
 }
 
 // Exact selection of the min(k, candidates) largest composites of the transformed segment into list (unordered);
-// returns their number.  MSB-first over 8-bit digits of the composites: count the digits of the composites that match
+// returns their number.  `bins`: 256 words.  MSB-first over 8-bit digits of the composites: count the digits of the composites that match
 // the prefix, walk the counts from the top, go on in the digit in which the k-th lies; stops early when a digit is
 // taken whole.  Every digit reads the segment again.  All threads call, after a barrier.
-__device__ __noinline__ int exact_select(const Segment& s, int k, u64* list, SharedCtl* ctl) {
+template <int T>
+__device__ __noinline__ int exact_select(const Segment s, int k, u64* list, unsigned* bins, SharedCtl* ctl) {
     const int tid = threadIdx.x, lane = tid & 31;
-    unsigned* bins = &ctl->keys[0][0];
-    static_assert(kNumWarps * 64 >= 256, "one counter per digit");
-    if (s.has_pen) set_bits(s, tid < s.hist_len ? s.hist[tid] : 0);
     u64 prefix = 0ull, mask = 0ull;
     int need = k;
-    const int rounds = (s.hi - s.lo + kThreads - 1) / kThreads;
+    const int rounds = (s.hi - s.lo + T - 1) / T;
     for (int shift = 56; shift >= 0; shift -= 8) {
         if (tid < 256) bins[tid] = 0u;
         __syncthreads();
         for (int i = 0; i < rounds; ++i) {
-            const int c = s.lo + i * kThreads + tid;
+            const int c = s.lo + i * T + tid;
             unsigned digit = 256u;
             if (c < s.hi) {
                 const float x = transform(__ldcg(s.row + c), c, s);
@@ -255,7 +239,7 @@ __device__ __noinline__ int exact_select(const Segment& s, int k, u64* list, Sha
     if (tid == 0) ctl->kept_n = 0;
     __syncthreads();
     for (int i = 0; i < rounds; ++i) {
-        const int c = s.lo + i * kThreads + tid;
+        const int c = s.lo + i * T + tid;
         if (c >= s.hi) continue;
         const float x = transform(__ldcg(s.row + c), c, s);
         const u64 m = make_comp(x, c + s.id_base);
@@ -267,21 +251,20 @@ __device__ __noinline__ int exact_select(const Segment& s, int k, u64* list, Sha
 
 // A segment with fewer than k logits above minus infinity (masked vocabularies): its first columns that hold minus
 // infinity are candidates too.  Appends up to k - n of them to the list; returns the new length.  All threads call.
-__device__ __noinline__ int append_masked(const Segment& s, int n, int k, u64* list, SharedCtl* ctl) {
+template <int T>
+__device__ __noinline__ int append_masked(const Segment s, int n, int k, u64* list, unsigned* counts) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __syncthreads();
-    if (s.has_pen) set_bits(s, tid < s.hist_len ? s.hist[tid] : 0);
-    __syncthreads();
-    for (int c0 = s.lo; c0 < s.hi && n < k; c0 += kThreads) {
+    for (int c0 = s.lo; c0 < s.hi && n < k; c0 += T) {
         const int c = c0 + tid;
         const bool hit = c < s.hi && transform(__ldcg(s.row + c), c, s) == -__int_as_float(0x7f800000);
         const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) ctl->keys[0][warp] = (unsigned)__popc(m);
+        if (lane == 0) counts[warp] = (unsigned)__popc(m);
         __syncthreads();
         int before = n, total = 0;
-        for (int w = 0; w < kWarps; ++w) {
-            if (w < warp) before += (int)ctl->keys[0][w];
-            total += (int)ctl->keys[0][w];
+        for (int w = 0; w < T / 32; ++w) {
+            if (w < warp) before += (int)counts[w];
+            total += (int)counts[w];
         }
         before += __popc(m & ((1u << lane) - 1u));
         if (hit && before < k) list[before] = make_comp(-__int_as_float(0x7f800000), c + s.id_base);
@@ -292,18 +275,19 @@ __device__ __noinline__ int append_masked(const Segment& s, int n, int k, u64* l
 }
 
 // Write-back: the transformed logits go to the caller's row.  Nothing reads the raw row after this.
-__device__ __noinline__ void write_back(const Segment& s) {
+template <int T>
+__device__ __noinline__ void write_back(const Segment s) {
     float* row = const_cast<float*>(s.row);
     __syncthreads();
-    if (s.has_pen) set_bits(s, threadIdx.x < s.hist_len ? s.hist[threadIdx.x] : 0);
-    __syncthreads();
     if (s.cap != 0.0f) {
-        for (int c = s.lo + threadIdx.x; c < s.hi; c += kThreads) row[c] = transform(__ldcg(row + c), c, s);
+        for (int c = s.lo + threadIdx.x; c < s.hi; c += T) row[c] = transform(__ldcg(row + c), c, s);
         return;
     }
-    for (int i = threadIdx.x; i < s.hist_len; i += kThreads) {
+    for (int i = threadIdx.x; i < s.hist_len; i += T) {
         const int c = s.hist[i] - s.id_base;
-        if (c >= s.lo && c < s.hi && claim(s, c)) row[c] = penalise(__ldcg(row + c), s.pen);
+        if (c < s.lo || c >= s.hi) continue;
+        const unsigned bit = 1u << ((c - s.bit0) & 31);   // an id counts once however often it occurs in the window
+        if (atomicAnd(&s.bitmap[(c - s.bit0) >> 5], ~bit) & bit) row[c] = penalise(__ldcg(row + c), s.pen);
     }
 }
 
@@ -344,19 +328,27 @@ struct SelectArgs {
     RowDesc rows[NDESC > 0 ? NDESC : 1];
 };
 
-template <int NDESC>
-__global__ void __launch_bounds__(kThreads, 4) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
+template <int T, int NDESC>
+__global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
+    using G = Geometry<T>;
+    constexpr int kChunkCells = G::kChunkCells, kWarps = G::kWarps;
     const StreamArgs& a = args.a;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float4* ring = reinterpret_cast<float4*>(smem_raw);
     u64* picked = reinterpret_cast<u64*>(smem_raw);   // after the stream: candidates, the row's candidates in order, merge list
-    u64* out = picked + kPickCap + 8;
+    u64* out = picked + kPickCap + 32;
     u64* list = out + kMaxK;
-    float4* listed = reinterpret_cast<float4*>(smem_raw + kRingBytes);
-    int* listed_num = reinterpret_cast<int*>(listed + kCellCap);
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(listed_num + kCellCap);
-    u64* recv = reinterpret_cast<u64*>(ctl + 1);
-    const int tid = threadIdx.x;
+    float4* listed = reinterpret_cast<float4*>(smem_raw + G::kRingBytes);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int cell_cap = a.kmax > 64 ? G::kWarpCellsLong : G::kWarpCells;
+    int* listed_num = reinterpret_cast<int*>(listed + kWarps * cell_cap);
+    float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
+    int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised ? kPenCap : 0));
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised ? kPenCap : 0));
+    listed += (tid >> 5) * cell_cap;   // the warp's own
+    listed_num += (tid >> 5) * cell_cap;
+    unsigned* maxima = reinterpret_cast<unsigned*>(ctl + 1);
+    u64* recv = reinterpret_cast<u64*>(maxima + (a.kmax > 64 ? kWarps * 64 : 0));
     pdl_launch_dependents();
     trace_mark(a, 0);
     // Mode 1 waits only before its first write (unless it stores into the logits); otherwise only the launch's latency -
@@ -379,25 +371,24 @@ __global__ void __launch_bounds__(kThreads, 4) stream_select_kernel(const __grid
     const float4* cells = reinterpret_cast<const float4*>(row_ptr + head);
     const float qnan = __int_as_float(0x7fc00000), ninf = -__int_as_float(0x7f800000);
     const unsigned slot0 = smem_u32(ring + tid);
-    // chunk c of this thread: cells j, j + kThreads, ... go to stage c % kStages
+    // chunk c of this thread: cells j, j + T, ... go to stage c % kStages
     auto fetch = [&](int c) {
         const int j = c_lo + c * kChunkCells + tid;
         const unsigned dst = slot0 + (unsigned)((c % kStages) * kChunkCells) * (unsigned)sizeof(float4);
 #pragma unroll
         for (int u = 0; u < kCells; ++u)
-            if (j + u * kThreads < c_hi) cp_async16(dst + (unsigned)(u * kThreads * sizeof(float4)), cells + j + u * kThreads);
+            if (j + u * T < c_hi) cp_async16(dst + (unsigned)(u * T * sizeof(float4)), cells + j + u * T);
         cp_async_commit();
     };
     for (int c = 0; c < kStages; ++c) fetch(c);
-    float edge = qnan;   // one of the logits outside the whole cells
-    int edge_col = -1;
-    if (seg == 0 && tid < head) edge_col = tid;
-    if (seg == nseg - 1 && tid >= 4 && tid < 4 + V - head - 4 * n_cells) edge_col = head + 4 * n_cells + tid - 4;
-    if (edge_col >= 0) edge = __ldcg(row_ptr + edge_col);
+    if (tid < 8) {   // the logits outside the whole cells
+        const int c = tid < 4 ? (seg == 0 && tid < head ? tid : -1) : (seg == nseg - 1 && tid < 4 + V - head - 4 * n_cells ? head + 4 * n_cells + tid - 4 : -1);
+        ctl->edge[tid] = c >= 0 ? __ldcg(row_ptr + c) : qnan;
+    }
 
     Segment s;
     s.row = row_ptr;
-    s.bitmap = reinterpret_cast<unsigned*>(recv + recv_entries(nseg));
+    s.bitmap = reinterpret_cast<unsigned*>(recv + (nseg > 1 ? nseg * kSendCap : 0));
     s.lo = seg == 0 ? 0 : head + 4 * c_lo;
     s.hi = seg == nseg - 1 ? V : head + 4 * c_hi;
     s.bit0 = head + 4 * c_lo - 32;
@@ -408,36 +399,53 @@ __global__ void __launch_bounds__(kThreads, 4) stream_select_kernel(const __grid
     s.hist = nullptr;
     s.hist_len = 0;
     const int k = dp.k;
-    int pen_col = -1;        // the first window id of this thread, if it is a column of the segment, and its logit
-    float pen_raw = qnan;
     if (tid == 0) {
-        ctl->list_n = 0;
+        ctl->lost = 0;
         ctl->kept_n = 0;
+        ctl->pen_n = 0;
     }
     if (nseg > 1) cluster_arrive_release();   // (waited for before the first store to another CTA's shared memory)
     if (s.has_pen) {
         s.hist = a.hist + dp.hist_begin;
         s.hist_len = dp.hist_len;
-        const int first_id = tid < s.hist_len ? s.hist[tid] : -1;
-        for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += kThreads) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+        int id = tid < s.hist_len ? s.hist[tid] : -1;
+        for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
-        set_bits(s, first_id);
-        const int c = first_id - s.id_base;
-        if (tid < s.hist_len && c >= s.lo && c < s.hi) {
-            pen_col = c;
-            pen_raw = __ldcg(row_ptr + c);
+        for (int i0 = tid & ~31; i0 < s.hist_len; i0 += T) {
+            const int next = i0 + T + lane < s.hist_len ? s.hist[i0 + T + lane] : -1;
+            const int c = id - s.id_base;
+            bool first = false;   // an id counts once however often it occurs in the window
+            if (i0 + lane < s.hist_len && c >= s.lo && c < s.hi) {
+                const unsigned bit = 1u << ((c - s.bit0) & 31);
+                first = (atomicOr(&s.bitmap[(c - s.bit0) >> 5], bit) & bit) == 0u;
+            }
+            const unsigned hits = __ballot_sync(0xffffffffu, first);
+            if (hits) {   // its logit is fetched now (with the next chunk's group) and needed at the end
+                int p = 0;
+                if (lane == 0) p = atomicAdd(&ctl->pen_n, __popc(hits));
+                p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
+                if (first && p < kPenCap) {
+                    pen_col[p] = c;
+                    cp_async4(smem_u32(pen_raw + p), row_ptr + c);
+                }
+            }
+            id = next;
         }
     }
     __syncthreads();
-    if (edge_col >= 0 && penalised(s, edge_col)) edge = qnan;   // penalised logits are looked at on their own
+    if (s.has_pen && tid < 8) {   // penalised logits are looked at on their own
+        const int c = tid < 4 ? tid : head + 4 * n_cells + tid - 4;
+        if (ctl->edge[tid] == ctl->edge[tid] && penalised(s, c)) ctl->edge[tid] = qnan;
+    }
     trace_mark(a, 1);
 
     // ---- the stream
     float run_a = ninf, run_b = ninf, thr = -FLT_MAX, admit = -FLT_MAX, seen = ninf;
+    int refreshes = 0;
+    int wn = 0;           // cells in the warp's list
     bool fresh = false;   // the bound takes in everything seen so far
     bool lost = false;    // a list was too short
     bool again = false;   // the second time through: the bound is final
-    int n = 0;
 again_from_the_start:
     for (int c = 0, j0 = c_lo + tid;; ++c, j0 += kChunkCells) {
         const int left = c_hi - (j0 - tid);   // cells of the segment from this chunk on
@@ -445,19 +453,14 @@ again_from_the_start:
         const float4* st = ring + (c % kStages) * kChunkCells + tid;
         float4 x[kCells];
 #pragma unroll
-        for (int u = 0; u < kCells; ++u) x[u] = st[u * kThreads];
-        if (left < kChunkCells) {
-#pragma unroll
-            for (int u = 0; u < kCells; ++u)
-                if (tid + u * kThreads >= left) x[u] = make_float4(ninf, ninf, ninf, ninf);
-        }
+        for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
         if (s.has_pen) {   // penalised logits are left out
             const unsigned* w = s.bitmap + ((j0 - c_lo) >> 3) + 1;
             const int sh = 4 * ((j0 - c_lo) & 7);
             unsigned bits[kCells];
 #pragma unroll
-            for (int u = 0; u < kCells; ++u) bits[u] = tid + u * kThreads < left ? (w[u * (kThreads / 8)] >> sh) & 15u : 0u;
-            if (bits[0] | bits[1] | bits[2] | bits[3]) {
+            for (int u = 0; u < kCells; ++u) bits[u] = tid + u * T < left ? w[u * (T / 8)] >> sh : 0u;
+            if ((bits[0] | bits[1] | bits[2] | bits[3]) & 15u) {
 #pragma unroll
                 for (int u = 0; u < kCells; ++u) {
                     if (bits[u] & 1u) x[u].x = ninf;
@@ -467,119 +470,139 @@ again_from_the_start:
                 }
             }
         }
-        const float m0 = cell_max(x[0]), m1 = cell_max(x[1]), m2 = cell_max(x[2]), m3 = cell_max(x[3]);
-        const float ma = fmaxf(m0, m1), mb = fmaxf(m2, m3);
-        run_a = fmaxf(run_a, ma);
-        run_b = fmaxf(run_b, mb);
+        float m[kCells];
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
+        if (left < kChunkCells) {
+#pragma unroll
+            for (int u = 0; u < kCells; ++u)
+                if (tid + u * T >= left) m[u] = ninf;
+        }
+        run_a = max3(run_a, m[0], m[1]);
+        run_b = max3(run_b, m[2], m[3]);
         fetch(c + kStages);   // into the stage just read
         fresh = !again && ((c & (c + 1)) == 0 || thr <= -FLT_MAX || (k > 64 && c < 8));
         if (fresh) {
-            thr = cta_bound(run_a, run_b, k, ctl, n);
+            thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl, maxima);
             admit = thr;
             if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
-            else seen = thr > -FLT_MAX ? thr : ninf;
-            lost = lost || n > kCellCap;
-            if (n > kCellCap / 2 && !lost) prune_cells(listed, listed_num, ctl, admit);
+            if (wn > cell_cap / 4) wn = prune_cells(listed, listed_num, wn, admit);
         }
-        if (__any_sync(0xffffffffu, fmaxf(ma, mb) >= admit)) {
-            const float m[kCells] = {m0, m1, m2, m3};
-            unsigned hit[kCells];
-            int p = warp_reserve<kCells>(m, admit, hit, &ctl->list_n);
+        if (__any_sync(0xffffffffu, fmaxf(max3(m[0], m[1], m[2]), m[3]) >= admit)) {   // the warp's own list: no atomics
 #pragma unroll
             for (int u = 0; u < kCells; ++u) {
-                const int q = p + __popc(hit[u] & lanes_below());
-                if (m[u] >= admit && q < kCellCap) {
+                const unsigned hits = __ballot_sync(0xffffffffu, m[u] >= admit);
+                const int q = wn + __popc(hits & lanes_below());
+                if (m[u] >= admit && q < cell_cap) {
                     listed[q] = x[u];
-                    listed_num[q] = j0 + u * kThreads;
+                    listed_num[q] = j0 + u * T;
                 }
-                p += __popc(hit[u]);
+                wn += __popc(hits);
+            }
+            if (wn > cell_cap) {
+                lost = true;
+                wn = cell_cap;
             }
         }
         if (left <= kChunkCells) break;
     }
     cp_async_wait<0>();
+    if (lost && lane == 0) ctl->lost = 1;
     trace_mark(a, 4);
 
     // ---- the segment's candidates: logits that reach the final bound
     if (fresh || again) {
         __syncthreads();
     } else {
-        thr = cta_bound(run_a, run_b, k, ctl, n);
+        thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl, maxima);
         admit = thr;
         if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
-        else seen = thr > -FLT_MAX ? thr : ninf;
     }
     const bool bounded = thr > -FLT_MAX;
-    n = ctl->list_n;
-    lost = lost || n > kCellCap;
+    if (s.cap == 0.0f) seen = thr;      // (minus infinity is not among the listed ones)
+    lost = ctl->lost != 0;
     if (lost && bounded && !again) {   // the early bounds let too much through: the final one will not, unless many logits are equal
         __syncthreads();
-        if (tid == 0) ctl->list_n = 0;
+        if (tid == 0) ctl->lost = 0;
         for (int c = 0; c < kStages; ++c) fetch(c);
+        wn = 0;
         lost = false;
         again = true;
         __syncthreads();
         goto again_from_the_start;
     }
     auto pick = [&](bool hit, float y, int col) {   // all lanes of the warp
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (m == 0u) return;
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (hits == 0u) return;
         int p = 0;
-        if ((tid & 31) == 0) p = atomicAdd(&ctl->kept_n, __popc(m));
-        p = __shfl_sync(0xffffffffu, p, 0) + __popc(m & lanes_below());
+        if (lane == 0) p = atomicAdd(&ctl->kept_n, __popc(hits));
+        p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
         if (hit && p < kPickCap) picked[p] = make_comp(y, col + s.id_base);
     };
     if (!lost) {
-        for (int p0 = tid & ~31; p0 < n; p0 += kThreads) {
-            const int p = p0 + (tid & 31);
-            float xs[4] = {ninf, ninf, ninf, ninf};
+        for (int p0 = 0; p0 < wn; p0 += 32) {
+            float4 v = make_float4(ninf, ninf, ninf, ninf);
             int col = 0;
-            if (p < n) {
-                *reinterpret_cast<float4*>(xs) = listed[p];
-                col = head + 4 * listed_num[p];
+            if (p0 + lane < wn) {
+                v = listed[p0 + lane];
+                col = head + 4 * listed_num[p0 + lane];
             }
+            float xs[4] = {v.x, v.y, v.z, v.w};
             if (s.cap != 0.0f) {
-#pragma unroll 1
+#pragma unroll
                 for (int e = 0; e < 4; ++e) xs[e] = xs[e] >= admit ? softcap_call(xs[e], s.cap) : ninf;
             }
+            const float least = fmaxf(seen, -FLT_MAX);
             unsigned hit[4];
-            int q = warp_reserve<4>(xs, fmaxf(seen, -FLT_MAX), hit, &ctl->kept_n);
+            int q = warp_reserve<4>(xs, least, hit, &ctl->kept_n);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int at = q + __popc(hit[e] & lanes_below());
-                if (xs[e] >= fmaxf(seen, -FLT_MAX) && at < kPickCap) picked[at] = make_comp(xs[e], col + e + s.id_base);
+                if (xs[e] >= least && at < kPickCap) picked[at] = make_comp(xs[e], col + e + s.id_base);
                 q += __popc(hit[e]);
             }
         }
         if (tid < 32 && V != 4 * n_cells) {
-            const float y = s.cap != 0.0f ? softcap_call(edge, s.cap) : edge;
-            pick(edge >= admit && y >= seen, y, edge_col);
+            const float x = lane < 8 ? ctl->edge[lane] : qnan;
+            const float y = s.cap != 0.0f ? softcap_call(x, s.cap) : x;
+            pick(x >= admit && y >= seen, y, lane < 4 ? lane : head + 4 * n_cells + lane - 4);
         }
         if (s.has_pen) {
-            for (int i0 = tid & ~31; i0 < s.hist_len; i0 += kThreads) {
-                const int i = i0 + (tid & 31);
-                float x = pen_raw;
-                int col = pen_col;
-                if (i != tid) {
-                    col = i < s.hist_len ? s.hist[i] - s.id_base : -1;
-                    x = col >= s.lo && col < s.hi ? __ldcg(row_ptr + col) : qnan;
+            const int n_pen = ctl->pen_n;
+            if (n_pen <= kPenCap) {
+                for (int i0 = tid & ~31; i0 < n_pen; i0 += T) {
+                    const bool in = i0 + lane < n_pen;
+                    const float x = in ? pen_raw[i0 + lane] : qnan;
+                    const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
+                    pick(y >= seen && y > ninf, y, in ? pen_col[i0 + lane] : 0);
                 }
-                const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
-                pick(y >= seen && y > ninf && claim(s, col), y, col);
+            } else {   // a long window: whatever the bitmap holds
+                const int words = (s.hi - s.bit0 + 31) >> 5;
+                for (int w0 = tid & ~31; w0 < words; w0 += T) {
+                    unsigned bits = w0 + lane < words ? s.bitmap[w0 + lane] : 0u;
+                    while (__any_sync(0xffffffffu, bits != 0u)) {
+                        const int col = s.bit0 + 32 * (w0 + lane) + __ffs(bits) - 1;
+                        const float x = bits ? __ldcg(row_ptr + col) : qnan;
+                        const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
+                        pick(y >= seen && y > ninf, y, col);
+                        bits &= bits - 1u;
+                    }
+                }
             }
         }
     }
     __syncthreads();
-    n = ctl->kept_n;
+    int n = ctl->kept_n;
     lost = lost || n > kPickCap;
-    if (lost || (n < k && (bounded || s.cap != 0.0f))) n = exact_select(s, k, picked, ctl);
-    else if (n < k) n = append_masked(s, n, k, picked, ctl);
-    if (a.write_back) write_back(s);
+    if (lost || (n < k && (bounded || s.cap != 0.0f))) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
+    else if (n < k) n = append_masked<T>(s, n, k, picked, reinterpret_cast<unsigned*>(list));
+    if (a.write_back) write_back<T>(s);
     trace_mark(a, 2);
     if (a.trace && tid == 0 && blockIdx.x < 4096u) a.trace[(size_t)blockIdx.x * 8 + 3] = (u64)n;
     if (a.overlap == 1) pdl_wait_prior();   // from here on this launch writes what the previous launch in the stream may still be using
 
     // ---- the row: the k best of all its segments' candidates, in order
+    if (tid >= kPost) return;   // eight warps finish the row (no barrier of the whole CTA or by all threads of the cluster from here on)
     u64* all = picked;
     if (nseg > 1) {
         const int lseg = nseg == 8 ? 3 : nseg == 4 ? 2 : 1;
@@ -604,16 +627,15 @@ again_from_the_start:
         const int q = tid & (nseg - 1), n_q = ctl->recv_n[q];
         const u64* from = recv + q * kSendCap;
         run_a = run_b = ninf;
-        for (int i = tid >> lseg; i < n_q; i += kThreads >> lseg) {
+        for (int i = tid >> lseg; i < n_q; i += kPost >> lseg) {
             const float y = comp_value(from[i]);
-            if (i & (kThreads >> lseg)) run_b = fmaxf(run_b, y);
+            if (i & (kPost >> lseg)) run_b = fmaxf(run_b, y);
             else run_a = fmaxf(run_a, y);
         }
-        const float floor_y = cta_bound(run_a, run_b, k, ctl, n);
+        const float floor_y = cta_bound<kPost, 1>(run_a, run_b, k, refreshes & 1, ctl, maxima);
         const float least = floor_y > -FLT_MAX ? floor_y : ninf;
-        int most = 0;
-        for (int g = 0; g < nseg; ++g) most = max(most, ctl->recv_n[g]);
-        for (int i = tid >> lseg; (i - (tid >> lseg)) < most; i += kThreads >> lseg) {
+        const int most = __reduce_max_sync(0xffffffffu, n_q);   // (every warp has threads of every segment)
+        for (int i = tid >> lseg; (i - (tid >> lseg)) < most; i += kPost >> lseg) {
             const u64 m = i < n_q ? from[i] : 0ull;
             const bool hit = m != 0ull && comp_value(m) >= least;
             const unsigned hits = __ballot_sync(0xffffffffu, hit);
@@ -623,12 +645,12 @@ again_from_the_start:
             p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
             if (hit) list[p] = m;
         }
-        __syncthreads();
+        block_sync<kPost, 1>();
         n = ctl->out_cnt;
         all = list;
     }
     rank_emit(all, n, k, all == list ? picked : list, ctl, [&](int rank, u64 m) { out[rank] = m; });
-    __syncthreads();
+    block_sync<kPost, 1>();
     trace_mark(a, 5);
     const RowDesc& d = dp;
     const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.flags, d.out_index, d.hist_begin + d.hist_len};
@@ -639,22 +661,36 @@ again_from_the_start:
 
 constexpr int kFewRows = 8, kArgRows = 64;   // batches of up to this many rows send their descriptors with the launch
 
-template <int NDESC>
-int launch_select(const cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows) {
+template <int T, int NDESC>
+int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows) {
+    const int seg_cols = a.penalised ? 4 * ((a.n_vocab / 4 + a.nseg - 1) / a.nseg) + 8 : 0;
+    cfg.blockDim = dim3(T);
+    cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols);
+    if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
     SelectArgs<NDESC> args;
     args.a = a;
     if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
-    return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<NDESC>, args);
+    return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC>, args);
+}
+template <int T>
+int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows) {
+    if (rows && a.n_rows <= kFewRows) return launch_select<T, kFewRows>(cfg, a, rows);
+    if (rows && a.n_rows <= kArgRows) return launch_select<T, kArgRows>(cfg, a, rows);
+    return launch_select<T, 0>(cfg, a, nullptr);
+}
+template <int T, int NDESC>
+int prepare_select() {
+    return (int)cudaFuncSetAttribute(stream_select_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
 }
 
 }  // namespace
 
 // Per-device set-up (the current device): opt in to the large dynamic shared memory.
 int prepare_device_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(stream_select_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<kFewRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<kArgRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
-    return (int)e;
+    for (int e : {prepare_select<256, 0>(), prepare_select<256, kFewRows>(), prepare_select<256, kArgRows>(), prepare_select<1024, 0>(),
+                  prepare_select<1024, kFewRows>(), prepare_select<1024, kArgRows>()})
+        if (e != 0) return e;
+    return 0;
 }
 
 int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* stream) {
@@ -670,28 +706,26 @@ int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* st
         attr[n].val.clusterDim.z = 1;
         ++n;
     }
-    const int seg_cols = a.penalised ? 4 * ((a.n_vocab / 4 + a.nseg - 1) / a.nseg) + 8 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(a.n_rows * a.nseg));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = select_smem_bytes(a.nseg, seg_cols);
-    if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    if (host_rows && a.n_rows <= kFewRows) return launch_select<kFewRows>(cfg, a, host_rows);
-    if (host_rows && a.n_rows <= kArgRows) return launch_select<kArgRows>(cfg, a, host_rows);
-    return launch_select<0>(cfg, a, nullptr);
+    return a.wide ? launch_select<1024>(cfg, a, host_rows) : launch_select<256>(cfg, a, host_rows);
 }
 
-// Segments per row: up to eight, as long as there are not more CTAs than two per SM and a segment has at least two chunks.
-// Measured on B200 (1 / 2 / 4 / 8 segments, us per synchronous call): 1 x 65536 33 / 30 / 27 / 25, 32 x 131072 (four steps)
-// 176 / 153 / 130 / 124, 64 x 262144 (launch) 55 / 40 / 33 / 40, 72 x 131072 93 / 87 / 84 / 93, 136 x 65536 32 / 34 / 36 / 48,
-// 512 x 32768 73 / 91 / 106 / 160: a segment more costs every CTA its fixed steps once more.
-int plan_segments(int n_rows, int n_vocab, int sms) {
-    int nseg = 1;
-    while (nseg < 8 && (int64_t)n_rows * nseg * 2 <= 2 * sms && n_vocab / (nseg * 2) >= 8 * kChunkCells) nseg *= 2;
-    return nseg;
+// How a launch is laid out.  Measured on B200, k = 40 to 64, us per call (small CTAs with 1 / 2 / 4 / 8 segments per row;
+// large ones with 1 / 2 / 4): 1 x 65536 34 / 30 / 27 / 26; 29 / 28 / 27.  24 x 100003 48 / 43 / 39 / 38; 44 / 44 / 40.
+// 64 x 262144 61 / 42 / 33 / 38; 35 / 31 / 43.  72 x 131072 95 / 85 / 85 / 89; 81 / 80 / 98.  512 x 32768 72 / 93 / 106 / 141.
+// Few rows: small CTAs, the row cut as finely as two per SM allow (a large CTA issues every step after the stream from
+// four times as many warps).  Medium batches: one large CTA per SM streams best.  Many rows: a small CTA per row, several
+// per SM, so that the steps of one run beside the stream of the others.
+SelectPlan plan_select(int n_rows, int n_vocab, int sms) {
+    SelectPlan pl;
+    pl.wide = n_rows > sms / 4 && n_rows <= sms;
+    const int most = pl.wide ? sms : 2 * sms;
+    while (pl.nseg < 8 && n_rows * pl.nseg * 2 <= most && n_vocab / (pl.nseg * 2) >= 8192) pl.nseg *= 2;
+    return pl;
 }
 
 }  // namespace fsb
@@ -774,7 +808,9 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
         a.n_rows = n_rows;
         a.n_vocab = n_vocab;
         a.kmax = 1;
-        a.nseg = plan_segments(n_rows, n_vocab, sd.sms);
+        const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms);
+        a.nseg = pl.nseg;
+        a.wide = pl.wide ? 1 : 0;
         if (rc == FSB_OK && launch_stream_kernel(a, nullptr, st) != 0) rc = FSB_ERR_CUDA;
         if (rc == FSB_OK && (flags & FSB_STATIC_WAIT)) {
             uint32_t word = 0;

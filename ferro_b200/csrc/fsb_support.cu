@@ -9,7 +9,8 @@
 namespace fsb {
 namespace {
 
-constexpr size_t kSmemMerge = (size_t)(kMergeCap + 8 + kMaxK) * sizeof(u64) + sizeof(SharedCtl);   // gathered lists, ordered candidates, control
+constexpr int kThreads = kPost;   // of the list merge
+constexpr size_t kSmemMerge = (size_t)(kMergeCap + 32 + kMaxK) * sizeof(u64) + sizeof(SharedCtl);   // gathered lists, ordered candidates, control
 
 // Merge of per-shard candidate lists: one CTA per row gathers the row's n_lists ordered lists (already in this
 // device's memory, list g of row r at lists + (g * n_rows + r) * list_stride) and finishes the row exactly as the
@@ -21,7 +22,7 @@ __global__ void __launch_bounds__(kThreads, 1) merge_lists_kernel(const u64* lis
                                                                  int32_t* kept_n, unsigned* status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     u64* buf = reinterpret_cast<u64*>(smem_raw);
-    u64* out = buf + kMergeCap + 8;
+    u64* out = buf + kMergeCap + 32;
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(out + kMaxK);
     const int row = blockIdx.x, tid = threadIdx.x;
     if (row >= n_rows) return;
@@ -39,11 +40,11 @@ __global__ void __launch_bounds__(kThreads, 1) merge_lists_kernel(const u64* lis
             atomicOr(status, kStatusMergeOverflow);
         }
     }
-    __syncthreads();
+    block_sync<kPost, 1>();
     const TailOut tout{tokens, nullptr, nullptr, nullptr, kept_ids, kept_pr, kept_n, nullptr, nullptr, 0, status};
     const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.flags & ~kRowAppend, d.out_index, 0};
     rank_emit(buf, total, d.k_global, out, ctl, [&](int rank, u64 c) { out[rank] = c; });
-    __syncthreads();
+    block_sync<kPost, 1>();
     row_epilogue(out, min(total, d.k_global), rt, reinterpret_cast<double*>(buf), ctl, tout);
 }
 
