@@ -52,6 +52,7 @@ struct fsb_batch {
     int n_cand = 0, n_full = 0;   // rows of the candidate kernel / of the full-row kernel
     int kmax = 1;
     fsb::SelectPlan plan;         // how the streaming kernel is laid out
+    bool all_greedy = false;      // every row of the streaming kernel is greedy
     bool penalised = false;       // some row of the streaming kernel has a penalty window
     int64_t hist_ids = 0;         // window ids staged with the batch
     int64_t gather_ids = 0;       // window values a write-back for a host caller brings back
@@ -243,10 +244,12 @@ int finalize_batch(fsb_handle* h, fsb_batch* b) {
     fsb::RowDesc* dst = b->h_rows();
     auto on_chip = [](const fsb::RowDesc& d) { return d.k <= fsb::kMaxK && d.k_global <= fsb::kMaxK; };
     b->penalised = false;
+    b->all_greedy = true;
     for (const auto& d : b->descs)
         if (on_chip(d)) {
             dst[n_cand++] = d;
             kmax = std::max(kmax, d.k);
+            b->all_greedy = b->all_greedy && (d.flags & fsb::kRowGreedy) != 0;
             b->penalised = b->penalised || (d.flags & fsb::kRowPenalty) != 0;
         }
     int n_full = 0;
@@ -328,6 +331,7 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.nseg = b->plan.nseg;
         a.wide = b->plan.wide ? 1 : 0;
         a.kmax = b->kmax;
+        a.all_greedy = b->all_greedy ? 1 : 0;
         a.penalised = b->penalised ? 1 : 0;
         a.write_back = (b->flags & FSB_WRITE_BACK) ? 1 : 0;
         a.vocab_offset = h->vocab_offset;

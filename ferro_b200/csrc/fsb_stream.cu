@@ -291,6 +291,135 @@ __device__ __noinline__ void write_back(const Segment s) {
     }
 }
 
+__device__ __forceinline__ unsigned lanes_below() {
+    unsigned m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
+__device__ __forceinline__ float cell_max(const float4& x) { return fmaxf(max3(x.x, x.y, x.z), x.w); }
+
+// Where a segment lies in its row: the row's whole 16-byte cells are cut into nseg runs.  Up to three logits before the
+// first cell belong to the first segment, up to three after the last cell to the last one: rows may start anywhere.
+struct RowSpan {
+    const float4* cells;   // cell 0
+    int head;              // columns before it
+    int n_cells, c_lo, c_hi;
+    // column of the segment's e-th logit outside the whole cells (e < 8), or -1
+    __device__ __forceinline__ int edge_column(int e, int n_vocab, int seg, int nseg) const {
+        if (e < 4) return seg == 0 && e < head ? e : -1;
+        return seg == nseg - 1 && e - 4 < n_vocab - head - 4 * n_cells ? head + 4 * n_cells + e - 4 : -1;
+    }
+};
+__device__ __forceinline__ RowSpan row_span(const float* row_ptr, int V, int seg, int nseg) {
+    RowSpan w;
+    w.head = min(V, (int)((0u - ((unsigned)reinterpret_cast<uintptr_t>(row_ptr) >> 2)) & 3u));
+    w.n_cells = (V - w.head) >> 2;
+    const int lseg = 31 - __clz(nseg), per = (w.n_cells + nseg - 1) >> lseg;   // nseg is a power of two
+    w.c_lo = min(seg * per, w.n_cells);
+    w.c_hi = min(w.c_lo + per, w.n_cells);
+    w.cells = reinterpret_cast<const float4*>(row_ptr + w.head);
+    return w;
+}
+__device__ __forceinline__ Segment make_segment(const StreamArgs& a, const RowSpan& w, const float* row_ptr, int seg, int nseg, unsigned* bitmap) {
+    Segment s;
+    s.row = row_ptr;
+    s.bitmap = bitmap;
+    s.hist = nullptr;
+    s.hist_len = 0;
+    s.lo = seg == 0 ? 0 : w.head + 4 * w.c_lo;
+    s.hi = seg == nseg - 1 ? a.n_vocab : w.head + 4 * w.c_hi;
+    s.bit0 = w.head + 4 * w.c_lo - 32;
+    s.id_base = a.vocab_offset;
+    s.has_pen = false;
+    s.pen = 1.0f;
+    s.cap = a.softcap;
+    return s;
+}
+
+// The window's columns of the segment: sets their bits, and lists each once - an id counts once however often it occurs -
+// with its logit, which is fetched now (the copies belong to the next group that the thread commits) and needed at the end.
+// All threads call; a barrier has to follow.
+template <int T>
+__device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* ctl, float* pen_raw, int* pen_col) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    int id = tid < s.hist_len ? s.hist[tid] : -1;
+    for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (int i0 = tid & ~31; i0 < s.hist_len; i0 += T) {
+        const int next = i0 + T + lane < s.hist_len ? s.hist[i0 + T + lane] : -1;
+        const int c = id - s.id_base;
+        bool first = false;
+        if (i0 + lane < s.hist_len && c >= s.lo && c < s.hi) {
+            const unsigned bit = 1u << ((c - s.bit0) & 31);
+            first = (atomicOr(&s.bitmap[(c - s.bit0) >> 5], bit) & bit) == 0u;
+        }
+        const unsigned hits = __ballot_sync(0xffffffffu, first);
+        if (hits) {
+            int p = 0;
+            if (lane == 0) p = atomicAdd(&ctl->pen_n, __popc(hits));
+            p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
+            if (first && p < kPenCap) {
+                pen_col[p] = c;
+                cp_async4(smem_u32(pen_raw + p), s.row + c);
+            }
+        }
+        id = next;
+    }
+}
+// Calls f(valid, raw logit, column) for every penalised column; whole warps call it together.
+template <int T, class F>
+__device__ __forceinline__ void for_each_penalised(const Segment& s, int n_pen, const float* pen_raw, const int* pen_col, F f) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (n_pen <= kPenCap) {
+        for (int i0 = tid & ~31; i0 < n_pen; i0 += T) {
+            const bool in = i0 + lane < n_pen;
+            f(in, in ? pen_raw[i0 + lane] : 0.0f, in ? pen_col[i0 + lane] : 0);
+        }
+    } else {   // a long window: whatever the bitmap holds
+        const int words = (s.hi - s.bit0 + 31) >> 5;
+        for (int w0 = tid & ~31; w0 < words; w0 += T) {
+            unsigned bits = w0 + lane < words ? s.bitmap[w0 + lane] : 0u;
+            while (__any_sync(0xffffffffu, bits != 0u)) {
+                const int col = s.bit0 + 32 * (w0 + lane) + __ffs(bits) - 1;
+                f(bits != 0u, bits ? __ldcg(s.row + col) : 0.0f, col);
+                bits &= bits - 1u;
+            }
+        }
+    }
+}
+// Penalised logits of a thread's cells of a chunk (`j`: its first cell, counted from the segment's first; `left`: cells of
+// the segment from this chunk on) become minus infinity: they are looked at on their own.
+template <int T>
+__device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const unsigned* bitmap, int j, int left) {
+    const float ninf = -__int_as_float(0x7f800000);
+    const unsigned* w = bitmap + (j >> 3) + 1;
+    const int sh = 4 * (j & 7);
+    unsigned bits[kCells];
+#pragma unroll
+    for (int u = 0; u < kCells; ++u) bits[u] = (int)threadIdx.x + u * T < left ? w[u * (T / 8)] >> sh : 0u;
+    if ((bits[0] | bits[1] | bits[2] | bits[3]) & 15u) {
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) {
+            if (bits[u] & 1u) x[u].x = ninf;
+            if (bits[u] & 2u) x[u].y = ninf;
+            if (bits[u] & 4u) x[u].z = ninf;
+            if (bits[u] & 8u) x[u].w = ninf;
+        }
+    }
+}
+// Largest of the lanes' composites.
+__device__ __forceinline__ u64 warp_max_u64(u64 v) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32) == hi ? (unsigned)v : 0u);
+    return ((u64)hi << 32) | lo;
+}
+// The row's candidates in order: softmax, cuts, draw, and whatever the caller wants of them.
+__device__ __forceinline__ void finish_row(const StreamArgs& a, const RowDesc& d, const u64* out, int kk, double* work, SharedCtl* ctl) {
+    const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.flags, d.out_index, d.hist_begin + d.hist_len};
+    const TailOut tout{a.tokens, a.tokens_host, a.status_host, a.pool, a.kept_ids, a.kept_pr, a.kept_n, reinterpret_cast<u64*>(a.shard_out), a.shard_n, a.shard_stride, a.status};
+    row_epilogue(out, kk, rt, work, ctl, tout);
+}
+
 __device__ __forceinline__ void trace_mark(const StreamArgs& a, int slot) {
     if (a.trace && threadIdx.x == 0 && blockIdx.x < 4096u) {
         a.trace[(size_t)blockIdx.x * 8 + slot] = slot == 0 ? global_timer_ns() : (u64)clock64();
@@ -298,11 +427,6 @@ __device__ __forceinline__ void trace_mark(const StreamArgs& a, int slot) {
     }
 }
 
-__device__ __forceinline__ unsigned lanes_below() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
 // Room in a list for every value of the warp that reaches `bound`: one shared-memory atomic per warp (lanes of a warp
 // that add to one word are served one after the other, 8 cycles each).  hit[i]: the lanes whose i-th value does; entries go
 // in order of i, then of lanes.  All lanes call.
@@ -318,7 +442,6 @@ __device__ __forceinline__ int warp_reserve(const float (&v)[N], float bound, un
     if ((threadIdx.x & 31) == 0 && total) p = atomicAdd(counter, total);
     return __shfl_sync(0xffffffffu, p, 0);
 }
-__device__ __forceinline__ float cell_max(const float4& x) { return fmaxf(max3(x.x, x.y, x.z), x.w); }
 
 // A launch's arguments: with NDESC > 0 the row descriptors come with them (a batch of few rows needs no copy to the
 // device before the launch, and no CTA waits for a read of global memory before it knows its row).
@@ -361,14 +484,10 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     const RowDesc& dp = NDESC > 0 ? args.rows[row] : a.rows[row];
     const float* row_ptr = a.logits + (a.row_ld >= 0 ? (int64_t)row * a.row_ld : dp.logits_off);
 
-    // The row's whole 16-byte cells, cut into nseg runs.  Up to three logits before the first cell belong to the first
-    // segment, up to three after the last cell to the last one: rows may start anywhere.
     const int V = a.n_vocab;
-    const int head = min(V, (int)((0u - ((unsigned)reinterpret_cast<uintptr_t>(row_ptr) >> 2)) & 3u));
-    const int n_cells = (V - head) >> 2;
-    const int per = (n_cells + nseg - 1) / nseg;
-    const int c_lo = min(seg * per, n_cells), c_hi = min(c_lo + per, n_cells);
-    const float4* cells = reinterpret_cast<const float4*>(row_ptr + head);
+    const RowSpan span = row_span(row_ptr, V, seg, nseg);
+    const int head = span.head, n_cells = span.n_cells, c_lo = span.c_lo, c_hi = span.c_hi;
+    const float4* cells = span.cells;
     const float qnan = __int_as_float(0x7fc00000), ninf = -__int_as_float(0x7f800000);
     const unsigned slot0 = smem_u32(ring + tid);
     // chunk c of this thread: cells j, j + T, ... go to stage c % kStages
@@ -382,22 +501,12 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     };
     for (int c = 0; c < kStages; ++c) fetch(c);
     if (tid < 8) {   // the logits outside the whole cells
-        const int c = tid < 4 ? (seg == 0 && tid < head ? tid : -1) : (seg == nseg - 1 && tid < 4 + V - head - 4 * n_cells ? head + 4 * n_cells + tid - 4 : -1);
+        const int c = span.edge_column(tid, V, seg, nseg);
         ctl->edge[tid] = c >= 0 ? __ldcg(row_ptr + c) : qnan;
     }
-
-    Segment s;
-    s.row = row_ptr;
-    s.bitmap = reinterpret_cast<unsigned*>(recv + (nseg > 1 ? nseg * kSendCap : 0));
-    s.lo = seg == 0 ? 0 : head + 4 * c_lo;
-    s.hi = seg == nseg - 1 ? V : head + 4 * c_hi;
-    s.bit0 = head + 4 * c_lo - 32;
-    s.id_base = a.vocab_offset;
+    Segment s = make_segment(a, span, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(recv + (nseg > 1 ? nseg * kSendCap : 0)));
     s.has_pen = (dp.flags & kRowPenalty) != 0;
     s.pen = dp.penalty;
-    s.cap = a.softcap;
-    s.hist = nullptr;
-    s.hist_len = 0;
     const int k = dp.k;
     if (tid == 0) {
         ctl->lost = 0;
@@ -408,29 +517,7 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     if (s.has_pen) {
         s.hist = a.hist + dp.hist_begin;
         s.hist_len = dp.hist_len;
-        int id = tid < s.hist_len ? s.hist[tid] : -1;
-        for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
-        __syncthreads();
-        for (int i0 = tid & ~31; i0 < s.hist_len; i0 += T) {
-            const int next = i0 + T + lane < s.hist_len ? s.hist[i0 + T + lane] : -1;
-            const int c = id - s.id_base;
-            bool first = false;   // an id counts once however often it occurs in the window
-            if (i0 + lane < s.hist_len && c >= s.lo && c < s.hi) {
-                const unsigned bit = 1u << ((c - s.bit0) & 31);
-                first = (atomicOr(&s.bitmap[(c - s.bit0) >> 5], bit) & bit) == 0u;
-            }
-            const unsigned hits = __ballot_sync(0xffffffffu, first);
-            if (hits) {   // its logit is fetched now (with the next chunk's group) and needed at the end
-                int p = 0;
-                if (lane == 0) p = atomicAdd(&ctl->pen_n, __popc(hits));
-                p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
-                if (first && p < kPenCap) {
-                    pen_col[p] = c;
-                    cp_async4(smem_u32(pen_raw + p), row_ptr + c);
-                }
-            }
-            id = next;
-        }
+        collect_penalised<T>(s, ctl, pen_raw, pen_col);
     }
     __syncthreads();
     if (s.has_pen && tid < 8) {   // penalised logits are looked at on their own
@@ -454,22 +541,7 @@ again_from_the_start:
         float4 x[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
-        if (s.has_pen) {   // penalised logits are left out
-            const unsigned* w = s.bitmap + ((j0 - c_lo) >> 3) + 1;
-            const int sh = 4 * ((j0 - c_lo) & 7);
-            unsigned bits[kCells];
-#pragma unroll
-            for (int u = 0; u < kCells; ++u) bits[u] = tid + u * T < left ? w[u * (T / 8)] >> sh : 0u;
-            if ((bits[0] | bits[1] | bits[2] | bits[3]) & 15u) {
-#pragma unroll
-                for (int u = 0; u < kCells; ++u) {
-                    if (bits[u] & 1u) x[u].x = ninf;
-                    if (bits[u] & 2u) x[u].y = ninf;
-                    if (bits[u] & 4u) x[u].z = ninf;
-                    if (bits[u] & 8u) x[u].w = ninf;
-                }
-            }
-        }
+        if (s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - c_lo, left);
         float m[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
@@ -567,29 +639,11 @@ again_from_the_start:
             const float y = s.cap != 0.0f ? softcap_call(x, s.cap) : x;
             pick(x >= admit && y >= seen, y, lane < 4 ? lane : head + 4 * n_cells + lane - 4);
         }
-        if (s.has_pen) {
-            const int n_pen = ctl->pen_n;
-            if (n_pen <= kPenCap) {
-                for (int i0 = tid & ~31; i0 < n_pen; i0 += T) {
-                    const bool in = i0 + lane < n_pen;
-                    const float x = in ? pen_raw[i0 + lane] : qnan;
-                    const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
-                    pick(y >= seen && y > ninf, y, in ? pen_col[i0 + lane] : 0);
-                }
-            } else {   // a long window: whatever the bitmap holds
-                const int words = (s.hi - s.bit0 + 31) >> 5;
-                for (int w0 = tid & ~31; w0 < words; w0 += T) {
-                    unsigned bits = w0 + lane < words ? s.bitmap[w0 + lane] : 0u;
-                    while (__any_sync(0xffffffffu, bits != 0u)) {
-                        const int col = s.bit0 + 32 * (w0 + lane) + __ffs(bits) - 1;
-                        const float x = bits ? __ldcg(row_ptr + col) : qnan;
-                        const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
-                        pick(y >= seen && y > ninf, y, col);
-                        bits &= bits - 1u;
-                    }
-                }
-            }
-        }
+        if (s.has_pen)
+            for_each_penalised<T>(s, ctl->pen_n, pen_raw, pen_col, [&](bool in, float x, int col) {
+                const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
+                pick(in && y >= seen && y > ninf, y, col);
+            });
     }
     __syncthreads();
     int n = ctl->kept_n;
@@ -652,10 +706,136 @@ again_from_the_start:
     rank_emit(all, n, k, all == list ? picked : list, ctl, [&](int rank, u64 m) { out[rank] = m; });
     block_sync<kPost, 1>();
     trace_mark(a, 5);
-    const RowDesc& d = dp;
-    const RowTail rt{d.rng_word, d.temperature, d.top_p, d.min_p, d.flags, d.out_index, d.hist_begin + d.hist_len};
-    const TailOut tout{a.tokens, a.tokens_host, a.status_host, a.pool, a.kept_ids, a.kept_pr, a.kept_n, reinterpret_cast<u64*>(a.shard_out), a.shard_n, a.shard_stride, a.status};
-    row_epilogue(out, min(n, k), rt, reinterpret_cast<double*>(list), ctl, tout);
+    finish_row(a, dp, out, min(n, k), reinterpret_cast<double*>(list), ctl);
+    trace_mark(a, 6);
+}
+
+// Launches whose rows are all greedy (a verification step at temperature 0, the static entry point): the same stream, but
+// a thread keeps the best cell it has seen in registers ("strictly larger" keeps the first of equals, because a thread
+// meets its cells in ascending order), the CTA takes the largest composite, and one warp finishes the row.  No bound, no
+// lists, no barrier before the end.  (Not with a softcap, which makes different logits equal, nor with write-back.)
+template <int T>
+size_t argmax_smem_bytes(int seg_cols) {
+    return Geometry<T>::kRingBytes + sizeof(SharedCtl) + (seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0);
+}
+
+template <int T, int NDESC>
+__global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
+    constexpr int kChunkCells = Geometry<T>::kChunkCells;
+    const StreamArgs& a = args.a;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    float4* ring = reinterpret_cast<float4*>(smem_raw);
+    u64* best_of = reinterpret_cast<u64*>(smem_raw);   // after the stream: the warps' best, then the first masked columns
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem_raw + Geometry<T>::kRingBytes);
+    float* pen_raw = reinterpret_cast<float*>(ctl + 1);
+    int* pen_col = reinterpret_cast<int*>(pen_raw + kPenCap);
+    const int tid = threadIdx.x, lane = tid & 31;
+    pdl_launch_dependents();
+    trace_mark(a, 0);
+    if (a.overlap != 1) pdl_wait_prior();
+
+    const int nseg = a.nseg, lseg = 31 - __clz(nseg);
+    const int row = (int)(blockIdx.x >> lseg), seg = (int)(blockIdx.x & (unsigned)(nseg - 1));
+    const RowDesc& dp = NDESC > 0 ? args.rows[row] : a.rows[row];
+    const float* row_ptr = a.logits + (a.row_ld >= 0 ? (int64_t)row * a.row_ld : dp.logits_off);
+    const RowSpan w = row_span(row_ptr, a.n_vocab, seg, nseg);
+    const float ninf = -__int_as_float(0x7f800000), qnan = __int_as_float(0x7fc00000);
+    const unsigned slot0 = smem_u32(ring + tid);
+    auto fetch = [&](int c) {
+        const int j = w.c_lo + c * kChunkCells + tid;
+        const unsigned dst = slot0 + (unsigned)((c % kStages) * kChunkCells) * (unsigned)sizeof(float4);
+#pragma unroll
+        for (int u = 0; u < kCells; ++u)
+            if (j + u * T < w.c_hi) cp_async16(dst + (unsigned)(u * T * sizeof(float4)), w.cells + j + u * T);
+        cp_async_commit();
+    };
+    for (int c = 0; c < kStages; ++c) fetch(c);
+    float edge = qnan;
+    int edge_col = -1;
+    if (tid < 8) {
+        edge_col = w.edge_column(tid, a.n_vocab, seg, nseg);
+        if (edge_col >= 0) edge = __ldcg(row_ptr + edge_col);
+    }
+    if (nseg > 1) cluster_arrive_release();
+    Segment s = make_segment(a, w, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(pen_col + kPenCap));
+    if (a.penalised) {   // (without windows nobody waits for the descriptor before the end)
+        s.has_pen = (dp.flags & kRowPenalty) != 0;
+        s.pen = dp.penalty;
+        if (s.has_pen) {
+            s.hist = a.hist + dp.hist_begin;
+            s.hist_len = dp.hist_len;
+            if (tid == 0) ctl->pen_n = 0;
+            collect_penalised<T>(s, ctl, pen_raw, pen_col);
+        }
+        __syncthreads();
+        if (s.has_pen && edge_col >= 0 && penalised(s, edge_col)) edge = qnan;
+    }
+    trace_mark(a, 1);
+
+    float best = ninf;
+    float4 best_cell = make_float4(0.f, 0.f, 0.f, 0.f);
+    int best_num = -1;
+    for (int c = 0, j0 = w.c_lo + tid;; ++c, j0 += kChunkCells) {
+        const int left = w.c_hi - (j0 - tid);
+        cp_async_wait<kStages - 1>();
+        const float4* st = ring + (c % kStages) * kChunkCells + tid;
+        float4 x[kCells];
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
+        if (s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - w.c_lo, left);
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) {
+            const float m = cell_max(x[u]);
+            if (m > best && tid + u * T < left) {
+                best = m;
+                best_cell = x[u];
+                best_num = j0 + u * T;
+            }
+        }
+        fetch(c + kStages);
+        if (left <= kChunkCells) break;
+    }
+    cp_async_wait<0>();
+    trace_mark(a, 4);
+
+    u64 top = 0ull;
+    if (best_num >= 0) {
+        const int e = best_cell.x == best ? 0 : best_cell.y == best ? 1 : best_cell.z == best ? 2 : 3;
+        top = make_comp(best, w.head + 4 * best_num + e + s.id_base);
+    }
+    if (edge > ninf) top = max(top, make_comp(edge, edge_col + s.id_base));
+    if (s.has_pen)
+        for_each_penalised<T>(s, ctl->pen_n, pen_raw, pen_col, [&](bool in, float x, int col) {
+            const float y = penalise(x, s.pen);
+            if (in && y > ninf) top = max(top, make_comp(y, col + s.id_base));
+        });
+    top = warp_max_u64(top);
+    __syncthreads();   // the ring's memory is free
+    if (lane == 0) best_of[tid >> 5] = top;
+    if (__syncthreads_or(top != 0ull) == 0) {   // nothing above minus infinity: the first column that holds it, if any
+        u64* found = best_of + 32;
+        const int n = append_masked<T>(s, 0, 1, found, reinterpret_cast<unsigned*>(found + 8));
+        __syncthreads();
+        if (tid == 0 && n > 0) best_of[0] = found[0];
+        __syncthreads();
+    }
+    trace_mark(a, 2);
+    if (tid >= 32) return;
+    top = warp_max_u64(lane < T / 32 ? best_of[lane] : 0ull);
+    if (a.overlap == 1) pdl_wait_prior();
+    if (nseg > 1) {
+        cluster_wait_acquire();   // every CTA of the row runs: the first one's shared memory may be written
+        if (lane == 0) cluster_store_u64(cluster_map_shared(smem_u32(&ctl->red[seg]), 0u), top);
+        __syncwarp();
+        cluster_arrive_release();
+        if (seg != 0) return;
+        cluster_wait_acquire();
+        top = warp_max_u64(lane < nseg ? ctl->red[lane] : 0ull);
+    }
+    trace_mark(a, 5);
+    if (lane == 0) best_of[0] = top;
+    __syncwarp();
+    finish_row(a, dp, best_of, top != 0ull ? 1 : 0, reinterpret_cast<double*>(best_of + 8), ctl);
     trace_mark(a, 6);
 }
 
@@ -670,6 +850,10 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
     SelectArgs<NDESC> args;
     args.a = a;
     if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
+    if (a.all_greedy && a.softcap == 0.0f && !a.write_back) {
+        cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols);
+        return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
+    }
     return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC>, args);
 }
 template <int T>
@@ -680,7 +864,8 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
 }
 template <int T, int NDESC>
 int prepare_select() {
-    return (int)cudaFuncSetAttribute(stream_select_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    const cudaError_t e = cudaFuncSetAttribute(argmax_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    return (int)(e != cudaSuccess ? e : cudaFuncSetAttribute(stream_select_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax));
 }
 
 }  // namespace
@@ -808,6 +993,7 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
         a.n_rows = n_rows;
         a.n_vocab = n_vocab;
         a.kmax = 1;
+        a.all_greedy = 1;
         const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms);
         a.nseg = pl.nseg;
         a.wide = pl.wide ? 1 : 0;
