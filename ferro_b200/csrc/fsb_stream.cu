@@ -796,6 +796,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         if (left <= kChunkCells) break;
     }
     cp_async_wait<0>();
+    if (s.has_pen) __syncthreads();   // the penalised logits were fetched by other threads
     trace_mark(a, 4);
 
     u64 top = 0ull;
