@@ -293,15 +293,20 @@ struct TailOut {
     unsigned* status;
 };
 
-// A status bit for the host: the device word collects the bits, the host mirror (if any) just becomes non-zero.
+// A status bit for the host: the device word collects the bits, the host mirror (if any) just becomes non-zero - before
+// the token that the host may be waiting for.
 __device__ __forceinline__ void report_status(unsigned* status, unsigned* status_host, unsigned bit) {
     atomicOr(status, bit);
-    if (status_host) *reinterpret_cast<volatile unsigned*>(status_host) = bit;
+    if (status_host) {
+        *reinterpret_cast<volatile unsigned*>(status_host) = bit;
+        __threadfence_system();
+    }
 }
-// A row's token: to the device array and, if the caller reads its own memory, to the host mirror.
+// A row's token: to the device array and, if the caller reads its own memory, to the host mirror, from where the host may
+// take it as soon as it lands.
 __device__ __forceinline__ void put_token(int32_t* tokens, int32_t* tokens_host, int index, int token) {
     tokens[index] = token;
-    if (tokens_host) tokens_host[index] = token;
+    if (tokens_host) *reinterpret_cast<volatile int32_t*>(tokens_host + index) = token;
 }
 
 // srt[0..kk) holds the row's candidates in order (largest first).  Either hands them out (vocabulary-sharded mode)

@@ -128,6 +128,7 @@ struct FullArgs {
     const float* logits;
     const RowDesc* rows;      // the rows of this kernel
     const int32_t* hist;
+    const int32_t* drafts;    // ids staged with a resident verification call
     int32_t* pool;            // id pool of the resident histories (rows with kRowAppend store their token there)
     int32_t* tokens;
     int32_t* tokens_host;     // mirror of the tokens in mapped host memory, or null
@@ -517,8 +518,9 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
         __syncthreads();
         const int32_t* h = a.hist + d.hist_begin;
-        for (int i = tid; i < d.hist_len; i += kFullThreads) {
-            const int c = h[i] - id_base - lo;
+        const int n_drafts = d.flags >> kRowDraftShift;
+        for (int i = tid; i < d.hist_len + n_drafts; i += kFullThreads) {
+            const int c = (i < d.hist_len ? h[i] : a.drafts[d.draft_off + i - d.hist_len]) - id_base - lo;
             if (c >= 0 && c < n) atomicOr(&bitmap[c >> 5], 1u << (c & 31));
         }
         __syncthreads();
@@ -793,7 +795,7 @@ int prepare_full_row_kernel(int max_vocab) {
     return (int)e;
 }
 
-int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
+int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, const int32_t* drafts, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
                            int32_t* kept_ids, double* kept_pr, int32_t* kept_n, int record, uint32_t* status, uint32_t* status_host, int n_vocab,
                            int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream) {
     if (n_vocab > (1 << 22)) return (int)cudaErrorInvalidValue;   // the histogram's limb sums are sized for 4 M logits
@@ -801,6 +803,7 @@ int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows,
     a.logits = logits;
     a.rows = rows;
     a.hist = hist;
+    a.drafts = drafts;
     a.pool = pool;
     a.tokens = tokens;
     a.tokens_host = tokens_host;

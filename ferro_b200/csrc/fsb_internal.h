@@ -19,9 +19,11 @@ enum : uint32_t {
 enum : int32_t {
     kRowGreedy = 1,       // temperature <= 0 or top_k == 1: argmax, no draw
     kRowPenalty = 2,      // the row has a non-empty penalty window and penalty != 1
-    kRowAppend = 4,       // resident histories: the row's token is appended at hist_begin + hist_len of the id pool
-    kRowDraft = 8         // resident verification windows: gather_off holds the draft id that is the last id of the row's window
+    kRowAppend = 4        // resident histories: the row's token is appended at hist_begin + hist_len of the id pool
 };
+// Resident verification windows: the drafts before a row are the last ids of its window.  They are not in the id pool:
+// bits 8 and up of the flags hold their number, draft_off the first one's place among the ids staged with the call.
+constexpr int kRowDraftShift = 8;
 
 constexpr int kWindowTableInts = 72;          // int32 words per stream of a resident verification call: 6 + up to 66 drafts
 
@@ -39,7 +41,10 @@ struct RowDesc {
     int32_t flags;
     int32_t out_index;     // position of the row's token in the output array
     int32_t k_global;      // vocabulary sharding: candidate count of the whole row (k is the shard's); otherwise == k
-    int32_t gather_off;    // where the row's window values go when patched entries are gathered for a host caller
+    union {
+        int32_t gather_off;   // where the row's window values go when patched entries are gathered for a host caller
+        int32_t draft_off;    // resident verification windows: see kRowDraftShift
+    };
 };
 static_assert(sizeof(RowDesc) == 64, "RowDesc layout");
 
@@ -47,7 +52,9 @@ static_assert(sizeof(RowDesc) == 64, "RowDesc layout");
 struct StreamArgs {
     const float* logits;       // base of the [rows][ld] matrix
     const RowDesc* rows;       // n_rows descriptors (only rows of the candidate path)
-    const int32_t* hist;       // packed penalty-window ids
+    const int32_t* hist;       // packed penalty-window ids (or the id pool)
+    const int32_t* drafts;     // ids staged with a resident verification call
+    float* patched;            // optional: the transformed logits at the window ids, indexed by RowDesc::gather_off + place in the window
     int32_t* pool;             // id pool of the resident histories (rows with kRowAppend store their token there)
     int32_t* tokens;           // output tokens, indexed by RowDesc::out_index
     uint32_t* status;          // one word, OR of kStatus* bits
@@ -89,8 +96,11 @@ SelectPlan plan_select(int n_rows, int n_vocab, int sms);
 
 // All return a cudaError_t as int (0 = success).
 int prepare_device_kernels();
-// host_rows: the descriptors in host memory (sent with the launch when they are few), or null.
-int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* stream);
+// Whether a batch's descriptors and staged ids can be arguments of the launch.
+bool rows_fit_launch(int n_rows, int64_t n_ids);
+// host_rows: the descriptors in host memory (sent with the launch when they are few), or null.  host_ids: n_ids staged ids
+// that go with the launch instead of a.hist (ids_are_windows) or a.drafts.
+int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* host_ids, int n_ids, bool ids_are_windows, void* stream);
 
 // One stream of a prompt-lookup drafting call: where its history lies in the id pool and what to look for.
 struct LookupDesc {
@@ -103,12 +113,13 @@ struct LookupDesc {
 static_assert(sizeof(LookupDesc) == 24, "LookupDesc layout");
 constexpr int kDraftStride = 68;              // int32 words per stream of a drafting call: the count, then up to 67 drafts
 
+constexpr int kLookupArgs = 64;               // drafting calls of up to this many streams send the descriptors with the launch
+
 // Defined in fsb_support.cu.
 int prepare_support_kernels();
-int launch_lookup_drafts(const int32_t* pool, const LookupDesc* desc, int n_streams, int32_t* out, int stride, void* stream);
+int launch_lookup_drafts(const int32_t* pool, const LookupDesc* host_desc, const LookupDesc* desc, int n_streams, int32_t* out, int stride, void* stream);
 int launch_merge_lists(const void* lists, const int32_t* list_n, int n_lists, int list_stride, int n_rows, const RowDesc* rows, int32_t* tokens,
                        int32_t* kept_ids, double* kept_pr, int32_t* kept_n, uint32_t* status, void* stream);
-int launch_write_drafts(const RowDesc* rows, int n_rows, int32_t* pool, void* stream);
 int launch_accept_windows(const int32_t* table, int n_streams, const int32_t* tokens, int32_t* pool, void* stream);
 int launch_gather_patched(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int n_vocab, int vocab_offset,
                           float* out, void* stream);
@@ -116,7 +127,7 @@ int launch_gather_patched(const float* logits, const RowDesc* rows, int n_rows, 
 // Defined in fsb_fullrow.cu.
 size_t full_row_smem_bytes(int n_vocab);
 int prepare_full_row_kernel(int max_vocab);
-int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
+int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, const int32_t* drafts, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
                            int32_t* kept_ids, double* kept_pr, int32_t* kept_n, int record, uint32_t* status, uint32_t* status_host, int n_vocab,
                            int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream);
 

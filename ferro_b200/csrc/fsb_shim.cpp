@@ -7,12 +7,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <optional>
 #include <random>
 #include <string>
 #include <vector>
@@ -55,6 +57,7 @@ struct fsb_batch {
     bool all_greedy = false;      // every row of the streaming kernel is greedy
     bool penalised = false;       // some row of the streaming kernel has a penalty window
     int64_t hist_ids = 0;         // window ids staged with the batch
+    bool sent_with_launch = false;   // descriptors and staged ids are arguments of the launch, the device copy is stale
     int64_t gather_ids = 0;       // window values a write-back for a host caller brings back
     int64_t table_ints = 0;       // int32 words of the per-stream table of a resident verification call, staged behind the window ids
     // pinned host staging: [RowDesc x cap_rows][int32 x cap_hist], tokens, gathered window values
@@ -63,6 +66,7 @@ struct fsb_batch {
     int32_t* h_tokens_dev = nullptr;   // the device's address of h_tokens (pinned memory is mapped): kernels mirror tokens and a status flag there
     bool mirrored = false;            // the last launch wrote the mirror: tokens need no copy back
     float* h_patched = nullptr;
+    float* h_patched_dev = nullptr;    // the device's address of h_patched
     // device
     unsigned char* d_in = nullptr;
     int32_t* d_tokens = nullptr;
@@ -75,11 +79,7 @@ struct fsb_batch {
 
     fsb::RowDesc* h_rows() const { return reinterpret_cast<fsb::RowDesc*>(h_in); }
     int32_t* h_hist() const { return reinterpret_cast<int32_t*>(h_in + sizeof(fsb::RowDesc) * (size_t)cap_rows); }
-    // where the kernels read the descriptors: the device copy, or the pinned host block itself through its device address
-    // (see upload_batch)
-    fsb::RowDesc* d_rows() const { return rows_from_host ? reinterpret_cast<fsb::RowDesc*>(h_in_dev) : reinterpret_cast<fsb::RowDesc*>(d_in); }
-    unsigned char* h_in_dev = nullptr;
-    bool rows_from_host = false;
+    fsb::RowDesc* d_rows() const { return reinterpret_cast<fsb::RowDesc*>(d_in); }
     int32_t* d_hist() const { return reinterpret_cast<int32_t*>(d_in + sizeof(fsb::RowDesc) * (size_t)cap_rows); }
     // the kernels' status word sits right behind the tokens, so that one copy brings both back
     uint32_t* d_status() const { return reinterpret_cast<uint32_t*>(d_tokens + cap_rows); }
@@ -107,13 +107,16 @@ struct fsb_handle {
     double* d_kept_pr = nullptr;
     int32_t* d_kept_n = nullptr;
     bool kept_valid = false;
-    // prompt-lookup drafting: descriptors up, drafts down (pinned host copies beside the device arrays)
+    // prompt-lookup drafting: descriptors up, drafts stored into pinned memory by the kernel
     fsb::LookupDesc* h_lookup = nullptr;
     fsb::LookupDesc* d_lookup = nullptr;
     int32_t* h_drafts = nullptr;
-    int32_t* d_drafts = nullptr;
+    int32_t* h_drafts_dev = nullptr;   // the device's address of h_drafts
     float* d_logits_stage = nullptr;   // device copy of host logits: max_rows x max_vocab, allocated with the engine
     size_t logits_stage_elems = 0;
+    float* h_logits = nullptr;         // pinned memory through which a few host rows go to the device
+    int32_t* h_ids = nullptr;          // ring through which new history ids go to the device without waiting
+    size_t h_ids_pos = 0;
     uint64_t* d_trace = nullptr;       // caller-owned diagnostics buffer, or null
     fsb_batch* own = nullptr;          // the batch behind fsb_sample_batch / fsb_verify_windows
     int32_t* d_pool = nullptr;         // resident histories: max_hist ids, carved into power-of-two regions
@@ -124,6 +127,11 @@ struct fsb_handle {
 };
 
 namespace {
+
+constexpr size_t kHostLogits = 256 * 1024;   // host logits that go through pinned memory of the engine's own (1 MB)
+constexpr size_t kIdRing = 64 * 1024;        // ids of the history ring
+constexpr int32_t kNoValue = 0x7fdeadff;     // what the host writes where it waits for a logit (a NaN that no kernel makes)
+constexpr int32_t kNoToken = INT32_MIN;      // ... for a token, a draft or a count
 
 int fail(fsb_handle* h, int code, const char* fmt, ...) {
     if (h) {
@@ -182,17 +190,13 @@ int alloc_batch(fsb_handle* h, int cap_rows, int64_t cap_hist, int64_t patched, 
     if (!b) return fail(h, FSB_ERR_INVALID, "out of host memory");
     b->cap_rows = cap_rows;
     b->cap_hist = std::max<int64_t>(cap_hist, 1);
-    cap_hist = b->cap_hist + (int64_t)fsb::kWindowTableInts * cap_rows;   // room for the table of a resident verification call
+    cap_hist = b->cap_hist + (int64_t)(fsb::kWindowTableInts + 1) * cap_rows;   // room for drafts and table of a resident verification call
     b->descs.reserve((size_t)cap_rows);
     b->sid.reserve((size_t)cap_rows);
     b->stochastic.reserve((size_t)cap_rows);
     const size_t in_bytes = sizeof(fsb::RowDesc) * (size_t)cap_rows + sizeof(int32_t) * (size_t)cap_hist;
     cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&b->h_in), in_bytes);
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&b->h_tokens), sizeof(int32_t) * ((size_t)cap_rows + 1));
-    if (e == cudaSuccess && cudaHostGetDevicePointer(reinterpret_cast<void**>(&b->h_in_dev), b->h_in, 0) != cudaSuccess) {
-        b->h_in_dev = nullptr;
-        cudaGetLastError();
-    }
     if (e == cudaSuccess && cudaHostGetDevicePointer(reinterpret_cast<void**>(&b->h_tokens_dev), b->h_tokens, 0) != cudaSuccess) {
         b->h_tokens_dev = nullptr;   // no mapping on this system: tokens come back by copy
         cudaGetLastError();
@@ -201,6 +205,10 @@ int alloc_batch(fsb_handle* h, int cap_rows, int64_t cap_hist, int64_t patched, 
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&b->d_tokens), sizeof(int32_t) * ((size_t)cap_rows + 1));
     if (e == cudaSuccess) e = cudaMemset(b->d_tokens, 0, sizeof(int32_t) * ((size_t)cap_rows + 1));
     if (e == cudaSuccess && patched > 0) e = cudaMallocHost(reinterpret_cast<void**>(&b->h_patched), sizeof(float) * (size_t)patched);
+    if (e == cudaSuccess && patched > 0 && cudaHostGetDevicePointer(reinterpret_cast<void**>(&b->h_patched_dev), b->h_patched, 0) != cudaSuccess) {
+        b->h_patched_dev = nullptr;
+        cudaGetLastError();
+    }
     if (e == cudaSuccess && patched > 0) e = cudaMalloc(reinterpret_cast<void**>(&b->d_patched), sizeof(float) * (size_t)patched);
     if (e != cudaSuccess) {
         free_batch_buffers(b);
@@ -262,31 +270,29 @@ int finalize_batch(fsb_handle* h, fsb_batch* b) {
     return FSB_OK;
 }
 
-// Sends what the kernels need to know about the batch.  `lone_launch`: the sampling kernels are the only readers of the
-// descriptors (nothing is gathered or drafted on the device around them).  Then, if only descriptors are to be
-// sent, the batch is one wave of CTAs and long enough to hide a read across PCIe behind its first tiles (measured on
-// B200: 64 x 262144 gains 6 us per call, 8 x 65536 nothing, one row loses 2 us), nothing is copied at all: the kernels
-// read the descriptors from the pinned host block.
-int upload_batch(fsb_handle* h, fsb_batch* b, bool lone_launch = false) {
+// Sends what the kernels need to know about the batch: nothing if it goes with the launch (few rows, few window ids, no
+// other kernel that reads them), else one copy.  (Letting the kernels read the pinned block across PCIe instead is far
+// slower on B200: one such read takes 2.3 us, 128 CTAs that each read a few hundred bytes 17 us, a copy 1.1 us in all.)
+int upload_batch(fsb_handle* h, fsb_batch* b, bool launched_often, bool other_readers) {
+    b->sent_with_launch = !launched_often && !other_readers && b->n_full == 0 && b->table_ints == 0 && fsb::rows_fit_launch(b->n_cand, b->hist_ids);
+    if (b->sent_with_launch) return FSB_OK;
     // descriptors, then (behind room for cap_rows of them) window ids and tables: one copy, cut short when only descriptors go up
-    b->rows_from_host = false;
-    if (lone_launch && b->hist_ids + b->table_ints == 0 && b->h_in_dev && b->n_rows <= h->sm_count &&
-        (int64_t)b->n_rows * b->n_vocab >= ((int64_t)4 << 20)) {
-        b->rows_from_host = true;
-        return FSB_OK;
-    }
     const size_t bytes = (b->hist_ids + b->table_ints == 0) ? sizeof(fsb::RowDesc) * (size_t)b->n_rows : b->in_bytes_used();
     FSB_CUDA(h, cudaMemcpyAsync(b->d_in, b->h_in, bytes, cudaMemcpyHostToDevice, h->stream));
     return FSB_OK;
 }
 
 int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep_kept, uint64_t* shard_out = nullptr,
-                 int32_t* shard_n = nullptr, int shard_stride = fsb::kMaxK, bool mirror = false) {
+                 int32_t* shard_n = nullptr, int shard_stride = fsb::kMaxK, bool mirror = false, bool patched = false) {
     // `mirror`: the caller is about to wait for the tokens - the kernels store them (and a flag for any status bit) into
-    // the batch's pinned host words as well, and fetch_tokens only waits for the stream
+    // the batch's pinned host words as well, and fetch_tokens copies nothing.  `patched`: the penalised values at the window
+    // ids go to pinned host memory instead of into the logits.
     int32_t* tokens_host = (mirror && b->h_tokens_dev) ? b->h_tokens_dev : nullptr;
     uint32_t* status_host = tokens_host ? reinterpret_cast<uint32_t*>(tokens_host + b->cap_rows) : nullptr;
-    if (tokens_host) b->h_tokens[b->cap_rows] = 0;
+    if (tokens_host) {
+        b->h_tokens[b->cap_rows] = 0;
+        std::fill(b->h_tokens, b->h_tokens + b->n_rows, kNoToken);
+    }
     b->mirrored = tokens_host != nullptr;
     if (shard_out && b->n_full > 0)
         return fail(h, FSB_ERR_RANGE, "rows whose candidate count exceeds %d (top_k = 0 or large) cannot be sharded by vocabulary", fsb::kMaxK);
@@ -301,7 +307,7 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
             FSB_CUDA(h, cudaStreamWaitEvent(h->side, h->ev_fork, 0));
             where = h->side;
         }
-        const int e = fsb::launch_full_row_kernel(logits_dev, b->d_rows() + b->n_cand, b->n_full, hist, h->d_pool, b->d_tokens, tokens_host,
+        const int e = fsb::launch_full_row_kernel(logits_dev, b->d_rows() + b->n_cand, b->n_full, hist, b->d_hist(), h->d_pool, b->d_tokens, tokens_host,
                                                   h->d_kept_ids, h->d_kept_pr, h->d_kept_n, keep_kept ? 1 : 0, b->d_status(), status_host, b->n_vocab, h->vocab_offset,
                                                   (b->flags & FSB_WRITE_BACK) ? 1 : 0, h->softcap, h->d_trace ? h->d_trace + 4096 * 8 : nullptr, where);
         if (e != 0) return fail(h, FSB_ERR_CUDA, "full-row kernel launch: %s", cudaGetErrorString((cudaError_t)e));
@@ -313,6 +319,8 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.logits = logits_dev;
         a.rows = b->d_rows();
         a.hist = hist;
+        a.drafts = b->d_hist();
+        a.patched = patched ? b->h_patched_dev : nullptr;
         a.pool = h->d_pool;
         a.tokens = b->d_tokens;
         a.status = b->d_status();
@@ -333,11 +341,12 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.kmax = b->kmax;
         a.all_greedy = b->all_greedy ? 1 : 0;
         a.penalised = b->penalised ? 1 : 0;
-        a.write_back = (b->flags & FSB_WRITE_BACK) ? 1 : 0;
+        a.write_back = (b->flags & FSB_WRITE_BACK) && !patched ? 1 : 0;
         a.vocab_offset = h->vocab_offset;
         a.softcap = h->softcap;
         a.overlap = h->launch_overlap;
-        const int e = fsb::launch_stream_kernel(a, b->h_rows(), h->stream);
+        const int e = fsb::launch_stream_kernel(a, b->h_rows(), b->sent_with_launch ? b->h_hist() : nullptr, b->sent_with_launch ? (int)b->hist_ids : 0,
+                                                b->hist_dev == nullptr, h->stream);
         if (e != 0) return fail(h, FSB_ERR_CUDA, "stream kernel launch: %s", cudaGetErrorString((cudaError_t)e));
         h->counters.kernel_launches++;
     }
@@ -347,13 +356,48 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
     return FSB_OK;
 }
 
-// Tokens and the status word behind them in one copy; `extra` floats of gathered window values in a second one.
-int fetch_tokens(fsb_handle* h, fsb_batch* b, int32_t* tokens_out, int64_t patched = 0) {
-    if (!b->mirrored)
-        FSB_CUDA(h, cudaMemcpyAsync(b->h_tokens, b->d_tokens, sizeof(int32_t) * ((size_t)b->cap_rows + 1), cudaMemcpyDeviceToHost, h->stream));
-    if (patched > 0) FSB_CUDA(h, cudaMemcpyAsync(b->h_patched, b->d_patched, sizeof(float) * (size_t)patched, cudaMemcpyDeviceToHost, h->stream));
-    FSB_CUDA(h, cudaStreamSynchronize(h->stream));
+// Waits until the kernels have stored something else than `none` into a word of pinned memory: it crosses PCIe about 3 us
+// before the stream reports the kernel complete.  Looks at the stream now and then, so that an error ends the wait; `done`
+// says that the stream was seen complete (a word that is still untouched then stays so).
+int poll_word(fsb_handle* h, const volatile int32_t* w, int32_t none, bool& done) {
+    for (unsigned spins = 1; *w == none; ++spins) {
+        if (done) return FSB_OK;
+        if (spins % 1024u == 0) {
+            const cudaError_t e = cudaStreamQuery(h->stream);
+            if (e == cudaSuccess) done = true;
+            else if (e != cudaErrorNotReady) return fail(h, FSB_ERR_CUDA, "waiting for results: %s", cudaGetErrorString(e));
+        }
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
+    }
+    return FSB_OK;
+}
+int poll_words(fsb_handle* h, const volatile int32_t* t, int n, int stride) {
+    bool done = false;
+    for (int i = 0; i < n; ++i) {
+        const int rc = poll_word(h, t + (size_t)i * stride, kNoToken, done);
+        if (rc) return rc;
+        if (t[(size_t)i * stride] == kNoToken) return fail(h, FSB_ERR_DEVICE, "no result for row %d", i);
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return FSB_OK;
+}
+
+// Brings the tokens (and `gathered` window values) to the caller and checks the status word.  `tokens_only`: nothing but the
+// mirrored tokens is waited for - the sampling kernels were the last of the call and left nothing else to be read.
+int fetch_tokens(fsb_handle* h, fsb_batch* b, int32_t* tokens_out, int64_t gathered = 0, bool tokens_only = false) {
+    if (b->mirrored && tokens_only) {
+        const int rc = poll_words(h, b->h_tokens, b->n_rows, 1);
+        if (rc) return rc;
+    } else {
+        if (!b->mirrored)
+            FSB_CUDA(h, cudaMemcpyAsync(b->h_tokens, b->d_tokens, sizeof(int32_t) * ((size_t)b->cap_rows + 1), cudaMemcpyDeviceToHost, h->stream));
+        if (gathered > 0) FSB_CUDA(h, cudaMemcpyAsync(b->h_patched, b->d_patched, sizeof(float) * (size_t)gathered, cudaMemcpyDeviceToHost, h->stream));
+        FSB_CUDA(h, cudaStreamSynchronize(h->stream));
+    }
     unsigned st = (unsigned)b->h_tokens[b->cap_rows];
+    if (st != 0u) cudaStreamSynchronize(h->stream);
     if (st != 0u && b->mirrored) {   // the mirror only says "something": the device word has the bits
         uint32_t word = 0;
         if (cudaMemcpy(&word, b->d_status(), sizeof word, cudaMemcpyDeviceToHost) == cudaSuccess && word != 0u) st = word;
@@ -421,9 +465,18 @@ int sync_history(fsb_handle* h, Stream* s) {
     if (n <= s->dev_len) return FSB_OK;
     const int rc = ensure_region(h, s, n);
     if (rc) return rc;
-    FSB_CUDA(h, cudaMemcpyAsync(h->d_pool + s->pool_off + s->dev_len, s->hist.data() + s->dev_len, sizeof(int32_t) * (size_t)(n - s->dev_len),
-                                cudaMemcpyHostToDevice, h->stream));
-    FSB_CUDA(h, cudaStreamSynchronize(h->stream));   // the source is pageable host memory that may change after return
+    const size_t count = (size_t)(n - s->dev_len);
+    const int32_t* src = s->hist.data() + s->dev_len;
+    if (count <= kIdRing) {   // through the pinned ring: nothing to wait for until it comes round again
+        if (h->h_ids_pos + count > kIdRing) {
+            FSB_CUDA(h, cudaStreamSynchronize(h->stream));
+            h->h_ids_pos = 0;
+        }
+        src = static_cast<const int32_t*>(std::memcpy(h->h_ids + h->h_ids_pos, src, sizeof(int32_t) * count));
+        h->h_ids_pos += count;
+    }
+    FSB_CUDA(h, cudaMemcpyAsync(h->d_pool + s->pool_off + s->dev_len, src, sizeof(int32_t) * count, cudaMemcpyHostToDevice, h->stream));
+    if (count > kIdRing) FSB_CUDA(h, cudaStreamSynchronize(h->stream));   // the source is pageable host memory that may change after return
     s->dev_len = n;
     return FSB_OK;
 }
@@ -506,6 +559,18 @@ int stage_host_logits(fsb_handle* h, const float* logits, int n_rows, int64_t ld
     if (elems > h->logits_stage_elems)
         return fail(h, FSB_ERR_CAPACITY, "host logits of %zu values (row stride %lld) exceed the engine's staging area of %zu", elems, (long long)ld,
                     h->logits_stage_elems);
+    if (elems <= kHostLogits) {
+        // A row or a few: through pinned memory in pieces, so that the copy engine works on one while the next is put there.
+        // (256 KB of pageable memory through one cudaMemcpyAsync take 25 us; nothing reads a piece after the call has returned.)
+        constexpr size_t kPiece = 32 * 1024;
+        for (size_t at = 0; at < elems; at += kPiece) {
+            const size_t n = std::min(kPiece, elems - at);
+            std::memcpy(h->h_logits + at, logits + at, n * sizeof(float));
+            FSB_CUDA(h, cudaMemcpyAsync(h->d_logits_stage + at, h->h_logits + at, n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+        }
+        *dev = h->d_logits_stage;
+        return FSB_OK;
+    }
     FSB_CUDA(h, cudaMemcpyAsync(h->d_logits_stage, logits, elems * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     *dev = h->d_logits_stage;
     return FSB_OK;
@@ -522,37 +587,48 @@ int launch_gather(fsb_handle* h, fsb_batch* b, const float* logits_dev) {
     h->counters.kernel_launches++;
     return FSB_OK;
 }
-void scatter_patched(const fsb_handle* h, const fsb_batch* b, float* logits_host, const int32_t* ids, int64_t n, int row, int gather_off) {
+int scatter_patched(fsb_handle* h, const fsb_batch* b, float* logits_host, const int32_t* ids, int64_t n, int row, int gather_off) {
     float* rowp = logits_host + (int64_t)row * b->ld;
+    const volatile int32_t* from = reinterpret_cast<const volatile int32_t*>(b->h_patched) + gather_off;
+    bool done = false;
     for (int64_t i = 0; i < n; ++i) {
         const int64_t c = (int64_t)ids[i] - h->vocab_offset;
-        if (c >= 0 && c < b->n_vocab) rowp[c] = b->h_patched[gather_off + i];
+        if (c < 0 || c >= b->n_vocab) continue;
+        const int rc = poll_word(h, from + i, kNoValue, done);   // (the kernels store every one of these)
+        if (rc) return rc;
+        const int32_t bits = from[i];
+        std::memcpy(rowp + c, &bits, sizeof bits);
     }
+    return FSB_OK;
 }
 
 // The common tail of the synchronous calls: upload, (stage host logits), launch, fetch, (write back to host).
-// `window_streams` > 0: a resident verification call - the drafts go into the id pool before the launch, and the last
-// accepted token of every stream after it (see verify_windows_impl).
-int run_staged(fsb_handle* h, fsb_batch* b, const float* logits, unsigned flags, int32_t* tokens_out, int window_streams = 0, bool window_append = false) {
+// `window_append` > 0: a resident verification call of that many streams whose accepted tokens are stored behind the
+// histories (see verify_windows_impl).
+int run_staged(fsb_handle* h, fsb_batch* b, const float* logits, unsigned flags, int32_t* tokens_out, int window_append = 0) {
     const bool on_host = (flags & FSB_LOGITS_ON_HOST) != 0;
     const bool host_wb = on_host && (flags & FSB_WRITE_BACK) && b->gather_ids > 0;
-    int rc = upload_batch(h, b, window_streams == 0 && !host_wb);
+    // the streaming kernel hands the penalised values over itself; rows of the full-vocabulary kernel have theirs gathered
+    const bool patched = host_wb && b->n_full == 0 && b->h_patched_dev;
+    const bool keep = (flags & FSB_KEEP_KEPT_SET) != 0;
     const float* dev = logits;
-    if (rc == FSB_OK && on_host) rc = stage_host_logits(h, logits, b->n_rows, b->ld, b->n_vocab, &dev);
-    if (rc == FSB_OK && window_streams > 0) {
-        const int e = fsb::launch_write_drafts(b->d_rows(), b->n_rows, h->d_pool, h->stream);
-        if (e != 0) rc = fail(h, FSB_ERR_CUDA, "draft kernel launch: %s", cudaGetErrorString((cudaError_t)e));
-        else h->counters.kernel_launches++;
-    }
-    if (rc == FSB_OK) rc = launch_batch(h, b, dev, (flags & FSB_KEEP_KEPT_SET) != 0, nullptr, nullptr, fsb::kMaxK, true);
-    if (rc == FSB_OK && window_streams > 0 && window_append) {
-        const int e = fsb::launch_accept_windows(b->d_hist() + b->hist_ids, window_streams, b->d_tokens, h->d_pool, h->stream);
+    int rc = FSB_OK;
+    if (on_host) rc = stage_host_logits(h, logits, b->n_rows, b->ld, b->n_vocab, &dev);
+    if (rc == FSB_OK) rc = upload_batch(h, b, false, host_wb && !patched);
+    if (patched) std::fill_n(reinterpret_cast<int32_t*>(b->h_patched), (size_t)b->gather_ids, kNoValue);
+    if (rc == FSB_OK) rc = launch_batch(h, b, dev, keep, nullptr, nullptr, fsb::kMaxK, true, patched);
+    if (rc == FSB_OK && window_append > 0) {
+        const int e = fsb::launch_accept_windows(b->d_hist() + b->hist_ids, window_append, b->d_tokens, h->d_pool, h->stream);
         if (e != 0) rc = fail(h, FSB_ERR_CUDA, "accept kernel launch: %s", cudaGetErrorString((cudaError_t)e));
         else h->counters.kernel_launches++;
     }
-    if (rc == FSB_OK && host_wb) rc = launch_gather(h, b, dev);
-    if (rc == FSB_OK) rc = fetch_tokens(h, b, tokens_out, host_wb ? b->gather_ids : 0);
-    if (rc) rollback_draws(h, b);
+    if (rc == FSB_OK && host_wb && !patched) rc = launch_gather(h, b, dev);
+    const bool tokens_only = !keep && window_append == 0 && (patched || !(flags & FSB_WRITE_BACK));
+    if (rc == FSB_OK) rc = fetch_tokens(h, b, tokens_out, host_wb && !patched ? b->gather_ids : 0, tokens_only);
+    if (rc) {
+        cudaStreamSynchronize(h->stream);   // nothing of this call may still write into the host's words
+        rollback_draws(h, b);
+    }
     return rc;
 }
 
@@ -631,9 +707,11 @@ int fsb_create(int device, int max_rows, int max_vocab, int64_t max_hist_ids, fs
         cudaMalloc(reinterpret_cast<void**>(&h->d_pool), sizeof(int32_t) * (size_t)std::max<int64_t>(max_hist_ids, 1)) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&h->d_logits_stage), sizeof(float) * h->logits_stage_elems) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&h->d_lookup), sizeof(fsb::LookupDesc) * (size_t)max_rows) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&h->d_drafts), sizeof(int32_t) * (size_t)max_rows * fsb::kDraftStride) != cudaSuccess ||
         cudaMallocHost(reinterpret_cast<void**>(&h->h_lookup), sizeof(fsb::LookupDesc) * (size_t)max_rows) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void**>(&h->h_drafts), sizeof(int32_t) * (size_t)max_rows * fsb::kDraftStride) != cudaSuccess)
+        cudaMallocHost(reinterpret_cast<void**>(&h->h_ids), sizeof(int32_t) * kIdRing) != cudaSuccess ||
+        cudaMallocHost(reinterpret_cast<void**>(&h->h_logits), sizeof(float) * std::min(kHostLogits, h->logits_stage_elems)) != cudaSuccess ||
+        cudaMallocHost(reinterpret_cast<void**>(&h->h_drafts), sizeof(int32_t) * (size_t)max_rows * fsb::kDraftStride) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void**>(&h->h_drafts_dev), h->h_drafts, 0) != cudaSuccess)
         return bail(FSB_ERR_CUDA);
     if (alloc_batch(h, max_rows, max_hist_ids, std::max<int64_t>(max_hist_ids, 1), &h->own) != FSB_OK) return bail(FSB_ERR_CUDA);
     *out = h;
@@ -654,9 +732,10 @@ int fsb_destroy(fsb_handle* h) {
     if (h->d_pool) cudaFree(h->d_pool);
     if (h->d_logits_stage) cudaFree(h->d_logits_stage);
     if (h->d_lookup) cudaFree(h->d_lookup);
-    if (h->d_drafts) cudaFree(h->d_drafts);
     if (h->h_lookup) cudaFreeHost(h->h_lookup);
     if (h->h_drafts) cudaFreeHost(h->h_drafts);
+    if (h->h_ids) cudaFreeHost(h->h_ids);
+    if (h->h_logits) cudaFreeHost(h->h_logits);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -787,7 +866,8 @@ static int sample_batch_impl(fsb_handle* h, int n_rows, const int* stream_ids, c
     if ((flags & FSB_LOGITS_ON_HOST) && (flags & FSB_WRITE_BACK)) {
         for (int i = 0; i < n_rows; ++i) {
             const fsb::RowDesc& d = b->descs[(size_t)i];
-            scatter_patched(h, b, const_cast<float*>(logits), b->h_hist() + d.hist_begin, d.hist_len, i, d.gather_off);
+            rc = scatter_patched(h, b, const_cast<float*>(logits), b->h_hist() + d.hist_begin, d.hist_len, i, d.gather_off);
+            if (rc) return rc;
         }
     }
     count_rows(h, b);
@@ -843,16 +923,22 @@ int fsb_lookup_drafts_resident(fsb_handle* h, int n_streams, const int* stream_i
         d.min_n = min_n[i];
         d.eos = eos;
     }
-    FSB_CUDA(h, cudaMemcpyAsync(h->d_lookup, h->h_lookup, sizeof(fsb::LookupDesc) * (size_t)n_streams, cudaMemcpyHostToDevice, h->stream));
-    const int e = fsb::launch_lookup_drafts(h->d_pool, h->d_lookup, n_streams, h->d_drafts, fsb::kDraftStride, h->stream);
+    if (n_streams > fsb::kLookupArgs)   // more descriptors than go with the launch
+        FSB_CUDA(h, cudaMemcpyAsync(h->d_lookup, h->h_lookup, sizeof(fsb::LookupDesc) * (size_t)n_streams, cudaMemcpyHostToDevice, h->stream));
+    std::fill_n(h->h_drafts, (size_t)n_streams * fsb::kDraftStride, kNoToken);
+    const int e = fsb::launch_lookup_drafts(h->d_pool, h->h_lookup, h->d_lookup, n_streams, h->h_drafts_dev, fsb::kDraftStride, h->stream);
     if (e != 0) return fail(h, FSB_ERR_CUDA, "draft kernel launch: %s", cudaGetErrorString((cudaError_t)e));
     h->counters.kernel_launches++;
-    FSB_CUDA(h, cudaMemcpyAsync(h->h_drafts, h->d_drafts, sizeof(int32_t) * (size_t)n_streams * fsb::kDraftStride, cudaMemcpyDeviceToHost, h->stream));
-    FSB_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (int i = 0; i < n_streams; ++i) {
+    int rc = poll_words(h, h->h_drafts, n_streams, fsb::kDraftStride);
+    for (int i = 0; i < n_streams && rc == FSB_OK; ++i) {
         const int32_t* src = h->h_drafts + (size_t)i * fsb::kDraftStride;
         n_out[i] = src[0];
-        for (int k = 0; k < src[0]; ++k) drafts_out[(size_t)i * stride + k] = src[1 + k];
+        rc = poll_words(h, src + 1, src[0], 1);
+        for (int k = 0; k < src[0] && rc == FSB_OK; ++k) drafts_out[(size_t)i * stride + k] = src[1 + k];
+    }
+    if (rc) {
+        cudaStreamSynchronize(h->stream);
+        return rc;
     }
     return FSB_OK;
 }
@@ -932,7 +1018,8 @@ int fsb_sample_batch_resident(fsb_handle* h, int n_rows, const int* stream_ids, 
         Stream* s = get_stream(h, stream_ids[i]);
         if (host_wb) {
             const fsb::RowDesc& d = b->descs[(size_t)i];
-            scatter_patched(h, b, const_cast<float*>(logits), s->hist.data() + (s->hist.size() - (size_t)d.hist_len), d.hist_len, i, d.gather_off);
+            rc = scatter_patched(h, b, const_cast<float*>(logits), s->hist.data() + (s->hist.size() - (size_t)d.hist_len), d.hist_len, i, d.gather_off);
+            if (rc) return rc;
         }
         if (append) {   // the device copy already holds the token
             s->hist.push_back(tokens_out[i]);
@@ -978,12 +1065,11 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
     if (need > b->cap_hist) return fail(h, FSB_ERR_CAPACITY, "%lld penalty-window ids exceed the capacity of %lld", (long long)need,
                                         (long long)b->cap_hist);
     if (resident) {
-        // The drafts of a window go behind the stream's history in its region of the id pool (they are what the history
-        // will hold if they are accepted), so that row r's window is a range of the pool like any other: make room.
+        // Accepted tokens go behind the stream's history in its region of the id pool: make room.
         for (int i = 0; i < n_streams; ++i) {
             Stream* s = get_stream(h, stream_ids[i]);
             rc = sync_history(h, s);
-            if (rc == FSB_OK) rc = ensure_region(h, s, (int64_t)s->hist.size() + (row_off[i + 1] - row_off[i]));
+            if (rc == FSB_OK && (flags & FSB_APPEND_SAMPLED)) rc = ensure_region(h, s, (int64_t)s->hist.size() + (row_off[i + 1] - row_off[i]));
             if (rc) return rc;
         }
     }
@@ -1004,33 +1090,45 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
         const int64_t len = resident ? (int64_t)s->hist.size() : hist->len(i);
         const bool pen_on = !(s->p.repetition_penalty == 1.0f || s->p.repeat_last_n == 0);
         // row r samples with history_i followed by draft_1..draft_r; the windows of successive rows only move
-        // forward, so one copy [b_0 .. len + m - 1) serves the whole stream: staged here, or the stream's pool region
+        // forward, so one copy [b_0 .. len + m - 1) serves the whole stream: staged here, or the stream's pool region and
+        // the drafts staged here
         const int64_t b0 = pen_on ? window_begin(s->p, len) : len;
         int64_t base = pos;
+        const int64_t drafts_at = pos;
         if (resident) {
-            base = s->pool_off + b0;
+            base = s->pool_off >= 0 ? s->pool_off : 0;
+            if (pen_on)
+                for (int r = 1; r < m; ++r) hs[pos++] = rows_flat[r0 + r];
         } else if (pen_on) {
             if (len > b0) std::memcpy(hs + pos, hist->data(i) + b0, sizeof(int32_t) * (size_t)(len - b0));
             pos += len - b0;
             for (int r = 1; r < m; ++r) hs[pos++] = rows_flat[r0 + r];
         }
-        std::mt19937_64 look = s->rng;   // draws are taken from a copy; the real engine advances by acc afterwards
         const bool greedy = is_greedy(s->p);
+        std::optional<std::mt19937_64> look;   // draws are taken from a copy; the real engine advances by acc afterwards
+        if (!greedy) look.emplace(s->rng);
         for (int r = 0; r < m; ++r) {
-            int64_t hb = 0, hl = 0;
+            int64_t hb = 0, hl = 0, db = 0, dl = 0;   // the window: a range of the history, then one of the staged drafts (resident)
             if (pen_on) {
                 const int64_t len_r = len + r;
                 const int64_t br = window_begin(s->p, len_r);
-                hb = base + (br - b0);
-                hl = len_r - br;
+                if (resident) {
+                    hb = base + std::min(br, len);
+                    hl = std::max<int64_t>(0, len - br);
+                    db = drafts_at + std::max<int64_t>(0, br - len);
+                    dl = len_r - br - hl;
+                } else {
+                    hb = base + (br - b0);
+                    hl = len_r - br;
+                }
             }
-            const uint64_t word = greedy ? 0ull : look();
+            const uint64_t word = greedy ? 0ull : (*look)();
             b->sid[(size_t)(r0 + r)] = stream_ids[i];
             fsb::RowDesc& d = b->descs[(size_t)(r0 + r)];
             fill_desc(h, d, s->p, n_vocab, (int64_t)(r0 + r) * ld, hb, hl, word, r0 + r);
-            if (resident && r >= 1 && hl >= 1) {   // draft_r is the last id of row r's window: a kernel puts it there before the launch
-                d.flags |= fsb::kRowDraft;
-                d.gather_off = rows_flat[r0 + r];
+            if (dl > 0) {
+                d.flags |= fsb::kRowPenalty | ((int32_t)dl << fsb::kRowDraftShift);
+                d.draft_off = (int32_t)db;
             }
         }
     }
@@ -1039,8 +1137,7 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
     const bool win_append = resident && (flags & FSB_APPEND_SAMPLED);
     if (win_append) {
         // per stream: first row, rows, accept limit, and where the stream's history ends in the id pool; the device walks
-        // the same accept loop as the host below and stores the last accepted token there (the confirmed drafts before
-        // it are in place already)
+        // the same accept loop as the host below and stores the accepted tokens there
         int32_t* tab = hs + pos;
         for (int i = 0; i < n_streams; ++i) {
             Stream* s = get_stream(h, stream_ids[i]);
@@ -1059,7 +1156,7 @@ static int verify_windows_impl(fsb_handle* h, int n_streams, const int* stream_i
     }
     rc = finalize_batch(h, b);
     if (rc) return rc;
-    rc = run_staged(h, b, logits, flags & ~FSB_APPEND_SAMPLED, nullptr, resident ? n_streams : 0, win_append);   // no engine was advanced: nothing to roll back
+    rc = run_staged(h, b, logits, flags & ~FSB_APPEND_SAMPLED, nullptr, win_append ? n_streams : 0);   // no engine was advanced: nothing to roll back
     if (rc) return rc;
     // accept loop of src/server.cpp:626-636 on the sampled tokens
     for (int i = 0; i < n_streams; ++i) {
@@ -1152,7 +1249,7 @@ int fsb_batch_prepare(fsb_handle* h, int n_rows, const int* stream_ids, int64_t 
     if (rc) return rc;
     rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, HistSource{hist_flat, hist_off, nullptr, nullptr}, flags);
     if (rc == FSB_OK) {
-        rc = upload_batch(h, b);
+        rc = upload_batch(h, b, true, true);
         if (rc == FSB_OK && cudaStreamSynchronize(h->stream) != cudaSuccess) rc = fail(h, FSB_ERR_CUDA, "upload failed");
         if (rc) rollback_draws(h, b);
     }

@@ -68,8 +68,9 @@ struct Geometry {
 struct Segment {
     const float* row;          // the row's logits
     unsigned* bitmap;          // penalised columns (bit 0 = column bit0), valid when has_pen
-    const int32_t* hist;       // the penalty window
-    int hist_len;
+    const int32_t* hist;       // the penalty window: these ids ...
+    const int32_t* drafts;     // ... then these
+    int hist_len, window_len;  // ids in the first part, in both
     int lo, hi;                // columns
     int bit0;
     int id_base;               // token id of column 0
@@ -77,6 +78,7 @@ struct Segment {
     float pen, cap;
 };
 
+__device__ __forceinline__ int window_id(const Segment& s, int i) { return i < s.hist_len ? s.hist[i] : s.drafts[i - s.hist_len]; }
 __device__ __forceinline__ float penalise(float x, float pen) { return x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen); }   // src/sampler.cpp:17
 __device__ __noinline__ float softcap_call(float x, float cap) { return __fmul_rn(cap, tanhf(__fdiv_rn(x, cap))); }          // src/model_gemma4.cpp:521
 __device__ __forceinline__ bool penalised(const Segment& s, int c) { return s.has_pen && ((s.bitmap[(c - s.bit0) >> 5] >> ((c - s.bit0) & 31)) & 1u); }
@@ -283,8 +285,8 @@ __device__ __noinline__ void write_back(const Segment s) {
         for (int c = s.lo + threadIdx.x; c < s.hi; c += T) row[c] = transform(__ldcg(row + c), c, s);
         return;
     }
-    for (int i = threadIdx.x; i < s.hist_len; i += T) {
-        const int c = s.hist[i] - s.id_base;
+    for (int i = threadIdx.x; i < s.window_len; i += T) {
+        const int c = window_id(s, i) - s.id_base;
         if (c < s.lo || c >= s.hi) continue;
         const unsigned bit = 1u << ((c - s.bit0) & 31);   // an id counts once however often it occurs in the window
         if (atomicAnd(&s.bitmap[(c - s.bit0) >> 5], ~bit) & bit) row[c] = penalise(__ldcg(row + c), s.pen);
@@ -324,8 +326,8 @@ __device__ __forceinline__ Segment make_segment(const StreamArgs& a, const RowSp
     Segment s;
     s.row = row_ptr;
     s.bitmap = bitmap;
-    s.hist = nullptr;
-    s.hist_len = 0;
+    s.hist = s.drafts = nullptr;
+    s.hist_len = s.window_len = 0;
     s.lo = seg == 0 ? 0 : w.head + 4 * w.c_lo;
     s.hi = seg == nseg - 1 ? a.n_vocab : w.head + 4 * w.c_hi;
     s.bit0 = w.head + 4 * w.c_lo - 32;
@@ -336,20 +338,27 @@ __device__ __forceinline__ Segment make_segment(const StreamArgs& a, const RowSp
     return s;
 }
 
+__device__ __forceinline__ void set_window(Segment& s, const int32_t* hist, const int32_t* drafts, const RowDesc& d) {
+    s.hist = hist + d.hist_begin;
+    s.hist_len = d.hist_len;
+    s.drafts = drafts + d.draft_off;
+    s.window_len = d.hist_len + (d.flags >> kRowDraftShift);
+}
+
 // The window's columns of the segment: sets their bits, and lists each once - an id counts once however often it occurs -
 // with its logit, which is fetched now (the copies belong to the next group that the thread commits) and needed at the end.
 // All threads call; a barrier has to follow.
 template <int T>
 __device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* ctl, float* pen_raw, int* pen_col) {
     const int tid = threadIdx.x, lane = tid & 31;
-    int id = tid < s.hist_len ? s.hist[tid] : -1;
+    int id = tid < s.window_len ? window_id(s, tid) : -1;
     for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    for (int i0 = tid & ~31; i0 < s.hist_len; i0 += T) {
-        const int next = i0 + T + lane < s.hist_len ? s.hist[i0 + T + lane] : -1;
+    for (int i0 = tid & ~31; i0 < s.window_len; i0 += T) {
+        const int next = i0 + T + lane < s.window_len ? window_id(s, i0 + T + lane) : -1;
         const int c = id - s.id_base;
         bool first = false;
-        if (i0 + lane < s.hist_len && c >= s.lo && c < s.hi) {
+        if (i0 + lane < s.window_len && c >= s.lo && c < s.hi) {
             const unsigned bit = 1u << ((c - s.bit0) & 31);
             first = (atomicOr(&s.bitmap[(c - s.bit0) >> 5], bit) & bit) == 0u;
         }
@@ -420,6 +429,16 @@ __device__ __forceinline__ void finish_row(const StreamArgs& a, const RowDesc& d
     row_epilogue(out, kk, rt, work, ctl, tout);
 }
 
+// For callers whose logits live in host memory: the penalised values at the window's ids, in window order, go straight to
+// pinned host memory, where the host waits for every one and stores it into its row (src/sampler.cpp:17); it computes nothing.
+template <int T>
+__device__ __noinline__ void send_patched(const Segment s, float* out) {
+    for (int i = threadIdx.x; i < s.window_len; i += T) {
+        const int c = window_id(s, i) - s.id_base;
+        if (c >= s.lo && c < s.hi) *reinterpret_cast<volatile float*>(out + i) = transform(__ldcg(s.row + c), c, s);
+    }
+}
+
 __device__ __forceinline__ void trace_mark(const StreamArgs& a, int slot) {
     if (a.trace && threadIdx.x == 0 && blockIdx.x < 4096u) {
         a.trace[(size_t)blockIdx.x * 8 + slot] = slot == 0 ? global_timer_ns() : (u64)clock64();
@@ -443,12 +462,17 @@ __device__ __forceinline__ int warp_reserve(const float (&v)[N], float bound, un
     return __shfl_sync(0xffffffffu, p, 0);
 }
 
-// A launch's arguments: with NDESC > 0 the row descriptors come with them (a batch of few rows needs no copy to the
-// device before the launch, and no CTA waits for a read of global memory before it knows its row).
+// A launch's arguments: with NDESC > 0 the row descriptors come with them - no CTA waits for a read of global memory before
+// it knows its row - and with few rows the staged window ids, too, if they are few: such a batch needs no copy to the device.
+// (4 KB of arguments cost 0.6 us, reading 256 ids from them 0.2; 1000 ids would take 1.3, more than a copy.)
+constexpr int kFewRows = 8, kArgRows = 64, kArgIds = 256;
 template <int NDESC>
 struct SelectArgs {
     StreamArgs a;
     RowDesc rows[NDESC > 0 ? NDESC : 1];
+    int32_t ids[NDESC == kFewRows ? kArgIds : 1];
+    __device__ __forceinline__ const int32_t* hist() const { return NDESC == kFewRows && !a.hist ? ids : a.hist; }
+    __device__ __forceinline__ const int32_t* drafts() const { return NDESC == kFewRows && !a.drafts ? ids : a.drafts; }
 };
 
 template <int T, int NDESC>
@@ -515,8 +539,7 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     }
     if (nseg > 1) cluster_arrive_release();   // (waited for before the first store to another CTA's shared memory)
     if (s.has_pen) {
-        s.hist = a.hist + dp.hist_begin;
-        s.hist_len = dp.hist_len;
+        set_window(s, args.hist(), args.drafts(), dp);
         collect_penalised<T>(s, ctl, pen_raw, pen_col);
     }
     __syncthreads();
@@ -651,6 +674,7 @@ again_from_the_start:
     if (lost || (n < k && (bounded || s.cap != 0.0f))) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
     else if (n < k) n = append_masked<T>(s, n, k, picked, reinterpret_cast<unsigned*>(list));
     if (a.write_back) write_back<T>(s);
+    if (a.patched && s.has_pen) send_patched<T>(s, a.patched + dp.gather_off);
     trace_mark(a, 2);
     if (a.trace && tid == 0 && blockIdx.x < 4096u) a.trace[(size_t)blockIdx.x * 8 + 3] = (u64)n;
     if (a.overlap == 1) pdl_wait_prior();   // from here on this launch writes what the previous launch in the stream may still be using
@@ -713,7 +737,7 @@ again_from_the_start:
 // Launches whose rows are all greedy (a verification step at temperature 0, the static entry point): the same stream, but
 // a thread keeps the best cell it has seen in registers ("strictly larger" keeps the first of equals, because a thread
 // meets its cells in ascending order), the CTA takes the largest composite, and one warp finishes the row.  No bound, no
-// lists, no barrier before the end.  (Not with a softcap, which makes different logits equal, nor with write-back.)
+// lists, no barrier before the end.  (Not with a softcap, which makes different logits equal, nor with write-back or patched values for the host.)
 template <int T>
 size_t argmax_smem_bytes(int seg_cols) {
     return Geometry<T>::kRingBytes + sizeof(SharedCtl) + (seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0);
@@ -762,8 +786,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         s.has_pen = (dp.flags & kRowPenalty) != 0;
         s.pen = dp.penalty;
         if (s.has_pen) {
-            s.hist = a.hist + dp.hist_begin;
-            s.hist_len = dp.hist_len;
+            set_window(s, args.hist(), args.drafts(), dp);
             if (tid == 0) ctl->pen_n = 0;
             collect_penalised<T>(s, ctl, pen_raw, pen_col);
         }
@@ -840,10 +863,8 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     trace_mark(a, 6);
 }
 
-constexpr int kFewRows = 8, kArgRows = 64;   // batches of up to this many rows send their descriptors with the launch
-
 template <int T, int NDESC>
-int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows) {
+int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows, const int32_t* ids, int n_ids) {
     const int seg_cols = a.penalised ? 4 * ((a.n_vocab / 4 + a.nseg - 1) / a.nseg) + 8 : 0;
     cfg.blockDim = dim3(T);
     cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols);
@@ -851,17 +872,18 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
     SelectArgs<NDESC> args;
     args.a = a;
     if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
-    if (a.all_greedy && a.softcap == 0.0f && !a.write_back) {
+    if (NDESC == kFewRows && n_ids > 0) std::memcpy(args.ids, ids, sizeof(int32_t) * (size_t)n_ids);
+    if (a.all_greedy && a.softcap == 0.0f && !a.write_back && !a.patched) {
         cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols);
         return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
     }
     return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC>, args);
 }
 template <int T>
-int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows) {
-    if (rows && a.n_rows <= kFewRows) return launch_select<T, kFewRows>(cfg, a, rows);
-    if (rows && a.n_rows <= kArgRows) return launch_select<T, kArgRows>(cfg, a, rows);
-    return launch_select<T, 0>(cfg, a, nullptr);
+int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows, const int32_t* ids, int n_ids) {
+    if (rows && a.n_rows <= kFewRows) return launch_select<T, kFewRows>(cfg, a, rows, ids, n_ids);
+    if (rows && a.n_rows <= kArgRows) return launch_select<T, kArgRows>(cfg, a, rows, nullptr, 0);
+    return launch_select<T, 0>(cfg, a, nullptr, nullptr, 0);
 }
 template <int T, int NDESC>
 int prepare_select() {
@@ -879,12 +901,20 @@ int prepare_device_kernels() {
     return 0;
 }
 
-int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* stream) {
+bool rows_fit_launch(int n_rows, int64_t n_ids) { return n_ids == 0 ? n_rows <= kArgRows : n_rows <= kFewRows && n_ids <= kArgIds; }
+
+int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* host_ids, int n_ids, bool ids_are_windows, void* stream) {
+    if (n_ids > 0) {   // the staged ids go with the launch: the windows themselves, or the drafts behind windows in the id pool
+        a.drafts = nullptr;
+        if (ids_are_windows) a.hist = nullptr;
+    }
     cudaLaunchAttribute attr[2];
     int n = 0;
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = a.overlap ? 1 : 0;
-    ++n;
+    if (a.overlap) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
     if (a.nseg > 1) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
         attr[n].val.clusterDim.x = (unsigned)a.nseg;
@@ -897,7 +927,7 @@ int launch_stream_kernel(const StreamArgs& a, const RowDesc* host_rows, void* st
     cfg.stream = static_cast<cudaStream_t>(stream);
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return a.wide ? launch_select<1024>(cfg, a, host_rows) : launch_select<256>(cfg, a, host_rows);
+    return a.wide ? launch_select<1024>(cfg, a, host_rows, host_ids, n_ids) : launch_select<256>(cfg, a, host_rows, host_ids, n_ids);
 }
 
 // How a launch is laid out.  Measured on B200, k = 40 to 64, us per call (small CTAs with 1 / 2 / 4 / 8 segments per row;
@@ -998,7 +1028,7 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
         const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms);
         a.nseg = pl.nseg;
         a.wide = pl.wide ? 1 : 0;
-        if (rc == FSB_OK && launch_stream_kernel(a, nullptr, st) != 0) rc = FSB_ERR_CUDA;
+        if (rc == FSB_OK && launch_stream_kernel(a, nullptr, nullptr, 0, false, st) != 0) rc = FSB_ERR_CUDA;
         if (rc == FSB_OK && (flags & FSB_STATIC_WAIT)) {
             uint32_t word = 0;
             if (cudaMemcpyAsync(&word, status, sizeof word, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) rc = FSB_ERR_CUDA;

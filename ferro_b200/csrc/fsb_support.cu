@@ -4,6 +4,8 @@
 // that lets a host caller see the penalised values without any host arithmetic.
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include "fsb_device.cuh"
 
 namespace fsb {
@@ -62,16 +64,10 @@ __global__ void gather_patched_kernel(const float* logits, const RowDesc* rows, 
     }
 }
 
-// Resident verification windows.  Before the launch: draft r of a stream is the last id of row r's window, and goes
-// to that place of the id pool.  After it: per stream the accept loop of src/server.cpp:630-636 over the sampled
-// tokens (accept while the token equals the next draft, at most `lim` rows), and the accepted tokens are stored
-// behind the history.  Table entry of a stream:
-// first row, rows m, limit, unused, end of the history in the pool (two words), then the m - 1 drafts.
-__global__ void write_drafts_kernel(const RowDesc* rows, int n_rows, int32_t* pool) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    if (rows[r].flags & kRowDraft) pool[rows[r].hist_begin + rows[r].hist_len - 1] = rows[r].gather_off;
-}
+// Resident verification windows, after the launch: per stream the accept loop of src/server.cpp:630-636 over the sampled
+// tokens (accept while the token equals the next draft, at most `lim` rows), and the accepted tokens are stored behind
+// the history.  Table entry of a stream: first row, rows m, limit, unused, end of the history in the pool (two words), then
+// the m - 1 drafts.
 __global__ void accept_windows_kernel(const int32_t* table, int n_streams, const int32_t* tokens, int32_t* pool) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_streams) return;
@@ -84,8 +80,6 @@ __global__ void accept_windows_kernel(const int32_t* table, int n_streams, const
         if (r + 1 < m && tokens[r0 + r] == t[6 + r]) continue;
         break;
     }
-    // every accepted token, not only the last: a row whose penalty window is empty (penalty off) never had its draft
-    // written into the pool before the launch
     for (int r = 0; r < acc; ++r) pool[end + r] = tokens[r0 + r];
 }
 
@@ -93,12 +87,16 @@ __global__ void accept_windows_kernel(const int32_t* table, int n_streams, const
 // the most recent earlier occurrence of the history's last n tokens, n = 4, 3, ... min_n - at most kmax of them, cut
 // at the end-of-sequence id; an occurrence whose continuation is empty is passed over.  One CTA per stream: every
 // thread tests some start positions of an n, the largest matching position wins, one thread copies the draft.
-// out[i * stride] = number of drafts of stream i, then the drafts.
-__global__ void lookup_drafts_kernel(const int32_t* pool, const LookupDesc* desc, int n_streams, int32_t* out, int stride) {
+// out[i * stride] = number of drafts of stream i, then the drafts; `out` is the caller's pinned memory, where the host
+// waits for the number and for every draft (a system-wide fence between the two would cost 7 us).
+struct LookupArgs {
+    LookupDesc d[kLookupArgs];
+};
+__global__ void lookup_drafts_kernel(const int32_t* pool, const __grid_constant__ LookupArgs args, const LookupDesc* desc, int n_streams, int32_t* out, int stride) {
     __shared__ int best;
     const int i = blockIdx.x;
     if (i >= n_streams) return;
-    const LookupDesc d = desc[i];
+    const LookupDesc d = desc ? desc[i] : args.d[i];
     const int32_t* h = pool + d.begin;
     const int L = d.len;
     int found_n = 0;
@@ -117,21 +115,28 @@ __global__ void lookup_drafts_kernel(const int32_t* pool, const LookupDesc* desc
         }
         __syncthreads();   // `best` is reset by thread 0 at the top of the next round
     }
-    if (threadIdx.x == 0) {
-        int cnt = 0;
-        if (found_n > 0)
-            for (int k = best + found_n; k < L && cnt < d.kmax && cnt < stride - 1; ++k) {
-                if (h[k] == d.eos) break;
-                out[(size_t)i * stride + 1 + cnt++] = h[k];
-            }
-        out[(size_t)i * stride] = cnt;
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x, most = found_n > 0 ? min(min(d.kmax, stride - 1), L - best - found_n) : 0;
+    volatile int32_t* to = out + (size_t)i * stride;
+    int cnt = 0;
+    for (int k0 = 0; k0 < most; k0 += 32) {
+        const int id = k0 + lane < most ? h[best + found_n + k0 + lane] : d.eos;
+        const unsigned stop = __ballot_sync(0xffffffffu, k0 + lane >= most || id == d.eos);
+        const int n = stop ? __ffs(stop) - 1 : 32;
+        if (lane < n) to[1 + k0 + lane] = id;
+        cnt = k0 + n;
+        if (n < 32) break;
     }
+    if (lane == 0) to[0] = cnt;
 }
 
 }  // namespace
 
-int launch_lookup_drafts(const int32_t* pool, const LookupDesc* desc, int n_streams, int32_t* out, int stride, void* stream) {
-    lookup_drafts_kernel<<<n_streams, 256, 0, static_cast<cudaStream_t>(stream)>>>(pool, desc, n_streams, out, stride);
+int launch_lookup_drafts(const int32_t* pool, const LookupDesc* host_desc, const LookupDesc* desc, int n_streams, int32_t* out, int stride, void* stream) {
+    LookupArgs args;
+    const bool sent = n_streams <= kLookupArgs;
+    if (sent) std::memcpy(args.d, host_desc, sizeof(LookupDesc) * (size_t)n_streams);
+    lookup_drafts_kernel<<<n_streams, 256, 0, static_cast<cudaStream_t>(stream)>>>(pool, args, sent ? nullptr : desc, n_streams, out, stride);
     return (int)cudaGetLastError();
 }
 
@@ -149,11 +154,6 @@ int launch_merge_lists(const void* lists, const int32_t* list_n, int n_lists, in
 int launch_gather_patched(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, int n_vocab, int vocab_offset, float* out,
                           void* stream) {
     gather_patched_kernel<<<n_rows, 128, 0, static_cast<cudaStream_t>(stream)>>>(logits, rows, n_rows, hist, n_vocab, vocab_offset, out);
-    return (int)cudaGetLastError();
-}
-
-int launch_write_drafts(const RowDesc* rows, int n_rows, int32_t* pool, void* stream) {
-    write_drafts_kernel<<<(n_rows + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(rows, n_rows, pool);
     return (int)cudaGetLastError();
 }
 
