@@ -2,22 +2,26 @@
 //
 // Rows whose effective candidate count k exceeds kMaxK - above all `top_k == 0`, where the reference sorts the
 // whole vocabulary (src/sampler.cpp:32-35 of paragontasx/ferro) - cannot keep their candidates in one CTA.  A
-// cluster of kFullCluster CTAs works on one such row.  Every CTA keeps its slice of the row in shared memory
+// cluster of eight (or four) CTAs works on one such row.  Every CTA keeps its slice of the row in shared memory
 // (softcap and penalty applied once, src/model_gemma4.cpp:521 and src/sampler.cpp:11-18), so the row is read from
 // HBM exactly once; everything after that reads shared memory:
 //   1. the row's largest and smallest candidate key                                            (src/sampler.cpp:38)
 //   2. if k < n: the k-th candidate, by a radix descent over the keys that counts                      (:27-31)
-//   3. the weights e_i = exp((double)(x_i - max) / T) of the candidates as 2^-62 fixed point, histogrammed by the
-//      leading digit of their keys; the sum of the histogram is the softmax denominator                    (:40-41)
-//   4. min-p bound (:43), top-p crossing (:44) and the draw (:45-49) by radix descents over accumulated weight.
-// A descent is MSB-first over 8-bit digits of the 64-bit candidate key.  At every level each CTA histograms the
-// candidates of its slice that match the prefix found so far (count and weight per digit), all CTAs of the
-// cluster read all histograms through distributed shared memory and walk the digits - each CTA does the same
-// integer arithmetic, so all arrive at the same digit without a broadcast - and the descent stops as soon as the
-// digit it lands on holds a single candidate.  Weights are recomputed from the values where they are needed
-// (the function is pure), never stored.  Sums of weights are integers, so they do not depend on the order in
-// which threads add: the result is deterministic and differs from the reference's sequential fp64 sums by
-// rounding only (~1e-13).
+//   3. one pass over the weights e_i = exp((double)(x_i - max) / T) as 2^-62 fixed point: their exact sum, the softmax
+//      denominator (:40-41), in registers, and a histogram of their upper 32 bits over kBins bins of equal width in the
+//      logit.  The cluster-wide cumulative histogram tells for any cumulative weight in which bin - or, because the
+//      lower bits are left out, in which few bins - it is reached.
+//   4. with top-p (:44) or min-p (:43): the bins that can hold kept candidates are known now.  Their candidates, tens to
+//      some hundreds as a rule, go to the first CTA, which orders them and does the rest of the row's work on the
+//      ordered list: exact cumulative weights, both cuts and the draw (:45-49).  Without a cut, or when there are too
+//      many, a cumulative weight is resolved on its own: exact weight above its bins, ordered candidates of its bins.
+// If even one bin's candidates do not fit the first CTA's list (thousands of equal logits), a radix descent over the
+// candidate keys resolves it: MSB-first over 8-bit digits, at every level each CTA histograms the candidates of its
+// slice that match the prefix, all CTAs read all histograms through distributed shared memory and walk the digits - the
+// same integer arithmetic everywhere, so no broadcast is needed - until a digit holds a single candidate.
+// Sums of weights are integers, so they do not depend on the order in which threads add: the result is deterministic
+// and differs from the reference's sequential fp64 sums by rounding only (~1e-13).
+// What bounds it: the fp64 exponentials (one per logit) and the chain of cluster-wide steps.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,8 +34,11 @@ namespace {
 constexpr int kFullThreads = 1024;
 constexpr int kFullWarps = kFullThreads / 32;
 static_assert(kFullWarps == 32, "the block reductions read one partial per lane");
-constexpr int kFullCluster = 8;                 // CTAs per row
-constexpr int kSliceCache = 32768;              // logits of a slice that are kept in shared memory (rows up to 8 x this)
+constexpr int kMaxCluster = 8;                  // most CTAs per row
+constexpr int kSliceCache = 32768;              // logits of a slice that are kept in shared memory
+constexpr int kBins = kFullThreads;             // a thread looks after one bin
+constexpr int kSendCap = 512;                   // candidates a CTA can hand to the first one
+constexpr int kShort = 256;                     // lists of up to this many candidates are ordered by counting
 constexpr int kStripes = 8;                     // copies of the level histogram (by warp): fewer warps hit one word at once
 constexpr int kLimbs = 4;                       // a weight is added to a histogram as four 16-bit limbs (32-bit native atomics)
 
@@ -96,19 +103,17 @@ __device__ __forceinline__ unsigned ld_cluster_u32(unsigned addr) {
 
 // ---- shared memory of a CTA -------------------------------------------------------------------------------------------
 struct FullShared {
-    // the level histogram being built (kStripes copies), then this CTA's sum of them, which the other CTAs read
-    // [stripe][limb 0..3, then the candidate count][digit], four words of padding between stripes: a limb sum stays
-    // below 2^32 while a stripe sees fewer than 65537 candidates, i.e. for rows of up to 4 M logits
+    // A descent's level histogram (kStripes copies): [stripe][limb 0..3, then the candidate count][digit], four words of
+    // padding between stripes; a limb sum stays below 2^32 while a stripe sees fewer than 65537 candidates, i.e. for
+    // rows of up to 4 M logits.  In the first CTA also the lists of candidates that the CTAs hand over (list()).
     alignas(16) unsigned h[kStripes][(kLimbs + 1) * 256 + 4];
-    u64 x_lo[2][256];          // double buffered by level: a CTA may build the next level while others still read this one
-    u64 x_hi[2][256];
+    u64 x_lo[2][256];          // this CTA's sum of them, which the other CTAs read; double buffered by level: a CTA may
+    u64 x_hi[2][256];          // build the next level while others still read this one
     unsigned x_cnt[2][256];
     u64 x_small[2][4];         // small values exchanged across the cluster (extremes, sums), double buffered by use
-    u64 x_all[2][kFullCluster * 4];   // ... and every CTA's copy of all of them
-    // the cluster-wide histogram of the first weighted level: the descents of step 4 all start from it
-    u64 l1_lo[256];
-    u64 l1_hi[256];
-    unsigned l1_cnt[256];
+    u64 x_all[2][kMaxCluster * 4];   // ... and every CTA's copy of all of them
+    unsigned hist[2][kBins];   // this CTA's weights by bin: sums of bits 46..62 and of bits 30..45
+    u64 cum[kBins];            // cluster-wide: weight of bins 0 .. b in units of 2^-32, rounded down per candidate
     // suffix sums of the walk
     u64 w_lo[8], w_hi[8];
     unsigned w_cnt[8];
@@ -116,13 +121,18 @@ struct FullShared {
     unsigned res_cnt;          // candidates in the chosen digit
     unsigned res_above_cnt;    // candidates before it
     u64 res_above_lo, res_above_hi;
-    u64 tot_lo, tot_hi;        // weight and number of all candidates of the level just walked (before-weight included)
-    unsigned tot_cnt;
     u64 red[kFullWarps];
     u64 red_hi[kFullWarps];
     unsigned red_cnt[kFullWarps];
-    int pick;                  // index of the drawn candidate in the ordered kept set
+    int bin_lo, bin_hi;        // bins that a cumulative weight may be reached in
+    int sent;                  // candidates this CTA has handed over
+    unsigned got[2][kMaxCluster];   // ... every CTA of the cluster has, double buffered by use
+    int first_p, first_u;      // places in the ordered list
+    u64 kw_lo, kw_hi;          // weight of the kept set
+    u64 cross[5];              // a resolved crossing: candidate, weight above (two words), count above, found
+    __device__ __forceinline__ u64* list() { return reinterpret_cast<u64*>(&h[0][0]); }
 };
+static_assert(sizeof(u64) * (kMaxCluster * kSendCap + kShort) <= sizeof(FullShared::h), "the lists, and room to order a short one, lie in the histogram's memory");
 
 struct FullArgs {
     const float* logits;
@@ -154,8 +164,9 @@ struct RowCtx {
     int lo, n;                // first column and number of columns of this CTA's slice
     int id_base;              // token id of column 0
     float mx;                 // the row's maximum
-    double temp;
-    u64* dbg;                 // diagnostics
+    double temp, inv_temp;    // T and 1 / T
+    u64 floor_c;              // candidates are those at or above this composite (0: all)
+    float bin_scale;          // bins per logit
     __device__ __forceinline__ float at(int i) const {   // logit i of the slice as the sampler sees it
         if (vals) return vals[i];
         float x = row[lo + i];
@@ -164,10 +175,19 @@ struct RowCtx {
         return x;
     }
     __device__ __forceinline__ u64 comp(float x, int i) const { return make_comp(x, lo + i + id_base); }
-    __device__ __forceinline__ u64 weight(float x) const {   // src/sampler.cpp:40, as 2^-62 fixed point
-        const double e = exp(__ddiv_rn((double)__fsub_rn(x, mx), temp));
-        return __double2ull_rn(__dmul_rn(e, 4611686018427387904.0));
+    // (x - max) / T, correctly rounded: a quotient from the rounded reciprocal and one exact correction step (Markstein 1990;
+    // T is a float, so its significand is never all ones) - three fused operations in place of a division.
+    __device__ __forceinline__ double scaled(float x) const {
+        const double d = (double)__fsub_rn(x, mx), q = __dmul_rn(d, inv_temp);
+        return __fma_rn(__fma_rn(-q, temp, d), inv_temp, q);
     }
+    __device__ __forceinline__ u64 weight(float x) const {   // src/sampler.cpp:40, as 2^-62 fixed point
+        if ((double)__fsub_rn(x, mx) < -43.8 * temp) return 0ull;   // below half of 2^-62
+        return __double2ull_rn(__dmul_rn(exp(scaled(x)), 4611686018427387904.0));
+    }
+    __device__ __forceinline__ bool is_candidate(float x, int i) const { return x == x && (floor_c == 0ull || comp(x, i) >= floor_c); }
+    // bin of a logit: never decreases as the logit falls
+    __device__ __forceinline__ int bin(float x) const { return min(kBins - 1, __float2int_rd(__fmul_rn(__fsub_rn(mx, x), bin_scale))); }
 };
 
 __device__ __forceinline__ u64 block_max_u64(u64 v, FullShared* sh) {
@@ -209,17 +229,18 @@ __device__ __forceinline__ void block_max2_u64(u64& hi, u64& lo, FullShared* sh)
     lo = ~b;
 }
 
-// Exchanges up to four 64-bit values per CTA across the cluster: every CTA gets all kFullCluster x 4 values.
+// Exchanges up to four 64-bit values per CTA across the cluster: every CTA gets all C x 4 values.
 // `use` alternates 0/1 between consecutive exchanges.  Contains one cluster barrier.
-__device__ __forceinline__ void cluster_exchange(FullShared* sh, int use, const u64 (&mine)[4], u64 (&all)[kFullCluster][4]) {
+template <int C>
+__device__ __forceinline__ void cluster_exchange(FullShared* sh, int use, const u64 (&mine)[4], u64 (&all)[C][4]) {
     if (threadIdx.x < 4) sh->x_small[use][threadIdx.x] = mine[threadIdx.x];
     cluster_sync_all();
     // one warp fetches the remote words; everybody else reads the local copy
-    if (threadIdx.x < kFullCluster * 4)
+    if (threadIdx.x < C * 4)
         sh->x_all[use][threadIdx.x] = ld_cluster_u64(map_to_rank(&sh->x_small[use][threadIdx.x & 3], threadIdx.x >> 2));
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kFullCluster; ++r)
+    for (int r = 0; r < C; ++r)
 #pragma unroll
         for (int j = 0; j < 4; ++j) all[r][j] = sh->x_all[use][r * 4 + j];
 }
@@ -279,55 +300,42 @@ struct Crossing {
 // barrier every CTA adds up all CTAs' histograms (thread d < 256 owns digit d) and walks the digits from the top:
 // the crossing digit is the highest digit d that holds a candidate and whose suffix sum (the weight of all higher
 // digits and its own, plus `above`) reaches the target.  Leaves digit, its candidate count and the weight and count
-// before it in shared memory; digit -1 if the target is beyond all candidates.  If `keep_l1`, the cluster-wide
-// histogram is also stored for later descents.  All threads of all CTAs of the cluster must call.
+// before it in shared memory; digit -1 if the target is beyond all candidates.  All threads of all CTAs of the cluster must call.
+template <int C>
 __device__ __forceinline__ void level_reduce_and_walk(FullShared* sh, int par, U128 target, U128 above, unsigned above_cnt, bool by_count,
-                                                      bool keep_l1, bool from_l1, unsigned stripe_mask) {
+                                                      unsigned stripe_mask) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     u64 lo = 0ull, hi = 0ull;
     unsigned cnt = 0u;
-    if (from_l1) {
-        if (tid < 256) {
-            lo = sh->l1_lo[tid];
-            hi = sh->l1_hi[tid];
-            cnt = sh->l1_cnt[tid];
-        }
-    } else {
-        if (tid < 256) {
-            u64 l0 = 0ull, l1 = 0ull, l2 = 0ull, l3 = 0ull;   // limb sums over the stripes: below 2^35 each
-            unsigned c = 0u;
+    if (tid < 256) {
+        u64 l0 = 0ull, l1 = 0ull, l2 = 0ull, l3 = 0ull;   // limb sums over the stripes: below 2^35 each
+        unsigned c = 0u;
 #pragma unroll
-            for (int s = 0; s <= (int)stripe_mask; ++s) {
-                l0 += sh->h[s][tid];
-                l1 += sh->h[s][256 + tid];
-                l2 += sh->h[s][512 + tid];
-                l3 += sh->h[s][768 + tid];
-                c += sh->h[s][kLimbs * 256 + tid];
-            }
-            U128 acc{0ull, l0};
-            acc = u128_add(acc, U128{l1 >> 48, l1 << 16});
-            acc = u128_add(acc, U128{l2 >> 32, l2 << 32});
-            acc = u128_add(acc, U128{l3 >> 16, l3 << 48});
-            sh->x_lo[par][tid] = acc.lo;
-            sh->x_hi[par][tid] = acc.hi;
-            sh->x_cnt[par][tid] = c;
+        for (int s = 0; s <= (int)stripe_mask; ++s) {
+            l0 += sh->h[s][tid];
+            l1 += sh->h[s][256 + tid];
+            l2 += sh->h[s][512 + tid];
+            l3 += sh->h[s][768 + tid];
+            c += sh->h[s][kLimbs * 256 + tid];
         }
-        cluster_sync_all();
-        if (tid < 256) {
+        U128 acc{0ull, l0};
+        acc = u128_add(acc, U128{l1 >> 48, l1 << 16});
+        acc = u128_add(acc, U128{l2 >> 32, l2 << 32});
+        acc = u128_add(acc, U128{l3 >> 16, l3 << 48});
+        sh->x_lo[par][tid] = acc.lo;
+        sh->x_hi[par][tid] = acc.hi;
+        sh->x_cnt[par][tid] = c;
+    }
+    cluster_sync_all();
+    if (tid < 256) {
 #pragma unroll
-            for (unsigned r = 0; r < (unsigned)kFullCluster; ++r) {
-                const u64 l = ld_cluster_u64(map_to_rank(&sh->x_lo[par][tid], r));
-                const u64 h = ld_cluster_u64(map_to_rank(&sh->x_hi[par][tid], r));
-                const unsigned c = ld_cluster_u32(map_to_rank(&sh->x_cnt[par][tid], r));
-                lo += l;
-                hi += h + (lo < l ? 1ull : 0ull);
-                cnt += c;
-            }
-            if (keep_l1) {
-                sh->l1_lo[tid] = lo;
-                sh->l1_hi[tid] = hi;
-                sh->l1_cnt[tid] = cnt;
-            }
+        for (unsigned r = 0; r < (unsigned)C; ++r) {
+            const u64 l = ld_cluster_u64(map_to_rank(&sh->x_lo[par][tid], r));
+            const u64 h = ld_cluster_u64(map_to_rank(&sh->x_hi[par][tid], r));
+            const unsigned c = ld_cluster_u32(map_to_rank(&sh->x_cnt[par][tid], r));
+            lo += l;
+            hi += h + (lo < l ? 1ull : 0ull);
+            cnt += c;
         }
     }
     if (by_count) {   // the "weight" of a digit is its number of candidates
@@ -368,11 +376,6 @@ __device__ __forceinline__ void level_reduce_and_walk(FullShared* sh, int par, U
         with = u128_add(suf, higher);        // everything from this digit up, and what came before the level
         with_c = sufc + higher_c;
         if (cnt != 0u && u128_ge(with, target)) atomicMax(&sh->res_digit, tid);   // the highest digit that reaches wins
-        if (tid == 0) {   // digit 0's suffix is everything
-            sh->tot_lo = with.lo;
-            sh->tot_hi = with.hi;
-            sh->tot_cnt = with_c;
-        }
     }
     __syncthreads();
     if (tid < 256 && tid == sh->res_digit) {
@@ -387,10 +390,9 @@ __device__ __forceinline__ void level_reduce_and_walk(FullShared* sh, int par, U
 
 // Radix descent over the candidates with composite in [floor_c, top_c] (the extremes of the candidate set): finds
 // the candidate at which the accumulated weight - or, with by_count, the number of candidates - counted from the
-// largest candidate down reaches `target`.  With use_l1 the first level is the stored histogram (the caller
-// guarantees it was built over the same candidate set with the same extremes).  All threads of the cluster call.
-__device__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_c, u64 top_c, U128 target, bool by_count, bool use_l1,
-                                    bool build_l1, int& par) {
+// largest candidate down reaches `target`.  All threads of the cluster call.
+template <int C>
+__device__ __noinline__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_c, u64 top_c, U128 target, bool by_count, int& par) {
     const int tid = threadIdx.x;
     Crossing out{0ull, U128{0ull, 0ull}, 0u, false};
     u64 mask, pfx;
@@ -411,19 +413,15 @@ __device__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_
     while (hb >= 0) {
         const int w = hb + 1 < 8 ? hb + 1 : 8, lo = hb + 1 - w;
         const unsigned dmask = (1u << w) - 1u;
-        const bool from_l1 = first && use_l1;
         // the first level sees every candidate, a few digits take most of them: eight stripes keep the lanes of a warp
         // apart.  Deeper levels see the few candidates that match the prefix: one stripe, an eighth of the clearing
         // and adding up.
         // (a 16-bit limb summed over one stripe stays below 2^32 for slices of up to 65536 logits)
         const unsigned stripe_mask = (first || rc.n > 65536) ? (unsigned)(kStripes - 1) : 0u;
-        const bool dbg = rc.dbg && build_l1;
-        if (dbg) rc.dbg[16] = global_timer_ns();
-        if (!from_l1) {
+        {
             for (int i = tid; i < (int)((stripe_mask + 1u) * sizeof(sh->h[0]) / sizeof(uint4)); i += kFullThreads)
                 reinterpret_cast<uint4*>(&sh->h[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
-            if (dbg) rc.dbg[17] = global_timer_ns();
             const int n_iter = (rc.n + kFullThreads - 1) / kFullThreads;
             for (int it = 0; it < n_iter; ++it) {
                 const int i = it * kFullThreads + tid;
@@ -444,11 +442,9 @@ __device__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_
                 hist_add(sh, active, digit, wgt, !by_count, stripe_mask);
             }
             __syncthreads();
-            if (dbg) rc.dbg[18] = global_timer_ns();
         }
-        level_reduce_and_walk(sh, par, target, above, above_cnt, by_count, first && build_l1, from_l1, stripe_mask);
-        if (dbg) rc.dbg[19] = global_timer_ns();
-        if (!from_l1) par ^= 1;
+        level_reduce_and_walk<C>(sh, par, target, above, above_cnt, by_count, stripe_mask);
+        par ^= 1;
         first = false;
         const int d = sh->res_digit;
         const unsigned in_digit = sh->res_cnt;
@@ -476,7 +472,7 @@ __device__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_
         // exactly one thread of the cluster holds it: that thread tells every CTA, one barrier makes it visible
         if (mine != 0ull) {
 #pragma unroll
-            for (unsigned r = 0; r < (unsigned)kFullCluster; ++r) cluster_store_u64(map_to_rank(&sh->x_small[par][0], r), mine);
+            for (unsigned r = 0; r < (unsigned)C; ++r) cluster_store_u64(map_to_rank(&sh->x_small[par][0], r), mine);
         }
         cluster_sync_all();
         pfx = sh->x_small[par][0];
@@ -489,15 +485,280 @@ __device__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_
     return out;
 }
 
+// ---- cumulative weights by bin ----------------------------------------------------------------------------------------
+// First bin whose cumulative weight reaches t (2^-62 units) for certain, and the first that may reach it, given that up to
+// n candidates were rounded down by less than one unit each.  All threads call; contains barriers.
+__device__ __forceinline__ void find_bins(FullShared* sh, U128 t, unsigned n) {
+    const int b = threadIdx.x;
+    const u64 t_lo = (t.hi << 34) | (t.lo >> 30), t_up = t_lo + ((t.lo & 0x3FFFFFFFull) ? 1ull : 0ull);   // t < 2^80
+    const u64 c = sh->cum[b], before = b > 0 ? sh->cum[b - 1] : 0ull;
+    if (b == 0) {
+        sh->bin_lo = kBins - 1;
+        sh->bin_hi = kBins - 1;
+    }
+    __syncthreads();
+    if (c >= t_up && (b == 0 || before < t_up)) sh->bin_hi = b;
+    if (c + n >= t_lo && (b == 0 || before + n < t_lo)) sh->bin_lo = b;
+    __syncthreads();
+}
+
+// Sum of two words and a count over the CTA, left in x_small[use][0..2].  Contains one barrier; the sums are there after the
+// next one.
+__device__ __forceinline__ void block_sums(FullShared* sh, int use, u64 lo, u64 hi, unsigned cnt) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+        sh->red[warp] = lo;
+        sh->red_hi[warp] = hi;
+        sh->red_cnt[warp] = cnt;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        lo = sh->red[lane];
+        hi = sh->red_hi[lane];
+        cnt = __reduce_add_sync(0xffffffffu, sh->red_cnt[lane]);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            lo += __shfl_xor_sync(0xffffffffu, lo, o);
+            hi += __shfl_xor_sync(0xffffffffu, hi, o);
+        }
+        if (lane == 0) {
+            sh->x_small[use][0] = lo;
+            sh->x_small[use][1] = hi;
+            sh->x_small[use][2] = cnt;
+        }
+    }
+}
+// A sum of weights kept as (sum of their low 32 bits, sum of their upper bits).
+__device__ __forceinline__ U128 join_words(u64 lo, u64 hi) { return u128_add(U128{0ull, lo}, U128{hi >> 32, hi << 32}); }
+
+// Hands this CTA's candidates of bins [b_lo, b_hi] to the first CTA of the cluster, and adds up its weights and candidates of
+// the bins before them.  Returns whether everybody's candidates fitted.  After it the first CTA has the lists (CTA r's
+// sh->got[par][r] candidates at list() + r * kSendCap), and every CTA's sums are in its x_small[par].
+template <int C>
+__device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsigned rank, int b_lo, int b_hi, bool sums, int par) {
+    const int tid = threadIdx.x;
+    if (tid == 0) sh->sent = 0;
+    __syncthreads();
+    const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u);
+    u64 lo = 0ull, hi = 0ull;
+    unsigned cnt = 0u;
+    for (int i = tid; i < rc.n; i += kFullThreads) {
+        const float x = rc.vals[i];
+        if (!(x == x)) continue;
+        const int b = rc.bin(x);
+        if (b > b_hi || !rc.is_candidate(x, i)) continue;
+        if (b >= b_lo) {
+            const int p = atomicAdd(&sh->sent, 1);
+            if (p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x, i));
+        } else if (sums) {
+            const u64 w = rc.weight(x);
+            lo += w & 0xFFFFFFFFull;
+            hi += w >> 32;
+            ++cnt;
+        }
+    }
+    if (sums) block_sums(sh, par, lo, hi, cnt);
+    else __syncthreads();
+    if (tid < C) cluster_store_u32(map_to_rank(&sh->got[par][rank], (unsigned)tid), (unsigned)sh->sent);
+    cluster_sync_all();
+    bool fits = true;
+#pragma unroll
+    for (int r = 0; r < C; ++r) fits = fits && sh->got[par][r] <= (unsigned)kSendCap;
+    return fits;
+}
+
+// Orders the lists that send_bins left in this (the first) CTA: one list, largest first, at the returned address; `n` entries.
+template <int C>
+__device__ __noinline__ u64* order_lists(FullShared* sh, int use, int& n) {
+    const int tid = threadIdx.x;
+    u64* list = sh->list();
+    u64* spare = list + kMaxCluster * kSendCap;
+    constexpr int kPer = kMaxCluster * kSendCap / kFullThreads;
+    int off[C + 1];
+    off[0] = 0;
+#pragma unroll
+    for (int r = 0; r < C; ++r) off[r + 1] = off[r] + (int)sh->got[use][r];
+    n = off[C];
+    u64 c[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int e = q * kFullThreads + tid;
+        int r = 0;
+#pragma unroll
+        for (int k = 1; k < C; ++k) r += e >= off[k] ? 1 : 0;
+        c[q] = 0ull;
+        if (e < n) {
+            int base = 0;
+#pragma unroll
+            for (int k = 1; k < C; ++k) base = r == k ? off[k] : base;
+            c[q] = list[r * kSendCap + e - base];
+        }
+    }
+    __syncthreads();
+    if (n <= kShort) {   // ranks by counting: four lanes for an entry, two entries per read
+        const int n8 = (n + 7) & ~7;
+        if (tid < n8) list[tid] = c[0];
+        __syncthreads();
+        const int part = tid & 3, e = tid >> 2;
+        if ((tid & ~31) >> 2 < n) {
+            const u64 mine = e < n ? list[e] : 0ull;
+            int larger = 0;
+#pragma unroll 4
+            for (int j = 2 * part; j < n8; j += 8) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(list + j);
+                larger += (v.x > mine ? 1 : 0) + (v.y > mine ? 1 : 0);
+            }
+            larger += __shfl_xor_sync(0xffffffffu, larger, 1);
+            larger += __shfl_xor_sync(0xffffffffu, larger, 2);
+            if (part == 0 && e < n) spare[larger] = mine;
+        }
+        __syncthreads();
+        return spare;
+    }
+    int m = kShort;
+    while (m < n) m <<= 1;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+        if (q * kFullThreads + tid < m) list[q * kFullThreads + tid] = c[q];
+    for (int k = 2; k <= m; k <<= 1)   // bitonic, descending
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (int i = tid; i < m / 2; i += kFullThreads) {
+                const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), up = lo | j;
+                const u64 x = list[lo], y = list[up];
+                if ((x < y) == ((lo & k) == 0)) {
+                    list[lo] = y;
+                    list[up] = x;
+                }
+            }
+        }
+    __syncthreads();
+    return list;
+}
+
+// Cumulative weights of the ordered list: every thread looks after up to four consecutive entries (`per` of them: fewer if
+// the list is short).  Contains barriers.
+struct ListScan {
+    static constexpr int kPer = kMaxCluster * kSendCap / kFullThreads;
+    U128 before;     // weight before the thread's first entry
+    u64 w[kPer];
+    int per;
+    // calls f(entry, weight before it, weight with it) for the thread's entries of the n
+    template <class F>
+    __device__ __forceinline__ void each(int n, F f) const {
+        U128 cum = before;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int e = (int)threadIdx.x * per + q;
+            if (q < per && e < n) {
+                const U128 with = u128_add(cum, U128{0ull, w[q]});
+                f(e, cum, with);
+                cum = with;
+            }
+        }
+    }
+};
+__device__ __forceinline__ ListScan scan_list(const RowCtx& rc, FullShared* sh, const u64* srt, int n, U128 above) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    ListScan ls;
+    ls.per = (n + kFullThreads - 1) / kFullThreads;
+    u64 lo = 0ull, hi = 0ull;
+#pragma unroll
+    for (int q = 0; q < ListScan::kPer; ++q) {
+        const int e = tid * ls.per + q;
+        ls.w[q] = q < ls.per && e < n ? rc.weight(comp_value(srt[e])) : 0ull;
+        lo += ls.w[q] & 0xFFFFFFFFull;
+        hi += ls.w[q] >> 32;
+    }
+    u64 ilo = lo, ihi = hi;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 l = __shfl_up_sync(0xffffffffu, ilo, o), h = __shfl_up_sync(0xffffffffu, ihi, o);
+        if (lane >= o) {
+            ilo += l;
+            ihi += h;
+        }
+    }
+    __syncthreads();
+    if (lane == 31) {
+        sh->red[warp] = ilo;
+        sh->red_hi[warp] = ihi;
+    }
+    __syncthreads();
+    u64 wl = sh->red[lane], wh = sh->red_hi[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 l = __shfl_up_sync(0xffffffffu, wl, o), h = __shfl_up_sync(0xffffffffu, wh, o);
+        if (lane >= o) {
+            wl += l;
+            wh += h;
+        }
+    }
+    wl = __shfl_sync(0xffffffffu, wl, max(0, warp - 1));
+    wh = __shfl_sync(0xffffffffu, wh, max(0, warp - 1));
+    if (warp == 0) wl = wh = 0ull;
+    ls.before = u128_add(above, join_words(wl + ilo - lo, wh + ihi - hi));
+    return ls;
+}
+
+// The candidate at which the cumulative weight reaches `target`; every CTA gets it.  Bins if they are of use, else a descent.
+template <int C>
+__device__ __noinline__ Crossing resolve(const RowCtx& rc, FullShared* sh, unsigned rank, bool binned, unsigned n_cand, u64 floor_c, u64 top_c, U128 target,
+                                         int& par) {
+    const int tid = threadIdx.x;
+    if (binned) {
+        find_bins(sh, target, n_cand);
+        if (tid == 0) sh->cross[4] = 0ull;
+        const bool fits = send_bins<C>(rc, sh, rank, sh->bin_lo, sh->bin_hi, true, par);
+        if (fits) {
+            if (rank == 0) {
+                u64 lo = 0ull, hi = 0ull, cnt = 0ull;
+                for (unsigned r = 0; r < (unsigned)C; ++r) {
+                    lo += ld_cluster_u64(map_to_rank(&sh->x_small[par][0], r));
+                    hi += ld_cluster_u64(map_to_rank(&sh->x_small[par][1], r));
+                    cnt += ld_cluster_u64(map_to_rank(&sh->x_small[par][2], r));
+                }
+                int n;
+                const u64* srt = order_lists<C>(sh, par, n);
+                const ListScan ls = scan_list(rc, sh, srt, n, join_words(lo, hi));
+                ls.each(n, [&](int e, U128 before, U128 with) {
+                    if (u128_ge(with, target) && (!u128_ge(before, target) || e == 0)) {
+#pragma unroll
+                        for (unsigned r = 0; r < (unsigned)C; ++r) {
+                            cluster_store_u64(map_to_rank(&sh->cross[0], r), srt[e]);
+                            cluster_store_u64(map_to_rank(&sh->cross[1], r), before.lo);
+                            cluster_store_u64(map_to_rank(&sh->cross[2], r), before.hi);
+                            cluster_store_u64(map_to_rank(&sh->cross[3], r), cnt + (u64)e);
+                            cluster_store_u64(map_to_rank(&sh->cross[4], r), 1ull);
+                        }
+                    }
+                });
+            }
+            par ^= 1;
+            cluster_sync_all();
+            return Crossing{sh->cross[0], U128{sh->cross[2], sh->cross[1]}, (unsigned)sh->cross[3], sh->cross[4] != 0ull};
+        }
+        par ^= 1;
+    }
+    return cluster_descent<C>(rc, sh, floor_c, top_c, target, false, par);
+}
+
+template <int C>
 __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArgs a, int cache_slice) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FullShared* sh = reinterpret_cast<FullShared*>(smem_raw);
     const int tid = threadIdx.x;
     const unsigned rank = cluster_rank();
-    const RowDesc d = a.rows[blockIdx.x / kFullCluster];
+    const RowDesc d = a.rows[blockIdx.x / C];
     const int V = a.n_vocab;
     // the slices: equal runs of columns, a multiple of four each
-    const int per = (((V + kFullCluster - 1) / kFullCluster) + 3) & ~3;
+    const int per = (((V + C - 1) / C) + 3) & ~3;
     const int lo = min(V, (int)rank * per), n = min(V, lo + per) - lo;
     unsigned* bitmap = reinterpret_cast<unsigned*>(smem_raw + sizeof(FullShared));
     float* vals = reinterpret_cast<float*>(smem_raw + sizeof(FullShared) + (size_t)((per + 31) / 32) * sizeof(unsigned));
@@ -505,11 +766,14 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     const float* row = a.logits + d.logits_off;
     const int id_base = a.vocab_offset;
     int par = 0;
-#define FTR(n)                                                                                                      \
-    do {                                                                                                            \
-        if (a.trace && blockIdx.x == gridDim.x - kFullCluster && tid == 0) a.trace[(n)] = global_timer_ns();        \
+#define FTR(n)                                                                                   \
+    do {                                                                                         \
+        if (a.trace && blockIdx.x == gridDim.x - C && tid == 0) a.trace[(n)] = global_timer_ns(); \
     } while (0)
     FTR(0);
+    cluster_arrive_release();   // (waited for before the first access to another CTA's shared memory)
+    sh->hist[0][tid] = 0u;
+    sh->hist[1][tid] = 0u;
 
     // ---- 0. the slice as the sampler sees it: penalty bitmap, softcap, penalty, optional write-back
     const bool has_pen = (d.flags & kRowPenalty) != 0;
@@ -525,151 +789,273 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         }
         __syncthreads();
     }
-    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature,
-              (a.trace && blockIdx.x == gridDim.x - kFullCluster && tid == 0) ? a.trace : nullptr};
-    u64 cmax = 0ull, cmin = ~0ull;
+    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, 0ull, 0.0f};
+    const float ninf = -__int_as_float(0x7f800000);
+    float mx = ninf, mn = -ninf;
+    unsigned valid = 0u;
     auto take = [&](float x, int i) {   // logit i of the slice as loaded: transform, keep, note the extremes, write back
         const bool hit = has_pen && ((bitmap[i >> 5] >> (i & 31)) & 1u);
         if (a.softcap != 0.0f) x = __fmul_rn(a.softcap, tanhf(__fdiv_rn(x, a.softcap)));
         if (hit) x = x > 0.0f ? __fdiv_rn(x, d.penalty) : __fmul_rn(x, d.penalty);
         if (cache_slice) vals[i] = x;
-        if (x == x) {   // NaNs take no part
-            const u64 c = rc.comp(x, i);
-            cmax = max(cmax, c);
-            cmin = min(cmin, c);
-        }
+        mx = fmaxf(mx, x);   // (NaNs take no part)
+        mn = fminf(mn, x);
+        valid += x == x ? 1u : 0u;
         if (a.write_back && (a.softcap != 0.0f || hit)) const_cast<float*>(row)[lo + i] = x;
     };
-    if (((reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0) && (n & 3) == 0) {
-        // 16-byte loads, four of them in flight per thread (the stores of a write-back come after the loads of a round)
-        const float4* src = reinterpret_cast<const float4*>(row + lo);
-        const int n4 = n >> 2;
-        for (int i0 = 0; i0 < n4; i0 += 4 * kFullThreads) {
-            float4 v[4];
+    // (the stores of a write-back come after the loads of a round)
+    const int n4 = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? n >> 2 : 0;
+    const float4* src = reinterpret_cast<const float4*>(row + lo);
+    for (int i0 = 0; i0 < n4; i0 += 4 * kFullThreads) {   // 16-byte loads, four of them in flight per thread
+        float4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = i0 + u * kFullThreads + tid;
-                v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * kFullThreads + tid;
+            v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = i0 + u * kFullThreads + tid;
-                if (i < n4) {
-                    take(v[u].x, 4 * i);
-                    take(v[u].y, 4 * i + 1);
-                    take(v[u].z, 4 * i + 2);
-                    take(v[u].w, 4 * i + 3);
-                }
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * kFullThreads + tid;
+            if (i < n4) {
+                take(v[u].x, 4 * i);
+                take(v[u].y, 4 * i + 1);
+                take(v[u].z, 4 * i + 2);
+                take(v[u].w, 4 * i + 3);
             }
         }
-    } else {
-        for (int i = tid; i < n; i += kFullThreads) take(row[lo + i], i);
     }
-    __syncthreads();
+    for (int i0 = 4 * n4; i0 < n; i0 += 8 * kFullThreads) {   // what is left, or a row that does not lie on 16-byte boundaries
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + u * kFullThreads + tid;
+            v[u] = i < n ? __ldcs(row + lo + i) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + u * kFullThreads + tid;
+            if (i < n) take(v[u], i);
+        }
+    }
     if (cache_slice) {
         rc.vals = vals;
     } else if (a.write_back) {   // the row in memory now holds the transformed values: read it as final
+        __syncthreads();
         rc.bitmap = nullptr;
         rc.cap = 0.0f;
     }
     FTR(1);
-    // ---- 1. the row's extremes
-    block_max2_u64(cmax, cmin, sh);
+    // ---- 1. the row's extremes and its number of logits
     {
-        u64 v[4] = {cmax, ~cmin, 0ull, 0ull}, all[kFullCluster][4];
-        cluster_exchange(sh, par, v, all);
-        par ^= 1;
-        for (int r = 0; r < kFullCluster; ++r) {
-            cmax = max(cmax, all[r][0]);
-            cmin = min(cmin, ~all[r][1]);
+        const int lane = tid & 31, warp = tid >> 5;
+        unsigned kx = __reduce_max_sync(0xffffffffu, float_key(mx)), kn = __reduce_min_sync(0xffffffffu, float_key(mn));
+        unsigned cnt = __reduce_add_sync(0xffffffffu, valid);
+        if (lane == 0) {
+            sh->red[warp] = ((u64)kx << 32) | kn;
+            sh->red_cnt[warp] = cnt;
         }
+        __syncthreads();
+        cluster_wait_acquire();
+        if (warp == 0) {
+            kx = __reduce_max_sync(0xffffffffu, (unsigned)(sh->red[lane] >> 32));
+            kn = __reduce_min_sync(0xffffffffu, (unsigned)sh->red[lane]);
+            cnt = __reduce_add_sync(0xffffffffu, sh->red_cnt[lane]);
+            // one lane per CTA of the cluster tells it
+            if (lane < C) {
+                cluster_store_u64(map_to_rank(&sh->x_all[0][rank], (unsigned)lane), ((u64)kx << 32) | kn);
+                cluster_store_u64(map_to_rank(&sh->x_all[0][kMaxCluster + rank], (unsigned)lane), cnt);
+            }
+        }
+        cluster_sync_all();
+        kx = 0u;
+        kn = ~0u;
+        valid = 0u;
+#pragma unroll
+        for (int r = 0; r < C; ++r) {
+            kx = max(kx, (unsigned)(sh->x_all[0][r] >> 32));
+            kn = min(kn, (unsigned)sh->x_all[0][r]);
+            valid += (unsigned)sh->x_all[0][kMaxCluster + r];
+        }
+        mx = key_float(kx);
+        mn = key_float(kn);
     }
+    // bounds of the candidates' composites, for the descents
+    const u64 cmax = ((u64)float_key(mx) << 32) | 0xFFFFFFFFull, cmin = (u64)float_key(mn) << 32;
     const int out = d.out_index;
     auto finish = [&](int token) {   // one thread: the row's token to wherever it is wanted
         if (d.flags & kRowAppend) a.pool[d.hist_begin + d.hist_len] = token;
         put_token(a.tokens, a.tokens_host, out, token);
     };
-    if (cmax == 0ull) {   // nothing but NaNs
+    if (valid == 0u) {   // nothing but NaNs
         if (rank == 0 && tid == 0) {
             report_status(a.status, a.status_host, kStatusEmptyRow);
-            finish(0);
             a.kept_n[out] = 0;
+            finish(0);
         }
-        cluster_sync_all();   // no CTA leaves while another may still read its shared memory
         return;
     }
-    rc.mx = comp_value(cmax);
+    rc.mx = mx;
+    rc.inv_temp = __ddiv_rn(1.0, rc.temp);
     FTR(2);
 
     // ---- 2. the k-th candidate (k < n only)
     u64 c_k = cmin;
     if (d.k < V) {
-        const Crossing ck = cluster_descent(rc, sh, 0ull, cmax, U128{0ull, (u64)d.k}, true, false, false, par);
-        if (ck.found) c_k = max(cmin, ck.c);
+        const Crossing ck = cluster_descent<C>(rc, sh, 0ull, cmax, U128{0ull, (u64)d.k}, true, par);
+        if (ck.found) c_k = rc.floor_c = max(cmin, ck.c);
     }
-
     FTR(3);
-    // ---- 3. the weights' histogram by leading digit (kept for the descents), their sum and the number of candidates
-    // (a descent towards an unreachable target builds the first level and stops there)
-    cluster_descent(rc, sh, c_k, cmax, U128{~0ull, ~0ull}, false, false, true, par);
-    U128 S{0ull, 0ull};
-    unsigned n_cand = 0u;
-    const bool have_l1 = cmax != c_k;
-    if (have_l1) {   // the walk left the level's totals behind
-        S = U128{sh->tot_hi, sh->tot_lo};
-        n_cand = sh->tot_cnt;
+    // ---- 3. the weights' exact sum, the number of candidates, and the histogram
+    // (a row whose largest logit is infinite, or that is too long for shared memory, is left to the descents)
+    const float inf = -ninf;
+    const bool binned = rc.vals != nullptr && mx < inf && mx > ninf;
+    // weights are zero 43.7 temperatures below the maximum: no bins are spent on what lies further down
+    rc.bin_scale = (float)kBins / fminf(44.0f * d.temperature, mx - mn);
+    if (!(rc.bin_scale < inf)) rc.bin_scale = 0.0f;
+    U128 S;
+    unsigned n_cand;
+    {
+        u64 wl = 0ull, wh = 0ull;
+        unsigned cnt = 0u;
+        auto weigh = [&](float x, int i) {
+            if (!rc.is_candidate(x, i)) return;
+            ++cnt;
+            const u64 w = rc.weight(x);
+            wl += w & 0xFFFFFFFFull;
+            wh += w >> 32;
+            const unsigned up = (unsigned)(w >> 46), down = (unsigned)(w >> 30) & 0xFFFFu;
+            if (binned && (up | down)) {
+                const int bin = rc.bin(x);
+                if (up) atomicAdd(&sh->hist[0][bin], up);
+                if (down) atomicAdd(&sh->hist[1][bin], down);
+            }
+        };
+#pragma unroll 4
+        for (int i = tid; i < n; i += kFullThreads) weigh(rc.at(i), i);
+        block_sums(sh, par, wl, wh, cnt);
+        cluster_sync_all();
+        u64 c = 0ull;
+#pragma unroll
+        for (unsigned r = 0; r < (unsigned)C; ++r)
+            c += ((u64)ld_cluster_u32(map_to_rank(&sh->hist[0][tid], r)) << 16) + ld_cluster_u32(map_to_rank(&sh->hist[1][tid], r));
+        if (tid < C * 4) sh->x_all[par][tid] = ld_cluster_u64(map_to_rank(&sh->x_small[par][tid & 3], (unsigned)tid >> 2));
+        // inclusive sums over the bins, largest logits first
+        const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u64 t = __shfl_up_sync(0xffffffffu, c, o);
+            if (lane >= o) c += t;
+        }
+        if (lane == 31) sh->red[warp] = c;
         __syncthreads();
-    } else {   // a single candidate: there was no level to build
-        S = U128{0ull, rc.weight(rc.mx)};
-        n_cand = 1u;
+        u64 t = lane < warp ? sh->red[lane] : 0ull;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        sh->cum[tid] = c + t;
+        wl = wh = 0ull;
+        n_cand = 0u;
+#pragma unroll
+        for (int r = 0; r < C; ++r) {
+            wl += sh->x_all[par][4 * r];
+            wh += sh->x_all[par][4 * r + 1];
+            n_cand += (unsigned)sh->x_all[par][4 * r + 2];
+        }
+        S = join_words(wl, wh);
+        par ^= 1;
+        __syncthreads();
     }
     const double sum = __dmul_rn(u128_to_double(S), 2.168404344971008868014905601739883422851562500e-19);   // * 2^-62
-
+    const double min_thr = __dmul_rn(__ddiv_rn(1.0, sum), (double)d.min_p);
+    // (top-p: the first candidate at which the cumulative probability reaches it, included)
+    const U128 target_p = double_to_u128_ceil(__dmul_rn(__dmul_rn((double)d.top_p, sum), 4611686018427387904.0));
+    // (min-p: the test is monotone in the logit and flips near mx + T * ln(min_p): only logits within a band around that value
+    // need the exact arithmetic, those above it are kept, those below it are not)
+    const double x_flip = d.min_p > 0.0f ? (double)mx + rc.temp * log((double)d.min_p) : (double)ninf;
+    const double band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
+    const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
+    double u = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
+    if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
     FTR(4);
-    // ---- 4a. min-p: the last candidate whose probability is not below pr[0] * min_p   (pr[0] = 1 / sum)
+
+    // ---- 4a. the usual way with a cut: everything that can be kept goes to the first CTA, which finishes the row
+    if (binned && (d.top_p < 1.0f || d.min_p > 0.0f)) {
+        int b_hi = kBins - 1;
+        if (d.top_p < 1.0f) {
+            find_bins(sh, target_p, n_cand);
+            b_hi = sh->bin_hi;
+        }
+        if (d.min_p > 0.0f) b_hi = min(b_hi, rc.bin(x_never));
+        if (send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
+            FTR(5);
+            if (rank != 0) return;   // nobody reads this CTA's memory any more
+            int m;
+            if (tid == 0) {
+                sh->first_p = 0x7fffffff;
+                sh->first_u = 0x7fffffff;
+            }
+            const u64* srt = order_lists<C>(sh, par, m);
+            const ListScan ls = scan_list(rc, sh, srt, m, U128{0ull, 0ull});
+            ls.each(m, [&](int e, U128 before, U128 with) {
+                if (d.top_p < 1.0f && u128_ge(with, target_p) && !u128_ge(before, target_p)) atomicMin(&sh->first_p, e + 1);
+                if (d.min_p > 0.0f && __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), sum) < min_thr) atomicMin(&sh->first_p, max(e, 1));
+            });
+            __syncthreads();
+            const int keep = min(sh->first_p, m);
+            ls.each(keep, [&](int e, U128, U128 with) {
+                if (e == keep - 1) {
+                    sh->kw_lo = with.lo;
+                    sh->kw_hi = with.hi;
+                }
+            });
+            __syncthreads();
+            const U128 target = double_to_u128_ceil(__dmul_rn(u, u128_to_double(U128{sh->kw_hi, sh->kw_lo})));
+            ls.each(keep, [&](int e, U128, U128 with) {
+                if (u128_ge(with, target)) atomicMin(&sh->first_u, e);
+                if (a.record && e < kMaxK) {
+                    a.kept_ids[(size_t)out * kMaxK + e] = comp_id(srt[e]);
+                    a.kept_pr[(size_t)out * kMaxK + e] = __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), sum);
+                }
+            });
+            __syncthreads();
+            if (tid == 0) {
+                if (a.record) a.kept_n[out] = keep;
+                finish(comp_id(srt[min(sh->first_u, keep - 1)]));   // (a target beyond the list, by rounding, takes the last)
+            }
+            FTR(6);
+            return;
+        }
+        par ^= 1;
+    }
+
+    // ---- 4b. the cuts one by one: min-p
     u64 c_keep = c_k;
     if (d.min_p > 0.0f) {
-        const double thr = __dmul_rn(__ddiv_rn(1.0, sum), (double)d.min_p);
-        // the test below is monotone in the logit and flips near mx + T * ln(min_p): only logits within a band around
-        // that value need the exact arithmetic, those above it are kept, those below it are not
-        const double x_flip = (double)rc.mx + rc.temp * log((double)d.min_p);
-        const double band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
-        const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
         u64 lowest = ~0ull;
         for (int i = tid; i < n; i += kFullThreads) {
             const float x = rc.at(i);
-            if (!(x == x) || x < x_never) continue;
-            const u64 c = rc.comp(x, i);
-            if (c < c_k) continue;
-            if (x > x_sure) {
-                lowest = min(lowest, c);
-                continue;
-            }
-            const double e = exp(__ddiv_rn((double)__fsub_rn(x, rc.mx), rc.temp));
-            if (!(__ddiv_rn(e, sum) < thr)) lowest = min(lowest, c);
+            if (!rc.is_candidate(x, i) || x < x_never) continue;
+            if (x > x_sure || !(__ddiv_rn(exp(rc.scaled(x)), sum) < min_thr)) lowest = min(lowest, rc.comp(x, i));
         }
         lowest = ~block_max_u64(~lowest, sh);
-        u64 v[4] = {~lowest, 0ull, 0ull, 0ull}, all[kFullCluster][4];
-        cluster_exchange(sh, par, v, all);
+        u64 v[4] = {~lowest, 0ull, 0ull, 0ull}, all[C][4];
+        cluster_exchange<C>(sh, par, v, all);
         par ^= 1;
-        for (int r = 0; r < kFullCluster; ++r) lowest = min(lowest, ~all[r][0]);
-        if (lowest == ~0ull) lowest = cmax;   // keep at least the best
+        for (int r = 0; r < C; ++r) lowest = min(lowest, ~all[r][0]);
+        if (lowest == ~0ull) lowest = cmax & 0xFFFFFFFF00000000ull;   // keep at least the best
         c_keep = max(c_keep, lowest);
     }
-    FTR(5);
-    // ---- 4b. top-p: the first candidate at which the cumulative probability reaches top_p, included
+    // ---- top-p
     bool keep_from_top_p = false;
     Crossing cp{0ull, U128{0ull, 0ull}, 0u, false};
     if (d.top_p < 1.0f) {
-        const U128 target = double_to_u128_ceil(__dmul_rn(__dmul_rn((double)d.top_p, sum), 4611686018427387904.0));
-        cp = cluster_descent(rc, sh, c_k, cmax, target, false, have_l1, false, par);
+        cp = resolve<C>(rc, sh, rank, binned, n_cand, c_k, cmax, target_p, par);
         if (cp.found && cp.c >= c_keep) {
             c_keep = cp.c;
             keep_from_top_p = true;
         }
     }
     FTR(6);
-    // ---- 4c. total weight and size of the kept set: known from the descent when top-p made the cut, the whole
+    // ---- 4c. total weight and size of the kept set: known from the crossing when top-p made the cut, the whole
     // candidate set when nothing cut, otherwise one pass
     U128 KW = S;
     unsigned n_keep = n_cand;
@@ -677,49 +1063,46 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         KW = u128_add(cp.above, U128{0ull, rc.weight(comp_value(cp.c))});
         n_keep = cp.above_cnt + 1u;
     } else if (c_keep != c_k) {
-        U128 part{0ull, 0ull};
+        u64 wl = 0ull, wh = 0ull;
         unsigned pc = 0u;
         for (int i = tid; i < n; i += kFullThreads) {
             const float x = rc.at(i);
             if (x == x && rc.comp(x, i) >= c_keep) {
                 const u64 w = rc.weight(x);
-                const u64 l = part.lo + w;
-                if (l < part.lo) part.hi += 1ull;
-                part.lo = l;
+                wl += w & 0xFFFFFFFFull;
+                wh += w >> 32;
                 ++pc;
             }
         }
-        block_sum_u128(part, pc, sh);
-        u64 v[4] = {part.lo, part.hi, (u64)pc, 0ull}, all[kFullCluster][4];
-        cluster_exchange(sh, par, v, all);
-        par ^= 1;
-        KW = U128{0ull, 0ull};
+        block_sums(sh, par, wl, wh, pc);
+        cluster_sync_all();
+        wl = wh = 0ull;
         n_keep = 0u;
-        for (int r = 0; r < kFullCluster; ++r) {
-            KW = u128_add(KW, U128{all[r][1], all[r][0]});
-            n_keep += (unsigned)all[r][2];
+        for (unsigned r = 0; r < (unsigned)C; ++r) {
+            wl += ld_cluster_u64(map_to_rank(&sh->x_small[par][0], r));
+            wh += ld_cluster_u64(map_to_rank(&sh->x_small[par][1], r));
+            n_keep += (unsigned)ld_cluster_u64(map_to_rank(&sh->x_small[par][2], r));
         }
+        KW = join_words(wl, wh);
+        par ^= 1;
     }
     FTR(7);
-    // ---- 4d. the draw: first kept candidate whose cumulative weight reaches u * (kept weight).  A kept set that fits
-    // the record is gathered for it anyway, and the first CTA then draws from the ordered list; otherwise a descent.
-    double u = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
-    if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
-    const U128 target = double_to_u128_ceil(__dmul_rn(u, u128_to_double(KW)));
-    const bool draw_from_list = n_keep <= (unsigned)kMaxK;
-    if (!draw_from_list) {
-        const Crossing ct = cluster_descent(rc, sh, c_k, cmax, target, false, have_l1, false, par);
-        const u64 c_tok = (ct.found && ct.c >= c_keep) ? ct.c : c_keep;
+    // ---- 4d. the draw: first kept candidate whose cumulative weight reaches u * (kept weight)
+    {
+        U128 target = double_to_u128_ceil(__dmul_rn(u, u128_to_double(KW)));
+        if (!u128_ge(KW, target)) target = KW;   // (beyond it by rounding: the last one)
+        const Crossing ct = resolve<C>(rc, sh, rank, binned, n_cand, c_k, cmax, target, par);
+        const u64 c_tok = ct.found && ct.c >= c_keep ? ct.c : c_keep;
         if (rank == 0 && tid == 0) finish(comp_id(c_tok));
     }
     FTR(8);
 
     // ---- 5. the kept set's record: its size, and its first kMaxK candidates in order with their probabilities
-    if (a.record || draw_from_list) {
+    if (a.record) {
         const int want = (int)min(n_keep, (unsigned)kMaxK);
         u64 c_first = c_keep;   // the last of the first `want` kept candidates
         if ((unsigned)want < n_keep) {
-            const Crossing cf = cluster_descent(rc, sh, c_k, cmax, U128{0ull, (u64)want}, true, false, false, par);
+            const Crossing cf = cluster_descent<C>(rc, sh, c_k, cmax, U128{0ull, (u64)want}, true, par);
             if (cf.found) c_first = max(c_keep, cf.c);
         }
         // every CTA appends its candidates >= c_first to the row's staging area (the probabilities' memory, as keys);
@@ -741,38 +1124,19 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         __threadfence();
         cluster_sync_all();
         if (rank == 0) {
-            // the first CTA's slice is no longer needed: the candidates, then (by rank) their ids' composites and weights
-            u64* srt = reinterpret_cast<u64*>(vals);
-            u64* by_rank_c = srt + kMaxK;
-            u64* by_rank_w = srt + 2 * kMaxK;
+            u64* srt = reinterpret_cast<u64*>(vals);   // the first CTA's slice is no longer needed
             u64 c = 0ull;
             if (tid < want) c = __ldcg(stage + tid);
             __syncthreads();
             if (tid < want) srt[tid] = c;
-            if (tid == 0) sh->pick = want - 1;   // a target beyond the list (rounding) takes the last kept candidate
             __syncthreads();
             if (tid < want) {
                 int rank_in = 0;
                 for (int j = 0; j < want; ++j) rank_in += srt[j] > c ? 1 : 0;
-                const float x = comp_value(c);
-                const double e = exp(__ddiv_rn((double)__fsub_rn(x, rc.mx), rc.temp));
                 a.kept_ids[(size_t)out * kMaxK + rank_in] = comp_id(c);
-                a.kept_pr[(size_t)out * kMaxK + rank_in] = __ddiv_rn(e, sum);
-                by_rank_c[rank_in] = c;
-                by_rank_w[rank_in] = rc.weight(x);
+                a.kept_pr[(size_t)out * kMaxK + rank_in] = __ddiv_rn(exp(rc.scaled(comp_value(c))), sum);
             }
-            __syncthreads();
-            if (draw_from_list && tid < want) {   // thread r: the weight of candidates 0 .. r
-                U128 cum{0ull, 0ull};
-                for (int j = 0; j <= tid; ++j) cum = u128_add(cum, U128{0ull, by_rank_w[j]});
-                const U128 before = u128_sub(cum, U128{0ull, by_rank_w[tid]});
-                if (u128_ge(cum, target) && (tid == 0 || !u128_ge(before, target))) sh->pick = tid;
-            }
-            __syncthreads();
-            if (tid == 0) {
-                if (draw_from_list) finish(comp_id(by_rank_c[sh->pick]));
-                a.kept_n[out] = (int)n_keep;
-            }
+            if (tid == 0) a.kept_n[out] = (int)n_keep;
         }
     }
     cluster_sync_all();   // no CTA leaves while another may still read its shared memory
@@ -780,24 +1144,45 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
 
 }  // namespace
 
-size_t full_row_smem_bytes(int n_vocab) {
-    const int per = (((n_vocab + kFullCluster - 1) / kFullCluster) + 3) & ~3;
+namespace {
+int slice_of(int n_vocab, int cluster) { return (((n_vocab + cluster - 1) / cluster) + 3) & ~3; }
+size_t full_row_smem_bytes(int n_vocab, int cluster) {
+    const int per = slice_of(n_vocab, cluster);
     const size_t bitmap = sizeof(unsigned) * (size_t)((per + 31) / 32);
-    // (the kept set is ordered in the slice's memory: three arrays of kMaxK 64-bit words)
-    const size_t slice = per <= kSliceCache ? sizeof(float) * (size_t)std::max(per, 6 * kMaxK) : 3 * sizeof(u64) * (size_t)kMaxK;
+    // (the kept set's record is ordered in the slice's memory: kMaxK 64-bit words)
+    const size_t slice = per <= kSliceCache ? sizeof(float) * (size_t)std::max(per, 2 * kMaxK) : sizeof(u64) * (size_t)kMaxK;
     return sizeof(FullShared) + bitmap + 16 + slice;
 }
+template <int C>
+int launch_full(const FullArgs& a, int n_rows, cudaStream_t stream) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(n_rows * C));
+    cfg.blockDim = dim3(kFullThreads);
+    cfg.dynamicSmemBytes = full_row_smem_bytes(a.n_vocab, C);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, full_row_kernel<C>, a, slice_of(a.n_vocab, C) <= kSliceCache ? 1 : 0);
+}
+}  // namespace
 
 int prepare_full_row_kernel(int max_vocab) {
     // the largest request of any row length up to max_vocab: rows that still fit the slice cache need the most
-    const size_t most = std::max(full_row_smem_bytes(max_vocab), full_row_smem_bytes(std::min(max_vocab, kFullCluster * kSliceCache)));
-    cudaError_t e = cudaFuncSetAttribute(full_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    const size_t most8 = std::max(full_row_smem_bytes(max_vocab, 8), full_row_smem_bytes(std::min(max_vocab, 8 * kSliceCache), 8));
+    const size_t most4 = full_row_smem_bytes(std::min(max_vocab, 4 * kSliceCache), 4);
+    cudaError_t e = cudaFuncSetAttribute(full_row_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most8);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(full_row_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most4);
     return (int)e;
 }
 
 int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, const int32_t* drafts, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
                            int32_t* kept_ids, double* kept_pr, int32_t* kept_n, int record, uint32_t* status, uint32_t* status_host, int n_vocab,
-                           int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream) {
+                           int vocab_offset, int write_back, float softcap, uint64_t* trace, int sms, void* stream) {
     if (n_vocab > (1 << 22)) return (int)cudaErrorInvalidValue;   // the histogram's limb sums are sized for 4 M logits
     FullArgs a{};
     a.logits = logits;
@@ -818,21 +1203,10 @@ int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows,
     a.record = record;
     a.softcap = softcap;
     a.trace = reinterpret_cast<u64*>(trace);
-    const int per = (((n_vocab + kFullCluster - 1) / kFullCluster) + 3) & ~3;
-    const int cache_slice = per <= kSliceCache ? 1 : 0;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kFullCluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(n_rows * kFullCluster));
-    cfg.blockDim = dim3(kFullThreads);
-    cfg.dynamicSmemBytes = full_row_smem_bytes(n_vocab);
-    cfg.stream = static_cast<cudaStream_t>(stream);
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, full_row_kernel, a, cache_slice);
+    // Eight CTAs per row while they fit the SMs at once, one each; with more rows four, which pay the steps between the passes
+    // half as often.
+    if ((int64_t)n_rows * 8 > sms && slice_of(n_vocab, 4) <= kSliceCache) return launch_full<4>(a, n_rows, static_cast<cudaStream_t>(stream));
+    return launch_full<8>(a, n_rows, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace fsb
