@@ -112,8 +112,11 @@ struct FullShared {
     unsigned x_cnt[2][256];
     u64 x_small[2][4];         // small values exchanged across the cluster (extremes, sums), double buffered by use
     u64 x_all[2][kMaxCluster * 4];   // ... and every CTA's copy of all of them
+    double table[64];          // 2^(j / 64)
     unsigned hist[2][kBins];   // this CTA's weights by bin: sums of bits 46..62 and of bits 30..45
     u64 cum[kBins];            // cluster-wide: weight of bins 0 .. b in units of 2^-32, rounded down per candidate
+    unsigned cum_n[kBins];     // ... and about how many candidates they hold (see estimated_count)
+    u64 part[kFullThreads];    // the CTAs' weights of the bins that this CTA adds up
     // suffix sums of the walk
     u64 w_lo[8], w_hi[8];
     unsigned w_cnt[8];
@@ -165,6 +168,8 @@ struct RowCtx {
     int id_base;              // token id of column 0
     float mx;                 // the row's maximum
     double temp, inv_temp;    // T and 1 / T
+    double cut;               // x - max below this weighs nothing
+    const double* table;      // 2^(j / 64)
     u64 floor_c;              // candidates are those at or above this composite (0: all)
     float bin_scale;          // bins per logit
     __device__ __forceinline__ float at(int i) const {   // logit i of the slice as the sampler sees it
@@ -181,9 +186,31 @@ struct RowCtx {
         const double d = (double)__fsub_rn(x, mx), q = __dmul_rn(d, inv_temp);
         return __fma_rn(__fma_rn(-q, temp, d), inv_temp, q);
     }
-    __device__ __forceinline__ u64 weight(float x) const {   // src/sampler.cpp:40, as 2^-62 fixed point
-        if ((double)__fsub_rn(x, mx) < -43.8 * temp) return 0ull;   // below half of 2^-62
-        return __double2ull_rn(__dmul_rn(exp(scaled(x)), 4611686018427387904.0));
+    // src/sampler.cpp:40, exp(y) as 2^-62 fixed point.  Table-driven (P. Tang, "Table-driven implementation of the exponential
+    // function", ACM TOMS 15, 1989): y = (64 e + j) ln2 / 64 + r, exp(y) = 2^e 2^(j/64) (1 + p(r)) with |r| <= ln2 / 128, where
+    // the Taylor polynomial of degree 5 is off by less than 2^-54.  Ten fp64 operations and a table look-up after the
+    // quotient; fixed point comes from the significand's bits.  (exp() and the conversion took three times as long.)
+    __device__ __forceinline__ u64 weight(float x) const {
+        const double d = (double)__fsub_rn(x, mx);
+        if (!(d >= cut)) return d != d ? 1ull << 62 : 0ull;   // below half of 2^-62 (or the maximum is infinite, and this is it)
+        const double y = scaled(x);
+        const double magic = 6755399441055744.0;   // 1.5 * 2^52: adding it rounds to an integer, which the low word then holds
+        const double t = __fma_rn(y, 92.33248261689366, magic);   // 64 / ln 2
+        const int n = __double2loint(t);
+        const double k = __dsub_rn(t, magic);
+        // ln2 / 64 in two parts, the first with 32 significant bits: k times it is exact
+        double r = __fma_rn(k, -0.010830424693267559632658958435, y);
+        r = __fma_rn(k, -2.9815858269852933e-12, r);
+        double q = __fma_rn(r, 1.0 / 120.0, 1.0 / 24.0);
+        q = __fma_rn(r, q, 1.0 / 6.0);
+        q = __fma_rn(r, q, 0.5);
+        q = __fma_rn(__dmul_rn(r, r), q, r);
+        const double s = table[n & 63];
+        const double v = __fma_rn(s, q, s);          // in [1, 2), or a hair below 1
+        const u64 bits = (u64)__double_as_longlong(v);
+        const u64 sig = (bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;          // v = sig * 2^(exponent - 52)
+        const int sh = (n >> 6) + (int)(bits >> 52) - 1023 + 10;                    // weight = sig * 2^sh, rounded
+        return sh >= 0 ? sig << sh : sh < -54 ? 0ull : (sig + (1ull << (-sh - 1))) >> -sh;
     }
     __device__ __forceinline__ bool is_candidate(float x, int i) const { return x == x && (floor_c == 0ull || comp(x, i) >= floor_c); }
     // bin of a logit: never decreases as the logit falls
@@ -392,7 +419,8 @@ __device__ __forceinline__ void level_reduce_and_walk(FullShared* sh, int par, U
 // the candidate at which the accumulated weight - or, with by_count, the number of candidates - counted from the
 // largest candidate down reaches `target`.  All threads of the cluster call.
 template <int C>
-__device__ __noinline__ Crossing cluster_descent(const RowCtx& rc, FullShared* sh, u64 floor_c, u64 top_c, U128 target, bool by_count, int& par) {
+__device__ __noinline__ Crossing cluster_descent(const RowCtx rc, FullShared* sh, u64 floor_c, u64 top_c, U128 target, bool by_count, int& use) {
+    int par = use;
     const int tid = threadIdx.x;
     Crossing out{0ull, U128{0ull, 0ull}, 0u, false};
     u64 mask, pfx;
@@ -451,7 +479,10 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx& rc, FullShared* s
         const U128 nabove{sh->res_above_hi, sh->res_above_lo};
         const unsigned nabove_cnt = sh->res_above_cnt;
         __syncthreads();   // the results may be overwritten
-        if (d < 0) return out;   // the target lies beyond the candidates
+        if (d < 0) {   // the target lies beyond the candidates
+            use = par;
+            return out;
+        }
         pfx |= (u64)(unsigned)d << lo;
         mask |= (u64)dmask << lo;
         above = nabove;
@@ -478,6 +509,7 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx& rc, FullShared* s
         pfx = sh->x_small[par][0];
         par ^= 1;
     }
+    use = par;
     out.c = pfx;
     out.above = above;
     out.above_cnt = above_cnt;
@@ -486,6 +518,14 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx& rc, FullShared* s
 }
 
 // ---- cumulative weights by bin ----------------------------------------------------------------------------------------
+// About how many candidates a bin holds, from its weight (units of 2^-32): right to a few per cent unless the bins are wide.
+// Clamped, so that sums do not overflow.
+__device__ __forceinline__ unsigned estimated_count(const RowCtx& rc, int bin, u64 weight) {
+    const float middle = ((float)bin + 0.5f) / (rc.bin_scale * (float)rc.temp);   // of the bin, below the maximum, in temperatures
+    const float n = (float)weight * exp2f(fminf(middle * 1.442695f, 60.0f) - 32.0f);
+    return n < 1e6f ? (unsigned)n + (weight ? 1u : 0u) : 1000000u;
+}
+
 // First bin whose cumulative weight reaches t (2^-62 units) for certain, and the first that may reach it, given that up to
 // n candidates were rounded down by less than one unit each.  All threads call; contains barriers.
 __device__ __forceinline__ void find_bins(FullShared* sh, U128 t, unsigned n) {
@@ -548,15 +588,24 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
     const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u);
     u64 lo = 0ull, hi = 0ull;
     unsigned cnt = 0u;
-    for (int i = tid; i < rc.n; i += kFullThreads) {
-        const float x = rc.vals[i];
-        if (!(x == x)) continue;
+    const int lane = tid & 31;
+    bool full = false;   // (then nothing more is handed over: the lists are of no use)
+    for (int i0 = tid - lane; i0 < rc.n; i0 += kFullThreads) {
+        const int i = i0 + lane;
+        const float x = i < rc.n ? rc.vals[i] : __int_as_float(0x7fc00000);
         const int b = rc.bin(x);
-        if (b > b_hi || !rc.is_candidate(x, i)) continue;
-        if (b >= b_lo) {
-            const int p = atomicAdd(&sh->sent, 1);
-            if (p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x, i));
-        } else if (sums) {
+        const bool in = x == x && b <= b_hi && rc.is_candidate(x, i), give = in && b >= b_lo && !full;
+        const unsigned hits = __ballot_sync(0xffffffffu, give);
+        if (hits) {
+            int p = 0;
+            if (lane == 0) p = atomicAdd(&sh->sent, __popc(hits));
+            p = __shfl_sync(0xffffffffu, p, 0);
+            full = p >= kSendCap;
+            p += __popc(hits & ((1u << lane) - 1u));
+            if (give && p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x, i));
+        }
+        if (!sums && full) break;
+        if (sums && in && b < b_lo) {
             const u64 w = rc.weight(x);
             lo += w & 0xFFFFFFFFull;
             hi += w >> 32;
@@ -573,40 +622,40 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
     return fits;
 }
 
-// Orders the lists that send_bins left in this (the first) CTA: one list, largest first, at the returned address; `n` entries.
-template <int C>
-__device__ __noinline__ u64* order_lists(FullShared* sh, int use, int& n) {
-    const int tid = threadIdx.x;
+// What the first CTA does with the lists that send_bins left there takes T threads: 256 of them, one candidate each, if
+// there are at most kShort (eight warps get through the barriers faster than thirty-two), else all.
+template <int T>
+__device__ __forceinline__ void list_sync() { block_sync<T, T == kFullThreads ? 0 : 1>(); }
+
+// Orders the lists: one list, largest first, at the returned address; `n` entries.
+template <int C, int T>
+__device__ __forceinline__ u64* order_lists(FullShared* sh, int use, int n) {
+    const int tid = threadIdx.x, lane = tid & 31;
     u64* list = sh->list();
     u64* spare = list + kMaxCluster * kSendCap;
-    constexpr int kPer = kMaxCluster * kSendCap / kFullThreads;
+    constexpr int kPer = T == kFullThreads ? kMaxCluster * kSendCap / kFullThreads : 1;
     int off[C + 1];
     off[0] = 0;
 #pragma unroll
     for (int r = 0; r < C; ++r) off[r + 1] = off[r] + (int)sh->got[use][r];
-    n = off[C];
     u64 c[kPer];
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
-        const int e = q * kFullThreads + tid;
-        int r = 0;
+        const int e = q * T + tid;
+        int from = 0;
 #pragma unroll
-        for (int k = 1; k < C; ++k) r += e >= off[k] ? 1 : 0;
-        c[q] = 0ull;
-        if (e < n) {
-            int base = 0;
-#pragma unroll
-            for (int k = 1; k < C; ++k) base = r == k ? off[k] : base;
-            c[q] = list[r * kSendCap + e - base];
-        }
+        for (int r = 0; r < C; ++r) from = e >= off[r] ? r * kSendCap + e - off[r] : from;
+        c[q] = e < n ? list[from] : 0ull;
     }
-    __syncthreads();
-    if (n <= kShort) {   // ranks by counting: four lanes for an entry, two entries per read
+    list_sync<T>();
+    if (T != kFullThreads) {   // ranks by counting: four lanes for an entry, two entries per read
         const int n8 = (n + 7) & ~7;
         if (tid < n8) list[tid] = c[0];
-        __syncthreads();
-        const int part = tid & 3, e = tid >> 2;
-        if ((tid & ~31) >> 2 < n) {
+        list_sync<T>();
+        const int part = tid & 3;
+        for (int e0 = 0; e0 < n; e0 += T / 4) {
+            const int e = e0 + (tid >> 2);
+            if (e0 + ((tid & ~31) >> 2) >= n) break;   // (whole warps)
             const u64 mine = e < n ? list[e] : 0ull;
             int larger = 0;
 #pragma unroll 4
@@ -618,18 +667,49 @@ __device__ __noinline__ u64* order_lists(FullShared* sh, int use, int& n) {
             larger += __shfl_xor_sync(0xffffffffu, larger, 2);
             if (part == 0 && e < n) spare[larger] = mine;
         }
-        __syncthreads();
+        list_sync<T>();
         return spare;
     }
-    int m = kShort;
+    if (n <= kFullThreads) {   // a run of 32 per warp, ordered across the lanes; then the places of an entry in all runs
+        u64 mine = c[0];
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const u64 o = __shfl_xor_sync(0xffffffffu, mine, j);
+                mine = (((lane & k) == 0) == ((lane & j) == 0)) ? max(mine, o) : min(mine, o);
+            }
+        }
+        list[tid] = mine;
+        __syncthreads();
+        const int runs = (n + 31) >> 5;
+        int rank = lane;
+        if (mine != 0ull) {
+#pragma unroll 4
+            for (int q = 0; q < runs; ++q) {
+                const u64* run = list + 32 * q;
+                int lo = 0;   // entries of the run above this one (0 .. 32)
+#pragma unroll
+                for (int st = 16; st > 0; st >>= 1)
+                    if (run[lo + st - 1] > mine) lo += st;
+                if (run[lo] > mine) lo += 1;
+                rank += q == tid >> 5 ? 0 : lo;
+            }
+        }
+        __syncthreads();
+        if (mine != 0ull) list[rank] = mine;
+        __syncthreads();
+        return list;
+    }
+    int m = 2 * kFullThreads;
     while (m < n) m <<= 1;
 #pragma unroll
     for (int q = 0; q < kPer; ++q)
-        if (q * kFullThreads + tid < m) list[q * kFullThreads + tid] = c[q];
+        if (q * T + tid < m) list[q * T + tid] = c[q];
     for (int k = 2; k <= m; k <<= 1)   // bitonic, descending
         for (int j = k >> 1; j > 0; j >>= 1) {
             __syncthreads();
-            for (int i = tid; i < m / 2; i += kFullThreads) {
+            for (int i = tid; i < m / 2; i += T) {
                 const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), up = lo | j;
                 const u64 x = list[lo], y = list[up];
                 if ((x < y) == ((lo & k) == 0)) {
@@ -644,8 +724,9 @@ __device__ __noinline__ u64* order_lists(FullShared* sh, int use, int& n) {
 
 // Cumulative weights of the ordered list: every thread looks after up to four consecutive entries (`per` of them: fewer if
 // the list is short).  Contains barriers.
+template <int T>
 struct ListScan {
-    static constexpr int kPer = kMaxCluster * kSendCap / kFullThreads;
+    static constexpr int kPer = T == kFullThreads ? kMaxCluster * kSendCap / kFullThreads : 1;
     U128 before;     // weight before the thread's first entry
     u64 w[kPer];
     int per;
@@ -664,13 +745,14 @@ struct ListScan {
         }
     }
 };
-__device__ __forceinline__ ListScan scan_list(const RowCtx& rc, FullShared* sh, const u64* srt, int n, U128 above) {
+template <int T>
+__device__ __forceinline__ ListScan<T> scan_list(const RowCtx& rc, FullShared* sh, const u64* srt, int n, U128 above) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    ListScan ls;
-    ls.per = (n + kFullThreads - 1) / kFullThreads;
+    ListScan<T> ls;
+    ls.per = ListScan<T>::kPer == 1 ? 1 : (n + T - 1) / T;
     u64 lo = 0ull, hi = 0ull;
 #pragma unroll
-    for (int q = 0; q < ListScan::kPer; ++q) {
+    for (int q = 0; q < ListScan<T>::kPer; ++q) {
         const int e = tid * ls.per + q;
         ls.w[q] = q < ls.per && e < n ? rc.weight(comp_value(srt[e])) : 0ull;
         lo += ls.w[q] & 0xFFFFFFFFull;
@@ -685,31 +767,103 @@ __device__ __forceinline__ ListScan scan_list(const RowCtx& rc, FullShared* sh, 
             ihi += h;
         }
     }
-    __syncthreads();
-    if (lane == 31) {
-        sh->red[warp] = ilo;
-        sh->red_hi[warp] = ihi;
-    }
-    __syncthreads();
-    u64 wl = sh->red[lane], wh = sh->red_hi[lane];
+    u64 wl = 0ull, wh = 0ull;
+    if (n > 32) {
+        list_sync<T>();
+        if (lane == 31) {
+            sh->red[warp] = ilo;
+            sh->red_hi[warp] = ihi;
+        }
+        list_sync<T>();
+        wl = lane < warp ? sh->red[lane] : 0ull;
+        wh = lane < warp ? sh->red_hi[lane] : 0ull;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u64 l = __shfl_up_sync(0xffffffffu, wl, o), h = __shfl_up_sync(0xffffffffu, wh, o);
-        if (lane >= o) {
-            wl += l;
-            wh += h;
+        for (int o = 16; o; o >>= 1) {
+            wl += __shfl_xor_sync(0xffffffffu, wl, o);
+            wh += __shfl_xor_sync(0xffffffffu, wh, o);
         }
     }
-    wl = __shfl_sync(0xffffffffu, wl, max(0, warp - 1));
-    wh = __shfl_sync(0xffffffffu, wh, max(0, warp - 1));
-    if (warp == 0) wl = wh = 0ull;
     ls.before = u128_add(above, join_words(wl + ilo - lo, wh + ihi - hi));
     return ls;
 }
 
+// The first CTA's share of resolve(): the crossing among the candidates it was sent goes to every CTA of the cluster.
+template <int C, int T>
+__device__ __forceinline__ void cross_list(const RowCtx& rc, FullShared* sh, int use, int n, U128 target) {
+    u64 lo = 0ull, hi = 0ull, cnt = 0ull;
+#pragma unroll
+    for (unsigned r = 0; r < (unsigned)C; ++r) {
+        lo += ld_cluster_u64(map_to_rank(&sh->x_small[use][0], r));
+        hi += ld_cluster_u64(map_to_rank(&sh->x_small[use][1], r));
+        cnt += ld_cluster_u64(map_to_rank(&sh->x_small[use][2], r));
+    }
+    const u64* srt = order_lists<C, T>(sh, use, n);
+    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, join_words(lo, hi));
+    ls.each(n, [&](int e, U128 before, U128 with) {
+        if (u128_ge(with, target) && (!u128_ge(before, target) || e == 0)) {
+#pragma unroll
+            for (unsigned r = 0; r < (unsigned)C; ++r) {
+                cluster_store_u64(map_to_rank(&sh->cross[0], r), srt[e]);
+                cluster_store_u64(map_to_rank(&sh->cross[1], r), before.lo);
+                cluster_store_u64(map_to_rank(&sh->cross[2], r), before.hi);
+                cluster_store_u64(map_to_rank(&sh->cross[3], r), cnt + (u64)e);
+                cluster_store_u64(map_to_rank(&sh->cross[4], r), 1ull);
+            }
+        }
+    });
+}
+template <int C>
+__device__ __forceinline__ int listed(const FullShared* sh, int use) {
+    int n = 0;
+#pragma unroll
+    for (int r = 0; r < C; ++r) n += (int)sh->got[use][r];
+    return n;
+}
+
+// The end of a row all of whose candidates that can be kept are in the first CTA's lists: min-p, top-p, draw, record.
+struct RowCuts {
+    U128 target_p;
+    double u, sum, min_thr;
+    bool top_p, min_p;
+};
+template <int C, int T>
+__device__ __forceinline__ int finish_list(const RowCtx& rc, FullShared* sh, int use, int n, const RowCuts& cuts, const FullArgs& a, int out) {
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        sh->first_p = 0x7fffffff;
+        sh->first_u = 0x7fffffff;
+    }
+    const u64* srt = order_lists<C, T>(sh, use, n);
+    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, U128{0ull, 0ull});
+    ls.each(n, [&](int e, U128 before, U128 with) {
+        if (cuts.top_p && u128_ge(with, cuts.target_p) && !u128_ge(before, cuts.target_p)) atomicMin(&sh->first_p, e + 1);
+        if (cuts.min_p && __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), cuts.sum) < cuts.min_thr) atomicMin(&sh->first_p, max(e, 1));
+    });
+    list_sync<T>();
+    const int keep = min(sh->first_p, n);
+    ls.each(keep, [&](int e, U128, U128 with) {
+        if (e == keep - 1) {
+            sh->kw_lo = with.lo;
+            sh->kw_hi = with.hi;
+        }
+    });
+    list_sync<T>();
+    const U128 target = double_to_u128_ceil(__dmul_rn(cuts.u, u128_to_double(U128{sh->kw_hi, sh->kw_lo})));
+    ls.each(keep, [&](int e, U128, U128 with) {
+        if (u128_ge(with, target)) atomicMin(&sh->first_u, e);
+        if (a.record && e < kMaxK) {
+            a.kept_ids[(size_t)out * kMaxK + e] = comp_id(srt[e]);
+            a.kept_pr[(size_t)out * kMaxK + e] = __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), cuts.sum);
+        }
+    });
+    list_sync<T>();
+    if (a.record && tid == 0) a.kept_n[out] = keep;
+    return comp_id(srt[min(sh->first_u, keep - 1)]);   // (a target beyond the list, by rounding, takes the last)
+}
+
 // The candidate at which the cumulative weight reaches `target`; every CTA gets it.  Bins if they are of use, else a descent.
 template <int C>
-__device__ __noinline__ Crossing resolve(const RowCtx& rc, FullShared* sh, unsigned rank, bool binned, unsigned n_cand, u64 floor_c, u64 top_c, U128 target,
+__device__ __noinline__ Crossing resolve(const RowCtx rc, FullShared* sh, unsigned rank, bool binned, unsigned n_cand, u64 floor_c, u64 top_c, U128 target,
                                          int& par) {
     const int tid = threadIdx.x;
     if (binned) {
@@ -718,27 +872,9 @@ __device__ __noinline__ Crossing resolve(const RowCtx& rc, FullShared* sh, unsig
         const bool fits = send_bins<C>(rc, sh, rank, sh->bin_lo, sh->bin_hi, true, par);
         if (fits) {
             if (rank == 0) {
-                u64 lo = 0ull, hi = 0ull, cnt = 0ull;
-                for (unsigned r = 0; r < (unsigned)C; ++r) {
-                    lo += ld_cluster_u64(map_to_rank(&sh->x_small[par][0], r));
-                    hi += ld_cluster_u64(map_to_rank(&sh->x_small[par][1], r));
-                    cnt += ld_cluster_u64(map_to_rank(&sh->x_small[par][2], r));
-                }
-                int n;
-                const u64* srt = order_lists<C>(sh, par, n);
-                const ListScan ls = scan_list(rc, sh, srt, n, join_words(lo, hi));
-                ls.each(n, [&](int e, U128 before, U128 with) {
-                    if (u128_ge(with, target) && (!u128_ge(before, target) || e == 0)) {
-#pragma unroll
-                        for (unsigned r = 0; r < (unsigned)C; ++r) {
-                            cluster_store_u64(map_to_rank(&sh->cross[0], r), srt[e]);
-                            cluster_store_u64(map_to_rank(&sh->cross[1], r), before.lo);
-                            cluster_store_u64(map_to_rank(&sh->cross[2], r), before.hi);
-                            cluster_store_u64(map_to_rank(&sh->cross[3], r), cnt + (u64)e);
-                            cluster_store_u64(map_to_rank(&sh->cross[4], r), 1ull);
-                        }
-                    }
-                });
+                const int n = listed<C>(sh, par);
+                if (n > kShort) cross_list<C, kFullThreads>(rc, sh, par, n, target);
+                else if (tid < kShort) cross_list<C, kShort>(rc, sh, par, n, target);
             }
             par ^= 1;
             cluster_sync_all();
@@ -774,67 +910,81 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     cluster_arrive_release();   // (waited for before the first access to another CTA's shared memory)
     sh->hist[0][tid] = 0u;
     sh->hist[1][tid] = 0u;
+    if (tid < 64) sh->table[tid] = exp2((double)tid / 64.0);
 
-    // ---- 0. the slice as the sampler sees it: penalty bitmap, softcap, penalty, optional write-back
+    // ---- 0. the slice as the sampler sees it: penalty bitmap, softcap, penalty, optional write-back.  The first loads of the
+    // slice (all of it, up to 16384 logits) are on their way while the bitmap is made.
+    const int n4 = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? n >> 2 : 0;
+    const float4* src = reinterpret_cast<const float4*>(row + lo);
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = u * kFullThreads + tid;
+        v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const bool has_pen = (d.flags & kRowPenalty) != 0;
     if (has_pen) {
-        const int words = (n + 31) >> 5;
+        const int32_t* h = a.hist + d.hist_begin;
+        const int n_drafts = d.flags >> kRowDraftShift, words = (n + 31) >> 5;
+        int id = tid < d.hist_len ? h[tid] : tid < d.hist_len + n_drafts ? a.drafts[d.draft_off + tid - d.hist_len] : 0;
         for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
         __syncthreads();
-        const int32_t* h = a.hist + d.hist_begin;
-        const int n_drafts = d.flags >> kRowDraftShift;
         for (int i = tid; i < d.hist_len + n_drafts; i += kFullThreads) {
-            const int c = (i < d.hist_len ? h[i] : a.drafts[d.draft_off + i - d.hist_len]) - id_base - lo;
+            if (i != tid) id = i < d.hist_len ? h[i] : a.drafts[d.draft_off + i - d.hist_len];
+            const int c = id - id_base - lo;
             if (c >= 0 && c < n) atomicOr(&bitmap[c >> 5], 1u << (c & 31));
         }
         __syncthreads();
     }
-    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, 0ull, 0.0f};
+    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, -43.8 * (double)d.temperature, sh->table, 0ull, 0.0f};
     const float ninf = -__int_as_float(0x7f800000);
     float mx = ninf, mn = -ninf;
     unsigned valid = 0u;
-    auto take = [&](float x, int i) {   // logit i of the slice as loaded: transform, keep, note the extremes, write back
-        const bool hit = has_pen && ((bitmap[i >> 5] >> (i & 31)) & 1u);
+    auto take = [&](float x, int i, bool hit) {   // logit i of the slice as loaded: transform, note the extremes, write back
         if (a.softcap != 0.0f) x = __fmul_rn(a.softcap, tanhf(__fdiv_rn(x, a.softcap)));
         if (hit) x = x > 0.0f ? __fdiv_rn(x, d.penalty) : __fmul_rn(x, d.penalty);
-        if (cache_slice) vals[i] = x;
         mx = fmaxf(mx, x);   // (NaNs take no part)
         mn = fminf(mn, x);
         valid += x == x ? 1u : 0u;
         if (a.write_back && (a.softcap != 0.0f || hit)) const_cast<float*>(row)[lo + i] = x;
+        return x;
     };
-    // (the stores of a write-back come after the loads of a round)
-    const int n4 = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? n >> 2 : 0;
-    const float4* src = reinterpret_cast<const float4*>(row + lo);
     for (int i0 = 0; i0 < n4; i0 += 4 * kFullThreads) {   // 16-byte loads, four of them in flight per thread
-        float4 v[4];
+        if (i0 > 0) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * kFullThreads + tid;
-            v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * kFullThreads + tid;
+                v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int i = i0 + u * kFullThreads + tid;
             if (i < n4) {
-                take(v[u].x, 4 * i);
-                take(v[u].y, 4 * i + 1);
-                take(v[u].z, 4 * i + 2);
-                take(v[u].w, 4 * i + 3);
+                const unsigned bits = has_pen ? bitmap[i >> 3] >> ((4 * i) & 31) : 0u;
+                float4 x = v[u];
+                x.x = take(x.x, 4 * i, bits & 1u);
+                x.y = take(x.y, 4 * i + 1, bits & 2u);
+                x.z = take(x.z, 4 * i + 2, bits & 4u);
+                x.w = take(x.w, 4 * i + 3, bits & 8u);
+                if (cache_slice) reinterpret_cast<float4*>(vals)[i] = x;
             }
         }
     }
     for (int i0 = 4 * n4; i0 < n; i0 += 8 * kFullThreads) {   // what is left, or a row that does not lie on 16-byte boundaries
-        float v[8];
+        float y[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * kFullThreads + tid;
-            v[u] = i < n ? __ldcs(row + lo + i) : 0.0f;
+            y[u] = i < n ? __ldcs(row + lo + i) : 0.0f;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * kFullThreads + tid;
-            if (i < n) take(v[u], i);
+            if (i < n) {
+                const float x = take(y[u], i, has_pen && ((bitmap[i >> 5] >> (i & 31)) & 1u));
+                if (cache_slice) vals[i] = x;
+            }
         }
     }
     if (cache_slice) {
@@ -912,6 +1062,11 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     // weights are zero 43.7 temperatures below the maximum: no bins are spent on what lies further down
     rc.bin_scale = (float)kBins / fminf(44.0f * d.temperature, mx - mn);
     if (!(rc.bin_scale < inf)) rc.bin_scale = 0.0f;
+    // (min-p: the test is monotone in the logit and flips near mx + T * ln(min_p): only logits within a band around that value
+    // need the exact arithmetic, those above it are kept, those below it are not)
+    const double x_flip = d.min_p > 0.0f ? (double)mx + rc.temp * log((double)d.min_p) : (double)ninf;
+    const double band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
+    const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
     U128 S;
     unsigned n_cand;
     {
@@ -934,24 +1089,44 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         for (int i = tid; i < n; i += kFullThreads) weigh(rc.at(i), i);
         block_sums(sh, par, wl, wh, cnt);
         cluster_sync_all();
-        u64 c = 0ull;
+        // Every CTA adds up kBins / C of the bins and hands the sums to all others: one load and one store per thread across the
+        // cluster (all bins read from all CTAs took 2.3 us).
+        {
+            constexpr int kMine = kBins / C;
+            const int src = tid / kMine, bin = (int)rank * kMine + tid % kMine;
+            sh->part[tid] = ((u64)ld_cluster_u32(map_to_rank(&sh->hist[0][bin], (unsigned)src)) << 16) + ld_cluster_u32(map_to_rank(&sh->hist[1][bin], (unsigned)src));
+            if (tid < C * 4) sh->x_all[par][tid] = ld_cluster_u64(map_to_rank(&sh->x_small[par][tid & 3], (unsigned)tid >> 2));
+            __syncthreads();
+            u64 c = 0ull;
 #pragma unroll
-        for (unsigned r = 0; r < (unsigned)C; ++r)
-            c += ((u64)ld_cluster_u32(map_to_rank(&sh->hist[0][tid], r)) << 16) + ld_cluster_u32(map_to_rank(&sh->hist[1][tid], r));
-        if (tid < C * 4) sh->x_all[par][tid] = ld_cluster_u64(map_to_rank(&sh->x_small[par][tid & 3], (unsigned)tid >> 2));
+            for (int r = 0; r < C; ++r) c += sh->part[r * kMine + tid % kMine];
+            cluster_store_u64(map_to_rank(&sh->cum[bin], (unsigned)src), c);
+        }
+        cluster_sync_all();
         // inclusive sums over the bins, largest logits first
         const int lane = tid & 31, warp = tid >> 5;
+        u64 c = sh->cum[tid];
+        unsigned est = estimated_count(rc, tid, c);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const u64 t = __shfl_up_sync(0xffffffffu, c, o);
-            if (lane >= o) c += t;
+            const unsigned e = __shfl_up_sync(0xffffffffu, est, o);
+            if (lane >= o) {
+                c += t;
+                est += e;
+            }
         }
-        if (lane == 31) sh->red[warp] = c;
+        if (lane == 31) {
+            sh->red[warp] = c;
+            sh->red_cnt[warp] = est;
+        }
         __syncthreads();
         u64 t = lane < warp ? sh->red[lane] : 0ull;
+        est += __reduce_add_sync(0xffffffffu, lane < warp ? sh->red_cnt[lane] : 0u);
 #pragma unroll
         for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         sh->cum[tid] = c + t;
+        sh->cum_n[tid] = est;
         wl = wh = 0ull;
         n_cand = 0u;
 #pragma unroll
@@ -968,11 +1143,6 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     const double min_thr = __dmul_rn(__ddiv_rn(1.0, sum), (double)d.min_p);
     // (top-p: the first candidate at which the cumulative probability reaches it, included)
     const U128 target_p = double_to_u128_ceil(__dmul_rn(__dmul_rn((double)d.top_p, sum), 4611686018427387904.0));
-    // (min-p: the test is monotone in the logit and flips near mx + T * ln(min_p): only logits within a band around that value
-    // need the exact arithmetic, those above it are kept, those below it are not)
-    const double x_flip = d.min_p > 0.0f ? (double)mx + rc.temp * log((double)d.min_p) : (double)ninf;
-    const double band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
-    const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
     double u = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
     if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
     FTR(4);
@@ -985,42 +1155,19 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             b_hi = sh->bin_hi;
         }
         if (d.min_p > 0.0f) b_hi = min(b_hi, rc.bin(x_never));
-        if (send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
+        if (sh->cum_n[b_hi] <= (unsigned)(C * kSendCap / 2) && send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
             FTR(5);
             if (rank != 0) return;   // nobody reads this CTA's memory any more
-            int m;
-            if (tid == 0) {
-                sh->first_p = 0x7fffffff;
-                sh->first_u = 0x7fffffff;
+            const RowCuts cuts{target_p, u, sum, min_thr, d.top_p < 1.0f, d.min_p > 0.0f};
+            const int m = listed<C>(sh, par);
+            int token;
+            if (m > kShort) {
+                token = finish_list<C, kFullThreads>(rc, sh, par, m, cuts, a, out);
+            } else {
+                if (tid >= kShort) return;
+                token = finish_list<C, kShort>(rc, sh, par, m, cuts, a, out);
             }
-            const u64* srt = order_lists<C>(sh, par, m);
-            const ListScan ls = scan_list(rc, sh, srt, m, U128{0ull, 0ull});
-            ls.each(m, [&](int e, U128 before, U128 with) {
-                if (d.top_p < 1.0f && u128_ge(with, target_p) && !u128_ge(before, target_p)) atomicMin(&sh->first_p, e + 1);
-                if (d.min_p > 0.0f && __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), sum) < min_thr) atomicMin(&sh->first_p, max(e, 1));
-            });
-            __syncthreads();
-            const int keep = min(sh->first_p, m);
-            ls.each(keep, [&](int e, U128, U128 with) {
-                if (e == keep - 1) {
-                    sh->kw_lo = with.lo;
-                    sh->kw_hi = with.hi;
-                }
-            });
-            __syncthreads();
-            const U128 target = double_to_u128_ceil(__dmul_rn(u, u128_to_double(U128{sh->kw_hi, sh->kw_lo})));
-            ls.each(keep, [&](int e, U128, U128 with) {
-                if (u128_ge(with, target)) atomicMin(&sh->first_u, e);
-                if (a.record && e < kMaxK) {
-                    a.kept_ids[(size_t)out * kMaxK + e] = comp_id(srt[e]);
-                    a.kept_pr[(size_t)out * kMaxK + e] = __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), sum);
-                }
-            });
-            __syncthreads();
-            if (tid == 0) {
-                if (a.record) a.kept_n[out] = keep;
-                finish(comp_id(srt[min(sh->first_u, keep - 1)]));   // (a target beyond the list, by rounding, takes the last)
-            }
+            if (tid == 0) finish(token);
             FTR(6);
             return;
         }
