@@ -2,7 +2,7 @@
 //
 // Rows whose effective candidate count k exceeds kMaxK - above all `top_k == 0`, where the reference sorts the
 // whole vocabulary (src/sampler.cpp:32-35 of paragontasx/ferro) - cannot keep their candidates in one CTA.  A
-// cluster of eight (or four) CTAs works on one such row.  Every CTA keeps its slice of the row in shared memory
+// cluster of four, six or eight CTAs works on one such row.  Every CTA keeps its slice of the row in shared memory
 // (softcap and penalty applied once, src/model_gemma4.cpp:521 and src/sampler.cpp:11-18), so the row is read from
 // HBM exactly once; everything after that reads shared memory:
 //   1. the row's largest and smallest candidate key                                            (src/sampler.cpp:38)
@@ -113,10 +113,10 @@ struct FullShared {
     u64 x_small[2][4];         // small values exchanged across the cluster (extremes, sums), double buffered by use
     u64 x_all[2][kMaxCluster * 4];   // ... and every CTA's copy of all of them
     double table[64];          // 2^(j / 64)
-    unsigned hist[2][kBins];   // this CTA's weights by bin: sums of bits 46..62 and of bits 30..45
-    u64 cum[kBins];            // cluster-wide: weight of bins 0 .. b in units of 2^-32, rounded down per candidate
+    unsigned hist[2][kBins];   // this CTA's weights (their upper parts) by bin: sums of bits 16..31 and of bits 0..15
+    u64 cum[kBins];            // cluster-wide: weight of bins 0 .. b in units of 2^-31, rounded per candidate
     unsigned cum_n[kBins];     // ... and about how many candidates they hold (see estimated_count)
-    u64 part[kFullThreads];    // the CTAs' weights of the bins that this CTA adds up
+    u64 part[kFullThreads + 8];   // the CTAs' weights of the bins that this CTA adds up
     // suffix sums of the walk
     u64 w_lo[8], w_hi[8];
     unsigned w_cnt[8];
@@ -158,6 +158,13 @@ struct FullArgs {
     u64* trace;               // diagnostics: time stamps of the last row's phases, or null
 };
 
+// A weight in 2^-62 units: up * 2^31 + down.
+struct Weight {
+    unsigned up;
+    int down;
+    __device__ __forceinline__ u64 value() const { return ((u64)up << 31) + (u64)(long long)down; }
+};
+
 // What the passes of a row share.
 struct RowCtx {
     const float* vals;        // the slice in shared memory (as the sampler sees it), or null: read and transform the row
@@ -168,7 +175,8 @@ struct RowCtx {
     int id_base;              // token id of column 0
     float mx;                 // the row's maximum
     double temp, inv_temp;    // T and 1 / T
-    double cut;               // x - max below this weighs nothing
+    float cut;                // x - max below this weighs nothing
+    bool odd;                 // an infinite maximum, or a temperature that makes `cut` overflow
     const double* table;      // 2^(j / 64)
     u64 floor_c;              // candidates are those at or above this composite (0: all)
     float bin_scale;          // bins per logit
@@ -182,19 +190,26 @@ struct RowCtx {
     __device__ __forceinline__ u64 comp(float x, int i) const { return make_comp(x, lo + i + id_base); }
     // (x - max) / T, correctly rounded: a quotient from the rounded reciprocal and one exact correction step (Markstein 1990;
     // T is a float, so its significand is never all ones) - three fused operations in place of a division.
-    __device__ __forceinline__ double scaled(float x) const {
-        const double d = (double)__fsub_rn(x, mx), q = __dmul_rn(d, inv_temp);
+    __device__ __forceinline__ double scaled(float diff) const {
+        const double d = (double)diff, q = __dmul_rn(d, inv_temp);
         return __fma_rn(__fma_rn(-q, temp, d), inv_temp, q);
     }
-    // src/sampler.cpp:40, exp(y) as 2^-62 fixed point.  Table-driven (P. Tang, "Table-driven implementation of the exponential
-    // function", ACM TOMS 15, 1989): y = (64 e + j) ln2 / 64 + r, exp(y) = 2^e 2^(j/64) (1 + p(r)) with |r| <= ln2 / 128, where
-    // the Taylor polynomial of degree 5 is off by less than 2^-54.  Ten fp64 operations and a table look-up after the
-    // quotient; fixed point comes from the significand's bits.  (exp() and the conversion took three times as long.)
-    __device__ __forceinline__ u64 weight(float x) const {
-        const double d = (double)__fsub_rn(x, mx);
-        if (!(d >= cut)) return d != d ? 1ull << 62 : 0ull;   // below half of 2^-62 (or the maximum is infinite, and this is it)
-        const double y = scaled(x);
-        const double magic = 6755399441055744.0;   // 1.5 * 2^52: adding it rounds to an integer, which the low word then holds
+    __device__ __forceinline__ double probability(float x, double sum) const { return __ddiv_rn(exp(scaled(__fsub_rn(x, mx))), sum); }   // src/sampler.cpp:40-41
+    // src/sampler.cpp:40, exp(y) as 2^-62 fixed point in two parts.  Table-driven (P. Tang, "Table-driven implementation of the
+    // exponential function", ACM TOMS 15, 1989): y = (64 e + j) ln2 / 64 + r, exp(y) = 2^e 2^(j/64) (1 + p(r)) with |r| <=
+    // ln2 / 128, where the Taylor polynomial of degree 5 is off by less than 2^-54.  Adding 1.5 * 2^(52 - b) rounds to a multiple
+    // of 2^-b and leaves that multiple in the low word: b = 31 gives the first part, b = 62 what is left.  Seventeen fp64
+    // operations and no branch; a pass over a slice is bound by them (exp() and conversions took twice as long).
+    // Logits 45 temperatures below the maximum and NaNs weigh nothing.
+    __device__ __noinline__ Weight odd_weight(float x) const {   // (an infinite maximum alone has weight)
+        const double e = x == mx ? 1.0 : x == x ? exp(__ddiv_rn((double)__fsub_rn(x, mx), temp)) : 0.0;
+        const u64 w = __double2ull_rn(__dmul_rn(e, 4611686018427387904.0));
+        return Weight{(unsigned)(w >> 31), (int)(w & 0x7FFFFFFFull)};
+    }
+    __device__ __forceinline__ Weight weight(float x) const {
+        if (odd) return odd_weight(x);
+        const double y = scaled(fmaxf(__fsub_rn(x, mx), cut));
+        const double magic = 6755399441055744.0;   // 1.5 * 2^52
         const double t = __fma_rn(y, 92.33248261689366, magic);   // 64 / ln 2
         const int n = __double2loint(t);
         const double k = __dsub_rn(t, magic);
@@ -206,11 +221,12 @@ struct RowCtx {
         q = __fma_rn(r, q, 0.5);
         q = __fma_rn(__dmul_rn(r, r), q, r);
         const double s = table[n & 63];
-        const double v = __fma_rn(s, q, s);          // in [1, 2), or a hair below 1
-        const u64 bits = (u64)__double_as_longlong(v);
-        const u64 sig = (bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;          // v = sig * 2^(exponent - 52)
-        const int sh = (n >> 6) + (int)(bits >> 52) - 1023 + 10;                    // weight = sig * 2^sh, rounded
-        return sh >= 0 ? sig << sh : sh < -54 ? 0ull : (sig + (1ull << (-sh - 1))) >> -sh;
+        const double v = __fma_rn(s, q, s);
+        const double w = __hiloint2double(__double2hiint(v) + ((n & ~63) << 14), __double2loint(v));   // times 2^(n >> 6)
+        const double m1 = 3145728.0, m2 = 0.00146484375;   // 1.5 * 2^21, 1.5 * 2^-10
+        const double t1 = __dadd_rn(w, m1);
+        const double t2 = __dadd_rn(__dsub_rn(w, __dsub_rn(t1, m1)), m2);
+        return Weight{(unsigned)__double2loint(t1), __double2loint(t2)};
     }
     __device__ __forceinline__ bool is_candidate(float x, int i) const { return x == x && (floor_c == 0ull || comp(x, i) >= floor_c); }
     // bin of a logit: never decreases as the logit falls
@@ -463,7 +479,7 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx rc, FullShared* sh
                         if (c >= floor_c && (c & mask) == pfx) {
                             active = true;
                             digit = (int)((unsigned)(c >> lo) & dmask);
-                            if (!by_count) wgt = rc.weight(x);
+                            if (!by_count) wgt = rc.weight(x).value();
                         }
                     }
                 }
@@ -518,19 +534,19 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx rc, FullShared* sh
 }
 
 // ---- cumulative weights by bin ----------------------------------------------------------------------------------------
-// About how many candidates a bin holds, from its weight (units of 2^-32): right to a few per cent unless the bins are wide.
+// About how many candidates a bin holds, from its weight (units of 2^-31): right to a few per cent unless the bins are wide.
 // Clamped, so that sums do not overflow.
 __device__ __forceinline__ unsigned estimated_count(const RowCtx& rc, int bin, u64 weight) {
     const float middle = ((float)bin + 0.5f) / (rc.bin_scale * (float)rc.temp);   // of the bin, below the maximum, in temperatures
-    const float n = (float)weight * exp2f(fminf(middle * 1.442695f, 60.0f) - 32.0f);
+    const float n = (float)weight * exp2f(fminf(middle * 1.442695f, 60.0f) - 31.0f);
     return n < 1e6f ? (unsigned)n + (weight ? 1u : 0u) : 1000000u;
 }
 
 // First bin whose cumulative weight reaches t (2^-62 units) for certain, and the first that may reach it, given that up to
-// n candidates were rounded down by less than one unit each.  All threads call; contains barriers.
+// n candidates were rounded by half a unit each.  All threads call; contains barriers.
 __device__ __forceinline__ void find_bins(FullShared* sh, U128 t, unsigned n) {
     const int b = threadIdx.x;
-    const u64 t_lo = (t.hi << 34) | (t.lo >> 30), t_up = t_lo + ((t.lo & 0x3FFFFFFFull) ? 1ull : 0ull);   // t < 2^80
+    const u64 slack = n / 2u + 1u, t_lo = (t.hi << 33) | (t.lo >> 31), t_up = t_lo + 1ull + slack;   // t < 2^80
     const u64 c = sh->cum[b], before = b > 0 ? sh->cum[b - 1] : 0ull;
     if (b == 0) {
         sh->bin_lo = kBins - 1;
@@ -538,7 +554,7 @@ __device__ __forceinline__ void find_bins(FullShared* sh, U128 t, unsigned n) {
     }
     __syncthreads();
     if (c >= t_up && (b == 0 || before < t_up)) sh->bin_hi = b;
-    if (c + n >= t_lo && (b == 0 || before + n < t_lo)) sh->bin_lo = b;
+    if (c + slack >= t_lo && (b == 0 || before + slack < t_lo)) sh->bin_lo = b;
     __syncthreads();
 }
 
@@ -574,8 +590,19 @@ __device__ __forceinline__ void block_sums(FullShared* sh, int use, u64 lo, u64 
         }
     }
 }
-// A sum of weights kept as (sum of their low 32 bits, sum of their upper bits).
-__device__ __forceinline__ U128 join_words(u64 lo, u64 hi) { return u128_add(U128{0ull, lo}, U128{hi >> 32, hi << 32}); }
+// A sum of weights kept as the sums of their parts.
+__device__ __forceinline__ U128 join_parts(u64 down, u64 up) { return u128_add(U128{(long long)down < 0 ? ~0ull : 0ull, down}, U128{up >> 33, up << 31}); }
+
+// Four consecutive logits of the slice; what lies past its end is NaN.
+__device__ __forceinline__ void load4(const RowCtx& rc, int i, float (&x)[4]) {
+    if (rc.vals && i + 4 <= rc.n) {
+        const float4 v = *reinterpret_cast<const float4*>(rc.vals + i);
+        x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[e] = i + e < rc.n ? rc.at(i + e) : __int_as_float(0x7fc00000);
+}
 
 // Hands this CTA's candidates of bins [b_lo, b_hi] to the first CTA of the cluster, and adds up its weights and candidates of
 // the bins before them.  Returns whether everybody's candidates fitted.  After it the first CTA has the lists (CTA r's
@@ -586,33 +613,50 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
     if (tid == 0) sh->sent = 0;
     __syncthreads();
     const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u);
-    u64 lo = 0ull, hi = 0ull;
+    u64 down = 0ull, up = 0ull;
     unsigned cnt = 0u;
     const int lane = tid & 31;
+    const float ninf = -__int_as_float(0x7f800000);
     bool full = false;   // (then nothing more is handed over: the lists are of no use)
-    for (int i0 = tid - lane; i0 < rc.n; i0 += kFullThreads) {
-        const int i = i0 + lane;
-        const float x = i < rc.n ? rc.vals[i] : __int_as_float(0x7fc00000);
-        const int b = rc.bin(x);
-        const bool in = x == x && b <= b_hi && rc.is_candidate(x, i), give = in && b >= b_lo && !full;
-        const unsigned hits = __ballot_sync(0xffffffffu, give);
-        if (hits) {
-            int p = 0;
-            if (lane == 0) p = atomicAdd(&sh->sent, __popc(hits));
-            p = __shfl_sync(0xffffffffu, p, 0);
-            full = p >= kSendCap;
-            p += __popc(hits & ((1u << lane) - 1u));
-            if (give && p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x, i));
+    for (int i0 = 4 * (tid - lane); i0 < rc.n; i0 += 4 * kFullThreads) {
+        float x[4];
+        load4(rc, i0 + 4 * lane, x);
+        bool give[4], above[4], some = false, any_above = false;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int b = rc.bin(x[e]);
+            const bool in = b <= b_hi && rc.is_candidate(x[e], i0 + 4 * lane + e);
+            give[e] = in && b >= b_lo;
+            above[e] = in && b < b_lo;
+            some = some || give[e];
+            any_above = any_above || above[e];
         }
-        if (!sums && full) break;
-        if (sums && in && b < b_lo) {
-            const u64 w = rc.weight(x);
-            lo += w & 0xFFFFFFFFull;
-            hi += w >> 32;
-            ++cnt;
+        if (__any_sync(0xffffffffu, some) && !full) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const unsigned hits = __ballot_sync(0xffffffffu, give[e]);
+                if (hits == 0u) continue;
+                int p = 0;
+                if (lane == 0) p = atomicAdd(&sh->sent, __popc(hits));
+                p = __shfl_sync(0xffffffffu, p, 0);
+                full = full || p >= kSendCap;
+                p += __popc(hits & ((1u << lane) - 1u));
+                if (give[e] && p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x[e], i0 + 4 * lane + e));
+            }
+        }
+        if (!sums) {
+            if (full) break;
+        } else if (any_above) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const Weight w = rc.weight(above[e] ? x[e] : ninf);
+                up += w.up;
+                down += (u64)(long long)w.down;
+                cnt += above[e] ? 1u : 0u;
+            }
         }
     }
-    if (sums) block_sums(sh, par, lo, hi, cnt);
+    if (sums) block_sums(sh, par, down, up, cnt);
     else __syncthreads();
     if (tid < C) cluster_store_u32(map_to_rank(&sh->got[par][rank], (unsigned)tid), (unsigned)sh->sent);
     cluster_sync_all();
@@ -754,9 +798,10 @@ __device__ __forceinline__ ListScan<T> scan_list(const RowCtx& rc, FullShared* s
 #pragma unroll
     for (int q = 0; q < ListScan<T>::kPer; ++q) {
         const int e = tid * ls.per + q;
-        ls.w[q] = q < ls.per && e < n ? rc.weight(comp_value(srt[e])) : 0ull;
-        lo += ls.w[q] & 0xFFFFFFFFull;
-        hi += ls.w[q] >> 32;
+        const Weight w = q < ls.per && e < n ? rc.weight(comp_value(srt[e])) : Weight{0u, 0};
+        ls.w[q] = w.value();
+        lo += (u64)(long long)w.down;
+        hi += w.up;
     }
     u64 ilo = lo, ihi = hi;
 #pragma unroll
@@ -783,7 +828,7 @@ __device__ __forceinline__ ListScan<T> scan_list(const RowCtx& rc, FullShared* s
             wh += __shfl_xor_sync(0xffffffffu, wh, o);
         }
     }
-    ls.before = u128_add(above, join_words(wl + ilo - lo, wh + ihi - hi));
+    ls.before = u128_add(above, join_parts(wl + ilo - lo, wh + ihi - hi));
     return ls;
 }
 
@@ -798,7 +843,7 @@ __device__ __forceinline__ void cross_list(const RowCtx& rc, FullShared* sh, int
         cnt += ld_cluster_u64(map_to_rank(&sh->x_small[use][2], r));
     }
     const u64* srt = order_lists<C, T>(sh, use, n);
-    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, join_words(lo, hi));
+    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, join_parts(lo, hi));
     ls.each(n, [&](int e, U128 before, U128 with) {
         if (u128_ge(with, target) && (!u128_ge(before, target) || e == 0)) {
 #pragma unroll
@@ -837,7 +882,7 @@ __device__ __forceinline__ int finish_list(const RowCtx& rc, FullShared* sh, int
     const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, U128{0ull, 0ull});
     ls.each(n, [&](int e, U128 before, U128 with) {
         if (cuts.top_p && u128_ge(with, cuts.target_p) && !u128_ge(before, cuts.target_p)) atomicMin(&sh->first_p, e + 1);
-        if (cuts.min_p && __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), cuts.sum) < cuts.min_thr) atomicMin(&sh->first_p, max(e, 1));
+        if (cuts.min_p && rc.probability(comp_value(srt[e]), cuts.sum) < cuts.min_thr) atomicMin(&sh->first_p, max(e, 1));
     });
     list_sync<T>();
     const int keep = min(sh->first_p, n);
@@ -853,7 +898,7 @@ __device__ __forceinline__ int finish_list(const RowCtx& rc, FullShared* sh, int
         if (u128_ge(with, target)) atomicMin(&sh->first_u, e);
         if (a.record && e < kMaxK) {
             a.kept_ids[(size_t)out * kMaxK + e] = comp_id(srt[e]);
-            a.kept_pr[(size_t)out * kMaxK + e] = __ddiv_rn(exp(rc.scaled(comp_value(srt[e]))), cuts.sum);
+            a.kept_pr[(size_t)out * kMaxK + e] = rc.probability(comp_value(srt[e]), cuts.sum);
         }
     });
     list_sync<T>();
@@ -936,7 +981,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         }
         __syncthreads();
     }
-    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, -43.8 * (double)d.temperature, sh->table, 0ull, 0.0f};
+    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, -45.0f * d.temperature, false, sh->table, 0ull, 0.0f};
     const float ninf = -__int_as_float(0x7f800000);
     float mx = ninf, mn = -ninf;
     unsigned valid = 0u;
@@ -1046,6 +1091,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     }
     rc.mx = mx;
     rc.inv_temp = __ddiv_rn(1.0, rc.temp);
+    rc.odd = !(mx < -ninf && mx > ninf) || d.temperature > 1e36f;
     FTR(2);
 
     // ---- 2. the k-th candidate (k < n only)
@@ -1058,7 +1104,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     // ---- 3. the weights' exact sum, the number of candidates, and the histogram
     // (a row whose largest logit is infinite, or that is too long for shared memory, is left to the descents)
     const float inf = -ninf;
-    const bool binned = rc.vals != nullptr && mx < inf && mx > ninf;
+    const bool binned = rc.vals != nullptr && !rc.odd;
     // weights are zero 43.7 temperatures below the maximum: no bins are spent on what lies further down
     rc.bin_scale = (float)kBins / fminf(44.0f * d.temperature, mx - mn);
     if (!(rc.bin_scale < inf)) rc.bin_scale = 0.0f;
@@ -1068,39 +1114,54 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     const double band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
     const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
     U128 S;
-    unsigned n_cand;
+    const unsigned n_cand = rc.floor_c != 0ull ? (unsigned)d.k : valid;
     {
-        u64 wl = 0ull, wh = 0ull;
-        unsigned cnt = 0u;
-        auto weigh = [&](float x, int i) {
-            if (!rc.is_candidate(x, i)) return;
-            ++cnt;
-            const u64 w = rc.weight(x);
-            wl += w & 0xFFFFFFFFull;
-            wh += w >> 32;
-            const unsigned up = (unsigned)(w >> 46), down = (unsigned)(w >> 30) & 0xFFFFu;
-            if (binned && (up | down)) {
-                const int bin = rc.bin(x);
-                if (up) atomicAdd(&sh->hist[0][bin], up);
-                if (down) atomicAdd(&sh->hist[1][bin], down);
+        u64 wl = 0ull, wh = 0ull;   // sums of the weights' lower and upper parts
+        for (int i = 4 * tid; i < n; i += 4 * kFullThreads) {
+            float x[4];
+            load4(rc, i, x);
+            if (rc.floor_c != 0ull) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = rc.is_candidate(x[e], i + e) ? x[e] : ninf;
             }
-        };
-#pragma unroll 4
-        for (int i = tid; i < n; i += kFullThreads) weigh(rc.at(i), i);
-        block_sums(sh, par, wl, wh, cnt);
+            Weight w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                w[e] = rc.weight(x[e]);
+                wl += (u64)(long long)w[e].down;
+                wh += w[e].up;
+            }
+            if (binned && (w[0].up | w[1].up | w[2].up | w[3].up)) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int bin = rc.bin(x[e]);
+                    if (w[e].up >> 16) atomicAdd(&sh->hist[0][bin], w[e].up >> 16);
+                    if (w[e].up & 0xFFFFu) atomicAdd(&sh->hist[1][bin], w[e].up & 0xFFFFu);
+                }
+            }
+        }
+        block_sums(sh, par, wl, wh, 0u);
         cluster_sync_all();
         // Every CTA adds up kBins / C of the bins and hands the sums to all others: one load and one store per thread across the
         // cluster (all bins read from all CTAs took 2.3 us).
         {
-            constexpr int kMine = kBins / C;
-            const int src = tid / kMine, bin = (int)rank * kMine + tid % kMine;
-            sh->part[tid] = ((u64)ld_cluster_u32(map_to_rank(&sh->hist[0][bin], (unsigned)src)) << 16) + ld_cluster_u32(map_to_rank(&sh->hist[1][bin], (unsigned)src));
+            constexpr int kMine = (kBins + C - 1) / C;   // (six CTAs: 171, and C * kMine is two more than there are threads)
+            static_assert(C * kMine <= kFullThreads + 8, "the parts' memory");
+            for (int t = tid; t < C * kMine; t += kFullThreads) {
+                const int src = t / kMine, bin = (int)rank * kMine + t % kMine;
+                if (bin < kBins)
+                    sh->part[t] = ((u64)ld_cluster_u32(map_to_rank(&sh->hist[0][bin], (unsigned)src)) << 16) + ld_cluster_u32(map_to_rank(&sh->hist[1][bin], (unsigned)src));
+            }
             if (tid < C * 4) sh->x_all[par][tid] = ld_cluster_u64(map_to_rank(&sh->x_small[par][tid & 3], (unsigned)tid >> 2));
             __syncthreads();
-            u64 c = 0ull;
+            for (int t = tid; t < C * kMine; t += kFullThreads) {
+                const int dst = t / kMine, bin = (int)rank * kMine + t % kMine;
+                if (bin >= kBins) continue;
+                u64 c = 0ull;
 #pragma unroll
-            for (int r = 0; r < C; ++r) c += sh->part[r * kMine + tid % kMine];
-            cluster_store_u64(map_to_rank(&sh->cum[bin], (unsigned)src), c);
+                for (int r = 0; r < C; ++r) c += sh->part[r * kMine + t % kMine];
+                cluster_store_u64(map_to_rank(&sh->cum[bin], (unsigned)dst), c);
+            }
         }
         cluster_sync_all();
         // inclusive sums over the bins, largest logits first
@@ -1128,14 +1189,12 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         sh->cum[tid] = c + t;
         sh->cum_n[tid] = est;
         wl = wh = 0ull;
-        n_cand = 0u;
 #pragma unroll
         for (int r = 0; r < C; ++r) {
             wl += sh->x_all[par][4 * r];
             wh += sh->x_all[par][4 * r + 1];
-            n_cand += (unsigned)sh->x_all[par][4 * r + 2];
         }
-        S = join_words(wl, wh);
+        S = join_parts(wl, wh);
         par ^= 1;
         __syncthreads();
     }
@@ -1181,7 +1240,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         for (int i = tid; i < n; i += kFullThreads) {
             const float x = rc.at(i);
             if (!rc.is_candidate(x, i) || x < x_never) continue;
-            if (x > x_sure || !(__ddiv_rn(exp(rc.scaled(x)), sum) < min_thr)) lowest = min(lowest, rc.comp(x, i));
+            if (x > x_sure || !(rc.probability(x, sum) < min_thr)) lowest = min(lowest, rc.comp(x, i));
         }
         lowest = ~block_max_u64(~lowest, sh);
         u64 v[4] = {~lowest, 0ull, 0ull, 0ull}, all[C][4];
@@ -1207,7 +1266,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     U128 KW = S;
     unsigned n_keep = n_cand;
     if (keep_from_top_p) {
-        KW = u128_add(cp.above, U128{0ull, rc.weight(comp_value(cp.c))});
+        KW = u128_add(cp.above, U128{0ull, rc.weight(comp_value(cp.c)).value()});
         n_keep = cp.above_cnt + 1u;
     } else if (c_keep != c_k) {
         u64 wl = 0ull, wh = 0ull;
@@ -1215,9 +1274,9 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         for (int i = tid; i < n; i += kFullThreads) {
             const float x = rc.at(i);
             if (x == x && rc.comp(x, i) >= c_keep) {
-                const u64 w = rc.weight(x);
-                wl += w & 0xFFFFFFFFull;
-                wh += w >> 32;
+                const Weight w = rc.weight(x);
+                wl += (u64)(long long)w.down;
+                wh += w.up;
                 ++pc;
             }
         }
@@ -1230,7 +1289,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             wh += ld_cluster_u64(map_to_rank(&sh->x_small[par][1], r));
             n_keep += (unsigned)ld_cluster_u64(map_to_rank(&sh->x_small[par][2], r));
         }
-        KW = join_words(wl, wh);
+        KW = join_parts(wl, wh);
         par ^= 1;
     }
     FTR(7);
@@ -1281,7 +1340,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
                 int rank_in = 0;
                 for (int j = 0; j < want; ++j) rank_in += srt[j] > c ? 1 : 0;
                 a.kept_ids[(size_t)out * kMaxK + rank_in] = comp_id(c);
-                a.kept_pr[(size_t)out * kMaxK + rank_in] = __ddiv_rn(exp(rc.scaled(comp_value(c))), sum);
+                a.kept_pr[(size_t)out * kMaxK + rank_in] = rc.probability(comp_value(c), sum);
             }
             if (tid == 0) a.kept_n[out] = (int)n_keep;
         }
@@ -1301,35 +1360,50 @@ size_t full_row_smem_bytes(int n_vocab, int cluster) {
     return sizeof(FullShared) + bitmap + 16 + slice;
 }
 template <int C>
-int launch_full(const FullArgs& a, int n_rows, cudaStream_t stream) {
-    cudaLaunchAttribute attr[1];
+void fill_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int n_rows, int n_vocab) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = C;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(n_rows * C));
     cfg.blockDim = dim3(kFullThreads);
-    cfg.dynamicSmemBytes = full_row_smem_bytes(a.n_vocab, C);
-    cfg.stream = stream;
+    cfg.dynamicSmemBytes = full_row_smem_bytes(n_vocab, C);
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+}
+template <int C>
+int launch_full(const FullArgs& a, int n_rows, cudaStream_t stream) {
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg{};
+    fill_config<C>(cfg, attr, n_rows, a.n_vocab);
+    cfg.stream = stream;
     return (int)cudaLaunchKernelEx(&cfg, full_row_kernel<C>, a, slice_of(a.n_vocab, C) <= kSliceCache ? 1 : 0);
+}
+// How many clusters of C CTAs run at once.  A cluster lies in one GPC, so this is less than SMs / C: 15 of eight on B200's
+// 148 SMs, 22 of six, 33 of four.
+int g_at_once[3] = {0, 0, 0};
+template <int C>
+int prepare_full(int max_vocab, int& at_once) {
+    // the largest request of any row length up to max_vocab: rows that still fit the slice cache need the most
+    const size_t most = std::max(C == kMaxCluster ? full_row_smem_bytes(max_vocab, C) : 0, full_row_smem_bytes(std::min(max_vocab, C * kSliceCache), C));
+    cudaError_t e = cudaFuncSetAttribute(full_row_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess || at_once > 0) return (int)e;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg{};
+    fill_config<C>(cfg, attr, 64, std::min(max_vocab, C * kSliceCache));
+    return (int)cudaOccupancyMaxActiveClusters(&at_once, full_row_kernel<C>, &cfg);
 }
 }  // namespace
 
 int prepare_full_row_kernel(int max_vocab) {
-    // the largest request of any row length up to max_vocab: rows that still fit the slice cache need the most
-    const size_t most8 = std::max(full_row_smem_bytes(max_vocab, 8), full_row_smem_bytes(std::min(max_vocab, 8 * kSliceCache), 8));
-    const size_t most4 = full_row_smem_bytes(std::min(max_vocab, 4 * kSliceCache), 4);
-    cudaError_t e = cudaFuncSetAttribute(full_row_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most8);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(full_row_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most4);
-    return (int)e;
+    for (int e : {prepare_full<8>(max_vocab, g_at_once[2]), prepare_full<6>(max_vocab, g_at_once[1]), prepare_full<4>(max_vocab, g_at_once[0])})
+        if (e != 0) return e;
+    return 0;
 }
 
 int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, const int32_t* drafts, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
                            int32_t* kept_ids, double* kept_pr, int32_t* kept_n, int record, uint32_t* status, uint32_t* status_host, int n_vocab,
-                           int vocab_offset, int write_back, float softcap, uint64_t* trace, int sms, void* stream) {
+                           int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream) {
     if (n_vocab > (1 << 22)) return (int)cudaErrorInvalidValue;   // the histogram's limb sums are sized for 4 M logits
     FullArgs a{};
     a.logits = logits;
@@ -1350,10 +1424,21 @@ int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows,
     a.record = record;
     a.softcap = softcap;
     a.trace = reinterpret_cast<u64*>(trace);
-    // Eight CTAs per row while they fit the SMs at once, one each; with more rows four, which pay the steps between the passes
-    // half as often.
-    if ((int64_t)n_rows * 8 > sms && slice_of(n_vocab, 4) <= kSliceCache) return launch_full<4>(a, n_rows, static_cast<cudaStream_t>(stream));
-    return launch_full<8>(a, n_rows, static_cast<cudaStream_t>(stream));
+    // The more CTAs per row the shorter the passes, but a second wave of clusters costs as much as the first.  Measured on B200
+    // (us, eight / six / four CTAs): see the rule's two terms, the steps between the passes and the passes.
+    int best = 8;
+    double cost = 1e30;
+    for (int i = 2; i >= 0; --i) {
+        const int c = 4 + 2 * i, per = slice_of(n_vocab, c), at_once = std::max(1, g_at_once[i]);
+        if (c < 8 && per > kSliceCache) continue;
+        const double t = ((n_rows + at_once - 1) / at_once) * (16.0 + 1.2 * per / 1024.0);
+        if (t < cost) {
+            cost = t;
+            best = c;
+        }
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return best == 8 ? launch_full<8>(a, n_rows, st) : best == 6 ? launch_full<6>(a, n_rows, st) : launch_full<4>(a, n_rows, st);
 }
 
 }  // namespace fsb
