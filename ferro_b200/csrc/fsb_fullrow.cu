@@ -246,32 +246,6 @@ __device__ __forceinline__ u64 block_max_u64(u64 v, FullShared* sh) {
     return r;
 }
 
-// Largest `hi` and smallest `lo` over the CTA in one go.
-__device__ __forceinline__ void block_max2_u64(u64& hi, u64& lo, FullShared* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    u64 a = hi, b = ~lo;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        a = max(a, __shfl_xor_sync(0xffffffffu, a, o));
-        b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    if (lane == 0) {
-        sh->red[warp] = a;
-        sh->red_hi[warp] = b;
-    }
-    __syncthreads();
-    a = sh->red[lane];
-    b = sh->red_hi[lane];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        a = max(a, __shfl_xor_sync(0xffffffffu, a, o));
-        b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    __syncthreads();
-    hi = a;
-    lo = ~b;
-}
-
 // Exchanges up to four 64-bit values per CTA across the cluster: every CTA gets all C x 4 values.
 // `use` alternates 0/1 between consecutive exchanges.  Contains one cluster barrier.
 template <int C>
@@ -286,31 +260,6 @@ __device__ __forceinline__ void cluster_exchange(FullShared* sh, int use, const 
     for (int r = 0; r < C; ++r)
 #pragma unroll
         for (int j = 0; j < 4; ++j) all[r][j] = sh->x_all[use][r * 4 + j];
-}
-
-// Exact sum of one 128-bit value and one count per thread over the CTA.
-__device__ __forceinline__ void block_sum_u128(U128& v, unsigned& cnt, FullShared* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const u64 l = __shfl_xor_sync(0xffffffffu, v.lo, o);
-        const u64 h = __shfl_xor_sync(0xffffffffu, v.hi, o);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        v = u128_add(v, U128{h, l});
-    }
-    if (lane == 0) {
-        sh->red[warp] = v.lo;
-        sh->red_hi[warp] = v.hi;
-        sh->red_cnt[warp] = cnt;
-    }
-    __syncthreads();
-    v = U128{0ull, 0ull};
-    cnt = 0u;
-    for (int w = 0; w < kFullWarps; ++w) {
-        v = u128_add(v, U128{sh->red_hi[w], sh->red[w]});
-        cnt += sh->red_cnt[w];
-    }
-    __syncthreads();
 }
 
 // Adds (digit, weight, one candidate) to the level histogram: native 32-bit shared-memory atomics on the count and on
@@ -618,6 +567,14 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
     const int lane = tid & 31;
     const float ninf = -__int_as_float(0x7f800000);
     bool full = false;   // (then nothing more is handed over: the lists are of no use)
+    float* pending = reinterpret_cast<float*>(sh->part) + (tid >> 5) * 64;
+    static_assert(sizeof(FullShared::part) >= kFullWarps * 64 * sizeof(float), "63 logits may wait per warp");
+    int waiting = 0;
+    auto add = [&](float x) {
+        const Weight w = rc.weight(x);
+        up += w.up;
+        down += (u64)(long long)w.down;
+    };
     for (int i0 = 4 * (tid - lane); i0 < rc.n; i0 += 4 * kFullThreads) {
         float x[4];
         load4(rc, i0 + 4 * lane, x);
@@ -646,15 +603,28 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
         }
         if (!sums) {
             if (full) break;
-        } else if (any_above) {
+            continue;
+        }
+        // the logits above are collected until the warp has 32 of them: often they are few, and a weight costs as much for one
+        // lane as for all
+        if (!__any_sync(0xffffffffu, any_above)) continue;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const Weight w = rc.weight(above[e] ? x[e] : ninf);
-                up += w.up;
-                down += (u64)(long long)w.down;
-                cnt += above[e] ? 1u : 0u;
+        for (int e = 0; e < 4; ++e) {
+            const unsigned hits = __ballot_sync(0xffffffffu, above[e]);
+            if (above[e]) pending[waiting + __popc(hits & ((1u << lane) - 1u))] = x[e];
+            waiting += __popc(hits);
+            __syncwarp();
+            if (waiting >= 32) {
+                waiting -= 32;
+                add(pending[waiting + lane]);
+                cnt += 1u;
+                __syncwarp();
             }
         }
+    }
+    if (sums && waiting > 0) {
+        add(lane < waiting ? pending[lane] : ninf);
+        cnt += lane < waiting ? 1u : 0u;
     }
     if (sums) block_sums(sh, par, down, up, cnt);
     else __syncthreads();
@@ -1214,7 +1184,8 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             b_hi = sh->bin_hi;
         }
         if (d.min_p > 0.0f) b_hi = min(b_hi, rc.bin(x_never));
-        if (sh->cum_n[b_hi] <= (unsigned)(C * kSendCap / 2) && send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
+        // (a list of more than a thousand is ordered too slowly: 22 us for 2000, two crossings take 15)
+        if (sh->cum_n[b_hi] <= (unsigned)(3 * kFullThreads / 4) && send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
             FTR(5);
             if (rank != 0) return;   // nobody reads this CTA's memory any more
             const RowCuts cuts{target_p, u, sum, min_thr, d.top_p < 1.0f, d.min_p > 0.0f};
