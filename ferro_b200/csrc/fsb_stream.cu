@@ -42,11 +42,12 @@ constexpr int kCells = 4;                               // cells of a thread per
 constexpr int kStages = 2;
 constexpr int kPenCap = 1024;                           // penalised columns of a segment that are looked up ahead
 constexpr int kPickCap = 1024;                          // candidates of a segment
-constexpr int kSendCap = 256;                           // candidates a segment sends to the row's first CTA
-constexpr int kMergeList = 8 * kSendCap;                // candidates of all segments
+constexpr int kMergeList = 2048;                        // candidates of all segments, an equal share of it each
+constexpr int kHashSlots = 2048, kHashIds = 1024;       // hashed penalty windows: slots, and the longest window that may use them
 constexpr int kSelectSmemMax = 224 * 1024;
 static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merge list's memory");
 
+size_t window_bytes(int seg_cols, bool hashed);
 // Sizes that go with T, the threads of a CTA.
 template <int T>
 struct Geometry {
@@ -56,18 +57,25 @@ struct Geometry {
     // cells a warp can list; with k > 64
     static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64;
     static_assert((kPickCap + 32 + kMaxK + kMergeList + 32) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
-    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns), control block, maxima
-    // (k > 64), receive buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
-    static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
-        return kRingBytes + (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int)) +
-               (seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0) + sizeof(SharedCtl) + (kmax > 64 ? (size_t)kWarps * 64 * sizeof(unsigned) : 0) +
-               (nseg > 1 ? (size_t)nseg * kSendCap * sizeof(u64) : 0);
+    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns; not with a hashed window),
+    // control block, receive buffer, and the segment's penalised columns (see Segment)
+    static size_t smem_bytes(int nseg, int kmax, int seg_cols, bool hashed) {
+        const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int));
+        return kRingBytes + cells + sizeof(SharedCtl) + (nseg > 1 ? kMergeList * sizeof(u64) : 0) + window_bytes(seg_cols, hashed);
     }
 };
+size_t window_bytes(int seg_cols, bool hashed) {
+    if (seg_cols <= 0) return 0;
+    const size_t bits = (size_t)seg_cols + 32;
+    return hashed ? (bits / 32 + 32 + 127) / 128 * 16 + kHashSlots * sizeof(int) : (bits + 127) / 128 * 16 + kPenCap * (sizeof(float) + sizeof(int));
+}
 
+// The penalised columns of a segment are a bitmap with a bit per column - or, where that would take the room of other CTAs
+// (32 KB for a row of 262144 logits), a hash table of the columns and a bitmap with a bit per 32 columns.
 struct Segment {
     const float* row;          // the row's logits
     unsigned* bitmap;          // penalised columns (bit 0 = column bit0), valid when has_pen
+    int* hash;                 // kHashSlots columns (-1: free), or null
     const int32_t* hist;       // the penalty window: these ids ...
     const int32_t* drafts;     // ... then these
     int hist_len, window_len;  // ids in the first part, in both
@@ -81,7 +89,20 @@ struct Segment {
 __device__ __forceinline__ int window_id(const Segment& s, int i) { return i < s.hist_len ? s.hist[i] : s.drafts[i - s.hist_len]; }
 __device__ __forceinline__ float penalise(float x, float pen) { return x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen); }   // src/sampler.cpp:17
 __device__ __noinline__ float softcap_call(float x, float cap) { return __fmul_rn(cap, tanhf(__fdiv_rn(x, cap))); }          // src/model_gemma4.cpp:521
-__device__ __forceinline__ bool penalised(const Segment& s, int c) { return s.has_pen && ((s.bitmap[(c - s.bit0) >> 5] >> ((c - s.bit0) & 31)) & 1u); }
+__device__ __forceinline__ bool bit_of(const unsigned* bits, int i) { return (bits[i >> 5] >> (i & 31)) & 1u; }
+__device__ __forceinline__ unsigned hash_slot(int c) { return ((unsigned)c * 2654435761u) / (0x80000000u / (kHashSlots / 2)); }
+__device__ __forceinline__ bool hashed_column(const int* hash, int c) {   // (at least half of the slots are free)
+    for (unsigned h = hash_slot(c);; h = (h + 1u) & (kHashSlots - 1u)) {
+        const int v = hash[h];
+        if (v == c) return true;
+        if (v < 0) return false;
+    }
+}
+__device__ __forceinline__ bool penalised(const Segment& s, int c) {
+    if (!s.has_pen) return false;
+    if (s.hash) return bit_of(s.bitmap, (c - s.bit0) >> 5) && hashed_column(s.hash, c);
+    return bit_of(s.bitmap, c - s.bit0);
+}
 
 // Logit of column c as the sampler sees it.
 __device__ __forceinline__ float transform(float x, int c, const Segment& s) {
@@ -93,39 +114,31 @@ __device__ __forceinline__ float transform(float x, int c, const Segment& s) {
 // A bound that at least k logits of the segment reach, from the threads' maxima (each a logit of its own; two per
 // thread, of different cells).  Minus infinity - and what is no number - never reaches a bound.  All threads get the same
 // value; contains one barrier; buffers alternate, so that the next call may write while a slow warp still reads.
-//  k <= 64: the r-th largest thread maximum of every warp, r = ceil(k / warps), minimum over the warps: 1.3 k to 2 k logits
-//    reach it.  r warp reductions take the largest out one after the other (equal ones together: the bound is lower then).
-//    (The k-th largest of all threads' maxima, found by counting, lets fewer through but cost more than it saved.)
-//  otherwise: the same over the 64 maxima of every warp, ranked by counting; keys give up their low bits to be distinct,
-//    which lowers the bound by less than 2^-16 of its value.
+//  The r-th largest maximum of every warp, r = ceil(k / warps), minimum over the warps: 1.3 k to 2 k logits reach it.  r warp
+//  reductions take the largest out one after the other; keys give up their low bits to be distinct, which lowers the bound
+//  by less than 2^-17 of its value.  k <= 64 does with one maximum per thread.  (Ranks by counting over shared memory took
+//  2.6 us per call with 32 warps, this 0.4; the k-th largest of all threads' maxima lets fewer through but costs more.)
 template <int T, int BAR>
-__device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, int buf, SharedCtl* ctl, unsigned* maxima) {
+__device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, int buf, SharedCtl* ctl) {
     constexpr int kWarps = T / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned ka = (float_key(run_a) & ~63u) | (unsigned)(2 * lane), kb = (float_key(run_b) & ~63u) | (unsigned)(2 * lane + 1), top;
     if (k <= 64) {
-        unsigned key = float_key(fmaxf(run_a, run_b)), top = __reduce_max_sync(0xffffffffu, key);
+        ka = max(ka, kb);
+        top = __reduce_max_sync(0xffffffffu, ka);
         for (int r = (k - 1) / kWarps; r > 0; --r) {
-            if (key == top) key = 0u;
-            top = __reduce_max_sync(0xffffffffu, key);
+            if (ka == top) ka = 0u;
+            top = __reduce_max_sync(0xffffffffu, ka);
         }
-        if (lane == 0) ctl->top[buf][warp] = top;
     } else {
-        const int r = (k + kWarps - 1) / kWarps;
-        const unsigned ka = (float_key(run_a) & ~127u) | (unsigned)lane, kb = (float_key(run_b) & ~127u) | (unsigned)(lane + 32);
-        unsigned* mine = maxima + 64 * warp;
-        mine[lane] = ka;
-        mine[lane + 32] = kb;
-        __syncwarp();
-        int rank_a = 0, rank_b = 0;
-#pragma unroll 4
-        for (int i = 0; i < 16; ++i) {
-            const uint4 v = *reinterpret_cast<const uint4*>(mine + 4 * i);
-            rank_a += (v.x > ka ? 1 : 0) + (v.y > ka ? 1 : 0) + (v.z > ka ? 1 : 0) + (v.w > ka ? 1 : 0);
-            rank_b += (v.x > kb ? 1 : 0) + (v.y > kb ? 1 : 0) + (v.z > kb ? 1 : 0) + (v.w > kb ? 1 : 0);
+        top = __reduce_max_sync(0xffffffffu, max(ka, kb));
+        for (int r = (k - 1) / kWarps; r > 0; --r) {
+            if (ka == top) ka = 0u;
+            if (kb == top) kb = 0u;
+            top = __reduce_max_sync(0xffffffffu, max(ka, kb));
         }
-        if (rank_a == r - 1) ctl->top[buf][warp] = ka & ~127u;
-        if (rank_b == r - 1) ctl->top[buf][warp] = kb & ~127u;
     }
+    if (lane == 0) ctl->top[buf][warp] = top & ~63u;
     block_sync<T, BAR>();
     const unsigned m = __reduce_min_sync(0xffffffffu, ctl->top[buf][lane & (kWarps - 1)]);
     return fmaxf(key_float(m), -FLT_MAX);   // (also for the patterns just below minus infinity's key, which are no numbers)
@@ -285,6 +298,11 @@ __device__ __noinline__ void write_back(const Segment s) {
         for (int c = s.lo + threadIdx.x; c < s.hi; c += T) row[c] = transform(__ldcg(row + c), c, s);
         return;
     }
+    if (s.hash) {
+        for (int i = threadIdx.x; i < kHashSlots; i += T)
+            if (s.hash[i] >= 0) row[s.hash[i]] = penalise(__ldcg(row + s.hash[i]), s.pen);
+        return;
+    }
     for (int i = threadIdx.x; i < s.window_len; i += T) {
         const int c = window_id(s, i) - s.id_base;
         if (c < s.lo || c >= s.hi) continue;
@@ -326,6 +344,11 @@ __device__ __forceinline__ Segment make_segment(const StreamArgs& a, const RowSp
     Segment s;
     s.row = row_ptr;
     s.bitmap = bitmap;
+    s.hash = nullptr;
+    if (a.hashed) {
+        s.hash = reinterpret_cast<int*>(bitmap);
+        s.bitmap = bitmap + kHashSlots;
+    }
     s.hist = s.drafts = nullptr;
     s.hist_len = s.window_len = 0;
     s.lo = seg == 0 ? 0 : w.head + 4 * w.c_lo;
@@ -352,8 +375,24 @@ template <int T>
 __device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* ctl, float* pen_raw, int* pen_col) {
     const int tid = threadIdx.x, lane = tid & 31;
     int id = tid < s.window_len ? window_id(s, tid) : -1;
-    for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+    const int bits = s.hash ? (s.hi - s.bit0 + 31) >> 5 : s.hi - s.bit0;
+    for (int i = tid; i < (bits + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (s.hash)
+        for (int i = tid; i < kHashSlots / 4; i += T) reinterpret_cast<int4*>(s.hash)[i] = make_int4(-1, -1, -1, -1);
     __syncthreads();
+    if (s.hash) {
+        for (int i = tid; i < s.window_len; i += T) {
+            const int c = (i == tid ? id : window_id(s, i)) - s.id_base;
+            if (c < s.lo || c >= s.hi) continue;
+            unsigned h = hash_slot(c);
+            for (;; h = (h + 1u) & (kHashSlots - 1u)) {   // (a window has at most kHashIds ids: half of the slots stay free)
+                const int v = atomicCAS(&s.hash[h], -1, c);
+                if (v == -1 || v == c) break;
+            }
+            atomicOr(&s.bitmap[(c - s.bit0) >> 10], 1u << (((c - s.bit0) >> 5) & 31));
+        }
+        return;
+    }
     for (int i0 = tid & ~31; i0 < s.window_len; i0 += T) {
         const int next = i0 + T + lane < s.window_len ? window_id(s, i0 + T + lane) : -1;
         const int c = id - s.id_base;
@@ -379,7 +418,12 @@ __device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* c
 template <int T, class F>
 __device__ __forceinline__ void for_each_penalised(const Segment& s, int n_pen, const float* pen_raw, const int* pen_col, F f) {
     const int tid = threadIdx.x, lane = tid & 31;
-    if (n_pen <= kPenCap) {
+    if (s.hash) {
+        for (int i = tid; i < kHashSlots; i += T) {   // (a multiple of T)
+            const int c = s.hash[i];
+            f(c >= 0, c >= 0 ? __ldcg(s.row + c) : 0.0f, c);
+        }
+    } else if (n_pen <= kPenCap) {
         for (int i0 = tid & ~31; i0 < n_pen; i0 += T) {
             const bool in = i0 + lane < n_pen;
             f(in, in ? pen_raw[i0 + lane] : 0.0f, in ? pen_col[i0 + lane] : 0);
@@ -399,13 +443,25 @@ __device__ __forceinline__ void for_each_penalised(const Segment& s, int n_pen, 
 // Penalised logits of a thread's cells of a chunk (`j`: its first cell, counted from the segment's first; `left`: cells of
 // the segment from this chunk on) become minus infinity: they are looked at on their own.
 template <int T>
-__device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const unsigned* bitmap, int j, int left) {
+__device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const Segment& s, int j, int left) {
     const float ninf = -__int_as_float(0x7f800000);
-    const unsigned* w = bitmap + (j >> 3) + 1;
-    const int sh = 4 * (j & 7);
     unsigned bits[kCells];
+    if (s.hash) {
 #pragma unroll
-    for (int u = 0; u < kCells; ++u) bits[u] = (int)threadIdx.x + u * T < left ? w[u * (T / 8)] >> sh : 0u;
+        for (int u = 0; u < kCells; ++u) {
+            bits[u] = 0u;
+            const int at = j + u * T, block = (at >> 3) + 1;   // (columns count from bit0: 32 before the first cell)
+            if ((int)threadIdx.x + u * T < left && bit_of(s.bitmap, block)) {
+#pragma unroll 1
+                for (int e = 0; e < 4; ++e) bits[u] |= hashed_column(s.hash, s.bit0 + 32 + 4 * at + e) ? 1u << e : 0u;
+            }
+        }
+    } else {
+        const unsigned* w = s.bitmap + (j >> 3) + 1;
+        const int sh = 4 * (j & 7);
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) bits[u] = (int)threadIdx.x + u * T < left ? w[u * (T / 8)] >> sh : 0u;
+    }
     if ((bits[0] | bits[1] | bits[2] | bits[3]) & 15u) {
 #pragma unroll
         for (int u = 0; u < kCells; ++u) {
@@ -488,14 +544,14 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     float4* listed = reinterpret_cast<float4*>(smem_raw + G::kRingBytes);
     const int tid = threadIdx.x, lane = tid & 31;
     const int cell_cap = a.kmax > 64 ? G::kWarpCellsLong : G::kWarpCells;
+    const int pen_cap = a.penalised && !a.hashed ? kPenCap : 0;
     int* listed_num = reinterpret_cast<int*>(listed + kWarps * cell_cap);
     float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
-    int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised ? kPenCap : 0));
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised ? kPenCap : 0));
+    int* pen_col = reinterpret_cast<int*>(pen_raw + pen_cap);
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + pen_cap);
+    u64* recv = reinterpret_cast<u64*>(ctl + 1);
     listed += (tid >> 5) * cell_cap;   // the warp's own
     listed_num += (tid >> 5) * cell_cap;
-    unsigned* maxima = reinterpret_cast<unsigned*>(ctl + 1);
-    u64* recv = reinterpret_cast<u64*>(maxima + (a.kmax > 64 ? kWarps * 64 : 0));
     pdl_launch_dependents();
     trace_mark(a, 0);
     // Mode 1 waits only before its first write (unless it stores into the logits); otherwise only the launch's latency -
@@ -528,7 +584,7 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
         const int c = span.edge_column(tid, V, seg, nseg);
         ctl->edge[tid] = c >= 0 ? __ldcg(row_ptr + c) : qnan;
     }
-    Segment s = make_segment(a, span, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(recv + (nseg > 1 ? nseg * kSendCap : 0)));
+    Segment s = make_segment(a, span, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(recv + (nseg > 1 ? kMergeList : 0)));
     s.has_pen = (dp.flags & kRowPenalty) != 0;
     s.pen = dp.penalty;
     const int k = dp.k;
@@ -564,7 +620,7 @@ again_from_the_start:
         float4 x[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
-        if (s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - c_lo, left);
+        if (s.has_pen) mask_penalised<T>(x, s, j0 - c_lo, left);
         float m[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
@@ -576,9 +632,9 @@ again_from_the_start:
         run_a = max3(run_a, m[0], m[1]);
         run_b = max3(run_b, m[2], m[3]);
         fetch(c + kStages);   // into the stage just read
-        fresh = !again && ((c & (c + 1)) == 0 || thr <= -FLT_MAX || (k > 64 && c < 8));
+        fresh = !again && ((c & (c + 1)) == 0 || thr <= -FLT_MAX || (k > 64 && c < 4));
         if (fresh) {
-            thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl, maxima);
+            thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
             admit = thr;
             if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
             if (wn > cell_cap / 4) wn = prune_cells(listed, listed_num, wn, admit);
@@ -609,7 +665,7 @@ again_from_the_start:
     if (fresh || again) {
         __syncthreads();
     } else {
-        thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl, maxima);
+        thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
         admit = thr;
         if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
     }
@@ -685,12 +741,13 @@ again_from_the_start:
     if (nseg > 1) {
         const int lseg = nseg == 8 ? 3 : nseg == 4 ? 2 : 1;
         cluster_wait_acquire();   // every CTA of the row runs: the first one's shared memory may be written
-        const unsigned dst = cluster_map_shared(smem_u32(recv + seg * kSendCap), 0u);
-        if (n > kSendCap) {       // (k > 64, or many equal logits)
+        const int send_cap = min(kPickCap, kMergeList >> lseg);
+        const unsigned dst = cluster_map_shared(smem_u32(recv + seg * send_cap), 0u);
+        if (n > send_cap) {       // (many equal logits, or k > 64 and eight segments)
             rank_emit(picked, n, k, list, ctl, [&](int rank, u64 m) { cluster_store_u64(dst + 8u * (unsigned)rank, m); });
             n = min(n, k);
-        } else if (tid < n) {
-            cluster_store_u64(dst + 8u * (unsigned)tid, picked[tid]);
+        } else {
+            for (int i = tid; i < n; i += kPost) cluster_store_u64(dst + 8u * (unsigned)i, picked[i]);
         }
         if (tid == 0) cluster_store_u32(cluster_map_shared(smem_u32(&ctl->recv_n[seg]), 0u), (unsigned)n);
         __syncwarp();
@@ -703,14 +760,14 @@ again_from_the_start:
         cluster_wait_acquire();
         // a bound that k of them reach, then those that reach it (thread t looks after every (256 / nseg)-th candidate of one segment)
         const int q = tid & (nseg - 1), n_q = ctl->recv_n[q];
-        const u64* from = recv + q * kSendCap;
+        const u64* from = recv + q * send_cap;
         run_a = run_b = ninf;
         for (int i = tid >> lseg; i < n_q; i += kPost >> lseg) {
             const float y = comp_value(from[i]);
             if (i & (kPost >> lseg)) run_b = fmaxf(run_b, y);
             else run_a = fmaxf(run_a, y);
         }
-        const float floor_y = cta_bound<kPost, 1>(run_a, run_b, k, refreshes & 1, ctl, maxima);
+        const float floor_y = cta_bound<kPost, 1>(run_a, run_b, k, refreshes & 1, ctl);
         const float least = floor_y > -FLT_MAX ? floor_y : ninf;
         const int most = __reduce_max_sync(0xffffffffu, n_q);   // (every warp has threads of every segment)
         for (int i = tid >> lseg; (i - (tid >> lseg)) < most; i += kPost >> lseg) {
@@ -739,8 +796,8 @@ again_from_the_start:
 // meets its cells in ascending order), the CTA takes the largest composite, and one warp finishes the row.  No bound, no
 // lists, no barrier before the end.  (Not with a softcap, which makes different logits equal, nor with write-back or patched values for the host.)
 template <int T>
-size_t argmax_smem_bytes(int seg_cols) {
-    return Geometry<T>::kRingBytes + sizeof(SharedCtl) + (seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0);
+size_t argmax_smem_bytes(int seg_cols, bool hashed) {
+    return Geometry<T>::kRingBytes + sizeof(SharedCtl) + window_bytes(seg_cols, hashed);
 }
 
 template <int T, int NDESC>
@@ -751,8 +808,9 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     float4* ring = reinterpret_cast<float4*>(smem_raw);
     u64* best_of = reinterpret_cast<u64*>(smem_raw);   // after the stream: the warps' best, then the first masked columns
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem_raw + Geometry<T>::kRingBytes);
+    const int pen_cap = a.penalised && !a.hashed ? kPenCap : 0;
     float* pen_raw = reinterpret_cast<float*>(ctl + 1);
-    int* pen_col = reinterpret_cast<int*>(pen_raw + kPenCap);
+    int* pen_col = reinterpret_cast<int*>(pen_raw + pen_cap);
     const int tid = threadIdx.x, lane = tid & 31;
     pdl_launch_dependents();
     trace_mark(a, 0);
@@ -781,7 +839,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         if (edge_col >= 0) edge = __ldcg(row_ptr + edge_col);
     }
     if (nseg > 1) cluster_arrive_release();
-    Segment s = make_segment(a, w, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(pen_col + kPenCap));
+    Segment s = make_segment(a, w, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(pen_col + pen_cap));
     if (a.penalised) {   // (without windows nobody waits for the descriptor before the end)
         s.has_pen = (dp.flags & kRowPenalty) != 0;
         s.pen = dp.penalty;
@@ -795,7 +853,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     }
     trace_mark(a, 1);
 
-    float best = ninf;
+    float best = ninf, floor_x = ninf;
     float4 best_cell = make_float4(0.f, 0.f, 0.f, 0.f);
     int best_num = -1;
     for (int c = 0, j0 = w.c_lo + tid;; ++c, j0 += kChunkCells) {
@@ -805,15 +863,26 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         float4 x[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
-        if (s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - w.c_lo, left);
+        float m[kCells];
 #pragma unroll
-        for (int u = 0; u < kCells; ++u) {
-            const float m = cell_max(x[u]);
-            if (m > best && tid + u * T < left) {
-                best = m;
-                best_cell = x[u];
-                best_num = j0 + u * T;
+        for (int u = 0; u < kCells; ++u) m[u] = tid + u * T < left ? cell_max(x[u]) : ninf;
+        // (`floor_x` is the warp's best so far: what does not exceed it cannot win, and a warp rarely sees more than ten such chunks)
+        if (__any_sync(0xffffffffu, fmaxf(max3(m[0], m[1], m[2]), m[3]) > floor_x)) {
+            if (s.has_pen) {
+                mask_penalised<T>(x, s, j0 - w.c_lo, left);
+#pragma unroll
+                for (int u = 0; u < kCells; ++u)
+                    if (tid + u * T < left) m[u] = cell_max(x[u]);
             }
+#pragma unroll
+            for (int u = 0; u < kCells; ++u) {
+                if (m[u] > best) {
+                    best = m[u];
+                    best_cell = x[u];
+                    best_num = j0 + u * T;
+                }
+            }
+            floor_x = key_float(__reduce_max_sync(0xffffffffu, float_key(best)));
         }
         fetch(c + kStages);
         if (left <= kChunkCells) break;
@@ -864,17 +933,22 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
 }
 
 template <int T, int NDESC>
-int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows, const int32_t* ids, int n_ids) {
+int launch_select(cudaLaunchConfig_t& cfg, StreamArgs a, const RowDesc* rows, const int32_t* ids, int n_ids) {
     const int seg_cols = a.penalised ? 4 * ((a.n_vocab / 4 + a.nseg - 1) / a.nseg) + 8 : 0;
     cfg.blockDim = dim3(T);
-    cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols);
+    a.hashed = 0;
+    cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols, false);
     if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
     SelectArgs<NDESC> args;
     args.a = a;
     if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
     if (NDESC == kFewRows && n_ids > 0) std::memcpy(args.ids, ids, sizeof(int32_t) * (size_t)n_ids);
     if (a.all_greedy && a.softcap == 0.0f && !a.write_back && !a.patched) {
-        cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols);
+        // Whole rows on small CTAs, four per SM: the bitmap of a row of more than 65536 logits would leave room for three or two.
+        // (512 x 262144 with windows of 512 ids: 109 us, hashed 91.  The general kernel, which meets the windows' columns in every
+        // chunk, loses more by the look-ups than it gains: 103 against 129.)
+        args.a.hashed = T == 256 && a.nseg == 1 && seg_cols > 65536 + 8 && a.window_max <= kHashIds ? 1 : 0;
+        cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols, args.a.hashed);
         return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
     }
     return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC>, args);
