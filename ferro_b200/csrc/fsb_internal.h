@@ -79,8 +79,6 @@ struct StreamArgs {
     int32_t wide;              // large CTAs (see SelectPlan)
     int32_t kmax;              // largest k of the rows
     int32_t all_greedy;        // every row is greedy
-    int32_t window_max;        // ids of the longest penalty window
-    int32_t hashed;            // the launch keeps the windows in hash tables (set by launch_stream_kernel)
     int32_t penalised;         // some row has a penalty window
     int32_t write_back;        // store penalised values into the caller's rows
     int32_t vocab_offset;      // token id of column 0
@@ -94,7 +92,7 @@ struct SelectPlan {
     int nseg = 1;
     bool wide = false;
 };
-SelectPlan plan_select(int n_rows, int n_vocab, int sms);
+SelectPlan plan_select(int n_rows, int n_vocab, int sms, int kmax, bool all_greedy, bool penalised);
 
 // All return a cudaError_t as int (0 = success).
 int prepare_device_kernels();

@@ -42,12 +42,16 @@ constexpr int kCells = 4;                               // cells of a thread per
 constexpr int kStages = 2;
 constexpr int kPenCap = 1024;                           // penalised columns of a segment that are looked up ahead
 constexpr int kPickCap = 1024;                          // candidates of a segment
+constexpr int kLongGap = 2;                              // unused words before the receive buffer if k > 64
 constexpr int kMergeList = 2048;                        // candidates of all segments, an equal share of it each
-constexpr int kHashSlots = 2048, kHashIds = 1024;       // hashed penalty windows: slots, and the longest window that may use them
 constexpr int kSelectSmemMax = 224 * 1024;
 static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merge list's memory");
 
-size_t window_bytes(int seg_cols, bool hashed);
+// Columns of the longest segment.
+int segment_columns(int n_vocab, int nseg) { return 4 * ((n_vocab / 4 + nseg - 1) / nseg) + 8; }
+// A segment's penalised columns: logits and numbers of the first kPenCap, and a bitmap.
+size_t window_bytes(int seg_cols) { return seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0; }
+
 // Sizes that go with T, the threads of a CTA.
 template <int T>
 struct Geometry {
@@ -57,25 +61,17 @@ struct Geometry {
     // cells a warp can list; with k > 64
     static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64;
     static_assert((kPickCap + 32 + kMaxK + kMergeList + 32) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
-    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns; not with a hashed window),
-    // control block, receive buffer, and the segment's penalised columns (see Segment)
-    static size_t smem_bytes(int nseg, int kmax, int seg_cols, bool hashed) {
+    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns), control block, receive
+    // buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
+    static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
         const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int));
-        return kRingBytes + cells + sizeof(SharedCtl) + (nseg > 1 ? kMergeList * sizeof(u64) : 0) + window_bytes(seg_cols, hashed);
+        return kRingBytes + cells + sizeof(SharedCtl) + (kLongGap + (nseg > 1 ? kMergeList : 0)) * sizeof(u64) + window_bytes(seg_cols);
     }
 };
-size_t window_bytes(int seg_cols, bool hashed) {
-    if (seg_cols <= 0) return 0;
-    const size_t bits = (size_t)seg_cols + 32;
-    return hashed ? (bits / 32 + 32 + 127) / 128 * 16 + kHashSlots * sizeof(int) : (bits + 127) / 128 * 16 + kPenCap * (sizeof(float) + sizeof(int));
-}
 
-// The penalised columns of a segment are a bitmap with a bit per column - or, where that would take the room of other CTAs
-// (32 KB for a row of 262144 logits), a hash table of the columns and a bitmap with a bit per 32 columns.
 struct Segment {
     const float* row;          // the row's logits
     unsigned* bitmap;          // penalised columns (bit 0 = column bit0), valid when has_pen
-    int* hash;                 // kHashSlots columns (-1: free), or null
     const int32_t* hist;       // the penalty window: these ids ...
     const int32_t* drafts;     // ... then these
     int hist_len, window_len;  // ids in the first part, in both
@@ -89,20 +85,7 @@ struct Segment {
 __device__ __forceinline__ int window_id(const Segment& s, int i) { return i < s.hist_len ? s.hist[i] : s.drafts[i - s.hist_len]; }
 __device__ __forceinline__ float penalise(float x, float pen) { return x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen); }   // src/sampler.cpp:17
 __device__ __noinline__ float softcap_call(float x, float cap) { return __fmul_rn(cap, tanhf(__fdiv_rn(x, cap))); }          // src/model_gemma4.cpp:521
-__device__ __forceinline__ bool bit_of(const unsigned* bits, int i) { return (bits[i >> 5] >> (i & 31)) & 1u; }
-__device__ __forceinline__ unsigned hash_slot(int c) { return ((unsigned)c * 2654435761u) / (0x80000000u / (kHashSlots / 2)); }
-__device__ __forceinline__ bool hashed_column(const int* hash, int c) {   // (at least half of the slots are free)
-    for (unsigned h = hash_slot(c);; h = (h + 1u) & (kHashSlots - 1u)) {
-        const int v = hash[h];
-        if (v == c) return true;
-        if (v < 0) return false;
-    }
-}
-__device__ __forceinline__ bool penalised(const Segment& s, int c) {
-    if (!s.has_pen) return false;
-    if (s.hash) return bit_of(s.bitmap, (c - s.bit0) >> 5) && hashed_column(s.hash, c);
-    return bit_of(s.bitmap, c - s.bit0);
-}
+__device__ __forceinline__ bool penalised(const Segment& s, int c) { return s.has_pen && ((s.bitmap[(c - s.bit0) >> 5] >> ((c - s.bit0) & 31)) & 1u); }
 
 // Logit of column c as the sampler sees it.
 __device__ __forceinline__ float transform(float x, int c, const Segment& s) {
@@ -298,11 +281,6 @@ __device__ __noinline__ void write_back(const Segment s) {
         for (int c = s.lo + threadIdx.x; c < s.hi; c += T) row[c] = transform(__ldcg(row + c), c, s);
         return;
     }
-    if (s.hash) {
-        for (int i = threadIdx.x; i < kHashSlots; i += T)
-            if (s.hash[i] >= 0) row[s.hash[i]] = penalise(__ldcg(row + s.hash[i]), s.pen);
-        return;
-    }
     for (int i = threadIdx.x; i < s.window_len; i += T) {
         const int c = window_id(s, i) - s.id_base;
         if (c < s.lo || c >= s.hi) continue;
@@ -344,11 +322,6 @@ __device__ __forceinline__ Segment make_segment(const StreamArgs& a, const RowSp
     Segment s;
     s.row = row_ptr;
     s.bitmap = bitmap;
-    s.hash = nullptr;
-    if (a.hashed) {
-        s.hash = reinterpret_cast<int*>(bitmap);
-        s.bitmap = bitmap + kHashSlots;
-    }
     s.hist = s.drafts = nullptr;
     s.hist_len = s.window_len = 0;
     s.lo = seg == 0 ? 0 : w.head + 4 * w.c_lo;
@@ -375,24 +348,8 @@ template <int T>
 __device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* ctl, float* pen_raw, int* pen_col) {
     const int tid = threadIdx.x, lane = tid & 31;
     int id = tid < s.window_len ? window_id(s, tid) : -1;
-    const int bits = s.hash ? (s.hi - s.bit0 + 31) >> 5 : s.hi - s.bit0;
-    for (int i = tid; i < (bits + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (s.hash)
-        for (int i = tid; i < kHashSlots / 4; i += T) reinterpret_cast<int4*>(s.hash)[i] = make_int4(-1, -1, -1, -1);
+    for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    if (s.hash) {
-        for (int i = tid; i < s.window_len; i += T) {
-            const int c = (i == tid ? id : window_id(s, i)) - s.id_base;
-            if (c < s.lo || c >= s.hi) continue;
-            unsigned h = hash_slot(c);
-            for (;; h = (h + 1u) & (kHashSlots - 1u)) {   // (a window has at most kHashIds ids: half of the slots stay free)
-                const int v = atomicCAS(&s.hash[h], -1, c);
-                if (v == -1 || v == c) break;
-            }
-            atomicOr(&s.bitmap[(c - s.bit0) >> 10], 1u << (((c - s.bit0) >> 5) & 31));
-        }
-        return;
-    }
     for (int i0 = tid & ~31; i0 < s.window_len; i0 += T) {
         const int next = i0 + T + lane < s.window_len ? window_id(s, i0 + T + lane) : -1;
         const int c = id - s.id_base;
@@ -418,12 +375,7 @@ __device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* c
 template <int T, class F>
 __device__ __forceinline__ void for_each_penalised(const Segment& s, int n_pen, const float* pen_raw, const int* pen_col, F f) {
     const int tid = threadIdx.x, lane = tid & 31;
-    if (s.hash) {
-        for (int i = tid; i < kHashSlots; i += T) {   // (a multiple of T)
-            const int c = s.hash[i];
-            f(c >= 0, c >= 0 ? __ldcg(s.row + c) : 0.0f, c);
-        }
-    } else if (n_pen <= kPenCap) {
+    if (n_pen <= kPenCap) {
         for (int i0 = tid & ~31; i0 < n_pen; i0 += T) {
             const bool in = i0 + lane < n_pen;
             f(in, in ? pen_raw[i0 + lane] : 0.0f, in ? pen_col[i0 + lane] : 0);
@@ -443,25 +395,13 @@ __device__ __forceinline__ void for_each_penalised(const Segment& s, int n_pen, 
 // Penalised logits of a thread's cells of a chunk (`j`: its first cell, counted from the segment's first; `left`: cells of
 // the segment from this chunk on) become minus infinity: they are looked at on their own.
 template <int T>
-__device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const Segment& s, int j, int left) {
+__device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const unsigned* bitmap, int j, int left) {
     const float ninf = -__int_as_float(0x7f800000);
+    const unsigned* w = bitmap + (j >> 3) + 1;
+    const int sh = 4 * (j & 7);
     unsigned bits[kCells];
-    if (s.hash) {
 #pragma unroll
-        for (int u = 0; u < kCells; ++u) {
-            bits[u] = 0u;
-            const int at = j + u * T, block = (at >> 3) + 1;   // (columns count from bit0: 32 before the first cell)
-            if ((int)threadIdx.x + u * T < left && bit_of(s.bitmap, block)) {
-#pragma unroll 1
-                for (int e = 0; e < 4; ++e) bits[u] |= hashed_column(s.hash, s.bit0 + 32 + 4 * at + e) ? 1u << e : 0u;
-            }
-        }
-    } else {
-        const unsigned* w = s.bitmap + (j >> 3) + 1;
-        const int sh = 4 * (j & 7);
-#pragma unroll
-        for (int u = 0; u < kCells; ++u) bits[u] = (int)threadIdx.x + u * T < left ? w[u * (T / 8)] >> sh : 0u;
-    }
+    for (int u = 0; u < kCells; ++u) bits[u] = (int)threadIdx.x + u * T < left ? w[u * (T / 8)] >> sh : 0u;
     if ((bits[0] | bits[1] | bits[2] | bits[3]) & 15u) {
 #pragma unroll
         for (int u = 0; u < kCells; ++u) {
@@ -531,7 +471,7 @@ struct SelectArgs {
     __device__ __forceinline__ const int32_t* drafts() const { return NDESC == kFewRows && !a.drafts ? ids : a.drafts; }
 };
 
-template <int T, int NDESC>
+template <int T, int NDESC, bool LONG>
 __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
     using G = Geometry<T>;
     constexpr int kChunkCells = G::kChunkCells, kWarps = G::kWarps;
@@ -543,13 +483,14 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     u64* list = out + kMaxK;
     float4* listed = reinterpret_cast<float4*>(smem_raw + G::kRingBytes);
     const int tid = threadIdx.x, lane = tid & 31;
-    const int cell_cap = a.kmax > 64 ? G::kWarpCellsLong : G::kWarpCells;
-    const int pen_cap = a.penalised && !a.hashed ? kPenCap : 0;
+    constexpr int cell_cap = LONG ? G::kWarpCellsLong : G::kWarpCells;
     int* listed_num = reinterpret_cast<int*>(listed + kWarps * cell_cap);
     float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
-    int* pen_col = reinterpret_cast<int*>(pen_raw + pen_cap);
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + pen_cap);
-    u64* recv = reinterpret_cast<u64*>(ctl + 1);
+    int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised ? kPenCap : 0));
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised ? kPenCap : 0));
+    // (The gap has no use but this: with an address that it knows the compiler's order of the stream loop is 12% slower, 512 x
+    // 262144 119 us against 105.)
+    u64* recv = reinterpret_cast<u64*>(ctl + 1) + (a.kmax > 64 ? kLongGap : 0);
     listed += (tid >> 5) * cell_cap;   // the warp's own
     listed_num += (tid >> 5) * cell_cap;
     pdl_launch_dependents();
@@ -620,7 +561,7 @@ again_from_the_start:
         float4 x[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
-        if (s.has_pen) mask_penalised<T>(x, s, j0 - c_lo, left);
+        if (s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - c_lo, left);
         float m[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
@@ -796,8 +737,8 @@ again_from_the_start:
 // meets its cells in ascending order), the CTA takes the largest composite, and one warp finishes the row.  No bound, no
 // lists, no barrier before the end.  (Not with a softcap, which makes different logits equal, nor with write-back or patched values for the host.)
 template <int T>
-size_t argmax_smem_bytes(int seg_cols, bool hashed) {
-    return Geometry<T>::kRingBytes + sizeof(SharedCtl) + window_bytes(seg_cols, hashed);
+size_t argmax_smem_bytes(int seg_cols) {
+    return Geometry<T>::kRingBytes + sizeof(SharedCtl) + window_bytes(seg_cols);
 }
 
 template <int T, int NDESC>
@@ -808,7 +749,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     float4* ring = reinterpret_cast<float4*>(smem_raw);
     u64* best_of = reinterpret_cast<u64*>(smem_raw);   // after the stream: the warps' best, then the first masked columns
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem_raw + Geometry<T>::kRingBytes);
-    const int pen_cap = a.penalised && !a.hashed ? kPenCap : 0;
+    const int pen_cap = a.penalised ? kPenCap : 0;
     float* pen_raw = reinterpret_cast<float*>(ctl + 1);
     int* pen_col = reinterpret_cast<int*>(pen_raw + pen_cap);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -869,7 +810,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         // (`floor_x` is the warp's best so far: what does not exceed it cannot win, and a warp rarely sees more than ten such chunks)
         if (__any_sync(0xffffffffu, fmaxf(max3(m[0], m[1], m[2]), m[3]) > floor_x)) {
             if (s.has_pen) {
-                mask_penalised<T>(x, s, j0 - w.c_lo, left);
+                mask_penalised<T>(x, s.bitmap, j0 - w.c_lo, left);
 #pragma unroll
                 for (int u = 0; u < kCells; ++u)
                     if (tid + u * T < left) m[u] = cell_max(x[u]);
@@ -933,25 +874,20 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
 }
 
 template <int T, int NDESC>
-int launch_select(cudaLaunchConfig_t& cfg, StreamArgs a, const RowDesc* rows, const int32_t* ids, int n_ids) {
-    const int seg_cols = a.penalised ? 4 * ((a.n_vocab / 4 + a.nseg - 1) / a.nseg) + 8 : 0;
+int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows, const int32_t* ids, int n_ids) {
+    const int seg_cols = a.penalised ? segment_columns(a.n_vocab, a.nseg) : 0;
     cfg.blockDim = dim3(T);
-    a.hashed = 0;
-    cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols, false);
+    cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols);
     if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
     SelectArgs<NDESC> args;
     args.a = a;
     if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
     if (NDESC == kFewRows && n_ids > 0) std::memcpy(args.ids, ids, sizeof(int32_t) * (size_t)n_ids);
     if (a.all_greedy && a.softcap == 0.0f && !a.write_back && !a.patched) {
-        // Whole rows on small CTAs, four per SM: the bitmap of a row of more than 65536 logits would leave room for three or two.
-        // (512 x 262144 with windows of 512 ids: 109 us, hashed 91.  The general kernel, which meets the windows' columns in every
-        // chunk, loses more by the look-ups than it gains: 103 against 129.)
-        args.a.hashed = T == 256 && a.nseg == 1 && seg_cols > 65536 + 8 && a.window_max <= kHashIds ? 1 : 0;
-        cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols, args.a.hashed);
+        cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols);
         return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
     }
-    return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC>, args);
+    return (int)(a.kmax > 64 ? cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, true>, args) : cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, false>, args));
 }
 template <int T>
 int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows, const int32_t* ids, int n_ids) {
@@ -961,8 +897,10 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
 }
 template <int T, int NDESC>
 int prepare_select() {
-    const cudaError_t e = cudaFuncSetAttribute(argmax_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
-    return (int)(e != cudaSuccess ? e : cudaFuncSetAttribute(stream_select_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax));
+    cudaError_t e = cudaFuncSetAttribute(argmax_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    return (int)e;
 }
 
 }  // namespace
@@ -1004,17 +942,39 @@ int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* 
     return a.wide ? launch_select<1024>(cfg, a, host_rows, host_ids, n_ids) : launch_select<256>(cfg, a, host_rows, host_ids, n_ids);
 }
 
-// How a launch is laid out.  Measured on B200, k = 40 to 64, us per call (small CTAs with 1 / 2 / 4 / 8 segments per row;
-// large ones with 1 / 2 / 4): 1 x 65536 34 / 30 / 27 / 26; 29 / 28 / 27.  24 x 100003 48 / 43 / 39 / 38; 44 / 44 / 40.
-// 64 x 262144 61 / 42 / 33 / 38; 35 / 31 / 43.  72 x 131072 95 / 85 / 85 / 89; 81 / 80 / 98.  512 x 32768 72 / 93 / 106 / 141.
-// Few rows: small CTAs, the row cut as finely as two per SM allow (a large CTA issues every step after the stream from
-// four times as many warps).  Medium batches: one large CTA per SM streams best.  Many rows: a small CTA per row, several
-// per SM, so that the steps of one run beside the stream of the others.
-SelectPlan plan_select(int n_rows, int n_vocab, int sms) {
+// How a launch is laid out: small CTAs (256 threads) or large ones (1024), and the segments of a row.  Measured on B200,
+// us per launch with windows of 512 ids; s1 = small, one segment.
+// Few rows: small CTAs, the row cut as finely as two per SM allow (a large CTA issues every step after the stream from four
+// times as many warps): 8 x 131072, k = 16: s4 16.5, s8 13.3, w4 14.5.  With longer lists the merge of eight costs more than
+// those steps: 24 x 262144, k = 64: s8 22.6, w4 20.6, but clusters of four large CTAs run on 132 SMs only (37 rows: w4 32.9, w2 24.7).
+// Medium batches: one large CTA per SM streams best (148 x 131072, k = 64: s1 39, s2 35, w1 27; 64: s4 24, w1 23, w2 21).
+// Many rows: a small CTA per row, several per SM, so that the steps of one run beside the stream of the others (200 x 131072,
+// k = 64: s1 43, s2 42, w1 47; 512 x 32768: s1 38, s2 54, w1 53).
+// Windows of more than 131072 columns leave room for two per SM, and three rounds of large ones beat what is not quite two of
+// those (262144, k = 64: 300 rows s1 104, w1 96; 400 s1 107, w1 100; 512 s1 119, w1 131).
+// k > 64: a small CTA lists every second logit at first.  Large ones from 32768 logits on however many rows there are (512 x
+// 262144, k = 256: s1 236, w1 164; 512 x 32768: s1 73, w1 72; 512 x 16384: s1 54, w1 60), in two segments while a pair per
+// row runs at once (32 x 262144: s8 48, w1 46, w2 33, w4 36; 148 x 262144: s1 122, w1 57, w2 68).
+// All greedy: little after the stream.  Up to three CTAs per SM two segments pay (200 x 262144: s1 43, s2 37; 296: s1 53, s2 60);
+// windows of more than 65536 columns leave room for three or two CTAs per SM, and one large one streams better than a
+// second wave (512 x 262144: s1 105, s2 94, w1 90; 400: s1 69, w1 70).
+SelectPlan plan_select(int n_rows, int n_vocab, int sms, int kmax, bool all_greedy, bool penalised) {
     SelectPlan pl;
-    pl.wide = n_rows > sms / 4 && n_rows <= sms;
-    const int most = pl.wide ? sms : 2 * sms;
-    while (pl.nseg < 8 && n_rows * pl.nseg * 2 <= most && n_vocab / (pl.nseg * 2) >= 8192) pl.nseg *= 2;
+    auto fits = [&](int nseg, int most) { return n_rows * nseg <= most && n_vocab / nseg >= 8192; };
+    if (kmax > 64) {
+        pl.wide = n_rows <= sms || n_vocab >= 32768;
+        if (fits(2, sms) && n_vocab >= 32768) pl.nseg = 2;
+    } else if (n_rows > sms) {
+        if (all_greedy && n_vocab >= 65536 && n_rows <= sms + sms / 2) pl.nseg = 2;
+        pl.wide = penalised && (all_greedy ? n_vocab > 65536 && n_rows > 3 * sms : n_vocab > 131072 && n_rows > 2 * sms && n_rows <= 3 * sms);
+    } else {
+        pl.wide = n_rows > sms / 4 || (kmax > 32 && n_rows > 8 && n_vocab >= 65536);
+        if (pl.wide) pl.nseg = fits(4, sms - sms / 10) ? 4 : fits(2, sms) ? 2 : 1;
+    }
+    // (the bitmap of a very long segment - above 380000 columns - does not fit beside a large CTA's ring, but always beside a small one's)
+    if (pl.wide && penalised && Geometry<1024>::smem_bytes(pl.nseg, kmax, segment_columns(n_vocab, pl.nseg)) > (size_t)kSelectSmemMax) pl = SelectPlan{};
+    if (!pl.wide && n_rows <= sms)
+        while (pl.nseg < 8 && fits(2 * pl.nseg, 2 * sms)) pl.nseg *= 2;
     return pl;
 }
 
@@ -1099,7 +1059,7 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
         a.n_vocab = n_vocab;
         a.kmax = 1;
         a.all_greedy = 1;
-        const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms);
+        const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms, 1, true, false);
         a.nseg = pl.nseg;
         a.wide = pl.wide ? 1 : 0;
         if (rc == FSB_OK && launch_stream_kernel(a, nullptr, nullptr, 0, false, st) != 0) rc = FSB_ERR_CUDA;
