@@ -698,7 +698,7 @@ int fsb_create(int device, int max_rows, int max_vocab, int64_t max_hist_ids, fs
         cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess)
         return bail(FSB_ERR_CUDA);
-    // Everything a call may need is allocated here, so that no call allocates: the rows' scratch, the counters, the
+    // Everything a call may need is allocated here, so that no call allocates: the status word, the
     // kept-set record, the id pool and the staging area of host logits.
     h->logits_stage_elems = (size_t)max_rows * (size_t)max_vocab;
     if (cudaMalloc(reinterpret_cast<void**>(&h->d_kept_ids), sizeof(int32_t) * (size_t)max_rows * fsb::kMaxK) != cudaSuccess ||

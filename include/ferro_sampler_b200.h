@@ -294,7 +294,7 @@ FSB_API int fsb_counters(const fsb_handle* h, fsb_counters_t* out);
  * in this call or any earlier one.  That is the situation of a decode loop whose device memory is owned entirely by
  * the serving engine's own pool, and of code that runs where an allocation would stall the device (a cudaMalloc
  * waits for running kernels).  All device memory the streaming kernel needs besides the caller's buffers (row
- * descriptors, the rows' candidate scratch, its counters and status word: about 1.2 MB) is one array inside the
+ * descriptors and the status word) is one array inside the
  * library's own image.  No penalty window, no softcap, no random draw: exactly the rows of a verification window
  * with repetition_penalty 1 (src/server.cpp:630-636).
  *   logits_dev [n_rows][ld] fp32 and tokens_dev [n_rows] int32 are device memory of `device`; the kernels are
