@@ -1354,20 +1354,21 @@ int launch_full(const FullArgs& a, int n_rows, cudaStream_t stream) {
 // 148 SMs, 22 of six, 33 of four.
 int g_at_once[3] = {0, 0, 0};
 template <int C>
-int prepare_full(int max_vocab, int& at_once) {
-    // the largest request of any row length up to max_vocab: rows that still fit the slice cache need the most
-    const size_t most = std::max(C == kMaxCluster ? full_row_smem_bytes(max_vocab, C) : 0, full_row_smem_bytes(std::min(max_vocab, C * kSliceCache), C));
+int prepare_full(int& at_once) {
+    // the largest request of any row length, whatever the engine's: the attribute is the kernel's, and engines of several sizes
+    // may be alive.  Rows that still fit the slice cache need the most.
+    const size_t most = full_row_smem_bytes(C * kSliceCache, C);
     cudaError_t e = cudaFuncSetAttribute(full_row_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess || at_once > 0) return (int)e;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg{};
-    fill_config<C>(cfg, attr, 64, std::min(max_vocab, C * kSliceCache));
+    fill_config<C>(cfg, attr, 64, C * kSliceCache);
     return (int)cudaOccupancyMaxActiveClusters(&at_once, full_row_kernel<C>, &cfg);
 }
 }  // namespace
 
-int prepare_full_row_kernel(int max_vocab) {
-    for (int e : {prepare_full<8>(max_vocab, g_at_once[2]), prepare_full<6>(max_vocab, g_at_once[1]), prepare_full<4>(max_vocab, g_at_once[0])})
+int prepare_full_row_kernel() {
+    for (int e : {prepare_full<8>(g_at_once[2]), prepare_full<6>(g_at_once[1]), prepare_full<4>(g_at_once[0])})
         if (e != 0) return e;
     return 0;
 }

@@ -125,7 +125,7 @@ int launch_gather_patched(const float* logits, const RowDesc* rows, int n_rows, 
                           float* out, void* stream);
 
 // Defined in fsb_fullrow.cu.
-int prepare_full_row_kernel(int max_vocab);
+int prepare_full_row_kernel();
 int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows, const int32_t* hist, const int32_t* drafts, int32_t* pool, int32_t* tokens, int32_t* tokens_host,
                            int32_t* kept_ids, double* kept_pr, int32_t* kept_n, int record, uint32_t* status, uint32_t* status_host, int n_vocab,
                            int vocab_offset, int write_back, float softcap, uint64_t* trace, void* stream);

@@ -691,7 +691,7 @@ int fsb_create(int device, int max_rows, int max_vocab, int64_t max_hist_ids, fs
     h->sm_count = prop.multiProcessorCount;
     if (fsb::prepare_device_kernels() != 0) return bail(FSB_ERR_CUDA);
     if (fsb::prepare_support_kernels() != 0) return bail(FSB_ERR_CUDA);
-    if (fsb::prepare_full_row_kernel(max_vocab) != 0) return bail(FSB_ERR_CUDA);
+    if (fsb::prepare_full_row_kernel() != 0) return bail(FSB_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(FSB_ERR_CUDA);
     h->own_stream = true;
     if (cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
