@@ -79,6 +79,7 @@ struct StreamArgs {
     int32_t wide;              // large CTAs (see SelectPlan)
     int32_t kmax;              // largest k of the rows
     int32_t all_greedy;        // every row is greedy
+    int32_t window_max;        // ids of the longest penalty window
     int32_t penalised;         // some row has a penalty window
     int32_t write_back;        // store penalised values into the caller's rows
     int32_t vocab_offset;      // token id of column 0

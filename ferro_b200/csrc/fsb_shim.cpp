@@ -55,6 +55,7 @@ struct fsb_batch {
     int kmax = 1;
     fsb::SelectPlan plan;         // how the streaming kernel is laid out
     bool all_greedy = false;      // every row of the streaming kernel is greedy
+    int window_max = 0;           // ids of the longest penalty window
     bool penalised = false;       // some row of the streaming kernel has a penalty window
     int64_t hist_ids = 0;         // window ids staged with the batch
     bool sent_with_launch = false;   // descriptors and staged ids are arguments of the launch, the device copy is stale
@@ -252,12 +253,14 @@ int finalize_batch(fsb_handle* h, fsb_batch* b) {
     fsb::RowDesc* dst = b->h_rows();
     auto on_chip = [](const fsb::RowDesc& d) { return d.k <= fsb::kMaxK && d.k_global <= fsb::kMaxK; };
     b->penalised = false;
+    b->window_max = 0;
     b->all_greedy = true;
     for (const auto& d : b->descs)
         if (on_chip(d)) {
             dst[n_cand++] = d;
             kmax = std::max(kmax, d.k);
             b->all_greedy = b->all_greedy && (d.flags & fsb::kRowGreedy) != 0;
+            if (d.flags & fsb::kRowPenalty) b->window_max = std::max(b->window_max, d.hist_len + (d.flags >> fsb::kRowDraftShift));
             b->penalised = b->penalised || (d.flags & fsb::kRowPenalty) != 0;
         }
     int n_full = 0;
@@ -340,6 +343,7 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.wide = b->plan.wide ? 1 : 0;
         a.kmax = b->kmax;
         a.all_greedy = b->all_greedy ? 1 : 0;
+        a.window_max = b->window_max;
         a.penalised = b->penalised ? 1 : 0;
         a.write_back = (b->flags & FSB_WRITE_BACK) && !patched ? 1 : 0;
         a.vocab_offset = h->vocab_offset;

@@ -9,6 +9,7 @@
 #include "../../include/ferro_sampler_b200.h"
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 #include <cstring>
 
 #include "fsb_device.cuh"
@@ -44,6 +45,7 @@ constexpr int kPenCap = 1024;                           // penalised columns of 
 constexpr int kPickCap = 1024;                          // candidates of a segment
 constexpr int kLongGap = 2;                              // unused words before the receive buffer if k > 64
 constexpr int kMergeList = 2048;                        // candidates of all segments, an equal share of it each
+constexpr int kCellSlots = 2048, kCellIds = 1024;       // penalised cells: slots of their table, and the longest window that may use it
 constexpr int kSelectSmemMax = 224 * 1024;
 static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merge list's memory");
 
@@ -51,6 +53,9 @@ static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merg
 int segment_columns(int n_vocab, int nseg) { return 4 * ((n_vocab / 4 + nseg - 1) / nseg) + 8; }
 // A segment's penalised columns: logits and numbers of the first kPenCap, and a bitmap.
 size_t window_bytes(int seg_cols) { return seg_cols > 0 ? kPenCap * (sizeof(float) + sizeof(int)) + (size_t)((seg_cols + 32 + 127) / 128) * 16 : 0; }
+
+// The same where a bit per cell will do (see CellSegment): a group of 32 words per chunk of small CTAs.
+size_t cell_bits_bytes(int seg_cols) { return seg_cols > 0 ? (size_t)(seg_cols / 4 + 1024) / 1024 * 128 : 0; }
 
 // Sizes that go with T, the threads of a CTA.
 template <int T>
@@ -87,8 +92,33 @@ __device__ __forceinline__ float penalise(float x, float pen) { return x > 0.0f 
 __device__ __noinline__ float softcap_call(float x, float cap) { return __fmul_rn(cap, tanhf(__fdiv_rn(x, cap))); }          // src/model_gemma4.cpp:521
 __device__ __forceinline__ bool penalised(const Segment& s, int c) { return s.has_pen && ((s.bitmap[(c - s.bit0) >> 5] >> ((c - s.bit0) & 31)) & 1u); }
 
+// A whole row whose penalised logits are kept by cells, on small CTAs: in the stream a bit per cell - a quarter of the
+// memory, and one 16-byte read per warp and chunk - sets whole cells aside; at the end a hash table in the ring's memory
+// says which columns of those cells the window holds.
+struct CellSegment : Segment {
+    int* table;                // kCellSlots x (cell << 4 | penalised columns of it), -1: free
+    const unsigned* edges;     // penalised ones of the logits outside the cells
+    int head, n_cells;
+};
+__device__ __forceinline__ int cell_word(int cell) { return (cell >> 10) * 32 + ((cell >> 5) & 7) * 4 + ((cell >> 8) & 3); }
+__device__ __forceinline__ unsigned cell_slot(int cell) { return ((unsigned)cell * 2654435761u) / (0x80000000u / (kCellSlots / 2)); }
+__device__ __forceinline__ int edge_index(const CellSegment& s, int c) { return c < s.head ? c : 4 + c - s.head - 4 * s.n_cells; }
+__device__ __forceinline__ bool outside_cells(const CellSegment& s, int c) { return c < s.head || c >= s.head + 4 * s.n_cells; }
+__device__ __forceinline__ bool penalised(const CellSegment& s, int c) {
+    if (!s.has_pen) return false;
+    if (outside_cells(s, c)) return (*s.edges >> edge_index(s, c)) & 1u;
+    const int cell = (c - s.head) >> 2, e = (c - s.head) & 3;
+    if (!((s.bitmap[cell_word(cell)] >> (cell & 31)) & 1u)) return false;
+    for (unsigned h = cell_slot(cell);; h = (h + 1u) & (kCellSlots - 1u)) {   // (at least half of the slots are free)
+        const int v = s.table[h];
+        if (v < 0) return false;
+        if ((v >> 4) == cell) return (v >> e) & 1;
+    }
+}
+
 // Logit of column c as the sampler sees it.
-__device__ __forceinline__ float transform(float x, int c, const Segment& s) {
+template <class S>
+__device__ __forceinline__ float transform(float x, int c, const S& s) {
     if (s.cap != 0.0f) x = softcap_call(x, s.cap);
     if (penalised(s, c)) x = penalise(x, s.pen);
     return x;
@@ -174,8 +204,8 @@ __device__ __noinline__ int prune_cells(float4* cells, int* nums, int n, float a
 // returns their number.  `bins`: 256 words.  MSB-first over 8-bit digits of the composites: count the digits of the composites that match
 // the prefix, walk the counts from the top, go on in the digit in which the k-th lies; stops early when a digit is
 // taken whole.  Every digit reads the segment again.  All threads call, after a barrier.
-template <int T>
-__device__ __noinline__ int exact_select(const Segment s, int k, u64* list, unsigned* bins, SharedCtl* ctl) {
+template <int T, class S>
+__device__ __noinline__ int exact_select(const S s, int k, u64* list, unsigned* bins, SharedCtl* ctl) {
     const int tid = threadIdx.x, lane = tid & 31;
     u64 prefix = 0ull, mask = 0ull;
     int need = k;
@@ -249,8 +279,8 @@ __device__ __noinline__ int exact_select(const Segment s, int k, u64* list, unsi
 
 // A segment with fewer than k logits above minus infinity (masked vocabularies): its first columns that hold minus
 // infinity are candidates too.  Appends up to k - n of them to the list; returns the new length.  All threads call.
-template <int T>
-__device__ __noinline__ int append_masked(const Segment s, int n, int k, u64* list, unsigned* counts) {
+template <int T, class S>
+__device__ __noinline__ int append_masked(const S s, int n, int k, u64* list, unsigned* counts) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __syncthreads();
     for (int c0 = s.lo; c0 < s.hi && n < k; c0 += T) {
@@ -412,6 +442,38 @@ __device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const unsign
         }
     }
 }
+// The window's cells: sets their bits before the stream, and fills the table after it.  All threads call; a barrier has to follow.
+template <int T>
+__device__ __forceinline__ void collect_cells(const CellSegment& s, unsigned* edges) {
+    for (int i = threadIdx.x; i < 8 * ((s.n_cells + 1023) >> 10); i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x == 0) *edges = 0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < s.window_len; i += T) {
+        const int c = window_id(s, i) - s.id_base;
+        if (c < s.lo || c >= s.hi) continue;
+        const int cell = (c - s.head) >> 2;
+        if (outside_cells(s, c)) atomicOr(edges, 1u << edge_index(s, c));
+        else atomicOr(&s.bitmap[cell_word(cell)], 1u << (cell & 31));
+    }
+}
+template <int T>
+__device__ __forceinline__ void fill_table(const CellSegment& s) {
+    for (int i = threadIdx.x; i < kCellSlots / 4; i += T) reinterpret_cast<int4*>(s.table)[i] = make_int4(-1, -1, -1, -1);
+    __syncthreads();
+    for (int i = threadIdx.x; i < s.window_len; i += T) {
+        const int c = window_id(s, i) - s.id_base;
+        if (c < s.lo || c >= s.hi || outside_cells(s, c)) continue;
+        const int cell = (c - s.head) >> 2, bit = 1 << ((c - s.head) & 3);
+        for (unsigned h = cell_slot(cell);; h = (h + 1u) & (kCellSlots - 1u)) {   // (no more cells than ids: at most half of the slots)
+            const int v = atomicCAS(&s.table[h], -1, cell << 4 | bit);
+            if (v == -1) break;
+            if ((v >> 4) == cell) {
+                atomicOr(&s.table[h], bit);
+                break;
+            }
+        }
+    }
+}
 // Largest of the lanes' composites.
 __device__ __forceinline__ u64 warp_max_u64(u64 v) {
     const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32));
@@ -471,7 +533,7 @@ struct SelectArgs {
     __device__ __forceinline__ const int32_t* drafts() const { return NDESC == kFewRows && !a.drafts ? ids : a.drafts; }
 };
 
-template <int T, int NDESC, bool LONG>
+template <int T, int NDESC, bool LONG, bool CELLS>
 __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
     using G = Geometry<T>;
     constexpr int kChunkCells = G::kChunkCells, kWarps = G::kWarps;
@@ -486,8 +548,8 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     constexpr int cell_cap = LONG ? G::kWarpCellsLong : G::kWarpCells;
     int* listed_num = reinterpret_cast<int*>(listed + kWarps * cell_cap);
     float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
-    int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised ? kPenCap : 0));
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised ? kPenCap : 0));
+    int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised && !CELLS ? kPenCap : 0));
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised && !CELLS ? kPenCap : 0));
     // (The gap has no use but this: with an address that it knows the compiler's order of the stream loop is 12% slower, 512 x
     // 262144 119 us against 105.)
     u64* recv = reinterpret_cast<u64*>(ctl + 1) + (a.kmax > 64 ? kLongGap : 0);
@@ -525,7 +587,14 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
         const int c = span.edge_column(tid, V, seg, nseg);
         ctl->edge[tid] = c >= 0 ? __ldcg(row_ptr + c) : qnan;
     }
-    Segment s = make_segment(a, span, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(recv + (nseg > 1 ? kMergeList : 0)));
+    std::conditional_t<CELLS, CellSegment, Segment> s;
+    static_cast<Segment&>(s) = make_segment(a, span, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(recv + (nseg > 1 ? kMergeList : 0)));
+    if constexpr (CELLS) {
+        s.table = reinterpret_cast<int*>(list + kMergeList / 2);   // (behind what the rare paths keep in the list's memory)
+        s.edges = reinterpret_cast<const unsigned*>(&ctl->pen_n);
+        s.head = head;
+        s.n_cells = n_cells;
+    }
     s.has_pen = (dp.flags & kRowPenalty) != 0;
     s.pen = dp.penalty;
     const int k = dp.k;
@@ -537,10 +606,11 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     if (nseg > 1) cluster_arrive_release();   // (waited for before the first store to another CTA's shared memory)
     if (s.has_pen) {
         set_window(s, args.hist(), args.drafts(), dp);
-        collect_penalised<T>(s, ctl, pen_raw, pen_col);
+        if constexpr (CELLS) collect_cells<T>(s, reinterpret_cast<unsigned*>(&ctl->pen_n));
+        else collect_penalised<T>(s, ctl, pen_raw, pen_col);
     }
     __syncthreads();
-    if (s.has_pen && tid < 8) {   // penalised logits are looked at on their own
+    if (!CELLS && s.has_pen && tid < 8) {   // penalised logits are looked at on their own
         const int c = tid < 4 ? tid : head + 4 * n_cells + tid - 4;
         if (ctl->edge[tid] == ctl->edge[tid] && penalised(s, c)) ctl->edge[tid] = qnan;
     }
@@ -561,10 +631,17 @@ again_from_the_start:
         float4 x[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
-        if (s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - c_lo, left);
+        if (!CELLS && s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - c_lo, left);
         float m[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
+        if (CELLS && s.has_pen) {
+            const uint4 aside = reinterpret_cast<const uint4*>(s.bitmap)[8 * c + (tid >> 5)];
+            if ((aside.x >> lane) & 1u) m[0] = ninf;
+            if ((aside.y >> lane) & 1u) m[1] = ninf;
+            if ((aside.z >> lane) & 1u) m[2] = ninf;
+            if ((aside.w >> lane) & 1u) m[3] = ninf;
+        }
         if (left < kChunkCells) {
 #pragma unroll
             for (int u = 0; u < kCells; ++u)
@@ -631,6 +708,33 @@ again_from_the_start:
         p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
         if (hit && p < kPickCap) picked[p] = make_comp(y, col + s.id_base);
     };
+    auto pick_cell = [&](const float4& v, int col, int pen) {   // a cell per lane, `pen`: penalised ones of its columns
+        float xs[4] = {v.x, v.y, v.z, v.w};
+        if (s.cap != 0.0f) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) xs[e] = xs[e] >= admit || (CELLS && ((pen >> e) & 1)) ? softcap_call(xs[e], s.cap) : ninf;
+        }
+        if (CELLS && pen) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if ((pen >> e) & 1) xs[e] = penalise(xs[e], s.pen);
+        }
+        const float least = fmaxf(seen, -FLT_MAX);
+        unsigned hit[4];
+        int q = warp_reserve<4>(xs, least, hit, &ctl->kept_n);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int at = q + __popc(hit[e] & lanes_below());
+            if (xs[e] >= least && at < kPickCap) picked[at] = make_comp(xs[e], col + e + s.id_base);
+            q += __popc(hit[e]);
+        }
+    };
+    if constexpr (CELLS) {
+        if (s.has_pen) {
+            fill_table<T>(s);
+            __syncthreads();
+        }
+    }
     if (!lost) {
         for (int p0 = 0; p0 < wn; p0 += 32) {
             float4 v = make_float4(ninf, ninf, ninf, ninf);
@@ -639,27 +743,28 @@ again_from_the_start:
                 v = listed[p0 + lane];
                 col = head + 4 * listed_num[p0 + lane];
             }
-            float xs[4] = {v.x, v.y, v.z, v.w};
-            if (s.cap != 0.0f) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) xs[e] = xs[e] >= admit ? softcap_call(xs[e], s.cap) : ninf;
-            }
-            const float least = fmaxf(seen, -FLT_MAX);
-            unsigned hit[4];
-            int q = warp_reserve<4>(xs, least, hit, &ctl->kept_n);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int at = q + __popc(hit[e] & lanes_below());
-                if (xs[e] >= least && at < kPickCap) picked[at] = make_comp(xs[e], col + e + s.id_base);
-                q += __popc(hit[e]);
-            }
+            pick_cell(v, col, 0);
         }
         if (tid < 32 && V != 4 * n_cells) {
             const float x = lane < 8 ? ctl->edge[lane] : qnan;
-            const float y = s.cap != 0.0f ? softcap_call(x, s.cap) : x;
-            pick(x >= admit && y >= seen, y, lane < 4 ? lane : head + 4 * n_cells + lane - 4);
+            const bool pen = CELLS && s.has_pen && lane < 8 && ((ctl->pen_n >> lane) & 1);
+            float y = s.cap != 0.0f ? softcap_call(x, s.cap) : x;
+            if (pen) y = penalise(y, s.pen);
+            pick((pen ? y > ninf : x >= admit) && y >= seen, y, lane < 4 ? lane : head + 4 * n_cells + lane - 4);
         }
-        if (s.has_pen)
+        if constexpr (CELLS) {
+            if (s.has_pen) {
+                for (int i0 = 0; i0 < kCellSlots; i0 += 4 * T) {   // (kCellSlots is a multiple)
+                    const int4 at = reinterpret_cast<const int4*>(s.table)[i0 / 4 + tid];
+                    const int v[4] = {at.x, at.y, at.z, at.w};
+                    float4 raw[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) raw[i] = v[i] >= 0 ? __ldcg(cells + (v[i] >> 4)) : make_float4(ninf, ninf, ninf, ninf);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) pick_cell(raw[i], head + 4 * (v[i] >> 4), v[i] >= 0 ? v[i] & 15 : 0);
+                }
+            }
+        } else if (s.has_pen)
             for_each_penalised<T>(s, ctl->pen_n, pen_raw, pen_col, [&](bool in, float x, int col) {
                 const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
                 pick(in && y >= seen && y > ninf, y, col);
@@ -670,8 +775,8 @@ again_from_the_start:
     lost = lost || n > kPickCap;
     if (lost || (n < k && (bounded || s.cap != 0.0f))) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
     else if (n < k) n = append_masked<T>(s, n, k, picked, reinterpret_cast<unsigned*>(list));
-    if (a.write_back) write_back<T>(s);
-    if (a.patched && s.has_pen) send_patched<T>(s, a.patched + dp.gather_off);
+    if (!CELLS && a.write_back) write_back<T>(s);
+    if (!CELLS && a.patched && s.has_pen) send_patched<T>(s, a.patched + dp.gather_off);
     trace_mark(a, 2);
     if (a.trace && tid == 0 && blockIdx.x < 4096u) a.trace[(size_t)blockIdx.x * 8 + 3] = (u64)n;
     if (a.overlap == 1) pdl_wait_prior();   // from here on this launch writes what the previous launch in the stream may still be using
@@ -887,7 +992,17 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
         cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols);
         return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
     }
-    return (int)(a.kmax > 64 ? cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, true>, args) : cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, false>, args));
+    if constexpr (T == 256 && NDESC == 0) {
+        // Whole rows on small CTAs, four per SM: a bitmap of more than 65536 columns leaves room for three or two, and costs every
+        // thread four words per chunk.  Windows of 512 ids, us before -> after: 512 x 262144, k = 64, 133 -> 100, 512 x 131072
+        // 86 -> 62, 512 x 65536 56 -> 45, 160 x 65536 32 -> 29; but 200 x 32768 25 -> 25, 200 x 16384 19 -> 21, 160 x 16384
+        // 16.5 -> 20: the second look at the window is then no longer hidden behind the stream of others.
+        if (a.nseg == 1 && a.kmax <= 64 && a.n_vocab >= 49152 && a.window_max <= kCellIds && !a.write_back && !a.patched) {
+            cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(1, a.kmax, 0) + cell_bits_bytes(seg_cols);
+            return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, false, true>, args);
+        }
+    }
+    return (int)(a.kmax > 64 ? cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, true, false>, args) : cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, false, false>, args));
 }
 template <int T>
 int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* rows, const int32_t* ids, int n_ids) {
@@ -898,8 +1013,10 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
 template <int T, int NDESC>
 int prepare_select() {
     cudaError_t e = cudaFuncSetAttribute(argmax_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if constexpr (T == 256 && NDESC == 0)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
     return (int)e;
 }
 
@@ -950,8 +1067,6 @@ int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* 
 // Medium batches: one large CTA per SM streams best (148 x 131072, k = 64: s1 39, s2 35, w1 27; 64: s4 24, w1 23, w2 21).
 // Many rows: a small CTA per row, several per SM, so that the steps of one run beside the stream of the others (200 x 131072,
 // k = 64: s1 43, s2 42, w1 47; 512 x 32768: s1 38, s2 54, w1 53).
-// Windows of more than 131072 columns leave room for two per SM, and three rounds of large ones beat what is not quite two of
-// those (262144, k = 64: 300 rows s1 104, w1 96; 400 s1 107, w1 100; 512 s1 119, w1 131).
 // k > 64: a small CTA lists every second logit at first.  Large ones from 32768 logits on however many rows there are (512 x
 // 262144, k = 256: s1 236, w1 164; 512 x 32768: s1 73, w1 72; 512 x 16384: s1 54, w1 60), in two segments while a pair per
 // row runs at once (32 x 262144: s8 48, w1 46, w2 33, w4 36; 148 x 262144: s1 122, w1 57, w2 68).
@@ -966,7 +1081,7 @@ SelectPlan plan_select(int n_rows, int n_vocab, int sms, int kmax, bool all_gree
         if (fits(2, sms) && n_vocab >= 32768) pl.nseg = 2;
     } else if (n_rows > sms) {
         if (all_greedy && n_vocab >= 65536 && n_rows <= sms + sms / 2) pl.nseg = 2;
-        pl.wide = penalised && (all_greedy ? n_vocab > 65536 && n_rows > 3 * sms : n_vocab > 131072 && n_rows > 2 * sms && n_rows <= 3 * sms);
+        pl.wide = penalised && all_greedy && n_vocab > 65536 && n_rows > 3 * sms;
     } else {
         pl.wide = n_rows > sms / 4 || (kmax > 32 && n_rows > 8 && n_vocab >= 65536);
         if (pl.wide) pl.nseg = fits(4, sms - sms / 10) ? 4 : fits(2, sms) ? 2 : 1;

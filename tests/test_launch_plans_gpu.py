@@ -17,7 +17,8 @@ PLANS = [
     (5, 40001, 33, 1030, 0.7, 30.0), (38, 32769, 64, 64, 1.1, 0.0), (75, 32769, 128, 64, 1.1, 0.0), (148, 16384, 7, 50, 1.1, 0.0),
     (149, 8191, 64, 200, 1.2, 0.0), (149, 32768, 256, 20, 1.2, 0.0), (150, 16000, 200, 2000, 1.2, 0.0),
     (149, 65536, 1, 40, 1.5, 0.0), (223, 65536, 1, 40, 1.5, 0.0), (8, 65536, 1, 1100, 1.5, 0.0), (445, 65540, 1, 20, 1.5, 0.0),
-    (300, 131076, 20, 40, 1.1, 0.0), (80, 400000, 40, 300, 1.1, 0.0), (2, 400003, 256, 300, 1.1, 0.0),  # bitmaps too long for large CTAs
+    (300, 131076, 20, 40, 1.1, 0.0), (149, 65545, 64, 1022, 1.3, 0.0), (150, 65547, 9, 1023, 0.6, 0.0), (151, 65551, 50, 300, 1.2, 30.0),   # penalised cells
+    (80, 400000, 40, 300, 1.1, 0.0), (2, 400003, 256, 300, 1.1, 0.0),  # bitmaps too long for large CTAs
 ]
 
 
