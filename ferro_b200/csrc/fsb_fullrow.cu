@@ -1397,13 +1397,15 @@ int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows,
     a.softcap = softcap;
     a.trace = reinterpret_cast<u64*>(trace);
     // The more CTAs per row the shorter the passes, but a second wave of clusters costs as much as the first.  Measured on B200
-    // (us, eight / six / four CTAs): see the rule's two terms, the steps between the passes and the passes.
+    // with top-p 0.95 (us, eight / six / four CTAs): 8 x 16384 30.4 / 29.7 / 28.8, 8 x 65536 38.8 / 41.1 / 45.3, 8 x 131072
+    // 51.3 / 60.0 / 72.1, 16 x 131072 92.7 / 60.4 / 72.3, 23 x 131072 96.4 / 106.6 / 73.4.  The rule's terms: steps, the
+    // exchanges of a step between more CTAs, passes over a slice.
     int best = 8;
     double cost = 1e30;
     for (int i = 2; i >= 0; --i) {
         const int c = 4 + 2 * i, per = slice_of(n_vocab, c), at_once = std::max(1, g_at_once[i]);
         if (c < 8 && per > kSliceCache) continue;
-        const double t = ((n_rows + at_once - 1) / at_once) * (16.0 + 1.2 * per / 1024.0);
+        const double t = ((n_rows + at_once - 1) / at_once) * (18.0 + 1.1 * c + 1.55 * per / 1024.0);
         if (t < cost) {
             cost = t;
             best = c;
