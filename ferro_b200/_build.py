@@ -19,9 +19,12 @@ HEADERS = ["fsb_internal.h", "fsb_device.cuh", os.path.join("..", "..", "include
 EXT_PATH = os.path.join(LIB_DIR, "_fsb_native.so")
 EXT_SOURCE = "fsb_python.cpp"
 
+# The soname is what the native half of the binding records as its dependency, to be found beside it ($ORIGIN): without one
+# the linker records the path of the library that it was built against, and a package that was moved would load that one, too.
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-cudart", "static", "-shared",
+    "-Xlinker", "-soname=" + os.path.basename(LIB_PATH),
 ]
 
 
@@ -36,7 +39,7 @@ def is_fresh() -> bool:
     if not os.path.exists(LIB_PATH):
         return False
     t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
+    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [os.path.abspath(__file__)]
     return all(os.path.getmtime(d) <= t for d in deps)
 
 
@@ -44,7 +47,8 @@ def ext_is_fresh() -> bool:
     if not os.path.exists(EXT_PATH):
         return False
     t = os.path.getmtime(EXT_PATH)
-    return all(os.path.getmtime(os.path.join(CSRC, f)) <= t for f in [EXT_SOURCE] + HEADERS if not f.endswith(".cuh"))
+    deps = [os.path.join(CSRC, f) for f in [EXT_SOURCE] + HEADERS if not f.endswith(".cuh")] + [os.path.abspath(__file__)]
+    return all(os.path.getmtime(d) <= t for d in deps)
 
 
 def build_ext(force: bool = False) -> str:

@@ -37,6 +37,22 @@ def test_library_does_not_link_torch_or_the_oracle():
     assert "torch" not in out and "oracle" not in out and "libferro_ref" not in out
 
 
+def test_a_moved_package_maps_its_own_library_once(tmp_path):
+    # the kernels' attributes are set in the copy that created the engine: the native half of the binding must be bound to it
+    import shutil
+    import subprocess
+    import sys
+    fb.load_library()
+    for d in ("ferro_b200", "include"):
+        shutil.copytree(os.path.join(ROOT, d), tmp_path / d, ignore=shutil.ignore_patterns("__pycache__"))
+    code = ("import ferro_b200 as fb; fb.load_library(build_if_missing=False); "
+            "print('\\n'.join(sorted({l.split()[-1] for l in open('/proc/self/maps') if 'libferro_sampler' in l or '_fsb_native' in l})))")
+    r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    lib = os.path.realpath(tmp_path / "ferro_b200" / "lib")
+    assert r.stdout.split() == [os.path.join(lib, "_fsb_native.so"), os.path.join(lib, "libferro_sampler_b200.so")]
+
+
 def test_params_struct_layout_matches_reference():
     assert fb.PARAMS_DTYPE.itemsize == 40
     assert fb.PARAMS_DTYPE.fields["seed"][1] == 32
