@@ -94,12 +94,12 @@ __device__ __forceinline__ int block_sync_count(bool pred) {
 }
 
 constexpr int kPost = 256;   // threads that finish a row
+static_assert(kPost == kMaxK && kMaxK % 16 == 0, "the epilogue has a thread per candidate and reads them 16 at a time");
 
 struct SharedCtl {
     alignas(16) unsigned top[2][32];          // per-warp bounds (keys), double buffered
     float edge[8];                            // the row's logits outside its whole 16-byte cells (NaN: none)
     u64 red[2 * kPost / 32];                  // cross-warp reduction scratch
-    double part[kMaxK / 32];                  // partial sums of the epilogue
     int sum[3];                               // rotating counters of the selection steps
     int lost;                                 // a warp's list of cells was too short
     int kept_n;                               // candidates picked from the lists
@@ -313,10 +313,10 @@ __device__ __forceinline__ void put_token(int32_t* tokens, int32_t* tokens_host,
 // or finishes the row: softmax over the candidates in fp64, sequential sums in candidate order, min-p, top-p,
 // draw.  `work` is scratch for 2 * kMaxK doubles that does not overlap srt.  The first kPost threads call it with the same
 // arguments; it is the last thing they do (no barrier at the end).
-// Exponentials, their sum (pairwise, like a tree) and the probabilities are one thread's work each.  The cumulative
-// probabilities follow the reference's order of additions exactly, since a cut may fall on a tie: one warp runs the chain
-// of dependent adds (15 cycles each), all lanes alike over broadcast reads, and stops soon after top-p is reached; the
-// cuts and the draw are warp votes.
+// Exponentials and probabilities are one thread's work each.  Their sum and the cumulative probabilities follow the
+// reference's order of additions exactly, since a cut may fall on a tie: a warp runs the chain of dependent adds, all lanes
+// alike over broadcast reads - the first in every warp that needs the sum (no barrier to hand it over), the second in one
+// warp, which stops soon after top-p is reached.  The cuts and the draw are warp votes.
 __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
     const int tid = threadIdx.x, lane = tid & 31;
     double* e = work;
@@ -338,15 +338,18 @@ __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTa
         // pr[i] = exp((double)(x_i - x_0) / T)   (fp32 subtraction, fp64 division, src/sampler.cpp:40)
         double x = 0.0;
         if (tid < kk) x = exp(__ddiv_rn((double)__fsub_rn(comp_value(srt[tid]), comp_value(srt[0])), (double)r.temperature));
-        double s = x;
-        if ((tid & ~31) < kk) {
-#pragma unroll
-            for (int d = 16; d; d >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, d));
-            if (lane == 0) ctl->part[tid >> 5] = s;
-        }
+        P[tid] = x;   // (kMaxK == kPost: zeros behind the last candidate)
         block_sync<kPost, 1>();
-        s = ctl->part[0];
-        for (int w = 1; 32 * w < kk; ++w) s = __dadd_rn(s, ctl->part[w]);
+        double s = 0.0;
+        if ((tid & ~31) < kk) {
+            for (int i = 0; i < kk; i += 16) {
+                double v[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) v[q] = P[i + q];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) s = __dadd_rn(s, v[q]);
+            }
+        }
         // probabilities; min-p keeps those not below pr[0] * min_p (they do not increase, pr[0] is 1 / sum)
         const double p = __ddiv_rn(x, s);
         if (tid < kk) e[tid] = p;
