@@ -76,6 +76,8 @@ struct fsb_batch {
     std::vector<unsigned char> stochastic;
     std::vector<fsb::RowDesc> descs;   // descriptors in row order while a batch is staged (capacity kept between calls)
     bool launched = false;
+    cudaEvent_t ev_sent = nullptr;       // prepared batches: recorded behind a redraw's copy, which reads h_in when its turn comes
+    bool sending = false;                // ... and that copy may not have run yet
     const int32_t* hist_dev = nullptr;   // where the rows' penalty windows live: the batch's staged copy, or the engine's id pool
 
     fsb::RowDesc* h_rows() const { return reinterpret_cast<fsb::RowDesc*>(h_in); }
@@ -182,6 +184,8 @@ void free_batch_buffers(fsb_batch* b) {
     if (b->d_in) cudaFree(b->d_in);
     if (b->d_tokens) cudaFree(b->d_tokens);
     if (b->d_patched) cudaFree(b->d_patched);
+    if (b->ev_sent) cudaEventDestroy(b->ev_sent);
+    b->ev_sent = nullptr;
     b->h_in = nullptr; b->h_tokens = nullptr; b->h_patched = nullptr; b->d_in = nullptr; b->d_tokens = nullptr; b->d_patched = nullptr;
 }
 
@@ -218,6 +222,13 @@ int alloc_batch(fsb_handle* h, int cap_rows, int64_t cap_hist, int64_t patched, 
     }
     *out = b;
     return FSB_OK;
+}
+
+bool is_capturing(const fsb_handle* h) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
 }
 
 Stream* get_stream(fsb_handle* h, int sid) {
@@ -1251,7 +1262,8 @@ int fsb_batch_prepare(fsb_handle* h, int n_rows, const int* stream_ids, int64_t 
     fsb_batch* b = nullptr;
     int rc = alloc_batch(h, n_rows, hist_off[n_rows] - hist_off[0], 0, &b);
     if (rc) return rc;
-    rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, HistSource{hist_flat, hist_off, nullptr, nullptr}, flags);
+    if (cudaEventCreateWithFlags(&b->ev_sent, cudaEventDisableTiming) != cudaSuccess) rc = fail(h, FSB_ERR_CUDA, "event creation failed");
+    if (rc == FSB_OK) rc = stage_rows(h, b, n_rows, stream_ids, ld, n_vocab, HistSource{hist_flat, hist_off, nullptr, nullptr}, flags);
     if (rc == FSB_OK) {
         rc = upload_batch(h, b, true, true);
         if (rc == FSB_OK && cudaStreamSynchronize(h->stream) != cudaSuccess) rc = fail(h, FSB_ERR_CUDA, "upload failed");
@@ -1276,6 +1288,15 @@ int fsb_batch_redraw(fsb_handle* h, fsb_batch* b) {
         Stream* s = get_stream(h, b->sid[(size_t)i]);
         if (!s) return fail(h, FSB_ERR_STREAM_ID, "stream id %d was closed", b->sid[(size_t)i]);
     }
+    // a copy that an earlier redraw queued takes the descriptors from this memory when its turn comes
+    if (b->sending) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (waiting is no part of a capture that may be under way)
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaEventSynchronize(b->ev_sent);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return fail(h, FSB_ERR_CUDA, "waiting for the previous upload: %s", cudaGetErrorString(e));
+        b->sending = false;
+    }
     // rows draw in row order, as a per-slot loop would
     std::vector<int> order((size_t)b->n_rows);
     for (int j = 0; j < b->n_rows; ++j) order[(size_t)rows[j].out_index] = j;
@@ -1286,6 +1307,10 @@ int fsb_batch_redraw(fsb_handle* h, fsb_batch* b) {
         s->draws++;
     }
     FSB_CUDA(h, cudaMemcpyAsync(b->d_in, b->h_in, sizeof(fsb::RowDesc) * (size_t)b->n_rows, cudaMemcpyHostToDevice, h->stream));
+    if (!is_capturing(h)) {   // (a captured copy reads whatever stands there when the graph is replayed)
+        FSB_CUDA(h, cudaEventRecord(b->ev_sent, h->stream));
+        b->sending = true;
+    }
     return FSB_OK;
 }
 
