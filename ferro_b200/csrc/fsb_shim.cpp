@@ -76,8 +76,12 @@ struct fsb_batch {
     std::vector<unsigned char> stochastic;
     std::vector<fsb::RowDesc> descs;   // descriptors in row order while a batch is staged (capacity kept between calls)
     bool launched = false;
-    cudaEvent_t ev_sent = nullptr;       // prepared batches: recorded behind a redraw's copy, which reads h_in when its turn comes
-    bool sending = false;                // ... and that copy may not have run yet
+    // Prepared batches: a redraw's copy reads h_in when its turn comes.  `ev_sent` is recorded behind it, but not for callers
+    // that were seen to wait for every step (it costs 3 us a step: 512 x 32768 sharded 72 -> 75).
+    bool sending = false;        // the copy may not have run yet
+    bool queues_steps = true;    // the caller does not wait for every step, as far as is known
+    bool redrawn = false;
+    cudaEvent_t ev_sent = nullptr;
     const int32_t* hist_dev = nullptr;   // where the rows' penalty windows live: the batch's staged copy, or the engine's id pool
 
     fsb::RowDesc* h_rows() const { return reinterpret_cast<fsb::RowDesc*>(h_in); }
@@ -410,6 +414,7 @@ int fetch_tokens(fsb_handle* h, fsb_batch* b, int32_t* tokens_out, int64_t gathe
             FSB_CUDA(h, cudaMemcpyAsync(b->h_tokens, b->d_tokens, sizeof(int32_t) * ((size_t)b->cap_rows + 1), cudaMemcpyDeviceToHost, h->stream));
         if (gathered > 0) FSB_CUDA(h, cudaMemcpyAsync(b->h_patched, b->d_patched, sizeof(float) * (size_t)gathered, cudaMemcpyDeviceToHost, h->stream));
         FSB_CUDA(h, cudaStreamSynchronize(h->stream));
+        b->sending = false;
     }
     unsigned st = (unsigned)b->h_tokens[b->cap_rows];
     if (st != 0u) cudaStreamSynchronize(h->stream);
@@ -1289,14 +1294,18 @@ int fsb_batch_redraw(fsb_handle* h, fsb_batch* b) {
         if (!s) return fail(h, FSB_ERR_STREAM_ID, "stream id %d was closed", b->sid[(size_t)i]);
     }
     // a copy that an earlier redraw queued takes the descriptors from this memory when its turn comes
+    const bool capturing = is_capturing(h);
     if (b->sending) {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (waiting is no part of a capture that may be under way)
+        if (capturing && !b->queues_steps) return fail(h, FSB_ERR_INVALID, "a redraw inside a capture, and the one before it has not been waited for");
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (waiting is no part of the capture)
         cudaThreadExchangeStreamCaptureMode(&mode);
-        const cudaError_t e = cudaEventSynchronize(b->ev_sent);
+        const cudaError_t e = b->queues_steps ? cudaEventSynchronize(b->ev_sent) : cudaStreamSynchronize(h->stream);
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) return fail(h, FSB_ERR_CUDA, "waiting for the previous upload: %s", cudaGetErrorString(e));
-        b->sending = false;
     }
+    b->queues_steps = b->sending || !b->redrawn;
+    b->sending = false;
+    b->redrawn = true;
     // rows draw in row order, as a per-slot loop would
     std::vector<int> order((size_t)b->n_rows);
     for (int j = 0; j < b->n_rows; ++j) order[(size_t)rows[j].out_index] = j;
@@ -1307,8 +1316,8 @@ int fsb_batch_redraw(fsb_handle* h, fsb_batch* b) {
         s->draws++;
     }
     FSB_CUDA(h, cudaMemcpyAsync(b->d_in, b->h_in, sizeof(fsb::RowDesc) * (size_t)b->n_rows, cudaMemcpyHostToDevice, h->stream));
-    if (!is_capturing(h)) {   // (a captured copy reads whatever stands there when the graph is replayed)
-        FSB_CUDA(h, cudaEventRecord(b->ev_sent, h->stream));
+    if (!capturing) {   // (a captured copy reads whatever stands there when the graph is replayed)
+        if (b->queues_steps) FSB_CUDA(h, cudaEventRecord(b->ev_sent, h->stream));
         b->sending = true;
     }
     return FSB_OK;

@@ -159,12 +159,13 @@ struct Setup {
 float logits_[1000];
 
 // Steps that are queued without waiting: every launch draws what the redraw before it drew.
-int queued_steps(int rows, bool merge) {
+// (`waited`: the first two of them are waited for, as by a caller that changes its ways.)
+int queued_steps(int rows, bool merge, bool waited = false) {
     Setup s(rows);
     fsb_batch* b = s.prepare();
     std::vector<uint64_t> lists((size_t)rows * 52);
-    std::vector<std::vector<int32_t>> seen(4, std::vector<int32_t>((size_t)rows)), want;
-    for (int step = 0; step < 4; ++step) {
+    std::vector<std::vector<int32_t>> seen(6, std::vector<int32_t>((size_t)rows)), want;
+    for (int step = 0; step < 6; ++step) {
         if (step > 0 && fsb_batch_redraw(s.h, b) != FSB_OK) return bad("redraw", step, 1, 0);
         want.push_back(s.next());
         const int rc = merge ? fsb_batch_merge_launch_packed(s.h, b, lists.data(), 52, 1, 0, rows) : fsb_batch_launch(s.h, b, logits_);
@@ -172,9 +173,10 @@ int queued_steps(int rows, bool merge) {
         int32_t* to = seen[(size_t)step].data();
         const int32_t* from = fsb_batch_tokens_device(b);
         enqueue([=] { std::memcpy(to, from, sizeof(int32_t) * (size_t)rows); });
+        if (waited && step < 2 && fsb_batch_check(s.h, b) != FSB_OK) return bad("check", step, 1, 0);
     }
     run_until(nullptr);
-    for (int step = 0; step < 4; ++step)
+    for (int step = 0; step < 6; ++step)
         for (int i = 0; i < rows; ++i)
             if (seen[(size_t)step][(size_t)i] != want[(size_t)step][(size_t)i])
                 return bad("token of a queued step", step * 1000 + i, seen[(size_t)step][(size_t)i], want[(size_t)step][(size_t)i]);
@@ -241,7 +243,8 @@ int any_draft() {
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     const int rows = argc > 2 ? std::atoi(argv[2]) : 8;
-    const int rc = what == "queued" ? queued_steps(rows, false) : what == "merged" ? queued_steps(rows, true) : what == "replayed" ? replayed_launch(rows)
+    const int rc = what == "queued" ? queued_steps(rows, false) : what == "merged" ? queued_steps(rows, true) : what == "waited" ? queued_steps(rows, false, true)
+                   : what == "replayed" ? replayed_launch(rows)
                    : what == "overlap" ? overlapped_windows() : what == "drafts" ? any_draft() : 2;
     if (rc == 0) std::puts("ok");
     return rc;
