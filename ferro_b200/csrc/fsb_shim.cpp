@@ -364,8 +364,10 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.vocab_offset = h->vocab_offset;
         a.softcap = h->softcap;
         a.overlap = h->launch_overlap;
-        const int e = fsb::launch_stream_kernel(a, b->h_rows(), b->sent_with_launch ? b->h_hist() : nullptr, b->sent_with_launch ? (int)b->hist_ids : 0,
-                                                b->hist_dev == nullptr, h->stream);
+        // Few descriptors go with the launch.  A captured launch of a prepared batch reads them on the device: it may be
+        // replayed after a redraw.
+        const int e = fsb::launch_stream_kernel(a, mirror || !is_capturing(h) ? b->h_rows() : nullptr, b->sent_with_launch ? b->h_hist() : nullptr,
+                                                b->sent_with_launch ? (int)b->hist_ids : 0, b->hist_dev == nullptr, h->stream);
         if (e != 0) return fail(h, FSB_ERR_CUDA, "stream kernel launch: %s", cudaGetErrorString((cudaError_t)e));
         h->counters.kernel_launches++;
     }
