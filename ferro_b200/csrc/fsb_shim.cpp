@@ -363,7 +363,8 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         a.write_back = (b->flags & FSB_WRITE_BACK) && !patched ? 1 : 0;
         a.vocab_offset = h->vocab_offset;
         a.softcap = h->softcap;
-        a.overlap = h->launch_overlap;
+        // Windows in the id pool: the launch before may have appended to them, so nothing is read before it is complete.
+        a.overlap = h->launch_overlap == 1 && b->hist_dev && b->penalised ? 2 : h->launch_overlap;
         // Few descriptors go with the launch.  A captured launch of a prepared batch reads them on the device: it may be
         // replayed after a redraw.
         const int e = fsb::launch_stream_kernel(a, mirror || !is_capturing(h) ? b->h_rows() : nullptr, b->sent_with_launch ? b->h_hist() : nullptr,

@@ -100,7 +100,8 @@ FSB_API int fsb_set_trace_buffer(fsb_handle* h, void* device_buffer);
  *    read logits while the previous kernel in the stream is still finishing; every write of the launch (tokens, kept
  *    sets, scratch) waits for that kernel to be complete.  Use it only if the logits of a launch are complete before
  *    the previous kernel in the stream starts (for instance logits that alternate between buffers filled well ahead);
- *    batches with FSB_WRITE_BACK wait before they read anything, so they gain nothing.
+ *    batches with FSB_WRITE_BACK wait before they read anything, so they gain nothing; so do the resident calls when a
+ *    row has a penalty window, since the launch before may have appended to it.
  * 2: the same launch attribute, but every CTA waits for the previous kernel to be complete before it reads or writes
  *    anything.  Results and ordering are those of plain stream order - the logits may be produced by the kernel just
  *    before - and only the launch latency (CTA placement, barrier set-up) is hidden behind that kernel's end.

@@ -27,6 +27,7 @@ def driver(tmp_path_factory):
     ("queued", 8), ("queued", 64), ("queued", 65), ("merged", 8), ("merged", 65),   # redraw, launch, redraw, launch, ... without waiting
     ("waited", 8), ("waited", 65),                                                  # ... after steps that were waited for
     ("replayed", 8), ("replayed", 64), ("replayed", 65),                            # a captured launch, replayed after redraws
+    ("overlap",),                                                                   # mode 1 over histories in the id pool
 ])
 def test_host_order(driver, args):
     r = subprocess.run([driver, *map(str, args)], capture_output=True, text=True, timeout=60)

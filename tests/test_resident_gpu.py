@@ -239,3 +239,33 @@ def test_resident_windows_of_streams_without_a_penalty_keep_their_device_history
     finally:
         for s in sids:
             engine.close_stream(int(s))
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+def test_decode_loop_with_overlapping_launches(engine, oracle, mode):
+    """In mode 1 a launch may begin before the one before it is complete; the window that one appended to is still read in order."""
+    import torch
+    B, V, steps = 16, 16384, 30
+    rng = np.random.default_rng(99 + mode)
+    p = fb.make_params(B, temperature=1.0, top_k=5, top_p=1.0, repetition_penalty=3.0)
+    p["temperature"][::4] = 0.0
+    p["seed"] = 10 + np.arange(B)
+    lg = (rng.standard_normal((B, V)) * 3).astype(np.float32)   # the same logits in every step: each token depends on the one before
+    dev = torch.from_numpy(lg).cuda()
+    torch.cuda.synchronize()
+    rngs = oracle.new_rngs(p["seed"])
+    hists = [rng.integers(0, V, size=20).astype(np.int32) for _ in range(B)]
+    sids = engine.open_streams(p)
+    engine.set_launch_overlap(mode)
+    try:
+        for i, s in enumerate(sids):
+            engine.history_set(int(s), hists[i])
+        for step in range(steps):
+            want = oracle.sample_rows(p, rngs, lg.copy(), hists)["tokens"]
+            tok = engine.sample_batch_resident(sids, dev.data_ptr(), n_vocab=V, flags=fb.APPEND_SAMPLED)
+            assert np.array_equal(tok, want), step
+            hists = [np.append(h, t).astype(np.int32) for h, t in zip(hists, want)]
+    finally:
+        engine.set_launch_overlap(0)
+        for s in sids:
+            engine.close_stream(int(s))
