@@ -395,12 +395,13 @@ int poll_word(fsb_handle* h, const volatile int32_t* w, int32_t none, bool& done
     }
     return FSB_OK;
 }
-int poll_words(fsb_handle* h, const volatile int32_t* t, int n, int stride) {
+// `any`: kNoToken itself is a value that may be stored.
+int poll_words(fsb_handle* h, const volatile int32_t* t, int n, int stride, bool any = false) {
     bool done = false;
     for (int i = 0; i < n; ++i) {
         const int rc = poll_word(h, t + (size_t)i * stride, kNoToken, done);
         if (rc) return rc;
-        if (t[(size_t)i * stride] == kNoToken) return fail(h, FSB_ERR_DEVICE, "no result for row %d", i);
+        if (!any && t[(size_t)i * stride] == kNoToken) return fail(h, FSB_ERR_DEVICE, "no result for row %d", i);
     }
     std::atomic_thread_fence(std::memory_order_acquire);
     return FSB_OK;
@@ -956,7 +957,7 @@ int fsb_lookup_drafts_resident(fsb_handle* h, int n_streams, const int* stream_i
     for (int i = 0; i < n_streams && rc == FSB_OK; ++i) {
         const int32_t* src = h->h_drafts + (size_t)i * fsb::kDraftStride;
         n_out[i] = src[0];
-        rc = poll_words(h, src + 1, src[0], 1);
+        rc = poll_words(h, src + 1, src[0], 1, true);   // (a history may hold any 32-bit value)
         for (int k = 0; k < src[0] && rc == FSB_OK; ++k) drafts_out[(size_t)i * stride + k] = src[1 + k];
     }
     if (rc) {
