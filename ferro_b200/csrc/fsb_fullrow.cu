@@ -188,13 +188,15 @@ struct RowCtx {
         return x;
     }
     __device__ __forceinline__ u64 comp(float x, int i) const { return make_comp(x, lo + i + id_base); }
-    // (x - max) / T, correctly rounded: a quotient from the rounded reciprocal and one exact correction step (Markstein 1990;
-    // T is a float, so its significand is never all ones) - three fused operations in place of a division.
+    // (x - max) / T for a finite difference, correctly rounded: a quotient from the rounded reciprocal and one exact correction
+    // step (Markstein 1990), three fused operations in place of a division.  Both operands are floats: a quotient of two 24-bit
+    // significands is at least 2^-25 ulp away from the middle of two doubles, and the correction is off by some 2^-52 ulp.
     __device__ __forceinline__ double scaled(float diff) const {
         const double d = (double)diff, q = __dmul_rn(d, inv_temp);
         return __fma_rn(__fma_rn(-q, temp, d), inv_temp, q);
     }
-    __device__ __forceinline__ double probability(float x, double sum) const { return __ddiv_rn(exp(scaled(__fsub_rn(x, mx))), sum); }   // src/sampler.cpp:40-41
+    // src/sampler.cpp:40-41 (a masked logit is infinitely far below the maximum: no correction step)
+    __device__ __forceinline__ double probability(float x, double sum) const { return __ddiv_rn(exp(__ddiv_rn((double)__fsub_rn(x, mx), temp)), sum); }
     // src/sampler.cpp:40, exp(y) as 2^-62 fixed point in two parts.  Table-driven (P. Tang, "Table-driven implementation of the
     // exponential function", ACM TOMS 15, 1989): y = (64 e + j) ln2 / 64 + r, exp(y) = 2^e 2^(j/64) (1 + p(r)) with |r| <=
     // ln2 / 128, where the Taylor polynomial of degree 5 is off by less than 2^-54.  Adding 1.5 * 2^(52 - b) rounds to a multiple
