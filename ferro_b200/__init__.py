@@ -179,7 +179,7 @@ def _logits_pointer(logits, n_vocab, flags):
         return logits.__array_interface__["data"][0], logits.strides[0] // 4, flags | LOGITS_ON_HOST, logits
     if hasattr(logits, "data_ptr"):
         ld = logits.stride(0) if logits.dim() == 2 else n_vocab
-        return logits.data_ptr(), ld, flags & ~LOGITS_ON_HOST, logits
+        return int(logits.data_ptr()), int(ld), flags & ~LOGITS_ON_HOST, logits
     raise TypeError("logits: numpy array or device tensor expected")
 
 
@@ -194,7 +194,7 @@ class Batch:
         self.engine._check(_native.batch_redraw(self.engine._hv, self._pv))
 
     def launch(self, logits_dev_ptr: int):
-        rc = _native.batch_launch(self.engine._hv, self._pv, logits_dev_ptr)
+        rc = _native.batch_launch(self.engine._hv, self._pv, int(logits_dev_ptr))
         if rc:
             self.engine._check(rc)
 

@@ -86,6 +86,30 @@ def test_null_arguments_are_errors_not_crashes():
     assert lib.fsb_counters(None, None) < 0
 
 
+@pytest.mark.parametrize("pointer", [4096, np.int64(4096), np.uint64(4096)])
+def test_addresses_may_be_any_integer(pointer):
+    # (the handles are null: the C ABI answers, whatever the pointer's Python type)
+    class Closed:
+        _hv = 0
+        _check = fb.Engine._check
+        lib, _h = fb.load_library(), None
+
+    class Tensor:
+        def data_ptr(self):
+            return pointer
+
+        def dim(self):
+            return 2
+
+        def stride(self, _):
+            return np.int64(8)
+
+    with pytest.raises(fb.SamplerError):
+        fb.Batch(Closed(), C.c_void_p(0), 1).launch(pointer)
+    with pytest.raises(fb.SamplerError):
+        fb.Engine.sample_batch(Closed(), [0], Tensor(), [[]], n_vocab=8)
+
+
 def test_no_cpu_fallback_without_a_device():
     import torch
     if torch.cuda.is_available():
