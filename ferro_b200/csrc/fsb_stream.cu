@@ -773,7 +773,8 @@ again_from_the_start:
     __syncthreads();
     int n = ctl->kept_n;
     lost = lost || n > kPickCap;
-    if (lost || (n < k && (bounded || s.cap != 0.0f))) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
+    // (the softcap makes a finite logit of minus infinity, equal to or above others: without a raw bound such columns count, too)
+    if (lost || (n < k && bounded) || (s.cap != 0.0f && admit <= -FLT_MAX)) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
     else if (n < k) n = append_masked<T>(s, n, k, picked, reinterpret_cast<unsigned*>(list));
     if (!CELLS && a.write_back) write_back<T>(s);
     if (!CELLS && a.patched && s.has_pen) send_patched<T>(s, a.patched + dp.gather_off);
