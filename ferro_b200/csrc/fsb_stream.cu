@@ -43,7 +43,6 @@ constexpr int kCells = 4;                               // cells of a thread per
 constexpr int kStages = 2;
 constexpr int kPenCap = 1024;                           // penalised columns of a segment that are looked up ahead
 constexpr int kPickCap = 1024;                          // candidates of a segment
-constexpr int kLongGap = 2;                              // unused words before the receive buffer if k > 64
 constexpr int kMergeList = 2048;                        // candidates of all segments, an equal share of it each
 constexpr int kCellSlots = 2048, kCellIds = 1024;       // penalised cells: slots of their table, and the longest window that may use it
 constexpr int kSelectSmemMax = 224 * 1024;
@@ -70,7 +69,7 @@ struct Geometry {
     // buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
     static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
         const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int));
-        return kRingBytes + cells + sizeof(SharedCtl) + (kLongGap + (nseg > 1 ? kMergeList : 0)) * sizeof(u64) + window_bytes(seg_cols);
+        return kRingBytes + cells + sizeof(SharedCtl) + (nseg > 1 ? kMergeList : 0) * sizeof(u64) + window_bytes(seg_cols);
     }
 };
 
@@ -550,9 +549,7 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
     int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised && !CELLS ? kPenCap : 0));
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised && !CELLS ? kPenCap : 0));
-    // (The gap has no use but this: with an address that it knows the compiler's order of the stream loop is 12% slower, 512 x
-    // 262144 119 us against 105.)
-    u64* recv = reinterpret_cast<u64*>(ctl + 1) + (a.kmax > 64 ? kLongGap : 0);
+    u64* recv = reinterpret_cast<u64*>(ctl + 1);
     listed += (tid >> 5) * cell_cap;   // the warp's own
     listed_num += (tid >> 5) * cell_cap;
     pdl_launch_dependents();
