@@ -992,9 +992,13 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
     }
     if constexpr (T == 256 && NDESC == 0) {
         // Whole rows on small CTAs, four per SM: a bitmap of more than 65536 columns leaves room for three or two, and costs every
-        // thread four words per chunk.  Windows of 512 ids, us before -> after: 512 x 262144, k = 64, 133 -> 100, 512 x 131072
-        // 86 -> 62, 512 x 65536 56 -> 45, 160 x 65536 32 -> 29; but 200 x 32768 25 -> 25, 200 x 16384 19 -> 21, 160 x 16384
-        // 16.5 -> 20: the second look at the window is then no longer hidden behind the stream of others.
+        // thread four words per chunk.  Windows of 512 ids, k = 64, us with a bit per column -> per cell: 512 x 262144 134 -> 107,
+        // 512 x 65536 57 -> 46, 512 x 49152 49 -> 41, 200 x 131072 49 -> 42, 160 x 65536 31.5 -> 29.5; near the limit 296 x 49152
+        // 28.2 -> 29.0, 200 x 49152 26.9 -> 27.6, 200 x 32768 25 -> 25, 512 x 32768 37 -> 35, and with fewer logits the second
+        // look at the window is no longer hidden behind the stream of others (160 x 16384 16.5 -> 20).
+        // Windows of more than kCellIds ids would fill more than half of the table: they go by columns.  The step there, 1024 ->
+        // 1025 ids: 512 x 262144 128 -> 162 us, 512 x 131072 72 -> 105, 160 x 262144 68 -> 91, 160 x 65536 33 -> 34.  (Beyond
+        // kPenCap = 1024 ids in a segment the columns are also found through the bitmap: 1100 ids 186, 122, 96, 41 us.)
         if (a.nseg == 1 && a.kmax <= 64 && a.n_vocab >= 49152 && a.window_max <= kCellIds && !a.write_back && !a.patched) {
             cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(1, a.kmax, 0) + cell_bits_bytes(seg_cols);
             return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, false, true>, args);
@@ -1058,19 +1062,21 @@ int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* 
 }
 
 // How a launch is laid out: small CTAs (256 threads) or large ones (1024), and the segments of a row.  Measured on B200,
-// us per launch with windows of 512 ids; s1 = small, one segment.
+// us per launch with windows of 512 ids; s1 = small, one segment (c: penalised logits by cells), w2 = large, two.
 // Few rows: small CTAs, the row cut as finely as two per SM allow (a large CTA issues every step after the stream from four
-// times as many warps): 8 x 131072, k = 16: s4 16.5, s8 13.3, w4 14.5.  With longer lists the merge of eight costs more than
-// those steps: 24 x 262144, k = 64: s8 22.6, w4 20.6, but clusters of four large CTAs run on 132 SMs only (37 rows: w4 32.9, w2 24.7).
-// Medium batches: one large CTA per SM streams best (148 x 131072, k = 64: s1 39, s2 35, w1 27; 64: s4 24, w1 23, w2 21).
+// times as many warps): 8 x 131072, k = 16: s4 17.7, s8 14.6, w4 14.7.  With longer lists the merge of eight costs more than
+// those steps: 24 x 262144, k = 64: s8 22.9, w4 20.8, but clusters of four large CTAs run on 132 SMs only (37 rows: w4 33.1, w2 25.0).
+// Medium batches: one large CTA per SM streams best (148 x 131072, k = 64: s1 39, s1c 35, s2 34, w1 27; 64: s4 22.9, w1 24.5, w2 21.5).
 // Many rows: a small CTA per row, several per SM, so that the steps of one run beside the stream of the others (200 x 131072,
-// k = 64: s1 43, s2 42, w1 47; 512 x 32768: s1 38, s2 54, w1 53).
+// k = 64: s1 48, s1c 41.7, s2 42.3, w1 47; 160 x 65536: s1 31.5, s1c 29.5, s2 30.9, w1 35; 296 x 262144: s1 79, s1c 72, s2 93, w1
+// 72; 512 x 32768: s1 37, s2 54, w1 54).  Two segments are level with one up to 200 rows below 65536 logits (200 x 49152: s1 26.9,
+// s1c 27.6, s2 27.0) and lose above (256: s1 27.4, s1c 28.8, s2 40).
 // k > 64: a small CTA lists every second logit at first.  Large ones from 32768 logits on however many rows there are (512 x
-// 262144, k = 256: s1 236, w1 164; 512 x 32768: s1 73, w1 72; 512 x 16384: s1 54, w1 60), in two segments while a pair per
-// row runs at once (32 x 262144: s8 48, w1 46, w2 33, w4 36; 148 x 262144: s1 122, w1 57, w2 68).
-// All greedy: little after the stream.  Up to three CTAs per SM two segments pay (200 x 262144: s1 43, s2 37; 296: s1 53, s2 60);
-// windows of more than 65536 columns leave room for three or two CTAs per SM, and one large one streams better than a
-// second wave (512 x 262144: s1 105, s2 94, w1 90; 400: s1 69, w1 70).
+// 262144, k = 256: s1 265, w1 170; 512 x 32768: s1 77, w1 80; 512 x 16384: s1 57, w1 68), in two segments while a pair per
+// row runs at once (32 x 262144: s8 47, w1 44, w2 35, w4 38; 148 x 262144: s1 121, w1 50, w2 72).
+// All greedy: little after the stream.  Up to three CTAs per SM two segments pay (200 x 262144: s1 37.3, s2 35.2; 296: s1 49.0, s2
+// 49.8); windows of more than 65536 columns leave room for three or two CTAs per SM, and one large one streams better than a
+// second wave (512 x 262144: s1 106, s2 95, w1 90; 400: s1 70, w1 71).
 SelectPlan plan_select(int n_rows, int n_vocab, int sms, int kmax, bool all_greedy, bool penalised) {
     SelectPlan pl;
     auto fits = [&](int nseg, int most) { return n_rows * nseg <= most && n_vocab / nseg >= 8192; };
