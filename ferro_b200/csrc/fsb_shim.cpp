@@ -745,7 +745,7 @@ int fsb_create(int device, int max_rows, int max_vocab, int64_t max_hist_ids, fs
 int fsb_destroy(fsb_handle* h) {
     if (!h) return FSB_ERR_INVALID;
     cudaSetDevice(h->device);
-    if (h->stream) cudaStreamSynchronize(h->stream);
+    cudaStreamSynchronize(h->stream);
     if (h->own) {
         free_batch_buffers(h->own);
         delete h->own;
@@ -773,7 +773,7 @@ const char* fsb_last_error(const fsb_handle* h) { return h ? h->err.c_str() : "n
 int fsb_set_cuda_stream(fsb_handle* h, void* cuda_stream) {
     if (!h) return FSB_ERR_INVALID;
     cudaSetDevice(h->device);
-    if (h->stream) cudaStreamSynchronize(h->stream);
+    cudaStreamSynchronize(h->stream);   // (null is the default stream; copies into the id pool may be under way)
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     h->stream = static_cast<cudaStream_t>(cuda_stream);
     h->own_stream = false;

@@ -224,6 +224,21 @@ int overlapped_windows() {
     return 0;
 }
 
+// An engine that leaves a stream, the default stream among them, leaves nothing behind that the next one would have to wait for.
+int switched_streams() {
+    Setup s(1);
+    const int32_t ids[3] = {1, 2, 3};
+    int n = 0;
+    for (uintptr_t to : {0, 32, 0}) {
+        if (fsb_set_cuda_stream(s.h, reinterpret_cast<void*>(to)) != FSB_OK) return bad("stream", n, 1, 0);
+        if (!queue_.empty()) return bad("operations left on a stream", n, (long long)queue_.size(), 0);
+        fsb_stream_history_set(s.h, s.sid[0], ids, 3);
+        ++n;
+    }
+    fsb_destroy(s.h);
+    return queue_.empty() ? 0 : bad("operations left on a stream", n, (long long)queue_.size(), 0);
+}
+
 // Every 32-bit value is a token id of a history, and of the drafts that are taken from it.
 int any_draft() {
     Setup s(1);
@@ -245,7 +260,7 @@ int main(int argc, char** argv) {
     const int rows = argc > 2 ? std::atoi(argv[2]) : 8;
     const int rc = what == "queued" ? queued_steps(rows, false) : what == "merged" ? queued_steps(rows, true) : what == "waited" ? queued_steps(rows, false, true)
                    : what == "replayed" ? replayed_launch(rows)
-                   : what == "overlap" ? overlapped_windows() : what == "drafts" ? any_draft() : 2;
+                   : what == "overlap" ? overlapped_windows() : what == "switched" ? switched_streams() : what == "drafts" ? any_draft() : 2;
     if (rc == 0) std::puts("ok");
     return rc;
 }

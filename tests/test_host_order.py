@@ -28,6 +28,7 @@ def driver(tmp_path_factory):
     ("waited", 8), ("waited", 65),                                                  # ... after steps that were waited for
     ("replayed", 8), ("replayed", 64), ("replayed", 65),                            # a captured launch, replayed after redraws
     ("overlap",),                                                                   # mode 1 over histories in the id pool
+    ("switched",),                                                                  # histories set on one stream, used on another
     ("drafts",),                                                                    # drafts of any 32-bit value
 ])
 def test_host_order(driver, args):
