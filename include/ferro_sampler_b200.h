@@ -240,9 +240,14 @@ FSB_API int fsb_last_kept(fsb_handle* h, int row, int cap, int32_t* ids, double*
  * times on different logits buffers. */
 FSB_API int fsb_batch_prepare(fsb_handle* h, int n_rows, const int* stream_ids, int64_t ld, int n_vocab,
                       const int32_t* hist_flat, const int64_t* hist_off, unsigned flags, fsb_batch** out);
-/* Draw fresh engine outputs for the batch's stochastic rows and upload them (8 bytes per row). */
+/* Draw fresh engine outputs for the batch's stochastic rows and upload the row descriptors that hold them (64 bytes per
+ * row).  Asynchronous: launches queued before keep the outputs they were queued with.  Steps may be queued without waiting
+ * for one another; the call then waits until the upload before it has run.  (Inside a stream capture it cannot wait for an
+ * upload that a caller who until then waited for every step left in flight: FSB_ERR_INVALID.) */
 FSB_API int fsb_batch_redraw(fsb_handle* h, fsb_batch* b);
-/* Enqueue the kernels for one step on `logits_dev` ([n_rows][ld] fp32 in device memory); asynchronous. */
+/* Enqueue the kernels for one step on `logits_dev` ([n_rows][ld] fp32 in device memory); asynchronous.  May be captured
+ * into a CUDA graph: a replay uses the engine outputs of the latest fsb_batch_redraw, and the logits buffer, softcap and
+ * launch mode of the capture. */
 FSB_API int fsb_batch_launch(fsb_handle* h, fsb_batch* b, const float* logits_dev);
 /* Wait for the last launch of `b` and copy its tokens (n_rows int32) to host memory. */
 FSB_API int fsb_batch_tokens(fsb_handle* h, fsb_batch* b, int32_t* tokens_out);
