@@ -316,7 +316,8 @@ __device__ __forceinline__ void put_token(int32_t* tokens, int32_t* tokens_host,
 // Exponentials and probabilities are one thread's work each.  Their sum and the cumulative probabilities follow the
 // reference's order of additions exactly, since a cut may fall on a tie: a warp runs the chain of dependent adds, all lanes
 // alike over broadcast reads - the first in every warp that needs the sum (no barrier to hand it over), the second in one
-// warp, which stops soon after top-p is reached.  The cuts and the draw are warp votes.
+// warp, which stops soon after top-p is reached.  The cuts and the draw are warp votes.  (The first sum over lanes instead, in another
+// order, would save 0.7 to 1.3 us a launch at k = 180 to 215, nothing that shows at k = 64.)
 __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
     const int tid = threadIdx.x, lane = tid & 31;
     double* e = work;
