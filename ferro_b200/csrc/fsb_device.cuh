@@ -309,15 +309,66 @@ __device__ __forceinline__ void put_token(int32_t* tokens, int32_t* tokens_host,
     if (tokens_host) *reinterpret_cast<volatile int32_t*>(tokens_host + index) = token;
 }
 
+// The cuts and the draw with the reference's own arithmetic, by one warp: probabilities p[i] = x[i] / s, their sequential sums
+// c[i] = p[0] + ... + p[i] (src/sampler.cpp:42-49).  Leaves p in `e` and c in `x`; returns keep | pick << 16.
+static __device__ __noinline__ int exact_cuts(double* x, double* e, int kk, double s, double min_p, double top_p, double u) {
+    const int lane = threadIdx.x & 31;
+    int keep = 0;
+    for (int b = 0; b < kk; b += 32) {   // min-p keeps those not below p[0] * min_p (they do not increase, p[0] is 1 / s)
+        const bool in = b + lane < kk;
+        const double p = in ? __ddiv_rn(x[b + lane], s) : 0.0;
+        if (in) e[b + lane] = p;
+        const bool cut = min_p > 0.0 && p < __dmul_rn(__ddiv_rn(1.0, s), min_p);
+        keep += __popc(__ballot_sync(0xffffffffu, in && !cut));
+    }
+    __syncwarp();
+    // top-p keeps the shortest prefix whose sum reaches top_p, the crossing candidate included
+    double c = 0.0;
+    int i = 0;
+    while (i < keep) {
+        double v[16];
+        const int n = min(16, keep - i);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = q < n ? e[i + q] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            c = __dadd_rn(c, v[q]);
+            if (lane == q) x[i + q] = c;
+        }
+        i += n;
+        if (c >= top_p) break;
+    }
+    __syncwarp();
+    for (int b = 0; b < i; b += 32) {
+        const unsigned m = __ballot_sync(0xffffffffu, b + lane < i && x[b + lane] >= top_p);
+        if (m) {
+            keep = min(keep, b + __ffs(m));
+            break;
+        }
+    }
+    const double r = __dadd_rn(__dmul_rn(u, x[keep - 1]), 0.0);   // r = u * tot + 0.0
+    int pick = keep - 1;
+    for (int b = 0; b < keep; b += 32) {
+        const unsigned m = __ballot_sync(0xffffffffu, b + lane < keep && r <= x[b + lane]);
+        if (m) {
+            pick = b + __ffs(m) - 1;
+            break;
+        }
+    }
+    return keep | pick << 16;
+}
+
 // srt[0..kk) holds the row's candidates in order (largest first).  Either hands them out (vocabulary-sharded mode)
 // or finishes the row: softmax over the candidates in fp64, sequential sums in candidate order, min-p, top-p,
-// draw.  `work` is scratch for 2 * kMaxK doubles that does not overlap srt.  The first kPost threads call it with the same
-// arguments; it is the last thing they do (no barrier at the end).
-// Exponentials and probabilities are one thread's work each.  Their sum and the cumulative probabilities follow the
-// reference's order of additions exactly, since a cut may fall on a tie: a warp runs the chain of dependent adds, all lanes
-// alike over broadcast reads - the first in every warp that needs the sum (no barrier to hand it over), the second in one
-// warp, which stops soon after top-p is reached.  The cuts and the draw are warp votes.  (The first sum over lanes instead, in another
-// order, would save 0.7 to 1.3 us a launch at k = 180 to 215, nothing that shows at k = 64.)
+// draw.  `work` is scratch for 2 * kMaxK doubles, 16-byte aligned, that does not overlap srt.  The first kPost threads call it
+// with the same arguments; it is the last thing they do (no barrier at the end).
+// Exponentials are one thread's work each.  Their sum follows the reference's order of additions exactly: a warp runs the
+// chain of dependent adds, 9 cycles each, all lanes alike over broadcast reads, and keeps the partial sums S[i].  The
+// reference then adds up the probabilities x[i] / S in the same way; both its cuts and its draw compare such a sum with a
+// number, and that sum differs from S[i] / S by less than (2 * 256 + 5) * 2^-53 of it, the rounding of three chains of at most
+// 256 terms.  A comparison that S[i] decides by more than 1e-12 - seventeen times that - comes out the same, so the second
+// chain and the divisions run only where one is closer (equal logits with a cut between them), or where the probabilities are
+// recorded.  Per launch, us: 24 x 100003, k = 50 18.6 -> 17.5; 64 x 262144, k = 64 26.9 -> 25.7; 512 x 65536, k = 200 94.8 -> 90.6.
 __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
     const int tid = threadIdx.x, lane = tid & 31;
     double* e = work;
@@ -336,67 +387,62 @@ __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTa
     }
     int token = 0, keep = 0;
     if (kk > 0 && !(r.flags & kRowGreedy)) {
-        // pr[i] = exp((double)(x_i - x_0) / T)   (fp32 subtraction, fp64 division, src/sampler.cpp:40)
+        // x[i] = exp((double)(x_i - x_0) / T)   (fp32 subtraction, fp64 division, src/sampler.cpp:40)
         double x = 0.0;
         if (tid < kk) x = exp(__ddiv_rn((double)__fsub_rn(comp_value(srt[tid]), comp_value(srt[0])), (double)r.temperature));
         P[tid] = x;   // (kMaxK == kPost: zeros behind the last candidate)
         block_sync<kPost, 1>();
-        double s = 0.0;
-        if ((tid & ~31) < kk) {
-            for (int i = 0; i < kk; i += 16) {
-                double v[16];
-#pragma unroll
-                for (int q = 0; q < 16; ++q) v[q] = P[i + q];
-#pragma unroll
-                for (int q = 0; q < 16; ++q) s = __dadd_rn(s, v[q]);
-            }
-        }
-        // probabilities; min-p keeps those not below pr[0] * min_p (they do not increase, pr[0] is 1 / sum)
-        const double p = __ddiv_rn(x, s);
-        if (tid < kk) e[tid] = p;
-        const bool cut = r.min_p > 0.0f && p < __dmul_rn(__ddiv_rn(1.0, s), (double)r.min_p);
-        keep = block_sync_count<kPost, 1>(tid < kk && !cut);
         if (tid >= 32) return;
-        // cumulative sums P[i] = pr[0] + ... + pr[i]; top-p keeps the shortest prefix whose sum reaches top_p, the crossing
-        // candidate included
-        const double top_p = r.top_p < 1.0f ? (double)r.top_p : 2.0;
-        double c = 0.0;
-        int i = 0;
-        while (i < keep) {
-            double v[16];
-            const int n = min(16, keep - i);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = q < n ? e[i + q] : 0.0;
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                c = __dadd_rn(c, v[q]);
-                if (lane == q) P[i + q] = c;
-            }
-            i += n;
-            if (c >= top_p) break;
-        }
-        __syncwarp();
-        if (r.top_p < 1.0f) {
-            for (int b = 0; b < i; b += 32) {
-                const unsigned m = __ballot_sync(0xffffffffu, b + lane < i && P[b + lane] >= top_p);
-                if (m) {
-                    keep = min(keep, b + __ffs(m));
-                    break;
-                }
-            }
-        }
-        const double tot = P[keep - 1];
-        // one engine output -> U[0,1) as libstdc++ does it, then r = u * tot + 0.0
+        // one engine output -> U[0,1) as libstdc++ does it
         double u = __dmul_rn(__ull2double_rn(r.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
         if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
-        const double rr = __dadd_rn(__dmul_rn(u, tot), 0.0);
-        int pick = keep - 1;
-        for (int b = 0; b < keep; b += 32) {
-            const unsigned m = __ballot_sync(0xffffffffu, b + lane < keep && rr <= P[b + lane]);
-            if (m) {
-                pick = b + __ffs(m) - 1;
-                break;
+        double s = 0.0;
+        for (int i = 0; i < kk; i += 16) {
+            double2 v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = *reinterpret_cast<const double2*>(P + i + 2 * q);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                v[q].x = s = __dadd_rn(s, v[q].x);
+                v[q].y = s = __dadd_rn(s, v[q].y);
             }
+            if (lane == 0) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) *reinterpret_cast<double2*>(e + i + 2 * q) = v[q];
+            }
+        }
+        __syncwarp();
+        int pick = 0;
+        const double close = 1e-12 * s;
+        bool sure = s < 1e300 && !o.kept_n;   // (an infinite logit makes the sum no number)
+        keep = kk;
+        if (sure && r.min_p > 0.0f) {
+            const double min_p = (double)r.min_p;
+            keep = 0;
+            for (int b = 0; b < kk; b += 32) {
+                const double v = b + lane < kk ? P[b + lane] : 0.0;
+                keep += __popc(__ballot_sync(0xffffffffu, v >= min_p));
+                sure = sure && !__any_sync(0xffffffffu, fabs(v - min_p) <= 1e-12 * min_p);
+            }
+        }
+        // first of the n kept candidates whose sum reaches t (n if there is none); notes when one is too close to tell
+        auto first_to_reach = [&](double t, int n) {
+            for (int b = 0; b < n; b += 32) {
+                const double v = b + lane < n ? e[b + lane] : 0.0;
+                const unsigned m = __ballot_sync(0xffffffffu, b + lane < n && v >= t);
+                sure = sure && !__any_sync(0xffffffffu, b + lane < n && fabs(v - t) <= close);
+                if (m) return b + __ffs(m) - 1;
+            }
+            return n;
+        };
+        if (sure) {
+            if (r.top_p < 1.0f) keep = min(keep, first_to_reach((double)r.top_p * s, keep) + 1);
+            pick = min(first_to_reach(u * e[keep - 1], keep), keep - 1);
+        }
+        if (!sure) {
+            const int both = exact_cuts(P, e, kk, s, (double)r.min_p, r.top_p < 1.0f ? (double)r.top_p : 2.0, u);
+            keep = both & 0xFFFF;
+            pick = both >> 16;
         }
         token = comp_id(srt[pick]);
     } else {
