@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         if (a.trace && blockIdx.x == gridDim.x - C && tid == 0) a.trace[(n)] = global_timer_ns(); \
     } while (0)
     FTR(0);
-    cluster_arrive_release();   // (waited for before the first access to another CTA's shared memory)
+    cluster_arrive_relaxed();   // (waited for before the first access to another CTA's shared memory)
     sh->hist[0][tid] = 0u;
     sh->hist[1][tid] = 0u;
     if (tid < 64) sh->table[tid] = exp2((double)tid / 64.0);

@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
         ctl->kept_n = 0;
         ctl->pen_n = 0;
     }
-    if (nseg > 1) cluster_arrive_release();   // (waited for before the first store to another CTA's shared memory)
+    if (nseg > 1) cluster_arrive_relaxed();   // (waited for before the first store to another CTA's shared memory)
     if (s.has_pen) {
         set_window(s, args.hist(), args.drafts(), dp);
         if constexpr (CELLS) collect_cells<T>(s, reinterpret_cast<unsigned*>(&ctl->pen_n));
@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         edge_col = w.edge_column(tid, a.n_vocab, seg, nseg);
         if (edge_col >= 0) edge = __ldcg(row_ptr + edge_col);
     }
-    if (nseg > 1) cluster_arrive_release();
+    if (nseg > 1) cluster_arrive_relaxed();
     Segment s = make_segment(a, w, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(pen_col + pen_cap));
     if (a.penalised) {   // (without windows nobody waits for the descriptor before the end)
         s.has_pen = (dp.flags & kRowPenalty) != 0;
