@@ -78,11 +78,6 @@ __device__ __forceinline__ U128 double_to_u128_ceil(double d) {
 }
 
 // ---- the cluster ---------------------------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // The cluster's barrier: arrive releases this thread's shared-memory writes to the cluster, wait acquires the others'.
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -12,7 +12,8 @@ constexpr int kMergeCap = 2400;               // candidates of one row that the 
 // status word bits written by kernels (0 = fine)
 enum : uint32_t {
     kStatusMergeOverflow = 4u,   // the candidate lists of a row hold more than the merge has room for
-    kStatusEmptyRow = 8u         // a row produced no candidate (all logits NaN)
+    kStatusEmptyRow = 8u,        // a row produced no candidate (all logits NaN)
+    kStatusLate = 16u            // what another CTA of the row had to send did not come
 };
 
 // row flags

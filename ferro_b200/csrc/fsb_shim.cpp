@@ -430,7 +430,7 @@ int fetch_tokens(fsb_handle* h, fsb_batch* b, int32_t* tokens_out, int64_t gathe
         // put the status word back into its idle state
         cudaMemsetAsync(b->d_status(), 0, sizeof(uint32_t), h->stream);
         cudaStreamSynchronize(h->stream);
-        return fail(h, FSB_ERR_DEVICE, "kernel status 0x%x (4 merge overflow, 8 row without a finite logit)", st);
+        return fail(h, FSB_ERR_DEVICE, "kernel status 0x%x (4 merge overflow, 8 row without a finite logit, 16 no word from another CTA of the row)", st);
     }
     if (tokens_out) std::memcpy(tokens_out, b->h_tokens, sizeof(int32_t) * (size_t)b->n_rows);
     return FSB_OK;

@@ -26,18 +26,24 @@ namespace {
 // from all threads' maxima the CTA derives a bound that at least k logits of the segment reach (cta_bound), at chunks 0, 1,
 // 3, 7, 15, ...  A cell whose maximum reaches the bound is listed in shared memory, data and all: about 100 in each of these
 // intervals for k = 64.  Every warp has a list of its own and keeps its length in a register: votes, but no atomics and
-// nothing to wait for.  Should a list overflow, the segment is gone through once more with the final bound.
-// At the end the listed cells are taken apart: the logits that reach the final bound are the segment's candidates, and
-// with them the penalised logits of the window that do so once penalised, each id once.  The softcap is applied here too,
-// to candidates only: it is monotone up to the rounding of tanhf, and a margin under the bound covers that.
-// The candidates are ordered; a row of several segments sends each segment's k best to its first CTA through distributed
-// shared memory, which picks the k best of all and finishes the row.
+// nothing to wait for.  Should a list overflow, the segment is gone through once more with the final bound.  A segment that
+// fits the ring (8192 or 32768 logits) is not listed: it is looked at again when its bound is known.
+// At the end the listed cells are taken apart: the logits that reach the final bound are candidates, and with them the
+// penalised logits of the window that do so once penalised, each id once.  The softcap is applied here too, to candidates
+// only: it is monotone up to the rounding of tanhf, and a margin under the bound covers that.
+// For k <= 64 the final bound is the row's (publish_most, key_bound), so a row has about 1.4 k candidates however many CTAs work
+// on it, and the few in each go straight to the first CTA, which orders them and finishes the row.  For k > 64 a CTA keeps to
+// its segment's bound, and the first one picks the k best of what they send.
 // What bounds it: the stream (HBM) for large batches, for small ones a chain of about ten dependent steps.  A step's
-// latency is its instruction count: a warp alone issues a dependent instruction every four to five cycles, so the code
-// after the stream counts over broadcast reads instead of sorting and branches little.
+// latency is its instruction count: a warp alone issues a dependent instruction every four to five cycles, and 32 warps that
+// all do the same take eight times their share of a scheduler, so steps after the stream are left to one warp or eight, and
+// what several CTAs need of one another goes by counted stores (inbox_put) instead of the cluster's barrier and its fences.
+// us per launch with launches chained (form 2), before -> after the final bound became the row's: 1 x 65536, k = 40 10.2 -> 7.9,
+// 32 x 131072, k = 40 14.4 -> 11.2, 72 x 131072, k = 50 21.0 -> 16.9, 64 x 262144, k = 64 23.3 -> 20.6, 512 x 32768, k = 40
+// 25.5 -> 24.5.
 // The exact path (exact_select) makes no assumption: a radix selection over the transformed segment that reads it again
 // (from L2) per digit.  It runs when hundreds of equal logits reach the final bound.
-// Nobody waits for another CTA but at the cluster's two barriers.
+// Waits for another CTA end after a million looks at the latest; the row is then reported (kStatusLate).
 
 constexpr int kCells = 4;                               // cells of a thread per chunk
 constexpr int kStages = 2;
@@ -55,23 +61,6 @@ size_t window_bytes(int seg_cols) { return seg_cols > 0 ? kPenCap * (sizeof(floa
 
 // The same where a bit per cell will do (see CellSegment): a group of 32 words per chunk of small CTAs.
 size_t cell_bits_bytes(int seg_cols) { return seg_cols > 0 ? (size_t)(seg_cols / 4 + 1024) / 1024 * 128 : 0; }
-
-// Sizes that go with T, the threads of a CTA.
-template <int T>
-struct Geometry {
-    static constexpr int kWarps = T / 32;
-    static constexpr int kChunkCells = kCells * T;
-    static constexpr size_t kRingBytes = (size_t)kStages * kChunkCells * sizeof(float4);
-    // cells a warp can list; with k > 64
-    static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64;
-    static_assert((kPickCap + 32 + kMaxK + kMergeList + 32) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
-    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns), control block, receive
-    // buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
-    static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
-        const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int));
-        return kRingBytes + cells + sizeof(SharedCtl) + (nseg > 1 ? kMergeList : 0) * sizeof(u64) + window_bytes(seg_cols);
-    }
-};
 
 struct Segment {
     const float* row;          // the row's logits
@@ -115,6 +104,35 @@ __device__ __forceinline__ bool penalised(const CellSegment& s, int c) {
     }
 }
 
+struct StreamCtl : SharedCtl {
+    CellSegment seg;           // what the steps after the stream need to know: registers are scarce while it runs
+    RowDesc desc;
+    u64 keyed, counted, sent;  // barriers: the row's keys have come; in its first CTA, the numbers of candidates, the candidates
+    u64 count[8];              // from segment r: its number of candidates, whether they are in the second part of its share, and how many words it has sent
+    unsigned bound;
+    int pad[3];
+};
+static_assert(sizeof(StreamCtl) % 16 == 0, "what follows the control block is read 16 bytes at a time");
+
+// Sizes that go with T, the threads of a CTA.
+template <int T>
+struct Geometry {
+    static constexpr int kWarps = T / 32;
+    static constexpr int kChunkCells = kCells * T;
+    static constexpr size_t kRingBytes = (size_t)kStages * kChunkCells * sizeof(float4);
+    // cells a warp can list; with k > 64
+    static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64;
+    static_assert((kPickCap + 32 + kMaxK + kMergeList + 32) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
+    // keys that the warps of a row hand over (publish_most): 8 per warp, at most 256
+    __host__ __device__ static constexpr int key_words(int nseg) { return T == 256 && nseg == 1 ? 64 : 256; }
+    // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns), control block, keys,
+    // receive buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
+    static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
+        const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int));
+        return kRingBytes + cells + sizeof(StreamCtl) + key_words(nseg) * sizeof(unsigned) + (nseg > 1 ? kMergeList : 0) * sizeof(u64) + window_bytes(seg_cols);
+    }
+};
+
 // Logit of column c as the sampler sees it.
 template <class S>
 __device__ __forceinline__ float transform(float x, int c, const S& s) {
@@ -154,6 +172,70 @@ __device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, int 
     block_sync<T, BAR>();
     const unsigned m = __reduce_min_sync(0xffffffffu, ctl->top[buf][lane & (kWarps - 1)]);
     return fmaxf(key_float(m), -FLT_MAX);   // (also for the patterns just below minus infinity's key, which are no numbers)
+}
+
+// For k <= 64 the final bound is the row's, however many CTAs it has: every warp hands its `most` largest lane maxima - each lane's
+// is a logit of its own; keys, their low bits cut off - to all CTAs of the row, and each finds a value that at least k of all those
+// keys reach, and not many more: about 1.1 k to 1.7 k logits do.
+__device__ __forceinline__ int warps_with_data(int cells, int n_warps) { return min(n_warps, (cells + 31) >> 5); }
+template <int T>
+__device__ __forceinline__ void publish_most(float run, int most, int seg, int nseg, unsigned* keys, u64* inbox) {
+    constexpr int kWarps = T / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned key = (float_key(run) & ~31u) | (unsigned)lane;
+    unsigned* own = keys + (seg * kWarps + warp) * most;
+    unsigned at = 0u, bar = 0u;
+    if (nseg > 1 && lane < nseg) {
+        at = cluster_map_shared(smem_u32(own), (unsigned)lane);
+        bar = cluster_map_shared(smem_u32(inbox), (unsigned)lane);
+    }
+    for (int r = 0; r < most; ++r) {
+        const unsigned top = __reduce_max_sync(0xffffffffu, key);
+        if (key == top) key = 0u;
+        if (nseg == 1) {
+            if (lane == 0) own[r] = top & ~31u;
+        } else if (lane < nseg) {
+            inbox_put(at + 4u * (unsigned)r, top & ~31u, bar);
+        }
+    }
+}
+// One warp; `n` (8 .. 256) keys.  Bisection by votes, over the integers between the smallest and the largest key, until between k and
+// 9/8 k keys are at or above the middle (four or five steps of 50 cycles as a rule; counting all ranks took 1200).
+__device__ __forceinline__ unsigned key_bound(int n, int k, const unsigned* keys) {
+    const int lane = threadIdx.x & 31;
+    unsigned q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = 32 * i + lane < n ? keys[32 * i + lane] : 0u;
+    auto reach = [&](unsigned t) {
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) c += __popc(__ballot_sync(0xffffffffu, q[i] >= t));
+        if (n > 128) {
+#pragma unroll
+            for (int i = 4; i < 8; ++i) c += __popc(__ballot_sync(0xffffffffu, q[i] >= t));
+        }
+        return c;
+    };
+    unsigned top = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) top = max(top, q[i]);
+    unsigned lo = 0x00800000u, hi = __reduce_max_sync(0xffffffffu, top) + 1u;   // lo: the key of -FLT_MAX
+    if (hi <= lo || reach(lo) < k) return 0u;
+    unsigned low = hi;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) low = min(low, q[i] >= lo ? q[i] : hi);
+    lo = __reduce_min_sync(0xffffffffu, low);
+    while (hi - lo > 1u) {
+        const unsigned mid = lo + ((hi - lo) >> 1);
+        const int c = reach(mid);
+        if (c >= k) {
+            lo = mid;
+            if (8 * c <= 9 * k) break;
+        } else {
+            hi = mid;
+        }
+    }
+    return lo;
 }
 
 // The softcap y(x) = cap * tanhf(x / cap) is monotone up to rounding: the division, tanhf (2 ulp) and the product are
@@ -370,20 +452,39 @@ __device__ __forceinline__ void set_window(Segment& s, const int32_t* hist, cons
     s.window_len = d.hist_len + (d.flags >> kRowDraftShift);
 }
 
-// The window's columns of the segment: sets their bits, and lists each once - an id counts once however often it occurs -
-// with its logit, which is fetched now (the copies belong to the next group that the thread commits) and needed at the end.
-// All threads call; a barrier has to follow.
+// The first ids of the window, up to 1024, which a CTA asks for before its copies fill the memory pipes.
 template <int T>
-__device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* ctl, float* pen_raw, int* pen_col) {
-    const int tid = threadIdx.x, lane = tid & 31;
-    int id = tid < s.window_len ? window_id(s, tid) : -1;
-    for (int i = tid; i < (s.hi - s.bit0 + 127) >> 7; i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    for (int i0 = tid & ~31; i0 < s.window_len; i0 += T) {
-        const int next = i0 + T + lane < s.window_len ? window_id(s, i0 + T + lane) : -1;
+struct FirstIds {
+    static constexpr int kPer = 1024 / T;
+    int id[kPer];
+    __device__ __forceinline__ void load(const Segment& s) {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) id[q] = (int)threadIdx.x + q * T < s.window_len ? window_id(s, threadIdx.x + q * T) : 0;
+    }
+    // calls f(in the window, id) for every id of the window, whole warps at a time
+    template <class F>
+    __device__ __forceinline__ void each(const Segment& s, F f) const {
+        const int tid = threadIdx.x, i0 = tid & ~31;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+            if (i0 + q * T < s.window_len) f(tid + q * T < s.window_len, id[q]);
+        for (int i = tid + 1024; (i & ~31) < s.window_len; i += T) f(i < s.window_len, i < s.window_len ? window_id(s, i) : 0);
+    }
+};
+__device__ __forceinline__ void clear_bits(unsigned* bitmap, int quads, int threads) {
+    for (int i = threadIdx.x; i < quads; i += threads) reinterpret_cast<uint4*>(bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The window's columns of the segment: sets their bits (cleared before), and lists each once - an id counts once however often it
+// occurs - with its logit, which is fetched now (the copies belong to the next group that the thread commits) and needed at the end.
+// All threads call, after a barrier; another has to follow.
+template <int T>
+__device__ __forceinline__ void collect_penalised(const Segment& s, const FirstIds<T>& ids, SharedCtl* ctl, float* pen_raw, int* pen_col) {
+    const int lane = threadIdx.x & 31;
+    ids.each(s, [&](bool in, int id) {
         const int c = id - s.id_base;
         bool first = false;
-        if (i0 + lane < s.window_len && c >= s.lo && c < s.hi) {
+        if (in && c >= s.lo && c < s.hi) {
             const unsigned bit = 1u << ((c - s.bit0) & 31);
             first = (atomicOr(&s.bitmap[(c - s.bit0) >> 5], bit) & bit) == 0u;
         }
@@ -397,8 +498,7 @@ __device__ __forceinline__ void collect_penalised(const Segment& s, SharedCtl* c
                 cp_async4(smem_u32(pen_raw + p), s.row + c);
             }
         }
-        id = next;
-    }
+    });
 }
 // Calls f(valid, raw logit, column) for every penalised column; whole warps call it together.
 template <int T, class F>
@@ -441,19 +541,17 @@ __device__ __forceinline__ void mask_penalised(float4 (&x)[kCells], const unsign
         }
     }
 }
-// The window's cells: sets their bits before the stream, and fills the table after it.  All threads call; a barrier has to follow.
+// The window's cells: sets their bits (cleared before, as `edges` is) before the stream, and fills the table after it.  All threads
+// call; a barrier has to follow.
 template <int T>
-__device__ __forceinline__ void collect_cells(const CellSegment& s, unsigned* edges) {
-    for (int i = threadIdx.x; i < 8 * ((s.n_cells + 1023) >> 10); i += T) reinterpret_cast<uint4*>(s.bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x == 0) *edges = 0u;
-    __syncthreads();
-    for (int i = threadIdx.x; i < s.window_len; i += T) {
-        const int c = window_id(s, i) - s.id_base;
-        if (c < s.lo || c >= s.hi) continue;
+__device__ __forceinline__ void collect_cells(const CellSegment& s, const FirstIds<T>& ids, unsigned* edges) {
+    ids.each(s, [&](bool in, int id) {
+        const int c = id - s.id_base;
+        if (!in || c < s.lo || c >= s.hi) return;
         const int cell = (c - s.head) >> 2;
         if (outside_cells(s, c)) atomicOr(edges, 1u << edge_index(s, c));
         else atomicOr(&s.bitmap[cell_word(cell)], 1u << (cell & 31));
-    }
+    });
 }
 template <int T>
 __device__ __forceinline__ void fill_table(const CellSegment& s) {
@@ -533,7 +631,7 @@ struct SelectArgs {
 };
 
 template <int T, int NDESC, bool LONG, bool CELLS>
-__global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
+__global__ void __launch_bounds__(T, T == 256 && NDESC > 0 ? 2 : 1024 / T) stream_select_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
     using G = Geometry<T>;
     constexpr int kChunkCells = G::kChunkCells, kWarps = G::kWarps;
     const StreamArgs& a = args.a;
@@ -548,8 +646,10 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     int* listed_num = reinterpret_cast<int*>(listed + kWarps * cell_cap);
     float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
     int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised && !CELLS ? kPenCap : 0));
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(pen_col + (a.penalised && !CELLS ? kPenCap : 0));
-    u64* recv = reinterpret_cast<u64*>(ctl + 1);
+    StreamCtl* ctl = reinterpret_cast<StreamCtl*>(pen_col + (a.penalised && !CELLS ? kPenCap : 0));
+    unsigned* keys = reinterpret_cast<unsigned*>(ctl + 1);   // the largest logits that the row's warps have seen
+    u64* recv = reinterpret_cast<u64*>(keys + G::key_words(a.nseg));
+    u64* lists = reinterpret_cast<u64*>(listed);
     listed += (tid >> 5) * cell_cap;   // the warp's own
     listed_num += (tid >> 5) * cell_cap;
     pdl_launch_dependents();
@@ -558,9 +658,7 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
     // placing the CTAs on the SMs - overlaps the end of the launch before it.
     if (a.write_back || a.overlap != 1) pdl_wait_prior();
 
-    const int nseg = a.nseg;
-    const int row = nseg == 1 ? (int)blockIdx.x : (int)blockIdx.x / nseg;
-    const int seg = (int)blockIdx.x - row * nseg;
+    const int nseg = a.nseg, row = (int)cluster_id(), seg = (int)cluster_rank();
     const RowDesc& dp = NDESC > 0 ? args.rows[row] : a.rows[row];
     const float* row_ptr = a.logits + (a.row_ld >= 0 ? (int64_t)row * a.row_ld : dp.logits_off);
 
@@ -579,41 +677,71 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_select_kernel(const __grid
             if (j + u * T < c_hi) cp_async16(dst + (unsigned)(u * T * sizeof(float4)), cells + j + u * T);
         cp_async_commit();
     };
-    for (int c = 0; c < kStages; ++c) fetch(c);
+    using Seg = std::conditional_t<CELLS, CellSegment, Segment>;
+    unsigned* const bitmap = reinterpret_cast<unsigned*>(recv + (nseg > 1 ? kMergeList : 0));
+    const bool has_pen = (dp.flags & kRowPenalty) != 0;
+    const int k = dp.k;
+    int most = 1;   // keys that a warp hands over: 1.6 k of them in all, but no more than 8 a warp
+    if constexpr (!LONG) {
+        const int sources = nseg * warps_with_data((n_cells + nseg - 1) / nseg, kWarps);
+        while (most < 8 && 5 * most * sources < 8 * k) most *= 2;
+    }
     if (tid < 8) {   // the logits outside the whole cells
         const int c = span.edge_column(tid, V, seg, nseg);
-        ctl->edge[tid] = c >= 0 ? __ldcg(row_ptr + c) : qnan;
+        if (c >= 0) cp_async4(smem_u32(&ctl->edge[tid]), row_ptr + c);
+        else ctl->edge[tid] = qnan;
     }
-    std::conditional_t<CELLS, CellSegment, Segment> s;
-    static_cast<Segment&>(s) = make_segment(a, span, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(recv + (nseg > 1 ? kMergeList : 0)));
-    if constexpr (CELLS) {
-        s.table = reinterpret_cast<int*>(list + kMergeList / 2);   // (behind what the rare paths keep in the list's memory)
-        s.edges = reinterpret_cast<const unsigned*>(&ctl->pen_n);
-        s.head = head;
-        s.n_cells = n_cells;
-    }
-    s.has_pen = (dp.flags & kRowPenalty) != 0;
-    s.pen = dp.penalty;
-    const int k = dp.k;
+    if (tid >= 32 && tid < 40) reinterpret_cast<u64*>(&ctl->desc)[tid - 32] = reinterpret_cast<const u64*>(&dp)[tid - 32];
     if (tid == 0) {
         ctl->lost = 0;
         ctl->kept_n = 0;
         ctl->pen_n = 0;
+        if (nseg > 1 && !LONG) {
+            inbox_init(&ctl->keyed);
+            inbox_init(&ctl->counted);
+            inbox_init(&ctl->sent);
+            inbox_inits_fence();
+            inbox_expect(&ctl->keyed, (unsigned)(4 * most * kWarps * nseg));
+            inbox_expect(&ctl->counted, (unsigned)(8 * nseg));
+        }
     }
     if (nseg > 1) cluster_arrive_relaxed();   // (waited for before the first store to another CTA's shared memory)
-    if (s.has_pen) {
-        set_window(s, args.hist(), args.drafts(), dp);
-        if constexpr (CELLS) collect_cells<T>(s, reinterpret_cast<unsigned*>(&ctl->pen_n));
-        else collect_penalised<T>(s, ctl, pen_raw, pen_col);
+    {
+        Seg s;
+        static_cast<Segment&>(s) = make_segment(a, span, row_ptr, seg, nseg, bitmap);
+        s.has_pen = has_pen;
+        s.pen = dp.penalty;
+        if (has_pen) set_window(s, args.hist(), args.drafts(), dp);
+        if constexpr (CELLS) {
+            s.table = reinterpret_cast<int*>(list + kMergeList / 2);   // (behind what the rare paths keep in the list's memory)
+            s.edges = reinterpret_cast<const unsigned*>(&ctl->pen_n);
+            s.head = head;
+            s.n_cells = n_cells;
+        }
+        if (tid == 0) static_cast<Seg&>(ctl->seg) = s;
+        // Of the stream's copies those of the first chunk go out before the window's bits are set, the others after: a copy takes the
+        // load/store unit 16 cycles per warp, and what works on shared memory queues behind them.
+        if (has_pen) {
+            FirstIds<T> ids;
+            ids.load(s);
+            clear_bits(bitmap, CELLS ? 8 * ((n_cells + 1023) >> 10) : (s.hi - s.bit0 + 127) >> 7, T);
+            fetch(0);
+            __syncthreads();
+            if constexpr (CELLS) collect_cells<T>(s, ids, reinterpret_cast<unsigned*>(&ctl->pen_n));
+            else collect_penalised<T>(s, ids, ctl, pen_raw, pen_col);
+            for (int c = 1; c < kStages; ++c) fetch(c);
+        } else {
+            for (int c = 0; c < kStages; ++c) fetch(c);
+        }
     }
     __syncthreads();
-    if (!CELLS && s.has_pen && tid < 8) {   // penalised logits are looked at on their own
-        const int c = tid < 4 ? tid : head + 4 * n_cells + tid - 4;
-        if (ctl->edge[tid] == ctl->edge[tid] && penalised(s, c)) ctl->edge[tid] = qnan;
-    }
+    const Seg& s = ctl->seg;
     trace_mark(a, 1);
 
     // ---- the stream
+    const float cap = a.softcap;
+    // A segment that fits the ring is only looked at when its final bound is known: nothing is listed.
+    const bool held = !LONG && !CELLS && c_hi - c_lo <= kStages * kChunkCells;
     float run_a = ninf, run_b = ninf, thr = -FLT_MAX, admit = -FLT_MAX, seen = ninf;
     int refreshes = 0;
     int wn = 0;           // cells in the warp's list
@@ -628,12 +756,12 @@ again_from_the_start:
         float4 x[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) x[u] = st[u * T];
-        if (!CELLS && s.has_pen) mask_penalised<T>(x, s.bitmap, j0 - c_lo, left);
+        if (!CELLS && has_pen) mask_penalised<T>(x, bitmap, j0 - c_lo, left);
         float m[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
-        if (CELLS && s.has_pen) {
-            const uint4 aside = reinterpret_cast<const uint4*>(s.bitmap)[8 * c + (tid >> 5)];
+        if (CELLS && has_pen) {
+            const uint4 aside = reinterpret_cast<const uint4*>(bitmap)[8 * c + (tid >> 5)];
             if ((aside.x >> lane) & 1u) m[0] = ninf;
             if ((aside.y >> lane) & 1u) m[1] = ninf;
             if ((aside.z >> lane) & 1u) m[2] = ninf;
@@ -644,14 +772,22 @@ again_from_the_start:
             for (int u = 0; u < kCells; ++u)
                 if (tid + u * T >= left) m[u] = ninf;
         }
-        run_a = max3(run_a, m[0], m[1]);
-        run_b = max3(run_b, m[2], m[3]);
+        if (LONG) {
+            run_a = max3(run_a, m[0], m[1]);
+            run_b = max3(run_b, m[2], m[3]);
+        } else {
+            run_a = max3(run_a, max3(m[0], m[1], m[2]), m[3]);
+        }
         fetch(c + kStages);   // into the stage just read
+        if (held) {
+            if (left <= kChunkCells) break;
+            continue;
+        }
         fresh = !again && ((c & (c + 1)) == 0 || thr <= -FLT_MAX || (k > 64 && c < 4));
         if (fresh) {
             thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
             admit = thr;
-            if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
+            if (cap != 0.0f) softcap_bounds(thr, cap, admit, seen);
             if (wn > cell_cap / 4) wn = prune_cells(listed, listed_num, wn, admit);
         }
         if (__any_sync(0xffffffffu, fmaxf(max3(m[0], m[1], m[2]), m[3]) >= admit)) {   // the warp's own list: no atomics
@@ -672,20 +808,37 @@ again_from_the_start:
         }
         if (left <= kChunkCells) break;
     }
-    cp_async_wait<0>();
+    cp_async_wait<0>();   // (also the penalised logits and those outside the cells: a group has been committed after them)
     if (lost && lane == 0) ctl->lost = 1;
     trace_mark(a, 4);
 
-    // ---- the segment's candidates: logits that reach the final bound
-    if (fresh || again) {
+    // ---- candidates: logits that reach the final bound
+    if constexpr (LONG) {
+        if (fresh || again) {
+            __syncthreads();
+        } else {
+            thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
+            admit = thr;
+            if (cap != 0.0f) softcap_bounds(thr, cap, admit, seen);
+        }
+    } else if (again) {
         __syncthreads();
     } else {
-        thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
+        if (nseg > 1) cluster_wait_acquire();   // every CTA of the row runs: its shared memory may be written
+        publish_most<T>(run_a, most, seg, nseg, keys, &ctl->keyed);
+        if (nseg == 1) __syncthreads();
+        if (tid < 32) {
+            if (nseg > 1 && !inbox_wait(&ctl->keyed) && lane == 0) report_status(a.status, a.status_host, kStatusLate);
+            const unsigned least = key_bound(most * kWarps * nseg, k, keys);
+            if (lane == 0) ctl->bound = least;
+        }
+        __syncthreads();
+        thr = fmaxf(key_float(ctl->bound), -FLT_MAX);
         admit = thr;
-        if (s.cap != 0.0f) softcap_bounds(thr, s.cap, admit, seen);
+        if (cap != 0.0f) softcap_bounds(thr, cap, admit, seen);
     }
     const bool bounded = thr > -FLT_MAX;
-    if (s.cap == 0.0f) seen = thr;      // (minus infinity is not among the listed ones)
+    if (cap == 0.0f) seen = thr;      // (minus infinity is not among the listed ones)
     lost = ctl->lost != 0;
     if (lost && bounded && !again) {   // the early bounds let too much through: the final one will not, unless many logits are equal
         __syncthreads();
@@ -697,13 +850,29 @@ again_from_the_start:
         __syncthreads();
         goto again_from_the_start;
     }
+    // Candidates go to a list of this CTA; those of a row of several CTAs straight to the first one's (k <= 64).  A CTA's share of it
+    // ends with room for a list that it makes again (64).
+    const bool direct = !LONG && nseg > 1;
+    const int lseg = 31 - __clz(nseg), share = direct ? min(kPickCap, (kMergeList >> lseg) - 64) : kPickCap;
+    unsigned first_recv = 0u, sent_bar = 0u;
+    if (direct) {
+        first_recv = cluster_map_shared(smem_u32(recv + (kMergeList >> lseg) * seg), 0u);
+        sent_bar = cluster_map_shared(smem_u32(&ctl->sent), 0u);
+    } else if (held) {
+        picked = lists;   // (the ring is still being read)
+    }
+    auto put = [&](int p, u64 m) {
+        if (p >= share) return;
+        if (direct) inbox_put(first_recv + 8u * (unsigned)p, m, sent_bar);
+        else picked[p] = m;
+    };
     auto pick = [&](bool hit, float y, int col) {   // all lanes of the warp
         const unsigned hits = __ballot_sync(0xffffffffu, hit);
         if (hits == 0u) return;
         int p = 0;
         if (lane == 0) p = atomicAdd(&ctl->kept_n, __popc(hits));
         p = __shfl_sync(0xffffffffu, p, 0) + __popc(hits & lanes_below());
-        if (hit && p < kPickCap) picked[p] = make_comp(y, col + s.id_base);
+        if (hit) put(p, make_comp(y, col + s.id_base));
     };
     auto pick_cell = [&](const float4& v, int col, int pen) {   // a cell per lane, `pen`: penalised ones of its columns
         float xs[4] = {v.x, v.y, v.z, v.w};
@@ -717,13 +886,22 @@ again_from_the_start:
                 if ((pen >> e) & 1) xs[e] = penalise(xs[e], s.pen);
         }
         const float least = fmaxf(seen, -FLT_MAX);
-        unsigned hit[4];
-        int q = warp_reserve<4>(xs, least, hit, &ctl->kept_n);
+        if constexpr (LONG) {
+            unsigned hit[4];
+            int q = warp_reserve<4>(xs, least, hit, &ctl->kept_n);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int at = q + __popc(hit[e] & lanes_below());
-            if (xs[e] >= least && at < kPickCap) picked[at] = make_comp(xs[e], col + e + s.id_base);
-            q += __popc(hit[e]);
+            for (int e = 0; e < 4; ++e) {
+                if (xs[e] >= least) put(q + __popc(hit[e] & lanes_below()), make_comp(xs[e], col + e + s.id_base));
+                q += __popc(hit[e]);
+            }
+        } else {   // few: a lane reserves for itself
+            const int hits = (xs[0] >= least ? 1 : 0) + (xs[1] >= least ? 1 : 0) + (xs[2] >= least ? 1 : 0) + (xs[3] >= least ? 1 : 0);
+            if (hits) {
+                int q = atomicAdd(&ctl->kept_n, hits);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (xs[e] >= least) put(q++, make_comp(xs[e], col + e + s.id_base));
+            }
         }
     };
     if constexpr (CELLS) {
@@ -733,18 +911,47 @@ again_from_the_start:
         }
     }
     if (!lost) {
-        for (int p0 = 0; p0 < wn; p0 += 32) {
-            float4 v = make_float4(ninf, ninf, ninf, ninf);
-            int col = 0;
-            if (p0 + lane < wn) {
-                v = listed[p0 + lane];
-                col = head + 4 * listed_num[p0 + lane];
+        if (held) {
+            auto cell = [&](int i) {   // the thread's i-th cell of the ring, which holds the segment in order
+                const int j = i * T + tid;
+                float4 v = make_float4(ninf, ninf, ninf, ninf);
+                if (j < c_hi - c_lo) {
+                    v = ring[j];
+                    if (s.has_pen) {
+                        const unsigned bits = s.bitmap[(j >> 3) + 1] >> (4 * (j & 7));
+                        if (bits & 1u) v.x = ninf;
+                        if (bits & 2u) v.y = ninf;
+                        if (bits & 4u) v.z = ninf;
+                        if (bits & 8u) v.w = ninf;
+                    }
+                }
+                return v;
+            };
+            unsigned mine = 0u;
+            if (run_a >= admit) {
+#pragma unroll
+                for (int i = 0; i < kStages * kCells; ++i) mine |= (cell_max(cell(i)) >= admit ? 1u : 0u) << i;
             }
-            pick_cell(v, col, 0);
+            while (mine) {   // (lanes on their own)
+                const int i = __ffs(mine) - 1;
+                mine &= mine - 1u;
+                pick_cell(cell(i), head + 4 * (c_lo + i * T + tid), 0);
+            }
+        } else {
+            for (int p0 = 0; p0 < wn; p0 += 32) {
+                float4 v = make_float4(ninf, ninf, ninf, ninf);
+                int col = 0;
+                if (p0 + lane < wn) {
+                    v = listed[p0 + lane];
+                    col = head + 4 * listed_num[p0 + lane];
+                }
+                if (LONG || cell_max(v) >= admit) pick_cell(v, col, 0);
+            }
         }
         if (tid < 32 && V != 4 * n_cells) {
-            const float x = lane < 8 ? ctl->edge[lane] : qnan;
+            float x = lane < 8 ? ctl->edge[lane] : qnan;
             const bool pen = CELLS && s.has_pen && lane < 8 && ((ctl->pen_n >> lane) & 1);
+            if (!CELLS && s.has_pen && x == x && penalised(s, lane < 4 ? lane : head + 4 * n_cells + lane - 4)) x = qnan;   // (looked at on its own)
             float y = s.cap != 0.0f ? softcap_call(x, s.cap) : x;
             if (pen) y = penalise(y, s.pen);
             pick((pen ? y > ninf : x >= admit) && y >= seen, y, lane < 4 ? lane : head + 4 * n_cells + lane - 4);
@@ -769,10 +976,23 @@ again_from_the_start:
     }
     __syncthreads();
     int n = ctl->kept_n;
-    lost = lost || n > kPickCap;
+    lost = lost || n > share;
     // (the softcap makes a finite logit of minus infinity, equal to or above others: without a raw bound such columns count, too)
-    if (lost || (n < k && bounded) || (s.cap != 0.0f && admit <= -FLT_MAX)) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
-    else if (n < k) n = append_masked<T>(s, n, k, picked, reinterpret_cast<unsigned*>(list));
+    const bool exact = lost || (LONG && n < k && bounded) || (cap != 0.0f && admit <= -FLT_MAX);
+    u64 report = 0ull;   // (to the first CTA)
+    if (exact || (n < k && !(direct && bounded))) {
+        const int kept = min(n, share);
+        if (exact) n = exact_select<T>(s, k, picked, reinterpret_cast<unsigned*>(list), ctl);
+        else n = append_masked<T>(s, n, k, picked, reinterpret_cast<unsigned*>(list));
+        if (direct) {   // (these work on a list of the CTA's own)
+            __syncthreads();
+            const int from = exact ? 0 : kept;
+            for (int i = from + tid; i < n; i += T) inbox_put(first_recv + 8u * (unsigned)((exact ? share : 0) + i), picked[i], sent_bar);
+            report = (u64)(unsigned)(kept + n - from) << 32 | (exact ? 1ull << 16 : 0ull) | (u64)(unsigned)n;
+        }
+    } else {
+        report = (u64)(unsigned)n << 32 | (u64)(unsigned)n;
+    }
     if (!CELLS && a.write_back) write_back<T>(s);
     if (!CELLS && a.patched && s.has_pen) send_patched<T>(s, a.patched + dp.gather_off);
     trace_mark(a, 2);
@@ -780,10 +1000,30 @@ again_from_the_start:
     if (a.overlap == 1) pdl_wait_prior();   // from here on this launch writes what the previous launch in the stream may still be using
 
     // ---- the row: the k best of all its segments' candidates, in order
+    if (direct) {
+        if (tid == 0) inbox_put(cluster_map_shared(smem_u32(&ctl->count[seg]), 0u), report, cluster_map_shared(smem_u32(&ctl->counted), 0u));
+        if (seg != 0) {
+            trace_mark(a, 6);
+            return;
+        }
+    }
     if (tid >= kPost) return;   // eight warps finish the row (no barrier of the whole CTA or by all threads of the cluster from here on)
     u64* all = picked;
-    if (nseg > 1) {
-        const int lseg = nseg == 8 ? 3 : nseg == 4 ? 2 : 1;
+    if (direct) {
+        if (!inbox_wait(&ctl->counted) && tid == 0) report_status(a.status, a.status_host, kStatusLate);
+        const u64 said = lane < nseg ? ctl->count[lane] : 0ull;
+        const int n_q = (int)(said & 0xFFFFu);
+        n = __reduce_add_sync(0xffffffffu, n_q);
+        const int words = __reduce_add_sync(0xffffffffu, (int)(said >> 32));
+        if (tid == 0) inbox_expect(&ctl->sent, 8u * (unsigned)words);
+        const int from = tid >> 5;   // one list: warp w copies segment w's part
+        const int before = __reduce_add_sync(0xffffffffu, lane < from ? n_q : 0), mine = __shfl_sync(0xffffffffu, n_q, from);
+        const u64* src = recv + (kMergeList >> lseg) * from + ((__shfl_sync(0xffffffffu, (unsigned)said, from) >> 16) & 1u ? share : 0);
+        if (!inbox_wait(&ctl->sent) && tid == 0) report_status(a.status, a.status_host, kStatusLate);
+        for (int i = lane; i < mine; i += 32) list[before + i] = src[i];
+        all = list;
+        block_sync<kPost, 1>();
+    } else if (LONG && nseg > 1) {
         cluster_wait_acquire();   // every CTA of the row runs: the first one's shared memory may be written
         const int send_cap = min(kPickCap, kMergeList >> lseg);
         const unsigned dst = cluster_map_shared(smem_u32(recv + seg * send_cap), 0u);
@@ -831,7 +1071,7 @@ again_from_the_start:
     rank_emit(all, n, k, all == list ? picked : list, ctl, [&](int rank, u64 m) { out[rank] = m; });
     block_sync<kPost, 1>();
     trace_mark(a, 5);
-    finish_row(a, dp, out, min(n, k), reinterpret_cast<double*>(list), ctl);
+    finish_row(a, ctl->desc, out, min(n, k), reinterpret_cast<double*>(list), ctl);
     trace_mark(a, 6);
 }
 
@@ -875,7 +1115,6 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
             if (j + u * T < w.c_hi) cp_async16(dst + (unsigned)(u * T * sizeof(float4)), w.cells + j + u * T);
         cp_async_commit();
     };
-    for (int c = 0; c < kStages; ++c) fetch(c);
     float edge = qnan;
     int edge_col = -1;
     if (tid < 8) {
@@ -887,13 +1126,21 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     if (a.penalised) {   // (without windows nobody waits for the descriptor before the end)
         s.has_pen = (dp.flags & kRowPenalty) != 0;
         s.pen = dp.penalty;
-        if (s.has_pen) {
-            set_window(s, args.hist(), args.drafts(), dp);
-            if (tid == 0) ctl->pen_n = 0;
-            collect_penalised<T>(s, ctl, pen_raw, pen_col);
-        }
+    }
+    if (s.has_pen) {
+        set_window(s, args.hist(), args.drafts(), dp);
+        FirstIds<T> ids;
+        ids.load(s);
+        if (tid == 0) ctl->pen_n = 0;
+        clear_bits(s.bitmap, (s.hi - s.bit0 + 127) >> 7, T);
+        fetch(0);
         __syncthreads();
-        if (s.has_pen && edge_col >= 0 && penalised(s, edge_col)) edge = qnan;
+        collect_penalised<T>(s, ids, ctl, pen_raw, pen_col);
+        for (int c = 1; c < kStages; ++c) fetch(c);
+        __syncthreads();
+        if (edge_col >= 0 && penalised(s, edge_col)) edge = qnan;
+    } else {
+        for (int c = 0; c < kStages; ++c) fetch(c);
     }
     trace_mark(a, 1);
 
