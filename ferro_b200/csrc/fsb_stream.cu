@@ -50,9 +50,10 @@ constexpr int kStages = 2;
 constexpr int kPenCap = 1024;                           // penalised columns of a segment that are looked up ahead
 constexpr int kPickCap = 1024;                          // candidates of a segment
 constexpr int kMergeList = 2048;                        // candidates of all segments, an equal share of it each
-constexpr int kCellSlots = 2048, kCellIds = 1024;       // penalised cells: slots of their table, and the longest window that may use it
+constexpr int kCellSlots = 4096, kCellIds = 2048;       // penalised cells: slots of their table, and the longest window that may use it
 constexpr int kSelectSmemMax = 224 * 1024;
 static_assert(kMergeList >= 2 * kMaxK, "the epilogue's scratch lives in the merge list's memory");
+static_assert((kPickCap + 32 + kMaxK) * 8 + 256 * 4 <= kStages * kCells * 256 * 16 - kCellSlots * 4, "candidates, the rare paths' counters and the table lie in a small CTA's ring");
 
 // Columns of the longest segment.
 int segment_columns(int n_vocab, int nseg) { return 4 * ((n_vocab / 4 + nseg - 1) / nseg) + 8; }
@@ -80,28 +81,35 @@ __device__ __forceinline__ float penalise(float x, float pen) { return x > 0.0f 
 __device__ __noinline__ float softcap_call(float x, float cap) { return __fmul_rn(cap, tanhf(__fdiv_rn(x, cap))); }          // src/model_gemma4.cpp:521
 __device__ __forceinline__ bool penalised(const Segment& s, int c) { return s.has_pen && ((s.bitmap[(c - s.bit0) >> 5] >> ((c - s.bit0) & 31)) & 1u); }
 
-// A whole row whose penalised logits are kept by cells, on small CTAs: in the stream a bit per cell - a quarter of the
-// memory, and one 16-byte read per warp and chunk - sets whole cells aside; at the end a hash table in the ring's memory
-// says which columns of those cells the window holds.
+// A whole row whose penalised logits are kept by cells, on small CTAs: a bit per cell - a quarter of the memory, and one
+// 16-byte read per warp and chunk - marks the cells that hold some.  Marked cells take no part in the bounds, but are listed as
+// others are if the largest of them, penalised or not, can reach the bound; at the end a hash table in the ring's memory says
+// which columns of the listed ones the window holds.  (Set aside as a whole and fetched again at the end, 800 random reads for a
+// window of 1024, they took 16 us of the 106 of a launch of 512 x 262144, all rows at the same time.)
+constexpr int kMarked = 1 << 30;   // in a listed cell's number
 struct CellSegment : Segment {
-    int* table;                // kCellSlots x (cell << 4 | penalised columns of it), -1: free
+    int* table;                // kCellSlots, or half of them, x (cell << 4 | penalised columns of it), -1: free
     const unsigned* edges;     // penalised ones of the logits outside the cells
     int head, n_cells;
+    int slots;
 };
 __device__ __forceinline__ int cell_word(int cell) { return (cell >> 10) * 32 + ((cell >> 5) & 7) * 4 + ((cell >> 8) & 3); }
-__device__ __forceinline__ unsigned cell_slot(int cell) { return ((unsigned)cell * 2654435761u) / (0x80000000u / (kCellSlots / 2)); }
+__device__ __forceinline__ unsigned cell_slot(int cell, int slots) { return __umulhi((unsigned)cell * 2654435761u, (unsigned)slots); }
 __device__ __forceinline__ int edge_index(const CellSegment& s, int c) { return c < s.head ? c : 4 + c - s.head - 4 * s.n_cells; }
 __device__ __forceinline__ bool outside_cells(const CellSegment& s, int c) { return c < s.head || c >= s.head + 4 * s.n_cells; }
+// The penalised columns of a marked cell.
+__device__ __forceinline__ int penalised_of(const CellSegment& s, int cell) {
+    for (unsigned h = cell_slot(cell, s.slots);; h = (h + 1u) & (unsigned)(s.slots - 1)) {   // (at least half of the slots are free)
+        const int v = s.table[h];
+        if (v < 0) return 0;
+        if ((v >> 4) == cell) return v & 15;
+    }
+}
 __device__ __forceinline__ bool penalised(const CellSegment& s, int c) {
     if (!s.has_pen) return false;
     if (outside_cells(s, c)) return (*s.edges >> edge_index(s, c)) & 1u;
     const int cell = (c - s.head) >> 2, e = (c - s.head) & 3;
-    if (!((s.bitmap[cell_word(cell)] >> (cell & 31)) & 1u)) return false;
-    for (unsigned h = cell_slot(cell);; h = (h + 1u) & (kCellSlots - 1u)) {   // (at least half of the slots are free)
-        const int v = s.table[h];
-        if (v < 0) return false;
-        if ((v >> 4) == cell) return (v >> e) & 1;
-    }
+    return ((s.bitmap[cell_word(cell)] >> (cell & 31)) & 1u) && ((penalised_of(s, cell) >> e) & 1);
 }
 
 struct StreamCtl : SharedCtl {
@@ -120,15 +128,16 @@ struct Geometry {
     static constexpr int kWarps = T / 32;
     static constexpr int kChunkCells = kCells * T;
     static constexpr size_t kRingBytes = (size_t)kStages * kChunkCells * sizeof(float4);
-    // cells a warp can list; with k > 64
-    static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64;
+    // cells a warp can list; with k > 64; where penalised cells are listed with the others (a window of a thousand ids may hold the
+    // hundred largest logits: with 64 a few rows in 512 went through their segment twice)
+    static constexpr int kWarpCells = 64, kWarpCellsLong = T == 256 ? 128 : 64, kWarpCellsMarked = 88;
     static_assert((kPickCap + 32 + kMaxK + kMergeList + 32) * sizeof(u64) <= kRingBytes, "everything after the stream lives in the ring's memory");
     // keys that the warps of a row hand over (publish_most): 8 per warp, at most 256
     __host__ __device__ static constexpr int key_words(int nseg) { return T == 256 && nseg == 1 ? 64 : 256; }
     // dynamic shared memory: ring, listed cells (data, numbers), penalised logits (data, columns), control block, keys,
     // receive buffer, bitmap of the penalised columns of the segment (its first word: the up to three columns before the cells)
-    static size_t smem_bytes(int nseg, int kmax, int seg_cols) {
-        const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : kWarpCells) * (sizeof(float4) + sizeof(int));
+    static size_t smem_bytes(int nseg, int kmax, int seg_cols, bool marked = false) {
+        const size_t cells = (size_t)kWarps * (kmax > 64 ? kWarpCellsLong : marked ? kWarpCellsMarked : kWarpCells) * (sizeof(float4) + sizeof(int));
         return kRingBytes + cells + sizeof(StreamCtl) + key_words(nseg) * sizeof(unsigned) + (nseg > 1 ? kMergeList : 0) * sizeof(u64) + window_bytes(seg_cols);
     }
 };
@@ -256,8 +265,9 @@ __device__ __forceinline__ void softcap_bounds(float thr, float cap, float& admi
     admit = fmaxf(admit, -FLT_MAX);
 }
 
-// Keeps those of a warp's n <= 128 listed cells that reach `admit`, in order; returns their number.
-__device__ __noinline__ int prune_cells(float4* cells, int* nums, int n, float admit) {
+// Keeps those of a warp's n <= 128 listed cells that reach `admit`, in order, and those whose number has a bit of `always`;
+// returns how many they are.
+__device__ __noinline__ int prune_cells(float4* cells, int* nums, int n, float admit, int always) {
     const int lane = threadIdx.x & 31;
     int w = 0;
     for (int p0 = 0; p0 < n; p0 += 32) {
@@ -267,7 +277,7 @@ __device__ __noinline__ int prune_cells(float4* cells, int* nums, int n, float a
         if (p0 + lane < n) {
             x = cells[p0 + lane];
             num = nums[p0 + lane];
-            keep = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)) >= admit;
+            keep = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)) >= admit || (num & always) != 0;
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {   // (never ahead of what is still to be read)
@@ -555,13 +565,13 @@ __device__ __forceinline__ void collect_cells(const CellSegment& s, const FirstI
 }
 template <int T>
 __device__ __forceinline__ void fill_table(const CellSegment& s) {
-    for (int i = threadIdx.x; i < kCellSlots / 4; i += T) reinterpret_cast<int4*>(s.table)[i] = make_int4(-1, -1, -1, -1);
+    for (int i = threadIdx.x; i < s.slots / 4; i += T) reinterpret_cast<int4*>(s.table)[i] = make_int4(-1, -1, -1, -1);
     __syncthreads();
     for (int i = threadIdx.x; i < s.window_len; i += T) {
         const int c = window_id(s, i) - s.id_base;
         if (c < s.lo || c >= s.hi || outside_cells(s, c)) continue;
         const int cell = (c - s.head) >> 2, bit = 1 << ((c - s.head) & 3);
-        for (unsigned h = cell_slot(cell);; h = (h + 1u) & (kCellSlots - 1u)) {   // (no more cells than ids: at most half of the slots)
+        for (unsigned h = cell_slot(cell, s.slots);; h = (h + 1u) & (unsigned)(s.slots - 1)) {   // (no more cells than ids: at most half of the slots)
             const int v = atomicCAS(&s.table[h], -1, cell << 4 | bit);
             if (v == -1) break;
             if ((v >> 4) == cell) {
@@ -642,7 +652,7 @@ __global__ void __launch_bounds__(T, T == 256 && NDESC > 0 ? 2 : 1024 / T) strea
     u64* list = out + kMaxK;
     float4* listed = reinterpret_cast<float4*>(smem_raw + G::kRingBytes);
     const int tid = threadIdx.x, lane = tid & 31;
-    constexpr int cell_cap = LONG ? G::kWarpCellsLong : G::kWarpCells;
+    constexpr int cell_cap = LONG ? G::kWarpCellsLong : CELLS ? G::kWarpCellsMarked : G::kWarpCells;
     int* listed_num = reinterpret_cast<int*>(listed + kWarps * cell_cap);
     float* pen_raw = reinterpret_cast<float*>(listed_num + kWarps * cell_cap);
     int* pen_col = reinterpret_cast<int*>(pen_raw + (a.penalised && !CELLS ? kPenCap : 0));
@@ -713,7 +723,8 @@ __global__ void __launch_bounds__(T, T == 256 && NDESC > 0 ? 2 : 1024 / T) strea
         s.pen = dp.penalty;
         if (has_pen) set_window(s, args.hist(), args.drafts(), dp);
         if constexpr (CELLS) {
-            s.table = reinterpret_cast<int*>(list + kMergeList / 2);   // (behind what the rare paths keep in the list's memory)
+            s.table = reinterpret_cast<int*>(smem_raw + G::kRingBytes) - kCellSlots;   // (the list's memory, but for what the rare paths keep there)
+            s.slots = s.window_len <= kCellIds / 2 ? kCellSlots / 2 : kCellSlots;
             s.edges = reinterpret_cast<const unsigned*>(&ctl->pen_n);
             s.head = head;
             s.n_cells = n_cells;
@@ -748,6 +759,7 @@ __global__ void __launch_bounds__(T, T == 256 && NDESC > 0 ? 2 : 1024 / T) strea
     bool fresh = false;   // the bound takes in everything seen so far
     bool lost = false;    // a list was too short
     bool again = false;   // the second time through: the bound is final
+    const bool raised = CELLS && has_pen && s.pen < 1.0f;
 again_from_the_start:
     for (int c = 0, j0 = c_lo + tid;; ++c, j0 += kChunkCells) {
         const int left = c_hi - (j0 - tid);   // cells of the segment from this chunk on
@@ -760,19 +772,25 @@ again_from_the_start:
         float m[kCells];
 #pragma unroll
         for (int u = 0; u < kCells; ++u) m[u] = cell_max(x[u]);
-        if (CELLS && has_pen) {
-            const uint4 aside = reinterpret_cast<const uint4*>(bitmap)[8 * c + (tid >> 5)];
-            if ((aside.x >> lane) & 1u) m[0] = ninf;
-            if ((aside.y >> lane) & 1u) m[1] = ninf;
-            if ((aside.z >> lane) & 1u) m[2] = ninf;
-            if ((aside.w >> lane) & 1u) m[3] = ninf;
-        }
         if (left < kChunkCells) {
 #pragma unroll
             for (int u = 0; u < kCells; ++u)
                 if (tid + u * T >= left) m[u] = ninf;
         }
-        if (LONG) {
+        unsigned marked = 0u;
+        if (CELLS && has_pen) {
+            const uint4 bits = reinterpret_cast<const uint4*>(bitmap)[8 * c + (tid >> 5)];
+            marked = ((bits.x >> lane) & 1u) | ((bits.y >> lane) & 1u) << 1 | ((bits.z >> lane) & 1u) << 2 | ((bits.w >> lane) & 1u) << 3;
+            float r[kCells];
+#pragma unroll
+            for (int u = 0; u < kCells; ++u) r[u] = (marked >> u) & 1u ? ninf : m[u];
+            run_a = max3(run_a, max3(r[0], r[1], r[2]), r[3]);
+            if (raised) {   // a penalty below 1 makes logits larger
+#pragma unroll
+                for (int u = 0; u < kCells; ++u)
+                    if ((marked >> u) & 1u) m[u] = cap != 0.0f ? -ninf : penalise(m[u], s.pen);
+            }
+        } else if (LONG) {
             run_a = max3(run_a, m[0], m[1]);
             run_b = max3(run_b, m[2], m[3]);
         } else {
@@ -788,7 +806,7 @@ again_from_the_start:
             thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
             admit = thr;
             if (cap != 0.0f) softcap_bounds(thr, cap, admit, seen);
-            if (wn > cell_cap / 4) wn = prune_cells(listed, listed_num, wn, admit);
+            if (wn > cell_cap / 4) wn = prune_cells(listed, listed_num, wn, admit, CELLS && raised ? kMarked : 0);
         }
         if (__any_sync(0xffffffffu, fmaxf(max3(m[0], m[1], m[2]), m[3]) >= admit)) {   // the warp's own list: no atomics
 #pragma unroll
@@ -797,7 +815,7 @@ again_from_the_start:
                 const int q = wn + __popc(hits & lanes_below());
                 if (m[u] >= admit && q < cell_cap) {
                     listed[q] = x[u];
-                    listed_num[q] = j0 + u * T;
+                    listed_num[q] = (j0 + u * T) | (CELLS && ((marked >> u) & 1u) ? kMarked : 0);
                 }
                 wn += __popc(hits);
             }
@@ -940,12 +958,21 @@ again_from_the_start:
         } else {
             for (int p0 = 0; p0 < wn; p0 += 32) {
                 float4 v = make_float4(ninf, ninf, ninf, ninf);
-                int col = 0;
+                int col = 0, pen = 0;
+                bool reach = false;
                 if (p0 + lane < wn) {
                     v = listed[p0 + lane];
-                    col = head + 4 * listed_num[p0 + lane];
+                    const int num = listed_num[p0 + lane], cell = num & ~kMarked;
+                    col = head + 4 * cell;
+                    reach = cell_max(v) >= admit;
+                    if constexpr (CELLS) {
+                        if (num != cell && (reach || raised)) {
+                            pen = penalised_of(s, cell);
+                            reach = true;
+                        }
+                    }
                 }
-                if (LONG || cell_max(v) >= admit) pick_cell(v, col, 0);
+                if (LONG || reach) pick_cell(v, col, pen);
             }
         }
         if (tid < 32 && V != 4 * n_cells) {
@@ -956,19 +983,7 @@ again_from_the_start:
             if (pen) y = penalise(y, s.pen);
             pick((pen ? y > ninf : x >= admit) && y >= seen, y, lane < 4 ? lane : head + 4 * n_cells + lane - 4);
         }
-        if constexpr (CELLS) {
-            if (s.has_pen) {
-                for (int i0 = 0; i0 < kCellSlots; i0 += 4 * T) {   // (kCellSlots is a multiple)
-                    const int4 at = reinterpret_cast<const int4*>(s.table)[i0 / 4 + tid];
-                    const int v[4] = {at.x, at.y, at.z, at.w};
-                    float4 raw[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) raw[i] = v[i] >= 0 ? __ldcg(cells + (v[i] >> 4)) : make_float4(ninf, ninf, ninf, ninf);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) pick_cell(raw[i], head + 4 * (v[i] >> 4), v[i] >= 0 ? v[i] & 15 : 0);
-                }
-            }
-        } else if (s.has_pen)
+        if (!CELLS && s.has_pen)
             for_each_penalised<T>(s, ctl->pen_n, pen_raw, pen_col, [&](bool in, float x, int col) {
                 const float y = penalise(s.cap != 0.0f ? softcap_call(x, s.cap) : x, s.pen);
                 pick(in && y >= seen && y > ninf, y, col);
@@ -1238,16 +1253,12 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
         return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
     }
     if constexpr (T == 256 && NDESC == 0) {
-        // Whole rows on small CTAs, four per SM: a bitmap of more than 65536 columns leaves room for three or two, and costs every
-        // thread four words per chunk.  Windows of 512 ids, k = 64, us with a bit per column -> per cell: 512 x 262144 134 -> 107,
-        // 512 x 65536 57 -> 46, 512 x 49152 49 -> 41, 200 x 131072 49 -> 42, 160 x 65536 31.5 -> 29.5; near the limit 296 x 49152
-        // 28.2 -> 29.0, 200 x 49152 26.9 -> 27.6, 200 x 32768 25 -> 25, 512 x 32768 37 -> 35, and with fewer logits the second
-        // look at the window is no longer hidden behind the stream of others (160 x 16384 16.5 -> 20).
-        // Windows of more than kCellIds ids would fill more than half of the table: they go by columns.  The step there, 1024 ->
-        // 1025 ids: 512 x 262144 128 -> 162 us, 512 x 131072 72 -> 105, 160 x 262144 68 -> 91, 160 x 65536 33 -> 34.  (Beyond
-        // kPenCap = 1024 ids in a segment the columns are also found through the bitmap: 1100 ids 186, 122, 96, 41 us.)
-        if (a.nseg == 1 && a.kmax <= 64 && a.n_vocab >= 49152 && a.window_max <= kCellIds && !a.write_back && !a.patched) {
-            cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(1, a.kmax, 0) + cell_bits_bytes(seg_cols);
+        // Whole rows on small CTAs, four per SM, that do not fit the ring: a bit per column costs every thread four words per chunk, and
+        // above 65536 columns the bitmap leaves room for three CTAs or two.  us per launch (chained), bit per column -> per cell, windows
+        // of 512 ids: 512 x 16384 22.6 -> 17.6, 200 x 49152 31.0 -> 27.5, 512 x 49152 35.0 -> 31.2, 160 x 16384 22.3 -> 19.3; of 128 ids 512 x
+        // 32768 24.4 -> 21.0, of 1024 36.2 -> 26.6.  Windows of more than kCellIds ids would fill more than half of the table.
+        if (a.penalised && a.nseg == 1 && a.kmax <= 64 && a.n_vocab >= 4 * kStages * Geometry<T>::kChunkCells + 8 && a.window_max <= kCellIds && !a.write_back && !a.patched) {
+            cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(1, a.kmax, 0, true) + cell_bits_bytes(seg_cols);
             return (int)cudaLaunchKernelEx(&cfg, stream_select_kernel<T, NDESC, false, true>, args);
         }
     }
