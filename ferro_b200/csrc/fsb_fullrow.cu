@@ -7,14 +7,13 @@
 // HBM exactly once; everything after that reads shared memory:
 //   1. the row's largest and smallest candidate key                                            (src/sampler.cpp:38)
 //   2. if k < n: the k-th candidate, by a radix descent over the keys that counts                      (:27-31)
-//   3. one pass over the weights e_i = exp((double)(x_i - max) / T) as 2^-62 fixed point: their exact sum, the softmax
-//      denominator (:40-41), in registers, and a histogram of their upper 32 bits over kBins bins of equal width in the
-//      logit.  The cluster-wide cumulative histogram tells for any cumulative weight in which bin - or, because the
-//      lower bits are left out, in which few bins - it is reached.
+//   3. one pass over the weights e_i = exp((double)(x_i - max) / T) as 2^-62 fixed point: a histogram of them, exact,
+//      over kBins bins of equal width in the logit.  Its cluster-wide cumulative sums end with the softmax denominator
+//      (:40-41) and tell for any cumulative weight in which bin it is reached, and what the bins before it weigh.
 //   4. with top-p (:44) or min-p (:43): the bins that can hold kept candidates are known now.  Their candidates, tens to
 //      some hundreds as a rule, go to the first CTA, which orders them and does the rest of the row's work on the
 //      ordered list: exact cumulative weights, both cuts and the draw (:45-49).  Without a cut, or when there are too
-//      many, a cumulative weight is resolved on its own: exact weight above its bins, ordered candidates of its bins.
+//      many, a cumulative weight is resolved on its own: the ordered candidates of its bin go there.
 // If even one bin's candidates do not fit the first CTA's list (thousands of equal logits), a radix descent over the
 // candidate keys resolves it: MSB-first over 8-bit digits, at every level each CTA histograms the candidates of its
 // slice that match the prefix, all CTAs read all histograms through distributed shared memory and walk the digits - the
@@ -105,17 +104,21 @@ struct FullShared {
     // A descent's level histogram (kStripes copies): [stripe][limb 0..3, then the candidate count][digit], four words of
     // padding between stripes; a limb sum stays below 2^32 while a stripe sees fewer than 65537 candidates, i.e. for
     // rows of up to 4 M logits.  In the first CTA also the lists of candidates that the CTAs hand over (list()).
-    alignas(16) unsigned h[kStripes][(kLimbs + 1) * 256 + 4];
+    union {
+        alignas(16) unsigned h[kStripes][(kLimbs + 1) * 256 + 4];
+        struct {   // while the weights are added up:
+            unsigned hist[kLimbs][kBins];      // this CTA's weights by bin, as sums of their 16-bit limbs
+            u64 part[2][kFullThreads + 8];     // the CTAs' weights of the bins that this CTA adds up (upper and lower 32 bits' sums)
+        };
+    };
     u64 x_lo[2][256];          // this CTA's sum of them, which the other CTAs read; double buffered by level: a CTA may
     u64 x_hi[2][256];          // build the next level while others still read this one
     unsigned x_cnt[2][256];
     u64 x_small[2][4];         // small values exchanged across the cluster (extremes, sums), double buffered by use
     u64 x_all[2][kMaxCluster * 4];   // ... and every CTA's copy of all of them
     double table[64];          // 2^(j / 64)
-    unsigned hist[2][kBins];   // this CTA's weights (their upper parts) by bin: sums of bits 16..31 and of bits 0..15
-    u64 cum[kBins];            // cluster-wide: weight of bins 0 .. b in units of 2^-31, rounded per candidate
+    u64 cum[2][kBins];         // cluster-wide: weight of bins 0 .. b, the sums of the weights' lower 32 bits and of the rest
     unsigned cum_n[kBins];     // ... and about how many candidates they hold (see estimated_count)
-    u64 part[kFullThreads + 8];   // the CTAs' weights of the bins that this CTA adds up
     // suffix sums of the walk
     u64 w_lo[8], w_hi[8];
     unsigned w_cnt[8];
@@ -126,12 +129,15 @@ struct FullShared {
     u64 red[kFullWarps];
     u64 red_hi[kFullWarps];
     unsigned red_cnt[kFullWarps];
-    int bin_lo, bin_hi;        // bins that a cumulative weight may be reached in
+    int bin;                   // where a cumulative weight is reached
     int sent;                  // candidates this CTA has handed over
     unsigned got[2][kMaxCluster];   // ... every CTA of the cluster has, double buffered by use
     int first_p, first_u;      // places in the ordered list
     u64 kw_lo, kw_hi;          // weight of the kept set
     u64 cross[5];              // a resolved crossing: candidate, weight above (two words), count above, found
+    __device__ __forceinline__ U128 weight_to(int b) const {   // of the bins up to b, b included (-1: none)
+        return b < 0 ? U128{0ull, 0ull} : u128_add(U128{0ull, cum[0][b]}, U128{cum[1][b] >> 32, cum[1][b] << 32});
+    }
     __device__ __forceinline__ u64* list() { return reinterpret_cast<u64*>(&h[0][0]); }
 };
 static_assert(sizeof(u64) * (kMaxCluster * kSendCap + kShort) <= sizeof(FullShared::h), "the lists, and room to order a short one, lie in the histogram's memory");
@@ -492,20 +498,14 @@ __device__ __forceinline__ unsigned estimated_count(const RowCtx& rc, int bin, u
     return n < 1e6f ? (unsigned)n + (weight ? 1u : 0u) : 1000000u;
 }
 
-// First bin whose cumulative weight reaches t (2^-62 units) for certain, and the first that may reach it, given that up to
-// n candidates were rounded by half a unit each.  All threads call; contains barriers.
-__device__ __forceinline__ void find_bins(FullShared* sh, U128 t, unsigned n) {
+// First bin whose cumulative weight reaches t (the last one if none does).  All threads call; contains barriers.
+__device__ __forceinline__ int find_bin(FullShared* sh, U128 t) {
     const int b = threadIdx.x;
-    const u64 slack = n / 2u + 1u, t_lo = (t.hi << 33) | (t.lo >> 31), t_up = t_lo + 1ull + slack;   // t < 2^80
-    const u64 c = sh->cum[b], before = b > 0 ? sh->cum[b - 1] : 0ull;
-    if (b == 0) {
-        sh->bin_lo = kBins - 1;
-        sh->bin_hi = kBins - 1;
-    }
+    if (b == 0) sh->bin = kBins - 1;
     __syncthreads();
-    if (c >= t_up && (b == 0 || before < t_up)) sh->bin_hi = b;
-    if (c + slack >= t_lo && (b == 0 || before + slack < t_lo)) sh->bin_lo = b;
+    if (u128_ge(sh->weight_to(b), t) && (b == 0 || !u128_ge(sh->weight_to(b - 1), t))) sh->bin = b;
     __syncthreads();
+    return sh->bin;
 }
 
 // Sum of two words and a count over the CTA, left in x_small[use][0..2].  Contains one barrier; the sums are there after the
@@ -554,40 +554,29 @@ __device__ __forceinline__ void load4(const RowCtx& rc, int i, float (&x)[4]) {
     for (int e = 0; e < 4; ++e) x[e] = i + e < rc.n ? rc.at(i + e) : __int_as_float(0x7fc00000);
 }
 
-// Hands this CTA's candidates of bins [b_lo, b_hi] to the first CTA of the cluster, and adds up its weights and candidates of
-// the bins before them.  Returns whether everybody's candidates fitted.  After it the first CTA has the lists (CTA r's
-// sh->got[par][r] candidates at list() + r * kSendCap), and every CTA's sums are in its x_small[par].
+// Hands this CTA's candidates of bins [b_lo, b_hi] to the first CTA of the cluster, and counts its candidates of the bins before
+// them.  Returns whether everybody's candidates fitted.  After it the first CTA has the lists (CTA r's sh->got[par][r] candidates
+// at list() + r * kSendCap), and every CTA's count is in its x_small[par].
 template <int C>
-__device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsigned rank, int b_lo, int b_hi, bool sums, int par) {
+__device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsigned rank, int b_lo, int b_hi, bool count, int par) {
     const int tid = threadIdx.x;
     if (tid == 0) sh->sent = 0;
     __syncthreads();
     const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u);
-    u64 down = 0ull, up = 0ull;
     unsigned cnt = 0u;
     const int lane = tid & 31;
-    const float ninf = -__int_as_float(0x7f800000);
     bool full = false;   // (then nothing more is handed over: the lists are of no use)
-    float* pending = reinterpret_cast<float*>(sh->part) + (tid >> 5) * 64;
-    static_assert(sizeof(FullShared::part) >= kFullWarps * 64 * sizeof(float), "63 logits may wait per warp");
-    int waiting = 0;
-    auto add = [&](float x) {
-        const Weight w = rc.weight(x);
-        up += w.up;
-        down += (u64)(long long)w.down;
-    };
     for (int i0 = 4 * (tid - lane); i0 < rc.n; i0 += 4 * kFullThreads) {
         float x[4];
         load4(rc, i0 + 4 * lane, x);
-        bool give[4], above[4], some = false, any_above = false;
+        bool give[4], some = false;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int b = rc.bin(x[e]);
             const bool in = b <= b_hi && rc.is_candidate(x[e], i0 + 4 * lane + e);
             give[e] = in && b >= b_lo;
-            above[e] = in && b < b_lo;
+            cnt += in && b < b_lo ? 1u : 0u;
             some = some || give[e];
-            any_above = any_above || above[e];
         }
         if (__any_sync(0xffffffffu, some) && !full) {
 #pragma unroll
@@ -602,32 +591,9 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
                 if (give[e] && p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x[e], i0 + 4 * lane + e));
             }
         }
-        if (!sums) {
-            if (full) break;
-            continue;
-        }
-        // the logits above are collected until the warp has 32 of them: often they are few, and a weight costs as much for one
-        // lane as for all
-        if (!__any_sync(0xffffffffu, any_above)) continue;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const unsigned hits = __ballot_sync(0xffffffffu, above[e]);
-            if (above[e]) pending[waiting + __popc(hits & ((1u << lane) - 1u))] = x[e];
-            waiting += __popc(hits);
-            __syncwarp();
-            if (waiting >= 32) {
-                waiting -= 32;
-                add(pending[waiting + lane]);
-                cnt += 1u;
-                __syncwarp();
-            }
-        }
+        if (full && !count) break;
     }
-    if (sums && waiting > 0) {
-        add(lane < waiting ? pending[lane] : ninf);
-        cnt += lane < waiting ? 1u : 0u;
-    }
-    if (sums) block_sums(sh, par, down, up, cnt);
+    if (count) block_sums(sh, par, 0ull, 0ull, cnt);
     else __syncthreads();
     if (tid < C) cluster_store_u32(map_to_rank(&sh->got[par][rank], (unsigned)tid), (unsigned)sh->sent);
     cluster_sync_all();
@@ -805,16 +771,14 @@ __device__ __forceinline__ ListScan<T> scan_list(const RowCtx& rc, FullShared* s
 
 // The first CTA's share of resolve(): the crossing among the candidates it was sent goes to every CTA of the cluster.
 template <int C, int T>
-__device__ __forceinline__ void cross_list(const RowCtx& rc, FullShared* sh, int use, int n, U128 target) {
-    u64 lo = 0ull, hi = 0ull, cnt = 0ull;
+__device__ __forceinline__ void cross_list(const RowCtx& rc, FullShared* sh, int use, int n, U128 target, U128 above, bool count) {
+    u64 cnt = 0ull;
+    if (count) {
 #pragma unroll
-    for (unsigned r = 0; r < (unsigned)C; ++r) {
-        lo += ld_cluster_u64(map_to_rank(&sh->x_small[use][0], r));
-        hi += ld_cluster_u64(map_to_rank(&sh->x_small[use][1], r));
-        cnt += ld_cluster_u64(map_to_rank(&sh->x_small[use][2], r));
+        for (unsigned r = 0; r < (unsigned)C; ++r) cnt += ld_cluster_u64(map_to_rank(&sh->x_small[use][2], r));
     }
     const u64* srt = order_lists<C, T>(sh, use, n);
-    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, join_parts(lo, hi));
+    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, above);
     ls.each(n, [&](int e, U128 before, U128 with) {
         if (u128_ge(with, target) && (!u128_ge(before, target) || e == 0)) {
 #pragma unroll
@@ -878,19 +842,20 @@ __device__ __forceinline__ int finish_list(const RowCtx& rc, FullShared* sh, int
 }
 
 // The candidate at which the cumulative weight reaches `target`; every CTA gets it.  Bins if they are of use, else a descent.
+// `count`: the number of candidates before it is wanted.
 template <int C>
-__device__ __noinline__ Crossing resolve(const RowCtx rc, FullShared* sh, unsigned rank, bool binned, unsigned n_cand, u64 floor_c, u64 top_c, U128 target,
-                                         int& par) {
+__device__ __noinline__ Crossing resolve(const RowCtx rc, FullShared* sh, unsigned rank, bool binned, bool count, u64 floor_c, u64 top_c, U128 target, int& par) {
     const int tid = threadIdx.x;
     if (binned) {
-        find_bins(sh, target, n_cand);
+        const int bin = find_bin(sh, target);
         if (tid == 0) sh->cross[4] = 0ull;
-        const bool fits = send_bins<C>(rc, sh, rank, sh->bin_lo, sh->bin_hi, true, par);
+        const bool fits = send_bins<C>(rc, sh, rank, bin, bin, count, par);
         if (fits) {
             if (rank == 0) {
                 const int n = listed<C>(sh, par);
-                if (n > kShort) cross_list<C, kFullThreads>(rc, sh, par, n, target);
-                else if (tid < kShort) cross_list<C, kShort>(rc, sh, par, n, target);
+                const U128 above = sh->weight_to(bin - 1);
+                if (n > kShort) cross_list<C, kFullThreads>(rc, sh, par, n, target, above, count);
+                else if (tid < kShort) cross_list<C, kShort>(rc, sh, par, n, target, above, count);
             }
             par ^= 1;
             cluster_sync_all();
@@ -924,8 +889,6 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     } while (0)
     FTR(0);
     cluster_arrive_relaxed();   // (waited for before the first access to another CTA's shared memory)
-    sh->hist[0][tid] = 0u;
-    sh->hist[1][tid] = 0u;
     if (tid < 64) sh->table[tid] = exp2((double)tid / 64.0);
 
     // ---- 0. the slice as the sampler sees it: penalty bitmap, softcap, penalty, optional write-back.  The first loads of the
@@ -1086,8 +1049,10 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
     U128 S;
     const unsigned n_cand = rc.floor_c != 0ull ? (unsigned)d.k : valid;
-    {
-        u64 wl = 0ull, wh = 0ull;   // sums of the weights' lower and upper parts
+    if (binned) {
+#pragma unroll
+        for (int l = 0; l < kLimbs; ++l) sh->hist[l][tid] = 0u;
+        __syncthreads();
         for (int i = 4 * tid; i < n; i += 4 * kFullThreads) {
             float x[4];
             load4(rc, i, x);
@@ -1095,70 +1060,97 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
 #pragma unroll
                 for (int e = 0; e < 4; ++e) x[e] = rc.is_candidate(x[e], i + e) ? x[e] : ninf;
             }
-            Weight w[4];
+            u64 w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] = rc.weight(x[e]).value();
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                w[e] = rc.weight(x[e]);
-                wl += (u64)(long long)w[e].down;
-                wh += w[e].up;
-            }
-            if (binned && (w[0].up | w[1].up | w[2].up | w[3].up)) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int bin = rc.bin(x[e]);
-                    if (w[e].up >> 16) atomicAdd(&sh->hist[0][bin], w[e].up >> 16);
-                    if (w[e].up & 0xFFFFu) atomicAdd(&sh->hist[1][bin], w[e].up & 0xFFFFu);
+                unsigned* h = &sh->hist[0][rc.bin(x[e])];
+                const unsigned lo = (unsigned)w[e], hi = (unsigned)(w[e] >> 32);
+                if (lo & 0xFFFFu) atomicAdd(h, lo & 0xFFFFu);
+                if (lo >> 16) atomicAdd(h + kBins, lo >> 16);
+                if (hi) {
+                    if (hi & 0xFFFFu) atomicAdd(h + 2 * kBins, hi & 0xFFFFu);
+                    if (hi >> 16) atomicAdd(h + 3 * kBins, hi >> 16);
                 }
             }
         }
-        block_sums(sh, par, wl, wh, 0u);
         cluster_sync_all();
-        // Every CTA adds up kBins / C of the bins and hands the sums to all others: one load and one store per thread across the
-        // cluster (all bins read from all CTAs took 2.3 us).
-        {
-            constexpr int kMine = (kBins + C - 1) / C;   // (six CTAs: 171, and C * kMine is two more than there are threads)
-            static_assert(C * kMine <= kFullThreads + 8, "the parts' memory");
-            for (int t = tid; t < C * kMine; t += kFullThreads) {
-                const int src = t / kMine, bin = (int)rank * kMine + t % kMine;
-                if (bin < kBins)
-                    sh->part[t] = ((u64)ld_cluster_u32(map_to_rank(&sh->hist[0][bin], (unsigned)src)) << 16) + ld_cluster_u32(map_to_rank(&sh->hist[1][bin], (unsigned)src));
+        // Every CTA adds up kBins / C of the bins and hands the sums to all others: one load and one store per thread and word across
+        // the cluster (all bins read from all CTAs took 2.3 us).
+        constexpr int kMine = (kBins + C - 1) / C;   // (six CTAs: 171, and C * kMine is two more than there are threads)
+        static_assert(C * kMine <= kFullThreads + 8, "the parts' memory");
+        for (int t = tid; t < C * kMine; t += kFullThreads) {
+            const int src = t / kMine, bin = (int)rank * kMine + t % kMine;
+            if (bin < kBins) {
+                unsigned l[kLimbs];
+#pragma unroll
+                for (int q = 0; q < kLimbs; ++q) l[q] = ld_cluster_u32(map_to_rank(&sh->hist[q][bin], (unsigned)src));
+                sh->part[0][t] = (u64)l[0] + ((u64)l[1] << 16);
+                sh->part[1][t] = (u64)l[2] + ((u64)l[3] << 16);
             }
-            if (tid < C * 4) sh->x_all[par][tid] = ld_cluster_u64(map_to_rank(&sh->x_small[par][tid & 3], (unsigned)tid >> 2));
-            __syncthreads();
-            for (int t = tid; t < C * kMine; t += kFullThreads) {
-                const int dst = t / kMine, bin = (int)rank * kMine + t % kMine;
-                if (bin >= kBins) continue;
+        }
+        __syncthreads();
+        for (int t = tid; t < C * kMine; t += kFullThreads) {
+            const int dst = t / kMine, bin = (int)rank * kMine + t % kMine;
+            if (bin >= kBins) continue;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
                 u64 c = 0ull;
 #pragma unroll
-                for (int r = 0; r < C; ++r) c += sh->part[r * kMine + t % kMine];
-                cluster_store_u64(map_to_rank(&sh->cum[bin], (unsigned)dst), c);
+                for (int r = 0; r < C; ++r) c += sh->part[q][r * kMine + t % kMine];
+                cluster_store_u64(map_to_rank(&sh->cum[q][bin], (unsigned)dst), c);
             }
         }
         cluster_sync_all();
         // inclusive sums over the bins, largest logits first
         const int lane = tid & 31, warp = tid >> 5;
-        u64 c = sh->cum[tid];
-        unsigned est = estimated_count(rc, tid, c);
+        u64 c0 = sh->cum[0][tid], c1 = sh->cum[1][tid];
+        unsigned est = estimated_count(rc, tid, (c1 << 1) + (c0 >> 31));
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const u64 t = __shfl_up_sync(0xffffffffu, c, o);
+            const u64 t0 = __shfl_up_sync(0xffffffffu, c0, o), t1 = __shfl_up_sync(0xffffffffu, c1, o);
             const unsigned e = __shfl_up_sync(0xffffffffu, est, o);
             if (lane >= o) {
-                c += t;
+                c0 += t0;
+                c1 += t1;
                 est += e;
             }
         }
         if (lane == 31) {
-            sh->red[warp] = c;
+            sh->red[warp] = c0;
+            sh->red_hi[warp] = c1;
             sh->red_cnt[warp] = est;
         }
         __syncthreads();
-        u64 t = lane < warp ? sh->red[lane] : 0ull;
+        u64 t0 = lane < warp ? sh->red[lane] : 0ull, t1 = lane < warp ? sh->red_hi[lane] : 0ull;
         est += __reduce_add_sync(0xffffffffu, lane < warp ? sh->red_cnt[lane] : 0u);
 #pragma unroll
-        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        sh->cum[tid] = c + t;
+        for (int o = 16; o; o >>= 1) {
+            t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+            t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+        }
+        sh->cum[0][tid] = c0 + t0;
+        sh->cum[1][tid] = c1 + t1;
         sh->cum_n[tid] = est;
+        __syncthreads();
+        S = sh->weight_to(kBins - 1);
+    } else {
+        u64 wl = 0ull, wh = 0ull;   // sums of the weights' lower and upper parts
+        for (int i = 4 * tid; i < n; i += 4 * kFullThreads) {
+            float x[4];
+            load4(rc, i, x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const Weight w = rc.weight(rc.floor_c == 0ull || rc.is_candidate(x[e], i + e) ? x[e] : ninf);
+                wl += (u64)(long long)w.down;
+                wh += w.up;
+            }
+        }
+        block_sums(sh, par, wl, wh, 0u);
+        cluster_sync_all();
+        if (tid < C * 4) sh->x_all[par][tid] = ld_cluster_u64(map_to_rank(&sh->x_small[par][tid & 3], (unsigned)tid >> 2));
+        __syncthreads();
         wl = wh = 0ull;
 #pragma unroll
         for (int r = 0; r < C; ++r) {
@@ -1167,7 +1159,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         }
         S = join_parts(wl, wh);
         par ^= 1;
-        __syncthreads();
+        cluster_sync_all();   // (the next use of x_small)
     }
     const double sum = __dmul_rn(u128_to_double(S), 2.168404344971008868014905601739883422851562500e-19);   // * 2^-62
     const double min_thr = __dmul_rn(__ddiv_rn(1.0, sum), (double)d.min_p);
@@ -1180,10 +1172,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     // ---- 4a. the usual way with a cut: everything that can be kept goes to the first CTA, which finishes the row
     if (binned && (d.top_p < 1.0f || d.min_p > 0.0f)) {
         int b_hi = kBins - 1;
-        if (d.top_p < 1.0f) {
-            find_bins(sh, target_p, n_cand);
-            b_hi = sh->bin_hi;
-        }
+        if (d.top_p < 1.0f) b_hi = find_bin(sh, target_p);
         if (d.min_p > 0.0f) b_hi = min(b_hi, rc.bin(x_never));
         // (a list of more than a thousand is ordered too slowly: 22 us for 2000, two crossings take 15)
         if (sh->cum_n[b_hi] <= (unsigned)(3 * kFullThreads / 4) && send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
@@ -1226,7 +1215,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     bool keep_from_top_p = false;
     Crossing cp{0ull, U128{0ull, 0ull}, 0u, false};
     if (d.top_p < 1.0f) {
-        cp = resolve<C>(rc, sh, rank, binned, n_cand, c_k, cmax, target_p, par);
+        cp = resolve<C>(rc, sh, rank, binned, a.record != 0, c_k, cmax, target_p, par);
         if (cp.found && cp.c >= c_keep) {
             c_keep = cp.c;
             keep_from_top_p = true;
@@ -1269,7 +1258,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     {
         U128 target = double_to_u128_ceil(__dmul_rn(u, u128_to_double(KW)));
         if (!u128_ge(KW, target)) target = KW;   // (beyond it by rounding: the last one)
-        const Crossing ct = resolve<C>(rc, sh, rank, binned, n_cand, c_k, cmax, target, par);
+        const Crossing ct = resolve<C>(rc, sh, rank, binned, false, c_k, cmax, target, par);
         const u64 c_tok = ct.found && ct.c >= c_keep ? ct.c : c_keep;
         if (rank == 0 && tid == 0) finish(comp_id(c_tok));
     }
