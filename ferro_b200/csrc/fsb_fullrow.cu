@@ -129,7 +129,7 @@ struct FullShared {
     u64 red[kFullWarps];
     u64 red_hi[kFullWarps];
     unsigned red_cnt[kFullWarps];
-    int bin;                   // where a cumulative weight is reached
+    int bin, bin_two;          // where a cumulative weight is reached
     int sent;                  // candidates this CTA has handed over
     unsigned got[2][kMaxCluster];   // ... every CTA of the cluster has, double buffered by use
     int first_p, first_u;      // places in the ordered list
@@ -508,6 +508,19 @@ __device__ __forceinline__ int find_bin(FullShared* sh, U128 t) {
     return sh->bin;
 }
 
+// The same for two weights, t <= v.
+__device__ __forceinline__ void find_two_bins(FullShared* sh, U128 t, U128 v, int& b_t, int& b_v) {
+    const int b = threadIdx.x;
+    if (b == 0) sh->bin = sh->bin_two = kBins - 1;
+    __syncthreads();
+    const U128 with = sh->weight_to(b), before = sh->weight_to(b - 1);
+    if (u128_ge(with, t) && (b == 0 || !u128_ge(before, t))) sh->bin = b;
+    if (u128_ge(with, v) && (b == 0 || !u128_ge(before, v))) sh->bin_two = b;
+    __syncthreads();
+    b_t = sh->bin;
+    b_v = sh->bin_two;
+}
+
 // Sum of two words and a count over the CTA, left in x_small[use][0..2].  Contains one barrier; the sums are there after the
 // next one.
 __device__ __forceinline__ void block_sums(FullShared* sh, int use, u64 lo, u64 hi, unsigned cnt) {
@@ -595,6 +608,43 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
     }
     if (count) block_sums(sh, par, 0ull, 0ull, cnt);
     else __syncthreads();
+    if (tid < C) cluster_store_u32(map_to_rank(&sh->got[par][rank], (unsigned)tid), (unsigned)sh->sent);
+    cluster_sync_all();
+    bool fits = true;
+#pragma unroll
+    for (int r = 0; r < C; ++r) fits = fits && sh->got[par][r] <= (unsigned)kSendCap;
+    return fits;
+}
+
+// The same for the candidates of bins [b0, b1] and [b2, b3], without a count (b1 < b2, or the second range is empty).
+template <int C>
+__device__ __forceinline__ bool send_ranges(const RowCtx& rc, FullShared* sh, unsigned rank, int b0, int b1, int b2, int b3, int par) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) sh->sent = 0;
+    __syncthreads();
+    const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u);
+    // (a logit's bin is only worked out if the logit may lie in one of the ranges: a bin of room on either side covers the rounding)
+    const float width = 1.0f / rc.bin_scale, inf = __int_as_float(0x7f800000);
+    const float hi1 = b0 > 0 ? rc.mx - (float)(b0 - 1) * width : inf, lo1 = b1 < kBins - 1 ? rc.mx - (float)(b1 + 2) * width : -inf;
+    const float hi2 = b2 > 0 ? rc.mx - (float)(b2 - 1) * width : inf, lo2 = b3 < kBins - 1 ? rc.mx - (float)(b3 + 2) * width : -inf;
+    const bool two = b3 >= b2;
+    for (int i0 = 4 * (tid - lane); i0 < rc.n; i0 += 4 * kFullThreads) {
+        float x[4];
+        load4(rc, i0 + 4 * lane, x);
+        bool some = false;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) some = some || (x[e] <= hi1 && !(x[e] < lo1)) || (two && x[e] <= hi2 && !(x[e] < lo2));
+        if (!some) continue;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {   // (few: a lane reserves for itself)
+            const int b = rc.bin(x[e]), i = i0 + 4 * lane + e;
+            if (((b >= b0 && b <= b1) || (b >= b2 && b <= b3)) && rc.is_candidate(x[e], i)) {
+                const int p = atomicAdd(&sh->sent, 1);
+                if (p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x[e], i));
+            }
+        }
+    }
+    __syncthreads();
     if (tid < C) cluster_store_u32(map_to_rank(&sh->got[par][rank], (unsigned)tid), (unsigned)sh->sent);
     cluster_sync_all();
     bool fits = true;
@@ -839,6 +889,66 @@ __device__ __forceinline__ int finish_list(const RowCtx& rc, FullShared* sh, int
     list_sync<T>();
     if (a.record && tid == 0) a.kept_n[out] = keep;
     return comp_id(srt[min(sh->first_u, keep - 1)]);   // (a target beyond the list, by rounding, takes the last)
+}
+
+// The end of a row whose first CTA has the candidates of the bins [draw_lo, draw_hi] that the draw may fall into and [cut_lo, cut_hi]
+// where the kept set may end (none: nothing is cut): the cut, the weight of the kept set, the draw.
+struct RowEnds {
+    U128 target_p, S;
+    double u, sum, min_thr;
+    int draw_lo, draw_hi, cut_lo, cut_hi;
+    bool top_p, min_p;   // in the cut's bins
+};
+template <int C, int T>
+__device__ __forceinline__ int finish_bins(const RowCtx& rc, FullShared* sh, int use, int n, const RowEnds& ends) {
+    const int tid = threadIdx.x;
+    const bool cut = ends.cut_hi >= ends.cut_lo;
+    const U128 above = cut ? sh->weight_to(ends.cut_lo - 1) : ends.S;   // the kept set if it ends before the cut's bins
+    if (tid == 0) {
+        sh->first_p = 0x7fffffff;
+        sh->first_u = 0x7fffffff;
+        sh->kw_lo = above.lo;
+        sh->kw_hi = above.hi;
+    }
+    const u64* srt = order_lists<C, T>(sh, use, n);
+    const ListScan<T> ls = scan_list<T>(rc, sh, srt, n, sh->weight_to(ends.draw_lo - 1));
+    // what lies between the two ranges is not in the list
+    const U128 gap = cut ? u128_sub(sh->weight_to(max(ends.cut_lo - 1, ends.draw_hi)), sh->weight_to(ends.draw_hi)) : U128{0ull, 0ull};
+    list_sync<T>();
+    if (cut) {
+        ls.each(n, [&](int e, U128 before, U128 with) {
+            const float x = comp_value(srt[e]);
+            const int b = rc.bin(x);
+            if (b < ends.cut_lo) return;
+            if (b > ends.draw_hi) {
+                before = u128_add(before, gap);
+                with = u128_add(with, gap);
+            }
+            if (ends.top_p && u128_ge(with, ends.target_p) && !u128_ge(before, ends.target_p)) atomicMin(&sh->first_p, e + 1);
+            if (ends.min_p && rc.probability(x, ends.sum) < ends.min_thr) atomicMin(&sh->first_p, e);
+        });
+        list_sync<T>();
+    }
+    const int keep = min(sh->first_p, n);
+    if (cut) {
+        ls.each(keep, [&](int e, U128, U128 with) {
+            const int b = rc.bin(comp_value(srt[e]));
+            if (e != keep - 1 || b < ends.cut_lo) return;
+            if (b > ends.draw_hi) with = u128_add(with, gap);
+            sh->kw_lo = with.lo;
+            sh->kw_hi = with.hi;
+        });
+        list_sync<T>();
+    }
+    const U128 kept{sh->kw_hi, sh->kw_lo};
+    U128 target = double_to_u128_ceil(__dmul_rn(ends.u, u128_to_double(kept)));
+    if (!u128_ge(kept, target)) target = kept;   // (beyond it by rounding: the last one)
+    ls.each(keep, [&](int e, U128, U128 with) {
+        if (rc.bin(comp_value(srt[e])) > ends.draw_hi) with = u128_add(with, gap);
+        if (u128_ge(with, target)) atomicMin(&sh->first_u, e);
+    });
+    list_sync<T>();
+    return comp_id(srt[max(0, min(sh->first_u, keep - 1))]);
 }
 
 // The candidate at which the cumulative weight reaches `target`; every CTA gets it.  Bins if they are of use, else a descent.
@@ -1168,6 +1278,52 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     double u = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
     if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
     FTR(4);
+
+    // ---- 4. the usual way: the candidates of the bins where the kept set may end, and of those that the draw may fall into, go to the
+    // first CTA, which finishes the row
+    if (binned && !a.record) {
+        int cut_lo = 0, cut_hi = -1;
+        bool by_top_p = d.top_p < 1.0f && u128_ge(S, target_p), by_min_p = d.min_p > 0.0f;
+        if (by_top_p) cut_lo = cut_hi = find_bin(sh, target_p);
+        if (by_min_p) {
+            const int sure = max(0, rc.bin(x_sure)), never = max(0, rc.bin(x_never));
+            if (by_top_p && cut_hi < sure) {
+                by_min_p = false;   // (top-p ends the kept set earlier)
+            } else if (by_top_p && never < cut_lo) {
+                by_top_p = false;
+                cut_lo = sure;
+                cut_hi = never;
+            } else {
+                cut_lo = by_top_p ? min(cut_lo, sure) : sure;
+                cut_hi = by_top_p ? max(cut_hi, never) : never;
+            }
+        }
+        const bool cut = cut_hi >= cut_lo;
+        const U128 least = cut ? sh->weight_to(cut_lo - 1) : S, most = cut ? sh->weight_to(cut_hi) : S;
+        U128 t_least = double_to_u128_ceil(__dmul_rn(u, u128_to_double(least))), t_most = double_to_u128_ceil(__dmul_rn(u, u128_to_double(most)));
+        if (!u128_ge(least, t_least)) t_least = least;
+        if (!u128_ge(most, t_most)) t_most = most;
+        int draw_lo, draw_hi;
+        find_two_bins(sh, t_least, t_most, draw_lo, draw_hi);
+        const unsigned about = sh->cum_n[draw_hi] - (draw_lo > 0 ? sh->cum_n[draw_lo - 1] : 0u) + (cut ? sh->cum_n[cut_hi] - (cut_lo > 0 ? sh->cum_n[cut_lo - 1] : 0u) : 0u);
+        if (about <= (unsigned)(3 * kFullThreads / 4) && send_ranges<C>(rc, sh, rank, draw_lo, draw_hi, max(cut_lo, draw_hi + 1), cut_hi, par)) {
+            FTR(5);
+            if (rank != 0) return;   // nobody reads this CTA's memory any more
+            const RowEnds ends{target_p, S, u, sum, min_thr, draw_lo, draw_hi, cut_lo, cut_hi, by_top_p, by_min_p};
+            const int m = listed<C>(sh, par);
+            int token;
+            if (m > kShort) {
+                token = finish_bins<C, kFullThreads>(rc, sh, par, m, ends);
+            } else {
+                if (tid >= kShort) return;
+                token = finish_bins<C, kShort>(rc, sh, par, m, ends);
+            }
+            if (tid == 0) finish(token);
+            FTR(6);
+            return;
+        }
+        par ^= 1;
+    }
 
     // ---- 4a. the usual way with a cut: everything that can be kept goes to the first CTA, which finishes the row
     if (binned && (d.top_p < 1.0f || d.min_p > 0.0f)) {
