@@ -101,6 +101,10 @@ __device__ __forceinline__ void inbox_put(unsigned addr, unsigned v, unsigned ba
 __device__ __forceinline__ void inbox_put(unsigned addr, u64 v, unsigned bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar) : "memory");
 }
+// A bulk copy global -> own shared memory (16-byte aligned, a multiple of 16 bytes), counted by such a barrier, too.
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, u64* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 // Waits until everything expected has come; gives up after a million looks (false), each of which the hardware may itself suspend.
 __device__ __forceinline__ bool inbox_wait(u64* bar) {
     for (int i = 0; i < (1 << 20); ++i) {

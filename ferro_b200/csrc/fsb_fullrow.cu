@@ -20,11 +20,13 @@
 // same integer arithmetic everywhere, so no broadcast is needed - until a digit holds a single candidate.
 // Sums of weights are integers, so they do not depend on the order in which threads add: the result is deterministic
 // and differs from the reference's sequential fp64 sums by rounding only (~1e-13).
-// What bounds it: latency, of passes over a slice by one CTA per SM and of cluster-wide steps; neither HBM nor the fp64 units
-// (17 operations a logit would take 3 us of the 13 us of step 3 below; a third of the issue slots are used).  16 x 131072,
-// top-p 0.95, clusters of six, slices of 21848 logits, us by time stamps: load and transform 7.5, extremes 1.5, weights and
-// histogram with two exchanges 13, top-p crossing 20 and draw 10.5 (kept sets of thousands), or, with min-p 0.05, lists handed
-// over 4 and finished 2.  8 x 65536 in clusters of eight: 3.7, 1.3, 7.5, 11.7 and 8.3, or 2.6 and 1.6.
+// What bounds it: the instructions of the passes over a slice, one CTA per SM, and latency of cluster-wide steps; not HBM.  Weighing
+// a logit takes 19 fp64 operations, a conversion each way and some 40 others.  512 threads with 128 registers: with 1024 and 64 the
+// passes spilled, and what all warps compute alike was issued eight times per scheduler instead of four.  What one warp can compute for
+// all is left to one, and CTAs hand values to one another by counted stores (inbox_put): the cluster's barrier and its fences take 1 us.
+// us by time stamps, before -> after, 16 x 131072 in clusters of six, top-p 0.95: slice 5.8 -> 2.3, extremes 1.3 -> 0.6, weights and cumulative sums
+// 13.2 -> 15.3 (exact now, and the plan of what to look at), the rest 29 -> 7 (one look at the slice instead of two or three); 8 x 65536 in clusters of
+// eight: 2.7 -> 1.6, 1.3 -> 0.6, 8.1 -> 8.5, 11 -> 5.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,12 +36,14 @@
 namespace fsb {
 namespace {
 
-constexpr int kFullThreads = 1024;
+constexpr int kFullThreads = 512;
 constexpr int kFullWarps = kFullThreads / 32;
-static_assert(kFullWarps == 32, "the block reductions read one partial per lane");
+static_assert(kFullWarps <= 32, "the block reductions read one partial per lane");
 constexpr int kMaxCluster = 8;                  // most CTAs per row
 constexpr int kSliceCache = 32768;              // logits of a slice that are kept in shared memory
-constexpr int kBins = kFullThreads;             // a thread looks after one bin
+constexpr int kBins = 1024, kBinsEach = kBins / kFullThreads;   // a thread looks after two bins
+constexpr int kMostListed = 768;                // candidates that are worth a list
+constexpr float kBinned = 19.4f;                // the bins cover this many temperatures below the maximum (weights down to 2^-28), the last one all the rest
 constexpr int kSendCap = 512;                   // candidates a CTA can hand to the first one
 constexpr int kShort = 256;                     // lists of up to this many candidates are ordered by counting
 constexpr int kStripes = 8;                     // copies of the level histogram (by warp): fewer warps hit one word at once
@@ -100,6 +104,15 @@ __device__ __forceinline__ unsigned ld_cluster_u32(unsigned addr) {
 }
 
 // ---- shared memory of a CTA -------------------------------------------------------------------------------------------
+// What is known about a row once its weights have been added up; one warp works it out.
+struct RowPlan {
+    U128 S, target_p;          // all weights; the cumulative weight that top-p wants
+    double sum, min_thr, u, below;   // (below: where min-p flips, from the largest logit)
+    float x_sure, x_never;     // min-p keeps logits above the first and none below the second
+    int draw_lo, draw_hi, cut_lo, cut_hi;   // bins that the draw may fall into, and where the kept set may end (none: nothing is cut)
+    int top_p, min_p;          // which cuts may end it there
+    unsigned about;            // how many candidates those bins hold, about
+};
 struct FullShared {
     // A descent's level histogram (kStripes copies): [stripe][limb 0..3, then the candidate count][digit], four words of
     // padding between stripes; a limb sum stays below 2^32 while a stripe sees fewer than 65537 candidates, i.e. for
@@ -108,7 +121,6 @@ struct FullShared {
         alignas(16) unsigned h[kStripes][(kLimbs + 1) * 256 + 4];
         struct {   // while the weights are added up:
             unsigned hist[kLimbs][kBins];      // this CTA's weights by bin, as sums of their 16-bit limbs
-            u64 part[2][kFullThreads + 8];     // the CTAs' weights of the bins that this CTA adds up (upper and lower 32 bits' sums)
         };
     };
     u64 x_lo[2][256];          // this CTA's sum of them, which the other CTAs read; double buffered by level: a CTA may
@@ -117,6 +129,7 @@ struct FullShared {
     u64 x_small[2][4];         // small values exchanged across the cluster (extremes, sums), double buffered by use
     u64 x_all[2][kMaxCluster * 4];   // ... and every CTA's copy of all of them
     double table[64];          // 2^(j / 64)
+    u64 part[2][kBins + 8];   // the CTAs' weights of the bins that this CTA adds up: the sums of their lower 32 bits and of the rest
     u64 cum[2][kBins];         // cluster-wide: weight of bins 0 .. b, the sums of the weights' lower 32 bits and of the rest
     unsigned cum_n[kBins];     // ... and about how many candidates they hold (see estimated_count)
     // suffix sums of the walk
@@ -129,7 +142,11 @@ struct FullShared {
     u64 red[kFullWarps];
     u64 red_hi[kFullWarps];
     unsigned red_cnt[kFullWarps];
-    int bin, bin_two;          // where a cumulative weight is reached
+    RowPlan plan;
+    // counted stores from the cluster's CTAs (inbox_put): extremes, parts of bins, their sums, and at the end numbers of candidates,
+    // candidates and whether the first CTA takes them
+    u64 in_slice, in_extremes, in_parts, in_sums, in_counts, in_list, in_verdict;
+    u64 extremes[2][kMaxCluster], counts[kMaxCluster], verdict;
     int sent;                  // candidates this CTA has handed over
     unsigned got[2][kMaxCluster];   // ... every CTA of the cluster has, double buffered by use
     int first_p, first_u;      // places in the ordered list
@@ -140,6 +157,7 @@ struct FullShared {
     }
     __device__ __forceinline__ u64* list() { return reinterpret_cast<u64*>(&h[0][0]); }
 };
+static_assert(sizeof(FullShared) + kSliceCache / 8 + 16 + kSliceCache * sizeof(float) <= 227 * 1024, "a CTA's shared memory");
 static_assert(sizeof(u64) * (kMaxCluster * kSendCap + kShort) <= sizeof(FullShared::h), "the lists, and room to order a short one, lie in the histogram's memory");
 
 struct FullArgs {
@@ -246,7 +264,7 @@ __device__ __forceinline__ u64 block_max_u64(u64 v, FullShared* sh) {
     for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
     if (lane == 0) sh->red[warp] = v;
     __syncthreads();
-    u64 r = sh->red[lane];   // kFullWarps == 32: one partial per lane
+    u64 r = lane < kFullWarps ? sh->red[lane] : 0ull;   // one partial per lane
 #pragma unroll
     for (int o = 16; o; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
     __syncthreads();
@@ -498,27 +516,13 @@ __device__ __forceinline__ unsigned estimated_count(const RowCtx& rc, int bin, u
     return n < 1e6f ? (unsigned)n + (weight ? 1u : 0u) : 1000000u;
 }
 
-// First bin whose cumulative weight reaches t (the last one if none does).  All threads call; contains barriers.
-__device__ __forceinline__ int find_bin(FullShared* sh, U128 t) {
-    const int b = threadIdx.x;
-    if (b == 0) sh->bin = kBins - 1;
-    __syncthreads();
-    if (u128_ge(sh->weight_to(b), t) && (b == 0 || !u128_ge(sh->weight_to(b - 1), t))) sh->bin = b;
-    __syncthreads();
-    return sh->bin;
-}
-
-// The same for two weights, t <= v.
-__device__ __forceinline__ void find_two_bins(FullShared* sh, U128 t, U128 v, int& b_t, int& b_v) {
-    const int b = threadIdx.x;
-    if (b == 0) sh->bin = sh->bin_two = kBins - 1;
-    __syncthreads();
-    const U128 with = sh->weight_to(b), before = sh->weight_to(b - 1);
-    if (u128_ge(with, t) && (b == 0 || !u128_ge(before, t))) sh->bin = b;
-    if (u128_ge(with, v) && (b == 0 || !u128_ge(before, v))) sh->bin_two = b;
-    __syncthreads();
-    b_t = sh->bin;
-    b_v = sh->bin_two;
+// First bin whose cumulative weight reaches t (the last one if none does).  Whole warps call.
+__device__ __forceinline__ int find_bin(const FullShared* sh, U128 t) {
+    const int lane = threadIdx.x & 31;
+    const unsigned group = __ballot_sync(0xffffffffu, u128_ge(sh->weight_to(32 * lane + 31), t));
+    if (group == 0u) return kBins - 1;
+    const int b = 32 * (__ffs(group) - 1);
+    return b + __ffs(__ballot_sync(0xffffffffu, u128_ge(sh->weight_to(b + lane), t))) - 1;
 }
 
 // Sum of two words and a count over the CTA, left in x_small[use][0..2].  Contains one barrier; the sums are there after the
@@ -538,9 +542,9 @@ __device__ __forceinline__ void block_sums(FullShared* sh, int use, u64 lo, u64 
     }
     __syncthreads();
     if (warp == 0) {
-        lo = sh->red[lane];
-        hi = sh->red_hi[lane];
-        cnt = __reduce_add_sync(0xffffffffu, sh->red_cnt[lane]);
+        lo = lane < kFullWarps ? sh->red[lane] : 0ull;
+        hi = lane < kFullWarps ? sh->red_hi[lane] : 0ull;
+        cnt = __reduce_add_sync(0xffffffffu, lane < kFullWarps ? sh->red_cnt[lane] : 0u);
 #pragma unroll
         for (int o = 16; o; o >>= 1) {
             lo += __shfl_xor_sync(0xffffffffu, lo, o);
@@ -616,40 +620,57 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
     return fits;
 }
 
-// The same for the candidates of bins [b0, b1] and [b2, b3], without a count (b1 < b2, or the second range is empty).
+// The same for the candidates of bins [b0, b1] and [b2, b3] (b1 < b2, or the second range is empty), without a count; once per row.
+// Nobody but the first CTA waits for the candidates: it counts what comes, and tells the others whether it has all of them.
 template <int C>
-__device__ __forceinline__ bool send_ranges(const RowCtx& rc, FullShared* sh, unsigned rank, int b0, int b1, int b2, int b3, int par) {
-    const int tid = threadIdx.x, lane = tid & 31;
-    if (tid == 0) sh->sent = 0;
-    __syncthreads();
-    const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u);
-    // (a logit's bin is only worked out if the logit may lie in one of the ranges: a bin of room on either side covers the rounding)
-    const float width = 1.0f / rc.bin_scale, inf = __int_as_float(0x7f800000);
-    const float hi1 = b0 > 0 ? rc.mx - (float)(b0 - 1) * width : inf, lo1 = b1 < kBins - 1 ? rc.mx - (float)(b1 + 2) * width : -inf;
-    const float hi2 = b2 > 0 ? rc.mx - (float)(b2 - 1) * width : inf, lo2 = b3 < kBins - 1 ? rc.mx - (float)(b3 + 2) * width : -inf;
+__device__ __forceinline__ bool send_ranges(const RowCtx& rc, FullShared* sh, unsigned rank, int b0, int b1, int b2, int b3, int par, bool& late) {
+    const int tid = threadIdx.x;
+    const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u), bar = map_to_rank(&sh->in_list, 0u);
+    // (a logit's bin is only worked out if the logit may lie in one of the ranges: the room on either side covers the rounding of the
+    // bin, 2^-13 of its width, and of these limits)
+    const float width = 1.0f / rc.bin_scale, room = 0.03f * width + 5e-7f * fabsf(rc.mx), inf = __int_as_float(0x7f800000);
     const bool two = b3 >= b2;
-    for (int i0 = 4 * (tid - lane); i0 < rc.n; i0 += 4 * kFullThreads) {
-        float x[4];
-        load4(rc, i0 + 4 * lane, x);
-        bool some = false;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) some = some || (x[e] <= hi1 && !(x[e] < lo1)) || (two && x[e] <= hi2 && !(x[e] < lo2));
-        if (!some) continue;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {   // (few: a lane reserves for itself)
-            const int b = rc.bin(x[e]), i = i0 + 4 * lane + e;
-            if (((b >= b0 && b <= b1) || (b >= b2 && b <= b3)) && rc.is_candidate(x[e], i)) {
-                const int p = atomicAdd(&sh->sent, 1);
-                if (p < kSendCap) cluster_store_u64(to + 8u * (unsigned)p, rc.comp(x[e], i));
-            }
+    const float hi1 = b0 > 0 ? rc.mx - (float)b0 * width + room : inf, lo1 = b1 < kBins - 1 ? rc.mx - (float)(b1 + 1) * width - room : -inf;
+    const float hi2 = !two ? -inf : b2 > 0 ? rc.mx - (float)b2 * width + room : inf, lo2 = !two ? inf : b3 < kBins - 1 ? rc.mx - (float)(b3 + 1) * width - room : -inf;
+    auto near = [&](float x) { return (x <= hi1 && x >= lo1) || (x <= hi2 && x >= lo2); };
+    auto look = [&](float x, int i) {   // (few: a lane reserves for itself)
+        const int b = rc.bin(x);
+        if (((b >= b0 && b <= b1) || (b >= b2 && b <= b3)) && rc.is_candidate(x, i)) {
+            const int p = atomicAdd(&sh->sent, 1);
+            if (p < kSendCap) inbox_put(to + 8u * (unsigned)p, rc.comp(x, i), bar);
+        }
+    };
+#pragma unroll 4
+    for (int i = tid; i < rc.n >> 2; i += kFullThreads) {
+        const float4 x = reinterpret_cast<const float4*>(rc.vals)[i];
+        unsigned hits = (near(x.x) ? 1u : 0u) | (near(x.y) ? 2u : 0u) | (near(x.z) ? 4u : 0u) | (near(x.w) ? 8u : 0u);
+        while (hits) {
+            const int e = __ffs(hits) - 1;
+            hits &= hits - 1u;
+            look(e == 0 ? x.x : e == 1 ? x.y : e == 2 ? x.z : x.w, 4 * i + e);
         }
     }
+    for (int i = (rc.n & ~3) + tid; i < rc.n; i += kFullThreads) look(rc.vals[i], i);
     __syncthreads();
-    if (tid < C) cluster_store_u32(map_to_rank(&sh->got[par][rank], (unsigned)tid), (unsigned)sh->sent);
-    cluster_sync_all();
+    if (tid == 0) inbox_put(map_to_rank(&sh->counts[rank], 0u), (u64)(unsigned)sh->sent, map_to_rank(&sh->in_counts, 0u));
+    if (rank != 0) {
+        late = !inbox_wait(&sh->in_verdict) || late;
+        return sh->verdict != 0ull;
+    }
+    late = !inbox_wait(&sh->in_counts) || late;
     bool fits = true;
+    unsigned words = 0u;
 #pragma unroll
-    for (int r = 0; r < C; ++r) fits = fits && sh->got[par][r] <= (unsigned)kSendCap;
+    for (int r = 0; r < C; ++r) {
+        const unsigned n = (unsigned)sh->counts[r];
+        fits = fits && n <= (unsigned)kSendCap;
+        words += min(n, (unsigned)kSendCap);
+        if (tid == r) sh->got[par][r] = n;
+    }
+    if (tid == 0) inbox_expect(&sh->in_list, 8u * words);
+    late = !inbox_wait(&sh->in_list) || late;   // (also what is of no use: the lists' memory may be needed for a descent)
+    if (tid > 0 && tid < C) inbox_put(map_to_rank(&sh->verdict, (unsigned)tid), fits ? 1ull : 0ull, map_to_rank(&sh->in_verdict, (unsigned)tid));
+    __syncthreads();
     return fits;
 }
 
@@ -701,38 +722,45 @@ __device__ __forceinline__ u64* order_lists(FullShared* sh, int use, int n) {
         list_sync<T>();
         return spare;
     }
-    if (n <= kFullThreads) {   // a run of 32 per warp, ordered across the lanes; then the places of an entry in all runs
-        u64 mine = c[0];
-#pragma unroll
-        for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                const u64 o = __shfl_xor_sync(0xffffffffu, mine, j);
-                mine = (((lane & k) == 0) == ((lane & j) == 0)) ? max(mine, o) : min(mine, o);
-            }
-        }
-        list[tid] = mine;
-        __syncthreads();
+    if (n <= 2 * kFullThreads) {   // two runs of 32 per warp, ordered across the lanes; then the places of an entry in all runs
         const int runs = (n + 31) >> 5;
-        int rank = lane;
-        if (mine != 0ull) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (q * kFullWarps + (tid >> 5) >= runs) continue;   // (whole warps)
+#pragma unroll
+            for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    const u64 o = __shfl_xor_sync(0xffffffffu, c[q], j);
+                    c[q] = (((lane & k) == 0) == ((lane & j) == 0)) ? max(c[q], o) : min(c[q], o);
+                }
+            }
+            list[q * kFullThreads + tid] = c[q];
+        }
+        __syncthreads();
+        int rank[2] = {lane, lane};
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            if (c[p] == 0ull) continue;
 #pragma unroll 4
             for (int q = 0; q < runs; ++q) {
                 const u64* run = list + 32 * q;
                 int lo = 0;   // entries of the run above this one (0 .. 32)
 #pragma unroll
                 for (int st = 16; st > 0; st >>= 1)
-                    if (run[lo + st - 1] > mine) lo += st;
-                if (run[lo] > mine) lo += 1;
-                rank += q == tid >> 5 ? 0 : lo;
+                    if (run[lo + st - 1] > c[p]) lo += st;
+                if (run[lo] > c[p]) lo += 1;
+                rank[p] += q == p * kFullWarps + (tid >> 5) ? 0 : lo;
             }
         }
         __syncthreads();
-        if (mine != 0ull) list[rank] = mine;
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+            if (c[p] != 0ull) list[rank[p]] = c[p];
         __syncthreads();
         return list;
     }
-    int m = 2 * kFullThreads;
+    int m = 4 * kFullThreads;
     while (m < n) m <<= 1;
 #pragma unroll
     for (int q = 0; q < kPer; ++q)
@@ -891,16 +919,11 @@ __device__ __forceinline__ int finish_list(const RowCtx& rc, FullShared* sh, int
     return comp_id(srt[min(sh->first_u, keep - 1)]);   // (a target beyond the list, by rounding, takes the last)
 }
 
-// The end of a row whose first CTA has the candidates of the bins [draw_lo, draw_hi] that the draw may fall into and [cut_lo, cut_hi]
-// where the kept set may end (none: nothing is cut): the cut, the weight of the kept set, the draw.
-struct RowEnds {
-    U128 target_p, S;
-    double u, sum, min_thr;
-    int draw_lo, draw_hi, cut_lo, cut_hi;
-    bool top_p, min_p;   // in the cut's bins
-};
+// The end of a row whose first CTA has the candidates of the bins that the draw may fall into and of those where the kept set may
+// end: the cut, the weight of the kept set, the draw.
 template <int C, int T>
-__device__ __forceinline__ int finish_bins(const RowCtx& rc, FullShared* sh, int use, int n, const RowEnds& ends) {
+__device__ __forceinline__ int finish_bins(const RowCtx& rc, FullShared* sh, int use, int n) {
+    const RowPlan& ends = sh->plan;
     const int tid = threadIdx.x;
     const bool cut = ends.cut_hi >= ends.cut_lo;
     const U128 above = cut ? sh->weight_to(ends.cut_lo - 1) : ends.S;   // the kept set if it ends before the cut's bins
@@ -998,33 +1021,34 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         if (a.trace && blockIdx.x == gridDim.x - C && tid == 0) a.trace[(n)] = global_timer_ns(); \
     } while (0)
     FTR(0);
+    constexpr int kMine = (kBins + C - 1) / C;   // bins that a CTA adds up (six CTAs: 171, and C * kMine is two more than there are threads)
+    static_assert(C * kMine <= kBins + 8, "the parts' memory");
+    if (tid == 0) {
+        for (u64* bar : {&sh->in_slice, &sh->in_extremes, &sh->in_parts, &sh->in_sums, &sh->in_counts, &sh->in_list, &sh->in_verdict}) inbox_init(bar);
+        inbox_inits_fence();
+        inbox_expect(&sh->in_extremes, 16u * C);
+        inbox_expect(&sh->in_parts, 16u * C * (unsigned)max(0, min(kMine, kBins - (int)rank * kMine)));
+        inbox_expect(&sh->in_sums, 16u * kBins);
+        inbox_expect(&sh->in_counts, 8u * C);
+        inbox_expect(&sh->in_verdict, 8u);
+        sh->sent = 0;
+    }
+    if (tid == 32) {   // (while the first loads are on their way)
+        double w = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
+        if (w >= 1.0) w = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
+        sh->plan.u = w;
+        sh->plan.below = d.min_p > 0.0f ? (double)d.temperature * log((double)d.min_p) : 0.0;
+    }
+    bool late = false;   // something did not come
     cluster_arrive_relaxed();   // (waited for before the first access to another CTA's shared memory)
     if (tid < 64) sh->table[tid] = exp2((double)tid / 64.0);
 
-    // ---- 0. the slice as the sampler sees it: penalty bitmap, softcap, penalty, optional write-back.  The first loads of the
-    // slice (all of it, up to 16384 logits) are on their way while the bitmap is made.
+    // ---- 0. the slice as the sampler sees it: softcap, penalty, optional write-back
     const int n4 = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? n >> 2 : 0;
-    const float4* src = reinterpret_cast<const float4*>(row + lo);
-    float4 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int i = u * kFullThreads + tid;
-        v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
     const bool has_pen = (d.flags & kRowPenalty) != 0;
-    if (has_pen) {
-        const int32_t* h = a.hist + d.hist_begin;
-        const int n_drafts = d.flags >> kRowDraftShift, words = (n + 31) >> 5;
-        int id = tid < d.hist_len ? h[tid] : tid < d.hist_len + n_drafts ? a.drafts[d.draft_off + tid - d.hist_len] : 0;
-        for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
-        __syncthreads();
-        for (int i = tid; i < d.hist_len + n_drafts; i += kFullThreads) {
-            if (i != tid) id = i < d.hist_len ? h[i] : a.drafts[d.draft_off + i - d.hist_len];
-            const int c = id - id_base - lo;
-            if (c >= 0 && c < n) atomicOr(&bitmap[c >> 5], 1u << (c & 31));
-        }
-        __syncthreads();
-    }
+    const int32_t* const window = a.hist + d.hist_begin;
+    const int n_drafts = has_pen ? d.flags >> kRowDraftShift : 0, window_len = has_pen ? d.hist_len + n_drafts : 0, words = (n + 31) >> 5;
+    auto window_id = [&](int i) { return i < d.hist_len ? window[i] : a.drafts[d.draft_off + i - d.hist_len]; };
     RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, -45.0f * d.temperature, false, sh->table, 0ull, 0.0f};
     const float ninf = -__int_as_float(0x7f800000);
     float mx = ninf, mn = -ninf;
@@ -1038,41 +1062,80 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         if (a.write_back && (a.softcap != 0.0f || hit)) const_cast<float*>(row)[lo + i] = x;
         return x;
     };
-    for (int i0 = 0; i0 < n4; i0 += 4 * kFullThreads) {   // 16-byte loads, four of them in flight per thread
-        if (i0 > 0) {
+    const bool copied = cache_slice && n4 > 0;
+    if (copied) {
+        // A slice on a 16-byte boundary: one bulk copy, and the penalty where the window says so.  (Loads and stores by all threads, with a
+        // look at the window's bits for every logit: 5.7 us for 21848 logits, this way 2.3.)
+        if (tid == 0) {
+            inbox_expect(&sh->in_slice, 16u * (unsigned)n4);
+            bulk_copy(vals, row + lo, 16u * (unsigned)n4, &sh->in_slice);
+        }
+        int id = tid < window_len ? window_id(tid) : 0;
+        if (has_pen)
+            for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
+        for (int i = 4 * n4 + tid; i < n; i += kFullThreads) vals[i] = __ldcs(row + lo + i);
+        late = !inbox_wait(&sh->in_slice);
+        __syncthreads();
+        if (a.softcap != 0.0f) {
+            for (int i = tid; i < n; i += kFullThreads) {
+                const float x = __fmul_rn(a.softcap, tanhf(__fdiv_rn(vals[i], a.softcap)));
+                vals[i] = x;
+                if (a.write_back) const_cast<float*>(row)[lo + i] = x;
+            }
+            __syncthreads();
+        }
+        if (has_pen) {
+            for (int i = tid; i < window_len; i += kFullThreads) {
+                if (i != tid) id = window_id(i);
+                const int c = id - id_base - lo;
+                if (c < 0 || c >= n) continue;
+                const unsigned bit = 1u << (c & 31);
+                if (atomicOr(&bitmap[c >> 5], bit) & bit) continue;   // an id counts once however often it occurs
+                const float x = vals[c], y = x > 0.0f ? __fdiv_rn(x, d.penalty) : __fmul_rn(x, d.penalty);
+                vals[c] = y;
+                if (a.write_back) const_cast<float*>(row)[lo + c] = y;
+            }
+            __syncthreads();
+        }
+        auto seen = [&](float x) {   // (NaNs take no part)
+            mx = fmaxf(mx, x);
+            mn = fminf(mn, x);
+            valid += x == x ? 1u : 0u;
+        };
+#pragma unroll 4
+        for (int i = tid; i < n4; i += kFullThreads) {
+            const float4 x = reinterpret_cast<const float4*>(vals)[i];
+            seen(x.x);
+            seen(x.y);
+            seen(x.z);
+            seen(x.w);
+        }
+        for (int i = 4 * n4 + tid; i < n; i += kFullThreads) seen(vals[i]);
+    } else {
+        // anything else by loads, and the window's columns in a bitmap
+        if (has_pen) {
+            for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
+            __syncthreads();
+            for (int i = tid; i < window_len; i += kFullThreads) {
+                const int c = window_id(i) - id_base - lo;
+                if (c >= 0 && c < n) atomicOr(&bitmap[c >> 5], 1u << (c & 31));
+            }
+            __syncthreads();
+        }
+        for (int i0 = 0; i0 < n; i0 += 8 * kFullThreads) {   // what is left, or a row that does not lie on 16-byte boundaries
+            float y[8];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 8; ++u) {
                 const int i = i0 + u * kFullThreads + tid;
-                v[u] = i < n4 ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                y[u] = i < n ? __ldcs(row + lo + i) : 0.0f;
             }
-        }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * kFullThreads + tid;
-            if (i < n4) {
-                const unsigned bits = has_pen ? bitmap[i >> 3] >> ((4 * i) & 31) : 0u;
-                float4 x = v[u];
-                x.x = take(x.x, 4 * i, bits & 1u);
-                x.y = take(x.y, 4 * i + 1, bits & 2u);
-                x.z = take(x.z, 4 * i + 2, bits & 4u);
-                x.w = take(x.w, 4 * i + 3, bits & 8u);
-                if (cache_slice) reinterpret_cast<float4*>(vals)[i] = x;
-            }
-        }
-    }
-    for (int i0 = 4 * n4; i0 < n; i0 += 8 * kFullThreads) {   // what is left, or a row that does not lie on 16-byte boundaries
-        float y[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * kFullThreads + tid;
-            y[u] = i < n ? __ldcs(row + lo + i) : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * kFullThreads + tid;
-            if (i < n) {
-                const float x = take(y[u], i, has_pen && ((bitmap[i >> 5] >> (i & 31)) & 1u));
-                if (cache_slice) vals[i] = x;
+            for (int u = 0; u < 8; ++u) {
+                const int i = i0 + u * kFullThreads + tid;
+                if (i < n) {
+                    const float x = take(y[u], i, has_pen && ((bitmap[i >> 5] >> (i & 31)) & 1u));
+                    if (cache_slice) vals[i] = x;
+                }
             }
         }
     }
@@ -1096,24 +1159,25 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         __syncthreads();
         cluster_wait_acquire();
         if (warp == 0) {
-            kx = __reduce_max_sync(0xffffffffu, (unsigned)(sh->red[lane] >> 32));
-            kn = __reduce_min_sync(0xffffffffu, (unsigned)sh->red[lane]);
-            cnt = __reduce_add_sync(0xffffffffu, sh->red_cnt[lane]);
-            // one lane per CTA of the cluster tells it
-            if (lane < C) {
-                cluster_store_u64(map_to_rank(&sh->x_all[0][rank], (unsigned)lane), ((u64)kx << 32) | kn);
-                cluster_store_u64(map_to_rank(&sh->x_all[0][kMaxCluster + rank], (unsigned)lane), cnt);
+            const u64 both = lane < kFullWarps ? sh->red[lane] : 0xFFFFFFFFull;
+            kx = __reduce_max_sync(0xffffffffu, (unsigned)(both >> 32));
+            kn = __reduce_min_sync(0xffffffffu, (unsigned)both);
+            cnt = __reduce_add_sync(0xffffffffu, lane < kFullWarps ? sh->red_cnt[lane] : 0u);
+            if (lane < C) {   // one lane per CTA of the cluster tells it
+                const unsigned bar = map_to_rank(&sh->in_extremes, (unsigned)lane);
+                inbox_put(map_to_rank(&sh->extremes[0][rank], (unsigned)lane), ((u64)kx << 32) | kn, bar);
+                inbox_put(map_to_rank(&sh->extremes[1][rank], (unsigned)lane), (u64)cnt, bar);
             }
         }
-        cluster_sync_all();
+        late = !inbox_wait(&sh->in_extremes) || late;
         kx = 0u;
         kn = ~0u;
         valid = 0u;
 #pragma unroll
         for (int r = 0; r < C; ++r) {
-            kx = max(kx, (unsigned)(sh->x_all[0][r] >> 32));
-            kn = min(kn, (unsigned)sh->x_all[0][r]);
-            valid += (unsigned)sh->x_all[0][kMaxCluster + r];
+            kx = max(kx, (unsigned)(sh->extremes[0][r] >> 32));
+            kn = min(kn, (unsigned)sh->extremes[0][r]);
+            valid += (unsigned)sh->extremes[1][r];
         }
         mx = key_float(kx);
         mn = key_float(kn);
@@ -1149,74 +1213,114 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     // (a row whose largest logit is infinite, or that is too long for shared memory, is left to the descents)
     const float inf = -ninf;
     const bool binned = rc.vals != nullptr && !rc.odd;
-    // weights are zero 43.7 temperatures below the maximum: no bins are spent on what lies further down
-    rc.bin_scale = (float)kBins / fminf(44.0f * d.temperature, mx - mn);
+    // What lies further down than kBinned temperatures - most of a row, often - is one bin, added up in registers: the other bins are
+    // narrow, and a crossing's list short.  A cumulative weight that is reached there (all of it weighs less than 2^-28 of the largest per
+    // logit, 1 part in 1000 of a row of 262144 at the most) is resolved by a descent.
+    rc.bin_scale = (float)(kBins - 1) / fminf(kBinned * d.temperature, mx - mn);
     if (!(rc.bin_scale < inf)) rc.bin_scale = 0.0f;
-    // (min-p: the test is monotone in the logit and flips near mx + T * ln(min_p): only logits within a band around that value
-    // need the exact arithmetic, those above it are kept, those below it are not)
-    const double x_flip = d.min_p > 0.0f ? (double)mx + rc.temp * log((double)d.min_p) : (double)ninf;
-    const double band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
-    const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
     U128 S;
     const unsigned n_cand = rc.floor_c != 0ull ? (unsigned)d.k : valid;
     if (binned) {
 #pragma unroll
-        for (int l = 0; l < kLimbs; ++l) sh->hist[l][tid] = 0u;
+        for (int l = 0; l < kLimbs * kBinsEach; ++l) (&sh->hist[0][0])[l * kFullThreads + tid] = 0u;
+        u64 rest_lo = 0ull, rest_hi = 0ull;   // of the last bin
         __syncthreads();
-        for (int i = 4 * tid; i < n; i += 4 * kFullThreads) {
-            float x[4];
-            load4(rc, i, x);
+        auto add = [&](float x, u64 w) {
+            const int b = rc.bin(x);
+            const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);
+            if (b < kBins - 1) {
+                unsigned* h = &sh->hist[0][b];
+                atomicAdd(h, lo & 0xFFFFu);
+                atomicAdd(h + kBins, lo >> 16);
+                atomicAdd(h + 2 * kBins, hi & 0xFFFFu);
+                if (hi >> 16) atomicAdd(h + 3 * kBins, hi >> 16);
+            } else {
+                rest_lo += lo;
+                rest_hi += hi;
+            }
+        };
+        for (int i = tid; i < n >> 2; i += kFullThreads) {
+            const float4 v = reinterpret_cast<const float4*>(rc.vals)[i];
+            float x[4] = {v.x, v.y, v.z, v.w};
             if (rc.floor_c != 0ull) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) x[e] = rc.is_candidate(x[e], i + e) ? x[e] : ninf;
+                for (int e = 0; e < 4; ++e) x[e] = rc.is_candidate(x[e], 4 * i + e) ? x[e] : ninf;
             }
             u64 w[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) w[e] = rc.weight(x[e]).value();
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                unsigned* h = &sh->hist[0][rc.bin(x[e])];
-                const unsigned lo = (unsigned)w[e], hi = (unsigned)(w[e] >> 32);
-                if (lo & 0xFFFFu) atomicAdd(h, lo & 0xFFFFu);
-                if (lo >> 16) atomicAdd(h + kBins, lo >> 16);
-                if (hi) {
-                    if (hi & 0xFFFFu) atomicAdd(h + 2 * kBins, hi & 0xFFFFu);
-                    if (hi >> 16) atomicAdd(h + 3 * kBins, hi >> 16);
-                }
-            }
+            for (int e = 0; e < 4; ++e) add(x[e], w[e]);
         }
-        cluster_sync_all();
-        // Every CTA adds up kBins / C of the bins and hands the sums to all others: one load and one store per thread and word across
-        // the cluster (all bins read from all CTAs took 2.3 us).
-        constexpr int kMine = (kBins + C - 1) / C;   // (six CTAs: 171, and C * kMine is two more than there are threads)
-        static_assert(C * kMine <= kFullThreads + 8, "the parts' memory");
-        for (int t = tid; t < C * kMine; t += kFullThreads) {
-            const int src = t / kMine, bin = (int)rank * kMine + t % kMine;
-            if (bin < kBins) {
-                unsigned l[kLimbs];
+        for (int i = (n & ~3) + tid; i < n; i += kFullThreads)
+            if (rc.is_candidate(rc.vals[i], i)) add(rc.vals[i], rc.weight(rc.vals[i]).value());
+        const int lane = tid & 31, warp = tid >> 5;
+        {   // the last bin
 #pragma unroll
-                for (int q = 0; q < kLimbs; ++q) l[q] = ld_cluster_u32(map_to_rank(&sh->hist[q][bin], (unsigned)src));
-                sh->part[0][t] = (u64)l[0] + ((u64)l[1] << 16);
-                sh->part[1][t] = (u64)l[2] + ((u64)l[3] << 16);
+            for (int o = 16; o; o >>= 1) {
+                rest_lo += __shfl_xor_sync(0xffffffffu, rest_lo, o);
+                rest_hi += __shfl_xor_sync(0xffffffffu, rest_hi, o);
+            }
+            if (lane == 0) {
+                sh->red[warp] = rest_lo;
+                sh->red_hi[warp] = rest_hi;
             }
         }
         __syncthreads();
+        // Every CTA adds up kMine of the bins, from what the others send it, and sends the sums to all: a thread looks after one bin of
+        // its CTA, then after a bin and the CTA that its sum goes to.
+        {
+            u64 r0 = 0ull, r1 = 0ull;
+            if (warp == kFullWarps - 1) {
+                r0 = lane < kFullWarps ? sh->red[lane] : 0ull;
+                r1 = lane < kFullWarps ? sh->red_hi[lane] : 0ull;
+#pragma unroll
+                for (int o = 16; o; o >>= 1) {
+                    r0 += __shfl_xor_sync(0xffffffffu, r0, o);
+                    r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kBinsEach; ++q) {
+                const int bin = q * kFullThreads + tid;
+                u64 p0 = (u64)sh->hist[0][bin] + ((u64)sh->hist[1][bin] << 16), p1 = (u64)sh->hist[2][bin] + ((u64)sh->hist[3][bin] << 16);
+                if (bin == kBins - 1) {
+                    p0 += r0;
+                    p1 += r1;
+                }
+                const unsigned owner = (unsigned)(bin / kMine), at = rank * kMine + (unsigned)(bin % kMine), bar = map_to_rank(&sh->in_parts, owner);
+                inbox_put(map_to_rank(&sh->part[0][at], owner), p0, bar);
+                inbox_put(map_to_rank(&sh->part[1][at], owner), p1, bar);
+            }
+        }
+        late = !inbox_wait(&sh->in_parts) || late;
         for (int t = tid; t < C * kMine; t += kFullThreads) {
             const int dst = t / kMine, bin = (int)rank * kMine + t % kMine;
             if (bin >= kBins) continue;
+            u64 c0 = 0ull, c1 = 0ull;
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                u64 c = 0ull;
-#pragma unroll
-                for (int r = 0; r < C; ++r) c += sh->part[q][r * kMine + t % kMine];
-                cluster_store_u64(map_to_rank(&sh->cum[q][bin], (unsigned)dst), c);
+            for (int r = 0; r < C; ++r) {
+                c0 += sh->part[0][r * kMine + t % kMine];
+                c1 += sh->part[1][r * kMine + t % kMine];
             }
+            const unsigned bar = map_to_rank(&sh->in_sums, (unsigned)dst);
+            inbox_put(map_to_rank(&sh->cum[0][bin], (unsigned)dst), c0, bar);
+            inbox_put(map_to_rank(&sh->cum[1][bin], (unsigned)dst), c1, bar);
         }
-        cluster_sync_all();
+        late = !inbox_wait(&sh->in_sums) || late;
         // inclusive sums over the bins, largest logits first
-        const int lane = tid & 31, warp = tid >> 5;
-        u64 c0 = sh->cum[0][tid], c1 = sh->cum[1][tid];
-        unsigned est = estimated_count(rc, tid, (c1 << 1) + (c0 >> 31));
+        u64 own0[kBinsEach], own1[kBinsEach], c0 = 0ull, c1 = 0ull;
+        unsigned own_est[kBinsEach], est = 0u;
+#pragma unroll
+        for (int q = 0; q < kBinsEach; ++q) {   // (consecutive ones)
+            const int bin = kBinsEach * tid + q;
+            const u64 w0 = sh->cum[0][bin], w1 = sh->cum[1][bin];
+            own0[q] = c0 += w0;
+            own1[q] = c1 += w1;
+            own_est[q] = est += estimated_count(rc, bin, (w1 << 1) + (w0 >> 31));
+        }
+        const u64 mine0 = c0, mine1 = c1;
+        const unsigned mine_est = est;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const u64 t0 = __shfl_up_sync(0xffffffffu, c0, o), t1 = __shfl_up_sync(0xffffffffu, c1, o);
@@ -1227,7 +1331,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
                 est += e;
             }
         }
-        if (lane == 31) {
+        if (lane == 31) {   // (red was last read before this CTA's parts went out)
             sh->red[warp] = c0;
             sh->red_hi[warp] = c1;
             sh->red_cnt[warp] = est;
@@ -1240,9 +1344,13 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             t0 += __shfl_xor_sync(0xffffffffu, t0, o);
             t1 += __shfl_xor_sync(0xffffffffu, t1, o);
         }
-        sh->cum[0][tid] = c0 + t0;
-        sh->cum[1][tid] = c1 + t1;
-        sh->cum_n[tid] = est;
+#pragma unroll
+        for (int q = 0; q < kBinsEach; ++q) {
+            const int bin = kBinsEach * tid + q;
+            sh->cum[0][bin] = c0 - mine0 + t0 + own0[q];
+            sh->cum[1][bin] = c1 - mine1 + t1 + own1[q];
+            sh->cum_n[bin] = est - mine_est + own_est[q];
+        }
         __syncthreads();
         S = sh->weight_to(kBins - 1);
     } else {
@@ -1271,21 +1379,26 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         par ^= 1;
         cluster_sync_all();   // (the next use of x_small)
     }
-    const double sum = __dmul_rn(u128_to_double(S), 2.168404344971008868014905601739883422851562500e-19);   // * 2^-62
-    const double min_thr = __dmul_rn(__ddiv_rn(1.0, sum), (double)d.min_p);
-    // (top-p: the first candidate at which the cumulative probability reaches it, included)
-    const U128 target_p = double_to_u128_ceil(__dmul_rn(__dmul_rn((double)d.top_p, sum), 4611686018427387904.0));
-    double u = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
-    if (u >= 1.0) u = __longlong_as_double(0x3FEFFFFFFFFFFFFFll);
-    FTR(4);
-
-    // ---- 4. the usual way: the candidates of the bins where the kept set may end, and of those that the draw may fall into, go to the
-    // first CTA, which finishes the row
-    if (binned && !a.record) {
+    // what follows from it, by one warp: thirty-two of them would issue the same instructions eight times per scheduler
+    if (tid < 32) {
+        RowPlan& pl = sh->plan;   // (all lanes store the same)
+        const double total = __dmul_rn(u128_to_double(S), 2.168404344971008868014905601739883422851562500e-19);   // * 2^-62
+        // (top-p: the first candidate at which the cumulative probability reaches it, included)
+        const U128 reach = double_to_u128_ceil(__dmul_rn(__dmul_rn((double)d.top_p, total), 4611686018427387904.0));
+        pl.S = S;
+        pl.sum = total;
+        pl.target_p = reach;
+        bool by_top_p = d.top_p < 1.0f && u128_ge(S, reach), by_min_p = d.min_p > 0.0f;
         int cut_lo = 0, cut_hi = -1;
-        bool by_top_p = d.top_p < 1.0f && u128_ge(S, target_p), by_min_p = d.min_p > 0.0f;
-        if (by_top_p) cut_lo = cut_hi = find_bin(sh, target_p);
+        if (by_top_p && binned) cut_lo = cut_hi = find_bin(sh, reach);
         if (by_min_p) {
+            pl.min_thr = __dmul_rn(__ddiv_rn(1.0, total), (double)d.min_p);
+            // (the test is monotone in the logit and flips near mx + T * ln(min_p): only logits within a band around that value need the
+            // exact arithmetic, those above it are kept, those below it are not)
+            const double x_flip = (double)mx + pl.below, band = 1e-3 * (fabs(x_flip) + rc.temp + 1.0);
+            const float x_sure = (float)(x_flip + band), x_never = (float)(x_flip - band);
+            pl.x_sure = x_sure;
+            pl.x_never = x_never;
             const int sure = max(0, rc.bin(x_sure)), never = max(0, rc.bin(x_never));
             if (by_top_p && cut_hi < sure) {
                 by_min_p = false;   // (top-p ends the kept set earlier)
@@ -1298,25 +1411,46 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
                 cut_hi = by_top_p ? max(cut_hi, never) : never;
             }
         }
-        const bool cut = cut_hi >= cut_lo;
-        const U128 least = cut ? sh->weight_to(cut_lo - 1) : S, most = cut ? sh->weight_to(cut_hi) : S;
-        U128 t_least = double_to_u128_ceil(__dmul_rn(u, u128_to_double(least))), t_most = double_to_u128_ceil(__dmul_rn(u, u128_to_double(most)));
-        if (!u128_ge(least, t_least)) t_least = least;
-        if (!u128_ge(most, t_most)) t_most = most;
-        int draw_lo, draw_hi;
-        find_two_bins(sh, t_least, t_most, draw_lo, draw_hi);
-        const unsigned about = sh->cum_n[draw_hi] - (draw_lo > 0 ? sh->cum_n[draw_lo - 1] : 0u) + (cut ? sh->cum_n[cut_hi] - (cut_lo > 0 ? sh->cum_n[cut_lo - 1] : 0u) : 0u);
-        if (about <= (unsigned)(3 * kFullThreads / 4) && send_ranges<C>(rc, sh, rank, draw_lo, draw_hi, max(cut_lo, draw_hi + 1), cut_hi, par)) {
+        if (binned) {
+            // the kept set weighs between `least` and `most`: the draw's place follows, up to a bin or two
+            const bool cut = cut_hi >= cut_lo;
+            const double w = pl.u;
+            auto drawn = [&](U128 kept) {
+                const U128 t = double_to_u128_ceil(__dmul_rn(w, u128_to_double(kept)));
+                return find_bin(sh, u128_ge(kept, t) ? t : kept);
+            };
+            const int draw_hi = drawn(cut ? sh->weight_to(cut_hi) : S), draw_lo = cut ? drawn(sh->weight_to(cut_lo - 1)) : draw_hi;
+            auto held = [&](int lo, int hi) { return sh->cum_n[hi] - (lo > 0 ? sh->cum_n[lo - 1] : 0u); };
+            pl.about = held(draw_lo, draw_hi) + (cut ? held(cut_lo, cut_hi) : 0u);
+            pl.draw_lo = draw_lo;
+            pl.draw_hi = draw_hi;
+        }
+        pl.cut_lo = cut_lo;
+        pl.cut_hi = cut_hi;
+        pl.top_p = by_top_p ? 1 : 0;
+        pl.min_p = by_min_p ? 1 : 0;
+    }
+    __syncthreads();
+    const RowPlan& plan = sh->plan;
+    const double sum = plan.sum, min_thr = plan.min_thr, u = plan.u;
+    const U128 target_p = plan.target_p;
+    FTR(4);
+
+    // ---- 4. the usual way: the candidates of the bins where the kept set may end, and of those that the draw may fall into, go to the
+    // first CTA, which finishes the row
+    if (binned && !a.record) {
+        if (plan.about <= (unsigned)kMostListed &&
+            send_ranges<C>(rc, sh, rank, plan.draw_lo, plan.draw_hi, max(plan.cut_lo, plan.draw_hi + 1), plan.cut_hi, par, late)) {
             FTR(5);
+            if (late && tid == 0) report_status(a.status, a.status_host, kStatusLate);
             if (rank != 0) return;   // nobody reads this CTA's memory any more
-            const RowEnds ends{target_p, S, u, sum, min_thr, draw_lo, draw_hi, cut_lo, cut_hi, by_top_p, by_min_p};
             const int m = listed<C>(sh, par);
             int token;
             if (m > kShort) {
-                token = finish_bins<C, kFullThreads>(rc, sh, par, m, ends);
+                token = finish_bins<C, kFullThreads>(rc, sh, par, m);
             } else {
                 if (tid >= kShort) return;
-                token = finish_bins<C, kShort>(rc, sh, par, m, ends);
+                token = finish_bins<C, kShort>(rc, sh, par, m);
             }
             if (tid == 0) finish(token);
             FTR(6);
@@ -1324,14 +1458,15 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         }
         par ^= 1;
     }
+    if (late && tid == 0) report_status(a.status, a.status_host, kStatusLate);
 
     // ---- 4a. the usual way with a cut: everything that can be kept goes to the first CTA, which finishes the row
     if (binned && (d.top_p < 1.0f || d.min_p > 0.0f)) {
         int b_hi = kBins - 1;
         if (d.top_p < 1.0f) b_hi = find_bin(sh, target_p);
-        if (d.min_p > 0.0f) b_hi = min(b_hi, rc.bin(x_never));
+        if (d.min_p > 0.0f) b_hi = min(b_hi, rc.bin(plan.x_never));
         // (a list of more than a thousand is ordered too slowly: 22 us for 2000, two crossings take 15)
-        if (sh->cum_n[b_hi] <= (unsigned)(3 * kFullThreads / 4) && send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
+        if (sh->cum_n[b_hi] <= (unsigned)kMostListed && send_bins<C>(rc, sh, rank, 0, b_hi, false, par)) {
             FTR(5);
             if (rank != 0) return;   // nobody reads this CTA's memory any more
             const RowCuts cuts{target_p, u, sum, min_thr, d.top_p < 1.0f, d.min_p > 0.0f};
@@ -1356,8 +1491,8 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         u64 lowest = ~0ull;
         for (int i = tid; i < n; i += kFullThreads) {
             const float x = rc.at(i);
-            if (!rc.is_candidate(x, i) || x < x_never) continue;
-            if (x > x_sure || !(rc.probability(x, sum) < min_thr)) lowest = min(lowest, rc.comp(x, i));
+            if (!rc.is_candidate(x, i) || x < plan.x_never) continue;
+            if (x > plan.x_sure || !(rc.probability(x, sum) < min_thr)) lowest = min(lowest, rc.comp(x, i));
         }
         lowest = ~block_max_u64(~lowest, sh);
         u64 v[4] = {~lowest, 0ull, 0ull, 0ull}, all[C][4];
