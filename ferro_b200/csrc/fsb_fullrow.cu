@@ -2,7 +2,7 @@
 //
 // Rows whose effective candidate count k exceeds kMaxK - above all `top_k == 0`, where the reference sorts the
 // whole vocabulary (src/sampler.cpp:32-35 of paragontasx/ferro) - cannot keep their candidates in one CTA.  A
-// cluster of four, six or eight CTAs works on one such row.  Every CTA keeps its slice of the row in shared memory
+// cluster of four, five, six or eight CTAs works on one such row.  Every CTA keeps its slice of the row in shared memory
 // (softcap and penalty applied once, src/model_gemma4.cpp:521 and src/sampler.cpp:11-18), so the row is read from
 // HBM exactly once; everything after that reads shared memory:
 //   1. the row's largest and smallest candidate key                                            (src/sampler.cpp:38)
@@ -1632,8 +1632,8 @@ int launch_full(const FullArgs& a, int n_rows, cudaStream_t stream) {
     return (int)cudaLaunchKernelEx(&cfg, full_row_kernel<C>, a, slice_of(a.n_vocab, C) <= kSliceCache ? 1 : 0);
 }
 // How many clusters of C CTAs run at once.  A cluster lies in one GPC, so this is less than SMs / C: 15 of eight on B200's
-// 148 SMs, 22 of six, 33 of four.
-int g_at_once[3] = {0, 0, 0};
+// 148 SMs (of seven, too), 22 of six, 26 of five, 33 of four.
+int g_at_once[4] = {0, 0, 0, 0};   // of four, five, six, eight
 template <int C>
 int prepare_full(int& at_once) {
     // the largest request of any row length, whatever the engine's: the attribute is the kernel's, and engines of several sizes
@@ -1649,7 +1649,7 @@ int prepare_full(int& at_once) {
 }  // namespace
 
 int prepare_full_row_kernel() {
-    for (int e : {prepare_full<8>(g_at_once[2]), prepare_full<6>(g_at_once[1]), prepare_full<4>(g_at_once[0])})
+    for (int e : {prepare_full<8>(g_at_once[3]), prepare_full<6>(g_at_once[2]), prepare_full<5>(g_at_once[1]), prepare_full<4>(g_at_once[0])})
         if (e != 0) return e;
     return 0;
 }
@@ -1677,23 +1677,27 @@ int launch_full_row_kernel(const float* logits, const RowDesc* rows, int n_rows,
     a.record = record;
     a.softcap = softcap;
     a.trace = reinterpret_cast<u64*>(trace);
-    // The more CTAs per row the shorter the passes, but a second wave of clusters costs as much as the first.  Measured on B200
-    // with top-p 0.95 (us, eight / six / four CTAs): 8 x 16384 30.4 / 29.7 / 28.8, 8 x 65536 38.8 / 41.1 / 45.3, 8 x 131072
-    // 51.3 / 60.0 / 72.1, 16 x 131072 92.7 / 60.4 / 72.3, 23 x 131072 96.4 / 106.6 / 73.4.  The rule's terms: steps, the
-    // exchanges of a step between more CTAs, passes over a slice.
+    // The more CTAs per row the shorter the passes, but a second wave of clusters costs as much as the first.  Measured on B200 with top-p
+    // 0.95 (us, four / five / six / eight CTAs): 8 x 16384 14.7 each, 8 x 65536 23.7 / 22.9 / 21.2 / 18.8, 16 x 131072 42 / 34.2 / 32.1 / 43.1,
+    // 23 x 131072 42 / 33.1 / 49.3 / 44.4, 32 x 65536 24.9 / 40.0 / 37.4 / 45.4.  The rule's terms: steps, and passes over a slice.
     int best = 8;
     double cost = 1e30;
-    for (int i = 2; i >= 0; --i) {
-        const int c = 4 + 2 * i, per = slice_of(n_vocab, c), at_once = std::max(1, g_at_once[i]);
+    for (int i = 3; i >= 0; --i) {
+        const int c = i == 3 ? 8 : 4 + i, per = slice_of(n_vocab, c), at_once = std::max(1, g_at_once[i]);
         if (c < 8 && per > kSliceCache) continue;
-        const double t = ((n_rows + at_once - 1) / at_once) * (18.0 + 1.1 * c + 1.55 * per / 1024.0);
+        const double t = ((n_rows + at_once - 1) / at_once) * (11.0 + 0.92 * per / 1024.0);
         if (t < cost) {
             cost = t;
             best = c;
         }
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return best == 8 ? launch_full<8>(a, n_rows, st) : best == 6 ? launch_full<6>(a, n_rows, st) : launch_full<4>(a, n_rows, st);
+    switch (best) {
+        case 8: return launch_full<8>(a, n_rows, st);
+        case 6: return launch_full<6>(a, n_rows, st);
+        case 5: return launch_full<5>(a, n_rows, st);
+        default: return launch_full<4>(a, n_rows, st);
+    }
 }
 
 }  // namespace fsb
