@@ -86,6 +86,8 @@ struct StreamArgs {
     int32_t vocab_offset;      // token id of column 0
     float softcap;             // 0 = off
     int32_t overlap;           // see fsb_set_launch_overlap
+    int32_t sms;               // multiprocessors of the device
+    int32_t captured;          // the launch goes into a graph: no programmatic edges
 };
 
 // How a launch of n_rows rows is laid out on a device of `sms` multiprocessors: CTAs per row, and whether they are large

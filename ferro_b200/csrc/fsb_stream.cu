@@ -1297,9 +1297,16 @@ int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* 
         a.drafts = nullptr;
         if (ids_are_windows) a.hist = nullptr;
     }
+    // Plain stream order, too, is launched with programmatic serialization where that pays: every CTA waits for the launch before to be
+    // complete (pdl_wait_prior), and only placing the CTAs overlaps its end.  us per launch in a train, without -> with: 1 x 65536 10.4 ->
+    // 7.8, 32 x 131072 14.0 -> 11.1, 64 x 262144 22.8 -> 20.5, 148 x 131072 23.9 -> 21.2, 512 x 32768 22.8 -> 20.6.  Not where a few small CTAs
+    // per SM are the whole launch: placed while others still run, they pile up on some SMs (200 x 131072 31.4 -> 41.0, 300 x 65536 26.3 -> 29.3);
+    // clusters do not (37 x 65536, k = 16, 296 CTAs 15.4 -> 13.3).
+    const int ctas = a.n_rows * a.nseg;
+    const bool chained = a.overlap == 0 && !a.captured && (a.wide || ctas <= (a.nseg > 1 ? 2 : 1) * a.sms || ctas >= 3 * a.sms);
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (a.overlap) {
+    if (a.overlap || chained) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -1436,6 +1443,8 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
         a.n_vocab = n_vocab;
         a.kmax = 1;
         a.all_greedy = 1;
+        a.sms = sd.sms;
+        a.captured = 1;   // (for all that is known here)
         const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms, 1, true, false);
         a.nseg = pl.nseg;
         a.wide = pl.wide ? 1 : 0;

@@ -95,7 +95,8 @@ FSB_API int fsb_set_softcap(fsb_handle* h, float cap);
  * default) turns it off.  No reference counterpart. */
 FSB_API int fsb_set_trace_buffer(fsb_handle* h, void* device_buffer);
 
-/* How consecutive launches follow one another (0, the default: plain stream order).
+/* How consecutive launches follow one another (0, the default: plain stream order; the launch attribute of form 2 is used
+ * where it is measured to pay, and not in a stream that is being captured).
  * 1: fsb_batch_launch starts the streaming kernel with programmatic stream serialization and its CTAs may begin to
  *    read logits while the previous kernel in the stream is still finishing; every write of the launch (tokens, kept
  *    sets, scratch) waits for that kernel to be complete.  Use it only if the logits of a launch are complete before
