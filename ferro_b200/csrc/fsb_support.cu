@@ -31,15 +31,31 @@ __global__ void __launch_bounds__(kThreads, 1) merge_lists_kernel(const u64* lis
     const RowDesc d = rows[row];
     const int hdr = list_n ? 0 : 1;
     int total = 0;   // the same in every thread
-    for (int g = 0; g < n_lists; ++g) {
-        const u64* src = lists + ((size_t)g * n_rows + row) * (size_t)list_stride;
-        const long long stated = list_n ? (long long)list_n[(size_t)g * n_rows + row] : (long long)src[0];
-        const int n = (int)max(0ll, min(stated, (long long)min(kMaxK, list_stride - hdr)));
-        if (total + n <= kMergeCap) {
-            for (int i = tid; i < n; i += kThreads) buf[total + i] = src[hdr + i];
+    auto list_at = [&](int g) { return lists + ((size_t)g * n_rows + row) * (size_t)list_stride; };
+    auto length = [&](int g) {
+        const long long stated = list_n ? (long long)list_n[(size_t)g * n_rows + row] : (long long)list_at(g)[0];
+        return (int)max(0ll, min(stated, (long long)min(kMaxK, list_stride - hdr)));
+    };
+    // Thirty-two lists at a time: every warp reads all their lengths at once, and copies some of the lists, two words per lane on their
+    // way together.  (List after list, the next length read when the one before was known: 8.6 us for eight lists of 41, this way 6.6.)
+    const int lane = tid & 31;
+    for (int g0 = 0; g0 < n_lists; g0 += 32) {
+        const int mine = g0 + lane < n_lists ? length(g0 + lane) : 0;
+        for (int g = g0; g < min(g0 + 32, n_lists); ++g) {
+            const int n = __shfl_sync(0xffffffffu, mine, g - g0);
+            if (total + n > kMergeCap) {
+                if (tid == 0) atomicOr(status, kStatusMergeOverflow);
+                continue;
+            }
+            if ((g & (kThreads / 32 - 1)) == tid >> 5) {
+                const u64* src = list_at(g) + hdr;
+                for (int i = lane; i < n; i += 64) {
+                    const u64 c0 = src[i], c1 = i + 32 < n ? src[i + 32] : 0ull;
+                    buf[total + i] = c0;
+                    if (i + 32 < n) buf[total + i + 32] = c1;
+                }
+            }
             total += n;
-        } else if (tid == 0) {
-            atomicOr(status, kStatusMergeOverflow);
         }
     }
     block_sync<kPost, 1>();
@@ -85,35 +101,49 @@ __global__ void accept_windows_kernel(const int32_t* table, int n_streams, const
 
 // Prompt-lookup drafting over resident histories (lookup_draft, src/server.cpp:552-564): the tokens that followed
 // the most recent earlier occurrence of the history's last n tokens, n = 4, 3, ... min_n - at most kmax of them, cut
-// at the end-of-sequence id; an occurrence whose continuation is empty is passed over.  One CTA per stream: every
-// thread tests some start positions of an n, the largest matching position wins, one thread copies the draft.
+// at the end-of-sequence id; an occurrence whose continuation is empty is passed over.  One CTA per stream, one pass: at every
+// position a thread finds how many ids up to there are those the history ends with (up to four; the five ids it needs are on their
+// way at once), and the last position of every length is noted; the longest one wins, and a warp copies the draft.  (A pass per length,
+// an id read when the one before had matched: 5.5 us for eight histories of 1024 ids, this way 4.8.)
 // out[i * stride] = number of drafts of stream i, then the drafts; `out` is the caller's pinned memory, where the host
 // waits for the number and for every draft (a system-wide fence between the two would cost 7 us).
 struct LookupArgs {
     LookupDesc d[kLookupArgs];
 };
 __global__ void lookup_drafts_kernel(const int32_t* pool, const __grid_constant__ LookupArgs args, const LookupDesc* desc, int n_streams, int32_t* out, int stride) {
-    __shared__ int best;
+    __shared__ int last[5];   // of the positions whose longest match is n ids, the last (-1: none)
     const int i = blockIdx.x;
     if (i >= n_streams) return;
     const LookupDesc d = desc ? desc[i] : args.d[i];
     const int32_t* h = pool + d.begin;
     const int L = d.len;
-    int found_n = 0;
-    for (int n = min(4, L - 1); n >= d.min_n && d.kmax > 0; --n) {
-        if (threadIdx.x == 0) best = -1;
-        __syncthreads();
-        for (int p = L - n - 1 - (int)threadIdx.x; p >= 0; p -= (int)blockDim.x) {
-            bool eq = h[p + n] != d.eos;            // an occurrence followed by the end-of-sequence id drafts nothing
-            for (int k = 0; k < n && eq; ++k) eq = h[p + k] == h[L - n + k];
-            if (eq) atomicMax(&best, p);
+    if (threadIdx.x < 5) last[threadIdx.x] = -1;
+    __syncthreads();
+    if (d.kmax > 0 && L > 1) {
+        int32_t end[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) end[j] = h[max(L - 1 - j, 0)];
+#pragma unroll 4
+        for (int q = L - 2 - (int)threadIdx.x; q >= 0; q -= (int)blockDim.x) {   // the match ends at q
+            const int32_t next = h[q + 1];
+            int32_t id[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) id[j] = h[max(q - j, 0)];
+            int n = 0;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) n = q >= j && id[j] == end[j] ? n + 1 : 0;
+            if (n >= max(d.min_n, 1) && next != d.eos) atomicMax(&last[n], q);   // (an occurrence followed by the end-of-sequence id drafts nothing)
         }
-        __syncthreads();
-        if (best >= 0) {
+    }
+    __syncthreads();
+    int found_n = 0, best = -1;
+    for (int n = 4, q = -1; n >= max(d.min_n, 1); --n) {   // a match of n ids is one of n - 1, too
+        q = max(q, last[n]);
+        if (q >= 0) {
             found_n = n;
+            best = q - n + 1;
             break;
         }
-        __syncthreads();   // `best` is reset by thread 0 at the top of the next round
     }
     if (threadIdx.x >= 32) return;
     const int lane = threadIdx.x, most = found_n > 0 ? min(min(d.kmax, stride - 1), L - best - found_n) : 0;
