@@ -1328,25 +1328,26 @@ int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* 
 
 // How a launch is laid out: small CTAs (256 threads) or large ones (1024), and the segments of a row.  Measured on B200,
 // us per launch with windows of 512 ids; s1 = small, one segment (c: penalised logits by cells), w2 = large, two.
-// Few rows: small CTAs, the row cut as finely as two per SM allow (a large CTA issues every step after the stream from four
-// times as many warps): 8 x 131072, k = 16: s4 17.7, s8 14.6, w4 14.7.  With longer lists the merge of eight costs more than
-// those steps: 24 x 262144, k = 64: s8 22.9, w4 20.8, but clusters of four large CTAs run on 132 SMs only (37 rows: w4 33.1, w2 25.0).
-// Medium batches: one large CTA per SM streams best (148 x 131072, k = 64: s1 39, s1c 35, s2 34, w1 27; 64: s4 22.9, w1 24.5, w2 21.5).
-// Many rows: a small CTA per row, several per SM, so that the steps of one run beside the stream of the others (200 x 131072,
-// k = 64: s1 48, s1c 41.7, s2 42.3, w1 47; 160 x 65536: s1 31.5, s1c 29.5, s2 30.9, w1 35; 296 x 262144: s1 79, s1c 72, s2 93, w1
-// 72; 512 x 32768: s1 37, s2 54, w1 54).  Two segments are level with one up to 200 rows below 65536 logits (200 x 49152: s1 26.9,
-// s1c 27.6, s2 27.0) and lose above (256: s1 27.4, s1c 28.8, s2 40).
-// k > 64: a small CTA lists every second logit at first.  Large ones from 32768 logits on however many rows there are (512 x
-// 262144, k = 256: s1 265, w1 170; 512 x 32768: s1 77, w1 80; 512 x 16384: s1 57, w1 68), in two segments while a pair per
-// row runs at once (32 x 262144: s8 47, w1 44, w2 35, w4 38; 148 x 262144: s1 121, w1 50, w2 72).
-// All greedy: little after the stream.  Up to three CTAs per SM two segments pay (200 x 262144: s1 37.3, s2 35.2; 296: s1 49.0, s2
-// 49.8); windows of more than 65536 columns leave room for three or two CTAs per SM, and one large one streams better than a
-// second wave (512 x 262144: s1 106, s2 95, w1 90; 400: s1 70, w1 71).
+// Few rows: small CTAs, the row cut as finely as two per SM allow and segments of 2048 logits (4096, and a CTA per SM at the most, for
+// more than eight rows): 1 x 65536, k = 40: s2 11.8, s4 9.5, s8 7.9, w4 8.9; 8 x 16384: s2 9.2, s8 8.0; 30 x 16384: s2 8.7, s4 8.2, s8 8.5.
+// Long rows, as many as there are clusters of eight large CTAs that run at once (15): those, from 100000 logits on (1 x 262144: s8
+// 12.9, w8 10.7; 14 x 131072: s8 11.6, w4 11.1, w8 10.4; 6 x 90000: s8 9.5, w8 9.9; 16 x 131072: w4 10.4, w8 15.5).
+// Medium batches: large CTAs, one per SM, in clusters of four or two while those run at once (clusters of four on 132 SMs only: 37 x
+// 262144 w4 24.7, w2 19.6; 64 x 131072: s4 16.1, w1 19.5, w2 16.2; 148 x 131072: s1 28.8, s2 23.3, w1 21.3); four small ones below 65536
+// logits up to 64 rows (44 x 40000: s4 9.9, w2 10.8; 64 x 49152: 11.5, 12.8; 70 x 40000: 11.8 both; 50 x 65536: 12.3, 11.9).
+// Many rows: a small CTA per row, several per SM, so that the steps of one run beside the stream of the others (plain order: 200 x
+// 131072, k = 40: s1 31.5, s2 41.5, w1 38.2; 160 x 65536: s1 24.9, s2 24.8, w1 28.6; 296 x 262144: s1 57.3, s2 63.8, w1 63.0; 512 x 32768: s1
+// 20.8, w1 40.4).
+// k > 64: a small CTA has longer lists and more bounds to find: large ones, in two segments while a pair per row runs at once (32 x
+// 65536, k = 200: w1 22.3, w2 17.9, s4 23.0), and above that where logits times k are many (512 x 65536, k = 100: s1 51.4, w1 67.4; k = 200 66.5,
+// 80.9; k = 256 87.3, 86.2; 300 x 100000, k = 200 59.1, 68.8; 512 x 131072, k = 100 73.8, 86.1; k = 256 134, 109; 300 x 262144, k = 100 102, 92).
+// All greedy: little after the stream.  Up to three CTAs per SM two segments pay (200 x 262144: s1 37.4, s2 35.2); windows of more than
+// 65536 columns leave room for three or two CTAs per SM, and one large one streams better than a second wave (512 x 262144: s1 104, w1 88).
 SelectPlan plan_select(int n_rows, int n_vocab, int sms, int kmax, bool all_greedy, bool penalised) {
     SelectPlan pl;
-    auto fits = [&](int nseg, int most) { return n_rows * nseg <= most && n_vocab / nseg >= 8192; };
+    auto fits = [&](int nseg, int most, int columns = 8192) { return n_rows * nseg <= most && n_vocab / nseg >= columns; };
     if (kmax > 64) {
-        pl.wide = n_rows <= sms || n_vocab >= 32768;
+        pl.wide = n_rows <= sms || (int64_t)n_vocab * kmax >= (kmax > 224 ? 10000000 : 24000000);
         if (fits(2, sms) && n_vocab >= 32768) pl.nseg = 2;
     } else if (n_rows > sms) {
         if (all_greedy && n_vocab >= 65536 && n_rows <= sms + sms / 2) pl.nseg = 2;
@@ -1354,11 +1355,19 @@ SelectPlan plan_select(int n_rows, int n_vocab, int sms, int kmax, bool all_gree
     } else {
         pl.wide = n_rows > sms / 4 || (kmax > 32 && n_rows > 8 && n_vocab >= 65536);
         if (pl.wide) pl.nseg = fits(4, sms - sms / 10) ? 4 : fits(2, sms) ? 2 : 1;
+        if (n_vocab >= 100000 && fits(8, sms - sms / 5)) {
+            pl.wide = true;
+            pl.nseg = 8;
+        }
+        if (pl.wide && !all_greedy && n_vocab < 65536 && n_rows > sms / 4 && fits(4, 2 * sms - sms / 4)) {
+            pl.wide = false;
+            pl.nseg = 4;
+        }
     }
     // (the bitmap of a very long segment - above 380000 columns - does not fit beside a large CTA's ring, but always beside a small one's)
     if (pl.wide && penalised && Geometry<1024>::smem_bytes(pl.nseg, kmax, segment_columns(n_vocab, pl.nseg)) > (size_t)kSelectSmemMax) pl = SelectPlan{};
     if (!pl.wide && n_rows <= sms)
-        while (pl.nseg < 8 && fits(2 * pl.nseg, 2 * sms)) pl.nseg *= 2;
+        while (pl.nseg < 8 && (fits(2 * pl.nseg, 2 * sms) || fits(2 * pl.nseg, n_rows <= 8 ? 2 * sms : sms, n_rows <= 8 ? 2048 : 4096))) pl.nseg *= 2;
     return pl;
 }
 

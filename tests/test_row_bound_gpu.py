@@ -13,6 +13,8 @@ SHAPES = [  # rows, logits, top_k, window
     (12, 32768, 64, 30), (12, 32769, 63, 30), (20, 16391, 33, 12),                         # four, two
     (30, 131072, 40, 50), (30, 131077, 64, 50), (70, 65536, 50, 9), (70, 65543, 2, 9),     # four large CTAs, two
     (100, 32768, 64, 5), (100, 32773, 40, 5), (100, 1500, 64, 2), (60, 900, 64, 40), (90, 130, 64, 8), (60, 61, 64, 2), (60, 3, 2, 1),
+    (14, 100000, 40, 20), (14, 131077, 64, 30), (15, 100001, 40, 9), (1, 262144, 64, 9),   # eight large CTAs
+    (44, 40003, 64, 9), (64, 65535, 40, 5), (8, 16384, 64, 9), (9, 16384, 40, 9), (37, 16391, 5, 3), (2, 2050, 40, 3),   # four or eight small ones, short
     (200, 8192, 64, 5), (200, 8193, 40, 5), (200, 8188, 5, 0), (160, 70, 30, 3),           # one small CTA per row
 ]
 
