@@ -1130,6 +1130,8 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
             if (j + u * T < w.c_hi) cp_async16(dst + (unsigned)(u * T * sizeof(float4)), w.cells + j + u * T);
         cp_async_commit();
     };
+    if (!a.penalised)
+        for (int c = 0; c < kStages; ++c) fetch(c);
     float edge = qnan;
     int edge_col = -1;
     if (tid < 8) {
@@ -1154,7 +1156,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         for (int c = 1; c < kStages; ++c) fetch(c);
         __syncthreads();
         if (edge_col >= 0 && penalised(s, edge_col)) edge = qnan;
-    } else {
+    } else if (a.penalised) {
         for (int c = 0; c < kStages; ++c) fetch(c);
     }
     trace_mark(a, 1);
