@@ -42,6 +42,7 @@ static_assert(kFullWarps <= 32, "the block reductions read one partial per lane"
 constexpr int kMaxCluster = 8;                  // most CTAs per row
 constexpr int kSliceCache = 32768;              // logits of a slice that are kept in shared memory
 constexpr int kBins = 1024, kBinsEach = kBins / kFullThreads;   // a thread looks after two bins
+constexpr int kShiftedFrom = 512;               // rows from this length on have slices that start on 16-byte boundaries
 constexpr int kMostListed = 768;                // candidates that are worth a list
 constexpr float kBinned = 19.4f;                // the bins cover this many temperatures below the maximum (weights down to 2^-28), the last one all the rest
 constexpr int kSendCap = 512;                   // candidates a CTA can hand to the first one
@@ -157,7 +158,7 @@ struct FullShared {
     }
     __device__ __forceinline__ u64* list() { return reinterpret_cast<u64*>(&h[0][0]); }
 };
-static_assert(sizeof(FullShared) + kSliceCache / 8 + 16 + kSliceCache * sizeof(float) <= 227 * 1024, "a CTA's shared memory");
+static_assert(sizeof(FullShared) + kSliceCache / 8 + 4 + 16 + (kSliceCache + 4) * sizeof(float) <= 227 * 1024, "a CTA's shared memory");
 static_assert(sizeof(u64) * (kMaxCluster * kSendCap + kShort) <= sizeof(FullShared::h), "the lists, and room to order a short one, lie in the histogram's memory");
 
 struct FullArgs {
@@ -194,7 +195,7 @@ struct RowCtx {
     const float* row;         // the row in global memory
     const unsigned* bitmap;   // penalised columns of the slice (bit i = column lo + i), or null
     float pen, cap;
-    int lo, n;                // first column and number of columns of this CTA's slice
+    int lo, main, n;          // first column of this CTA's slice, columns from there on, and all its columns
     int id_base;              // token id of column 0
     float mx;                 // the row's maximum
     double temp, inv_temp;    // T and 1 / T
@@ -210,7 +211,8 @@ struct RowCtx {
         if (bitmap && ((bitmap[i >> 5] >> (i & 31)) & 1u)) x = x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen);
         return x;
     }
-    __device__ __forceinline__ u64 comp(float x, int i) const { return make_comp(x, lo + i + id_base); }
+    // (the up to three columns before the row's first 16-byte boundary come last in the first slice)
+    __device__ __forceinline__ u64 comp(float x, int i) const { return make_comp(x, (i < main ? lo + i : i - main) + id_base); }
     // (x - max) / T for a finite difference, correctly rounded: a quotient from the rounded reciprocal and one exact correction
     // step (Markstein 1990), three fused operations in place of a division.  Both operands are floats: a quotient of two 24-bit
     // significands is at least 2^-25 ulp away from the middle of two doubles, and the correction is off by some 2^-52 ulp.
@@ -1008,12 +1010,15 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     const RowDesc d = a.rows[blockIdx.x / C];
     const int V = a.n_vocab;
     // the slices: equal runs of columns, a multiple of four each
-    const int per = (((V + C - 1) / C) + 3) & ~3;
-    const int lo = min(V, (int)rank * per), n = min(V, lo + per) - lo;
-    unsigned* bitmap = reinterpret_cast<unsigned*>(smem_raw + sizeof(FullShared));
-    float* vals = reinterpret_cast<float*>(smem_raw + sizeof(FullShared) + (size_t)((per + 31) / 32) * sizeof(unsigned));
-    vals = reinterpret_cast<float*>(((uintptr_t)vals + 15) & ~(uintptr_t)15);
+    // (from the row's first 16-byte boundary on, so that they can be copied in one piece; the columns before it belong to the first CTA)
     const float* row = a.logits + d.logits_off;
+    const bool shifted = cache_slice && V >= kShiftedFrom;
+    const int head = shifted ? (int)((0u - ((unsigned)reinterpret_cast<uintptr_t>(row) >> 2)) & 3u) : 0;
+    const int per = (((V - head + C - 1) / C) + 3) & ~3;
+    const int lo = min(V, head + (int)rank * per), main = min(V, lo + per) - lo, n = main + (rank == 0 ? head : 0);
+    unsigned* bitmap = reinterpret_cast<unsigned*>(smem_raw + sizeof(FullShared));
+    float* vals = reinterpret_cast<float*>(smem_raw + sizeof(FullShared) + (size_t)((per + 3 + 31) / 32) * sizeof(unsigned));
+    vals = reinterpret_cast<float*>(((uintptr_t)vals + 15) & ~(uintptr_t)15);
     const int id_base = a.vocab_offset;
     int par = 0;
 #define FTR(n)                                                                                   \
@@ -1044,12 +1049,12 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     if (tid < 64) sh->table[tid] = exp2((double)tid / 64.0);
 
     // ---- 0. the slice as the sampler sees it: softcap, penalty, optional write-back
-    const int n4 = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? n >> 2 : 0;
+    const int n4 = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? main >> 2 : 0;
     const bool has_pen = (d.flags & kRowPenalty) != 0;
     const int32_t* const window = a.hist + d.hist_begin;
     const int n_drafts = has_pen ? d.flags >> kRowDraftShift : 0, window_len = has_pen ? d.hist_len + n_drafts : 0, words = (n + 31) >> 5;
     auto window_id = [&](int i) { return i < d.hist_len ? window[i] : a.drafts[d.draft_off + i - d.hist_len]; };
-    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, n, id_base, 0.0f, (double)d.temperature, 0.0, -45.0f * d.temperature, false, sh->table, 0ull, 0.0f};
+    RowCtx rc{nullptr, row, has_pen ? bitmap : nullptr, d.penalty, a.softcap, lo, main, n, id_base, 0.0f, (double)d.temperature, 0.0, -45.0f * d.temperature, false, sh->table, 0ull, 0.0f};
     const float ninf = -__int_as_float(0x7f800000);
     float mx = ninf, mn = -ninf;
     unsigned valid = 0u;
@@ -1064,7 +1069,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
     };
     const bool copied = cache_slice && n4 > 0;
     if (copied) {
-        // A slice on a 16-byte boundary: one bulk copy, and the penalty where the window says so.  (Loads and stores by all threads, with a
+        // The usual way, a slice on a 16-byte boundary: one bulk copy, and the penalty where the window says so.  (Loads and stores by all threads, with a
         // look at the window's bits for every logit: 5.7 us for 21848 logits, this way 2.3.)
         if (tid == 0) {
             inbox_expect(&sh->in_slice, 16u * (unsigned)n4);
@@ -1073,27 +1078,30 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         int id = tid < window_len ? window_id(tid) : 0;
         if (has_pen)
             for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
-        for (int i = 4 * n4 + tid; i < n; i += kFullThreads) vals[i] = __ldcs(row + lo + i);
+        auto column = [&](int i) { return i < main ? lo + i : i - main; };
+        for (int i = 4 * n4 + tid; i < n; i += kFullThreads) vals[i] = __ldcs(row + column(i));
         late = !inbox_wait(&sh->in_slice);
         __syncthreads();
         if (a.softcap != 0.0f) {
             for (int i = tid; i < n; i += kFullThreads) {
                 const float x = __fmul_rn(a.softcap, tanhf(__fdiv_rn(vals[i], a.softcap)));
                 vals[i] = x;
-                if (a.write_back) const_cast<float*>(row)[lo + i] = x;
+                if (a.write_back) const_cast<float*>(row)[column(i)] = x;
             }
             __syncthreads();
         }
         if (has_pen) {
             for (int i = tid; i < window_len; i += kFullThreads) {
                 if (i != tid) id = window_id(i);
-                const int c = id - id_base - lo;
-                if (c < 0 || c >= n) continue;
+                const int col = id - id_base;
+                if (col < 0 || col >= V) continue;   // (and no overflow)
+                const int c = col >= lo && col < lo + main ? col - lo : rank == 0 && col < head ? main + col : -1;
+                if (c < 0) continue;
                 const unsigned bit = 1u << (c & 31);
                 if (atomicOr(&bitmap[c >> 5], bit) & bit) continue;   // an id counts once however often it occurs
                 const float x = vals[c], y = x > 0.0f ? __fdiv_rn(x, d.penalty) : __fmul_rn(x, d.penalty);
                 vals[c] = y;
-                if (a.write_back) const_cast<float*>(row)[lo + c] = y;
+                if (a.write_back) const_cast<float*>(row)[col] = y;
             }
             __syncthreads();
         }
@@ -1606,9 +1614,9 @@ namespace {
 int slice_of(int n_vocab, int cluster) { return (((n_vocab + cluster - 1) / cluster) + 3) & ~3; }
 size_t full_row_smem_bytes(int n_vocab, int cluster) {
     const int per = slice_of(n_vocab, cluster);
-    const size_t bitmap = sizeof(unsigned) * (size_t)((per + 31) / 32);
+    const size_t bitmap = sizeof(unsigned) * (size_t)((per + 3 + 31) / 32);   // (three columns may come before the first slice)
     // (the kept set's record is ordered in the slice's memory: kMaxK 64-bit words)
-    const size_t slice = per <= kSliceCache ? sizeof(float) * (size_t)std::max(per, 2 * kMaxK) : sizeof(u64) * (size_t)kMaxK;
+    const size_t slice = per <= kSliceCache ? sizeof(float) * (size_t)std::max(per + 4, 2 * kMaxK) : sizeof(u64) * (size_t)kMaxK;
     return sizeof(FullShared) + bitmap + 16 + slice;
 }
 template <int C>
