@@ -87,7 +87,7 @@ struct StreamArgs {
     float softcap;             // 0 = off
     int32_t overlap;           // see fsb_set_launch_overlap
     int32_t sms;               // multiprocessors of the device
-    int32_t captured;          // the launch goes into a graph: no programmatic edges
+    int32_t unchained;         // no launch attribute unless `overlap` asks for it
 };
 
 // How a launch of n_rows rows is laid out on a device of `sms` multiprocessors: CTAs per row, and whether they are large

@@ -368,8 +368,9 @@ int launch_batch(fsb_handle* h, fsb_batch* b, const float* logits_dev, bool keep
         // Few descriptors go with the launch.  A captured launch of a prepared batch reads them on the device: it may be
         // replayed after a redraw.
         a.sms = h->sm_count;
-        a.captured = !mirror && is_capturing(h) ? 1 : 0;
-        const int e = fsb::launch_stream_kernel(a, !a.captured ? b->h_rows() : nullptr, b->sent_with_launch ? b->h_hist() : nullptr,
+        const bool captured = !mirror && is_capturing(h);
+        a.unchained = captured || side_by_side ? 1 : 0;   // (graphs, and launches between events, keep to plain edges)
+        const int e = fsb::launch_stream_kernel(a, !captured ? b->h_rows() : nullptr, b->sent_with_launch ? b->h_hist() : nullptr,
                                                 b->sent_with_launch ? (int)b->hist_ids : 0, b->hist_dev == nullptr, h->stream);
         if (e != 0) return fail(h, FSB_ERR_CUDA, "stream kernel launch: %s", cudaGetErrorString((cudaError_t)e));
         h->counters.kernel_launches++;

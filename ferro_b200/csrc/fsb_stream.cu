@@ -1305,7 +1305,7 @@ int launch_stream_kernel(StreamArgs a, const RowDesc* host_rows, const int32_t* 
     // per SM are the whole launch: placed while others still run, they pile up on some SMs (200 x 131072 31.4 -> 41.0, 300 x 65536 26.3 -> 29.3);
     // clusters do not (37 x 65536, k = 16, 296 CTAs 15.4 -> 13.3).
     const int ctas = a.n_rows * a.nseg;
-    const bool chained = a.overlap == 0 && !a.captured && (a.wide || ctas <= (a.nseg > 1 ? 2 : 1) * a.sms || ctas >= 3 * a.sms);
+    const bool chained = a.overlap == 0 && !a.unchained && (a.wide || ctas <= (a.nseg > 1 ? 2 : 1) * a.sms || ctas >= 3 * a.sms);
     cudaLaunchAttribute attr[2];
     int n = 0;
     if (a.overlap || chained) {
@@ -1455,7 +1455,7 @@ extern "C" int fsb_argmax_rows_static(int device, const float* logits_dev, int64
         a.kmax = 1;
         a.all_greedy = 1;
         a.sms = sd.sms;
-        a.captured = 1;   // (for all that is known here)
+        a.unchained = 1;   // (the stream may be capturing, for all that is known here)
         const SelectPlan pl = plan_select(n_rows, n_vocab, sd.sms, 1, true, false);
         a.nseg = pl.nseg;
         a.wide = pl.wide ? 1 : 0;
