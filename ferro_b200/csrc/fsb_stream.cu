@@ -186,7 +186,7 @@ __device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, int 
 // For k <= 64 the final bound is the row's, however many CTAs it has: every warp hands its `most` largest lane maxima - each lane's
 // is a logit of its own; keys, their low bits cut off - to all CTAs of the row, and each finds a value that at least k of all those
 // keys reach, and not many more: about 1.1 k to 1.7 k logits do.
-__device__ __forceinline__ int warps_with_data(int cells, int n_warps) { return min(n_warps, (cells + 31) >> 5); }
+__host__ __device__ __forceinline__ int warps_with_data(int cells, int n_warps) { return (cells + 31) >> 5 < n_warps ? (cells + 31) >> 5 : n_warps; }
 template <int T>
 __device__ __forceinline__ void publish_most(float run, int most, int seg, int nseg, unsigned* keys, u64* inbox) {
     constexpr int kWarps = T / 32;
@@ -1246,6 +1246,12 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
     cfg.blockDim = dim3(T);
     cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols);
     if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
+    if (a.kmax <= 64) {   // the keys that the warps of a row hand over have to fit (they do in every layout that plan_select gives)
+        const int cells = (a.n_vocab > 3 ? a.n_vocab - 3 : 0) / 4, sources = a.nseg * warps_with_data((cells + a.nseg - 1) / a.nseg, T / 32);
+        int most = 1;
+        while (most < 8 && 5 * most * sources < 8 * a.kmax) most *= 2;
+        if (most * (T / 32) * a.nseg > Geometry<T>::key_words(a.nseg)) return (int)cudaErrorInvalidValue;
+    }
     SelectArgs<NDESC> args;
     args.a = a;
     if (NDESC > 0) std::memcpy(args.rows, rows, sizeof(RowDesc) * (size_t)a.n_rows);
