@@ -846,8 +846,8 @@ again_from_the_start:
         } else {
             thr = cta_bound<T, 0>(run_a, run_b, k, refreshes++ & 1, ctl);
             admit = thr;
-            if (cap != 0.0f) softcap_bounds(thr, cap, admit, seen);
         }
+        if (cap != 0.0f && !again) softcap_bounds(thr, cap, admit, seen);   // (softcap_admit leaves `seen` to the final bound)
     } else if (again) {
         __syncthreads();
     } else {
