@@ -1103,12 +1103,15 @@ again_from_the_start:
 // a thread keeps the best cell it has seen in registers ("strictly larger" keeps the first of equals, because a thread
 // meets its cells in ascending order), the CTA takes the largest composite, and one warp finishes the row.  No bound, no
 // lists, no barrier before the end.  (Not with a softcap, which makes different logits equal, nor with write-back or patched values for the host.)
+// PEN: some row has a penalty window.  Where none has, the kernel does not know windows: their code between the first copies and the
+// stream, passed by, and the looks at whether there is one cost a launch that is waited for 700 cycles of 7550 (136 x 65536, by the SM's
+// counter); us per launch in a train, one kernel for both and two: 8.12, 8.03; with windows of 128 ids 9.28, 9.10.
 template <int T>
 size_t argmax_smem_bytes(int seg_cols) {
     return Geometry<T>::kRingBytes + sizeof(SharedCtl) + window_bytes(seg_cols);
 }
 
-template <int T, int NDESC>
+template <int T, int NDESC, bool PEN>
 __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_constant__ SelectArgs<NDESC> args) {
     constexpr int kChunkCells = Geometry<T>::kChunkCells;
     const StreamArgs& a = args.a;
@@ -1116,7 +1119,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     float4* ring = reinterpret_cast<float4*>(smem_raw);
     u64* best_of = reinterpret_cast<u64*>(smem_raw);   // after the stream: the warps' best, then the first masked columns
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem_raw + Geometry<T>::kRingBytes);
-    const int pen_cap = a.penalised ? kPenCap : 0;
+    constexpr int pen_cap = PEN ? kPenCap : 0;
     float* pen_raw = reinterpret_cast<float*>(ctl + 1);
     int* pen_col = reinterpret_cast<int*>(pen_raw + pen_cap);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -1139,7 +1142,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
             if (j + u * T < w.c_hi) cp_async16(dst + (unsigned)(u * T * sizeof(float4)), w.cells + j + u * T);
         cp_async_commit();
     };
-    if (!a.penalised)
+    if constexpr (!PEN)
         for (int c = 0; c < kStages; ++c) fetch(c);
     float edge = qnan;
     int edge_col = -1;
@@ -1149,11 +1152,11 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
     }
     if (nseg > 1) cluster_arrive_relaxed();
     Segment s = make_segment(a, w, row_ptr, seg, nseg, reinterpret_cast<unsigned*>(pen_col + pen_cap));
-    if (a.penalised) {   // (without windows nobody waits for the descriptor before the end)
+    if constexpr (PEN) {   // (without windows nobody waits for the descriptor before the end)
         s.has_pen = (dp.flags & kRowPenalty) != 0;
         s.pen = dp.penalty;
     }
-    if (s.has_pen) {
+    if (PEN && s.has_pen) {
         set_window(s, args.hist(), args.drafts(), dp);
         FirstIds<T> ids;
         ids.load(s);
@@ -1165,7 +1168,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         for (int c = 1; c < kStages; ++c) fetch(c);
         __syncthreads();
         if (edge_col >= 0 && penalised(s, edge_col)) edge = qnan;
-    } else if (a.penalised) {
+    } else if constexpr (PEN) {
         for (int c = 0; c < kStages; ++c) fetch(c);
     }
     trace_mark(a, 1);
@@ -1185,7 +1188,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         for (int u = 0; u < kCells; ++u) m[u] = tid + u * T < left ? cell_max(x[u]) : ninf;
         // (`floor_x` is the warp's best so far: what does not exceed it cannot win, and a warp rarely sees more than ten such chunks)
         if (__any_sync(0xffffffffu, fmaxf(max3(m[0], m[1], m[2]), m[3]) > floor_x)) {
-            if (s.has_pen) {
+            if (PEN && s.has_pen) {
                 mask_penalised<T>(x, s.bitmap, j0 - w.c_lo, left);
 #pragma unroll
                 for (int u = 0; u < kCells; ++u)
@@ -1205,7 +1208,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         if (left <= kChunkCells) break;
     }
     cp_async_wait<0>();
-    if (s.has_pen) __syncthreads();   // the penalised logits were fetched by other threads
+    if (PEN && s.has_pen) __syncthreads();   // the penalised logits were fetched by other threads
     trace_mark(a, 4);
 
     u64 top = 0ull;
@@ -1214,7 +1217,7 @@ __global__ void __launch_bounds__(T, 1024 / T) argmax_kernel(const __grid_consta
         top = make_comp(best, w.head + 4 * best_num + e + s.id_base);
     }
     if (edge > ninf) top = max(top, make_comp(edge, edge_col + s.id_base));
-    if (s.has_pen)
+    if (PEN && s.has_pen)
         for_each_penalised<T>(s, ctl->pen_n, pen_raw, pen_col, [&](bool in, float x, int col) {
             const float y = penalise(x, s.pen);
             if (in && y > ninf) top = max(top, make_comp(y, col + s.id_base));
@@ -1267,7 +1270,7 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
     if (NDESC == kFewRows && n_ids > 0) std::memcpy(args.ids, ids, sizeof(int32_t) * (size_t)n_ids);
     if (a.all_greedy && a.softcap == 0.0f && !a.write_back && !a.patched) {
         cfg.dynamicSmemBytes = argmax_smem_bytes<T>(seg_cols);
-        return (int)cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC>, args);
+        return (int)(a.penalised ? cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC, true>, args) : cudaLaunchKernelEx(&cfg, argmax_kernel<T, NDESC, false>, args));
     }
     if constexpr (T == 256 && NDESC == 0) {
         // Whole rows on small CTAs, four per SM, that do not fit the ring: a bit per column costs every thread four words per chunk, and
@@ -1289,7 +1292,8 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
 }
 template <int T, int NDESC>
 int prepare_select() {
-    cudaError_t e = cudaFuncSetAttribute(argmax_kernel<T, NDESC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    cudaError_t e = cudaFuncSetAttribute(argmax_kernel<T, NDESC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(argmax_kernel<T, NDESC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
     if constexpr (T == 256 && NDESC == 0)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(stream_select_kernel<T, NDESC, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelectSmemMax);
