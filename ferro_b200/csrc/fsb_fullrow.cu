@@ -1080,6 +1080,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             for (int i = tid; i < words; i += kFullThreads) bitmap[i] = 0u;
         auto column = [&](int i) { return i < main ? lo + i : i - main; };
         for (int i = 4 * n4 + tid; i < n; i += kFullThreads) vals[i] = __ldcs(row + column(i));
+        __syncthreads();   // (the barriers are initialised)
         late = !inbox_wait(&sh->in_slice);
         __syncthreads();
         if (a.softcap != 0.0f) {
