@@ -116,10 +116,16 @@ __device__ __forceinline__ void cluster_store_u32(unsigned addr, unsigned v) { a
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Ends when all other CTAs of the cluster have left or are here, too (the barrier does not count threads that have exited).  Whole warps.
+__device__ __forceinline__ void outlast_cluster() {
+    __syncwarp();
+    cluster_arrive_release();
+    cluster_wait_acquire();
+}
 
 // Stores to another CTA's shared memory that a barrier there counts, by bytes: the receiver waits for what it expects, and nobody
 // for a fence (a release of the cluster's barrier takes 1200 cycles).  One thread of the receiver initialises the barrier, and
-// expects the bytes, before or after they come; fenced_inits before that CTA arrives at the cluster's barrier.
+// expects the bytes, before or after they come; inbox_inits_fence before that CTA arrives at the cluster's barrier.
 __device__ __forceinline__ void inbox_init(u64* bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ void inbox_inits_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void inbox_expect(u64* bar, unsigned bytes) {
@@ -135,11 +141,15 @@ __device__ __forceinline__ void inbox_put(unsigned addr, u64 v, unsigned bar) {
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, u64* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
-// Waits until everything expected has come; gives up after a million looks (false), each of which the hardware may itself suspend.
+// Waits until everything expected has come; gives up (false) after a million looks, for each of which the hardware may suspend the
+// thread for a microsecond.  Threads of a CTA may differ in what they get.  (A test has waits run out.)
+#ifndef FSB_INBOX_LOOKS
+#define FSB_INBOX_LOOKS (1 << 20)
+#endif
 __device__ __forceinline__ bool inbox_wait(u64* bar) {
-    for (int i = 0; i < (1 << 20); ++i) {
+    for (int i = FSB_INBOX_LOOKS; i > 0; --i) {
         unsigned done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done) : "r"(smem_u32(bar)) : "memory");
         if (done) return true;
     }

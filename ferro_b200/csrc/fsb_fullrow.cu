@@ -148,6 +148,8 @@ struct FullShared {
     // candidates and whether the first CTA takes them
     u64 in_slice, in_extremes, in_parts, in_sums, in_counts, in_list, in_verdict;
     u64 extremes[2][kMaxCluster], counts[kMaxCluster], verdict;
+    int late;                  // a wait of this CTA has run out
+    unsigned gone;             // ... of another CTA of the cluster: see step_aside
     int sent;                  // candidates this CTA has handed over
     unsigned got[2][kMaxCluster];   // ... every CTA of the cluster has, double buffered by use
     int first_p, first_u;      // places in the ordered list
@@ -624,8 +626,9 @@ __device__ __forceinline__ bool send_bins(const RowCtx& rc, FullShared* sh, unsi
 
 // The same for the candidates of bins [b0, b1] and [b2, b3] (b1 < b2, or the second range is empty), without a count; once per row.
 // Nobody but the first CTA waits for the candidates: it counts what comes, and tells the others whether it has all of them.
+// 1: it has, 0: it has not, -1: this CTA's wait has run out (the first one has told nobody anything then).
 template <int C>
-__device__ __forceinline__ bool send_ranges(const RowCtx& rc, FullShared* sh, unsigned rank, int b0, int b1, int b2, int b3, int par, bool& late) {
+__device__ __forceinline__ int send_ranges(const RowCtx& rc, FullShared* sh, unsigned rank, int b0, int b1, int b2, int b3, int par) {
     const int tid = threadIdx.x;
     const unsigned to = map_to_rank(sh->list() + rank * kSendCap, 0u), bar = map_to_rank(&sh->in_list, 0u);
     // (a logit's bin is only worked out if the logit may lie in one of the ranges: the room on either side covers the rounding of the
@@ -655,11 +658,8 @@ __device__ __forceinline__ bool send_ranges(const RowCtx& rc, FullShared* sh, un
     for (int i = (rc.n & ~3) + tid; i < rc.n; i += kFullThreads) look(rc.vals[i], i);
     __syncthreads();
     if (tid == 0) inbox_put(map_to_rank(&sh->counts[rank], 0u), (u64)(unsigned)sh->sent, map_to_rank(&sh->in_counts, 0u));
-    if (rank != 0) {
-        late = !inbox_wait(&sh->in_verdict) || late;
-        return sh->verdict != 0ull;
-    }
-    late = !inbox_wait(&sh->in_counts) || late;
+    if (rank != 0) return __syncthreads_or(!inbox_wait(&sh->in_verdict)) ? -1 : sh->verdict != 0ull ? 1 : 0;
+    const bool counted = inbox_wait(&sh->in_counts);
     bool fits = true;
     unsigned words = 0u;
 #pragma unroll
@@ -669,11 +669,12 @@ __device__ __forceinline__ bool send_ranges(const RowCtx& rc, FullShared* sh, un
         words += min(n, (unsigned)kSendCap);
         if (tid == r) sh->got[par][r] = n;
     }
-    if (tid == 0) inbox_expect(&sh->in_list, 8u * words);
-    late = !inbox_wait(&sh->in_list) || late;   // (also what is of no use: the lists' memory may be needed for a descent)
-    if (tid > 0 && tid < C) inbox_put(map_to_rank(&sh->verdict, (unsigned)tid), fits ? 1ull : 0ull, map_to_rank(&sh->in_verdict, (unsigned)tid));
+    if (tid == 0 && counted) inbox_expect(&sh->in_list, 8u * words);
+    if (!counted || !inbox_wait(&sh->in_list)) sh->late = 1;   // (also what is of no use: the lists' memory may be needed for a descent)
     __syncthreads();
-    return fits;
+    if (sh->late) return -1;
+    if (tid > 0 && tid < C) inbox_put(map_to_rank(&sh->verdict, (unsigned)tid), fits ? 1ull : 0ull, map_to_rank(&sh->in_verdict, (unsigned)tid));
+    return fits ? 1 : 0;
 }
 
 // What the first CTA does with the lists that send_bins left there takes T threads: 256 of them, one candidate each, if
@@ -1001,6 +1002,35 @@ __device__ __noinline__ Crossing resolve(const RowCtx rc, FullShared* sh, unsign
     return cluster_descent<C>(rc, sh, floor_c, top_c, target, false, par);
 }
 
+// What a CTA does whose wait has run out, and those of its row that learn of it: the row is reported and gets token 0, nothing that
+// was waited for is used.  `tell`: the others learn of it at their next look at `gone` - all of them are still there, since none leaves the
+// kernel without a word from this CTA that it has not given, or its arrival at a barrier.  Then the CTA keeps to the cluster's barriers until
+// the others have left or do the same (the barrier does not count threads that have exited; kMostBarriers is more than a row has between
+// its last wait for a word and its look at `gone`: nine of a descent, two for the sums, one before the look): its memory is there for whoever
+// reads it or stores to it.
+constexpr int kMostBarriers = 32;
+struct RowOutputs {   // (by value: the address of a kernel's argument would put a copy of all of them in local memory)
+    unsigned *status, *status_host;
+    int32_t *tokens, *tokens_host, *append_at, *kept_n;
+    int out;
+};
+template <int C>
+__device__ __noinline__ void step_aside(FullShared* sh, unsigned rank, bool tell, bool copying, const RowOutputs o) {
+    const int tid = threadIdx.x;
+    if (tid == 0) report_status(o.status, o.status_host, kStatusLate);
+    if (tell && tid < C) cluster_store_u32(map_to_rank(&sh->gone, (unsigned)tid), 1u);
+    for (int i = 0; i < kMostBarriers; ++i) {
+        __syncwarp();
+        cluster_sync_all();
+    }
+    if (copying) inbox_wait(&sh->in_slice);   // (a copy that is still on its way)
+    if (rank == 0 && tid == 0) {
+        if (o.kept_n) o.kept_n[o.out] = 0;
+        if (o.append_at) *o.append_at = 0;
+        put_token(o.tokens, o.tokens_host, o.out, 0);
+    }
+}
+
 template <int C>
 __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArgs a, int cache_slice) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1037,6 +1067,8 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         inbox_expect(&sh->in_counts, 8u * C);
         inbox_expect(&sh->in_verdict, 8u);
         sh->sent = 0;
+        sh->late = 0;
+        sh->gone = 0u;
     }
     if (tid == 32) {   // (while the first loads are on their way)
         double w = __dmul_rn(__ull2double_rn(d.rng_word), 5.42101086242752217003726400434970855712890625e-20);   // 2^-64
@@ -1044,7 +1076,6 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         sh->plan.u = w;
         sh->plan.below = d.min_p > 0.0f ? (double)d.temperature * log((double)d.min_p) : 0.0;
     }
-    bool late = false;   // something did not come
     cluster_arrive_relaxed();   // (waited for before the first access to another CTA's shared memory)
     if (tid < 64) sh->table[tid] = exp2((double)tid / 64.0);
 
@@ -1068,6 +1099,10 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         return x;
     };
     const bool copied = cache_slice && n4 > 0;
+    auto aside = [&](bool tell) {
+        step_aside<C>(sh, rank, tell, copied,
+                      RowOutputs{a.status, a.status_host, a.tokens, a.tokens_host, d.flags & kRowAppend ? a.pool + d.hist_begin + d.hist_len : nullptr, a.record ? a.kept_n : nullptr, d.out_index});
+    };
     if (copied) {
         // The usual way, a slice on a 16-byte boundary: one bulk copy, and the penalty where the window says so.  (Loads and stores by all threads, with a
         // look at the window's bits for every logit: 5.7 us for 21848 logits, this way 2.3.)
@@ -1081,8 +1116,13 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         auto column = [&](int i) { return i < main ? lo + i : i - main; };
         for (int i = 4 * n4 + tid; i < n; i += kFullThreads) vals[i] = __ldcs(row + column(i));
         __syncthreads();   // (the barriers are initialised)
-        late = !inbox_wait(&sh->in_slice);
+        if (!inbox_wait(&sh->in_slice)) sh->late = 1;
         __syncthreads();
+        if (sh->late) {
+            cluster_wait_acquire();
+            aside(true);
+            return;
+        }
         if (a.softcap != 0.0f) {
             for (int i = tid; i < n; i += kFullThreads) {
                 const float x = __fmul_rn(a.softcap, tanhf(__fdiv_rn(vals[i], a.softcap)));
@@ -1178,7 +1218,12 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
                 inbox_put(map_to_rank(&sh->extremes[1][rank], (unsigned)lane), (u64)cnt, bar);
             }
         }
-        late = !inbox_wait(&sh->in_extremes) || late;
+        if (!inbox_wait(&sh->in_extremes)) sh->late = 1;
+        __syncthreads();
+        if (sh->late) {
+            aside(true);
+            return;
+        }
         kx = 0u;
         kn = ~0u;
         valid = 0u;
@@ -1204,6 +1249,8 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             a.kept_n[out] = 0;
             finish(0);
         }
+        __syncwarp();
+        cluster_sync_all();   // (a CTA that steps aside may still tell this one)
         return;
     }
     rc.mx = mx;
@@ -1302,8 +1349,9 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
                 inbox_put(map_to_rank(&sh->part[1][at], owner), p1, bar);
             }
         }
-        late = !inbox_wait(&sh->in_parts) || late;
-        for (int t = tid; t < C * kMine; t += kFullThreads) {
+        const bool parts = inbox_wait(&sh->in_parts);
+        if (!parts) sh->late = 1;
+        for (int t = tid; parts && t < C * kMine; t += kFullThreads) {
             const int dst = t / kMine, bin = (int)rank * kMine + t % kMine;
             if (bin >= kBins) continue;
             u64 c0 = 0ull, c1 = 0ull;
@@ -1316,7 +1364,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             inbox_put(map_to_rank(&sh->cum[0][bin], (unsigned)dst), c0, bar);
             inbox_put(map_to_rank(&sh->cum[1][bin], (unsigned)dst), c1, bar);
         }
-        late = !inbox_wait(&sh->in_sums) || late;
+        if (!inbox_wait(&sh->in_sums)) sh->late = 1;
         // inclusive sums over the bins, largest logits first
         u64 own0[kBinsEach], own1[kBinsEach], c0 = 0ull, c1 = 0ull;
         unsigned own_est[kBinsEach], est = 0u;
@@ -1346,6 +1394,10 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             sh->red_cnt[warp] = est;
         }
         __syncthreads();
+        if (sh->late) {
+            aside(true);
+            return;
+        }
         u64 t0 = lane < warp ? sh->red[lane] : 0ull, t1 = lane < warp ? sh->red_hi[lane] : 0ull;
         est += __reduce_add_sync(0xffffffffu, lane < warp ? sh->red_cnt[lane] : 0u);
 #pragma unroll
@@ -1447,11 +1499,11 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
 
     // ---- 4. the usual way: the candidates of the bins where the kept set may end, and of those that the draw may fall into, go to the
     // first CTA, which finishes the row
+    int sent = 0;
     if (binned && !a.record) {
-        if (plan.about <= (unsigned)kMostListed &&
-            send_ranges<C>(rc, sh, rank, plan.draw_lo, plan.draw_hi, max(plan.cut_lo, plan.draw_hi + 1), plan.cut_hi, par, late)) {
+        if (plan.about <= (unsigned)kMostListed) sent = send_ranges<C>(rc, sh, rank, plan.draw_lo, plan.draw_hi, max(plan.cut_lo, plan.draw_hi + 1), plan.cut_hi, par);
+        if (sent > 0) {
             FTR(5);
-            if (late && tid == 0) report_status(a.status, a.status_host, kStatusLate);
             if (rank != 0) return;   // nobody reads this CTA's memory any more
             const int m = listed<C>(sh, par);
             int token;
@@ -1466,8 +1518,24 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
             return;
         }
         par ^= 1;
+        if (sent < 0 && rank == 0) {
+            aside(true);
+            return;
+        }
     }
-    if (late && tid == 0) report_status(a.status, a.status_host, kStatusLate);
+    __syncwarp();
+    cluster_sync_all();   // whoever goes on from here needs all CTAs of the row
+    if (sh->gone) {
+        aside(false);
+        return;
+    }
+    if (sent < 0) {   // the first CTA's verdict came late: it is here by now, from a CTA that has passed the barrier with it or has left
+        if (__syncthreads_or(!inbox_wait(&sh->in_verdict))) {
+            aside(false);
+            return;
+        }
+        if (sh->verdict) return;   // (the row is finished)
+    }
 
     // ---- 4a. the usual way with a cut: everything that can be kept goes to the first CTA, which finishes the row
     if (binned && (d.top_p < 1.0f || d.min_p > 0.0f)) {

@@ -43,7 +43,10 @@ namespace {
 // 25.5 -> 24.5.
 // The exact path (exact_select) makes no assumption: a radix selection over the transformed segment that reads it again
 // (from L2) per digit.  It runs when hundreds of equal logits reach the final bound.
-// Waits for another CTA end after a million looks at the latest; the row is then reported (kStatusLate).
+// Waits for another CTA end after a second or so at the latest.  A CTA whose wait has run out reports the row (kStatusLate) and uses nothing of
+// what it waited for: without the row's keys it goes on with a bound that no finite logit (under the softcap: hardly one) reaches, and the
+// first one without all candidates finishes a row of none.  It stays until the others have left or gave up, too: what is still on its way to it
+// finds its memory there.
 
 constexpr int kCells = 4;                               // cells of a thread per chunk
 constexpr int kStages = 2;
@@ -117,7 +120,8 @@ struct StreamCtl : SharedCtl {
     u64 keyed, counted, sent;  // barriers: the row's keys have come; in its first CTA, the numbers of candidates, the candidates
     u64 count[8];              // from segment r: its number of candidates, whether they are in the second part of its share, and how many words it has sent
     unsigned bound;
-    int pad[3];
+    int late;                  // a wait has run out
+    int pad[2];
 };
 static_assert(sizeof(StreamCtl) % 16 == 0, "what follows the control block is read 16 bytes at a time");
 
@@ -687,6 +691,7 @@ __global__ void __launch_bounds__(T, T == 256 && NDESC > 0 ? 2 : 1024 / T) strea
         ctl->lost = 0;
         ctl->kept_n = 0;
         ctl->pen_n = 0;
+        ctl->late = 0;
         if (nseg > 1 && !LONG) {
             inbox_init(&ctl->keyed);
             inbox_init(&ctl->counted);
@@ -827,12 +832,16 @@ again_from_the_start:
         publish_most<T>(run_a, most, seg, nseg, keys, &ctl->keyed);
         if (nseg == 1) __syncthreads();
         if (tid < 32) {
-            if (nseg > 1 && !inbox_wait(&ctl->keyed) && lane == 0) report_status(a.status, a.status_host, kStatusLate);
+            if (nseg > 1 && !inbox_wait(&ctl->keyed)) {
+                ctl->late = 1;
+                report_status(a.status, a.status_host, kStatusLate);
+            }
+            __syncwarp();
             const unsigned least = key_bound(most * kWarps * nseg, k, keys);
             if (lane == 0) ctl->bound = least;
         }
         __syncthreads();
-        thr = fmaxf(key_float(ctl->bound), -FLT_MAX);
+        thr = ctl->late ? -ninf : fmaxf(key_float(ctl->bound), -FLT_MAX);
         admit = thr;
         if (cap != 0.0f) softcap_bounds(thr, cap, admit, seen);
     }
@@ -1000,25 +1009,33 @@ again_from_the_start:
         if (tid == 0) inbox_put(cluster_map_shared(smem_u32(&ctl->count[seg]), 0u), report, cluster_map_shared(smem_u32(&ctl->counted), 0u));
         if (seg != 0) {
             trace_mark(a, 6);
+            if (ctl->late) outlast_cluster();
             return;
         }
     }
     if (tid >= kPost) return;   // eight warps finish the row (no barrier of the whole CTA or by all threads of the cluster from here on)
     u64* all = picked;
     if (direct) {
-        if (!inbox_wait(&ctl->counted) && tid == 0) report_status(a.status, a.status_host, kStatusLate);
-        const u64 said = lane < nseg ? ctl->count[lane] : 0ull;
+        constexpr u64 kUnknown = 1ull << 48;   // (more words than there can be, and no candidate)
+        const bool counted = inbox_wait(&ctl->counted);
+        const u64 said = !counted ? kUnknown : lane < nseg ? ctl->count[lane] : 0ull;
         const int n_q = (int)(said & 0xFFFFu);
         n = __reduce_add_sync(0xffffffffu, n_q);
         const int words = __reduce_add_sync(0xffffffffu, (int)(said >> 32));
-        if (tid == 0) inbox_expect(&ctl->sent, 8u * (unsigned)words);
+        if (tid == 0 && words < (int)(kUnknown >> 32)) inbox_expect(&ctl->sent, 8u * (unsigned)words);
         const int from = tid >> 5;   // one list: warp w copies segment w's part
         const int before = __reduce_add_sync(0xffffffffu, lane < from ? n_q : 0), mine = __shfl_sync(0xffffffffu, n_q, from);
         const u64* src = recv + (kMergeList >> lseg) * from + ((__shfl_sync(0xffffffffu, (unsigned)said, from) >> 16) & 1u ? share : 0);
-        if (!inbox_wait(&ctl->sent) && tid == 0) report_status(a.status, a.status_host, kStatusLate);
-        for (int i = lane; i < mine; i += 32) list[before + i] = src[i];
+        const bool here = inbox_wait(&ctl->sent) && counted;
+        if (!here) ctl->late = 1;
+        for (int i = lane; here && i < mine; i += 32) list[before + i] = src[i];
         all = list;
         block_sync<kPost, 1>();
+        if (ctl->late) {
+            n = 0;
+            if (tid == 0) report_status(a.status, a.status_host, kStatusLate);
+            outlast_cluster();
+        }
     } else if (LONG && nseg > 1) {
         cluster_wait_acquire();   // every CTA of the row runs: the first one's shared memory may be written
         const int send_cap = min(kPickCap, kMergeList >> lseg);
