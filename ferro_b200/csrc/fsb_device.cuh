@@ -168,13 +168,6 @@ __device__ __forceinline__ u64 global_timer_ns() {
 // often).
 template <int T, int BAR>
 __device__ __forceinline__ void block_sync() { asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(T) : "memory"); }
-// The same, with the number of threads whose `pred` holds.
-template <int T, int BAR>
-__device__ __forceinline__ int block_sync_count(bool pred) {
-    int n;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.popc.u32 %0, %2, %3, p;\n\t}" : "=r"(n) : "r"((int)pred), "n"(BAR), "n"(T) : "memory");
-    return n;
-}
 
 constexpr int kPost = 256;   // threads that finish a row
 static_assert(kPost == kMaxK && kMaxK % 16 == 0, "the epilogue has a thread per candidate and reads them 16 at a time");

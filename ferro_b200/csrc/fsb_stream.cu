@@ -189,7 +189,13 @@ __device__ __forceinline__ float cta_bound(float run_a, float run_b, int k, int 
 // For k <= 64 the final bound is the row's, however many CTAs it has: every warp hands its `most` largest lane maxima - each lane's
 // is a logit of its own; keys, their low bits cut off - to all CTAs of the row, and each finds a value that at least k of all those
 // keys reach, and not many more: about 1.1 k to 1.7 k logits do.
-__host__ __device__ __forceinline__ int warps_with_data(int cells, int n_warps) { return (cells + 31) >> 5 < n_warps ? (cells + 31) >> 5 : n_warps; }
+// How many that is in a row of `cells` cells and nseg CTAs of n_warps warps: 1.6 k of them in all, but no more than 8 a warp.
+__host__ __device__ __forceinline__ int keys_per_warp(int cells, int nseg, int n_warps, int k) {
+    const int groups = ((cells + nseg - 1) / nseg + 31) >> 5, sources = nseg * (groups < n_warps ? groups : n_warps);   // (warps that have any cells)
+    int most = 1;
+    while (most < 8 && 5 * most * sources < 8 * k) most *= 2;
+    return most;
+}
 template <int T>
 __device__ __forceinline__ void publish_most(float run, int most, int seg, int nseg, unsigned* keys, u64* inbox) {
     constexpr int kWarps = T / 32;
@@ -676,11 +682,7 @@ __global__ void __launch_bounds__(T, T == 256 && NDESC > 0 ? 2 : 1024 / T) strea
     unsigned* const bitmap = reinterpret_cast<unsigned*>(recv + (nseg > 1 ? kMergeList : 0));
     const bool has_pen = (dp.flags & kRowPenalty) != 0;
     const int k = dp.k;
-    int most = 1;   // keys that a warp hands over: 1.6 k of them in all, but no more than 8 a warp
-    if constexpr (!LONG) {
-        const int sources = nseg * warps_with_data((n_cells + nseg - 1) / nseg, kWarps);
-        while (most < 8 && 5 * most * sources < 8 * k) most *= 2;
-    }
+    const int most = LONG ? 0 : keys_per_warp(n_cells, nseg, kWarps, k);
     if (tid < 8) {   // the logits outside the whole cells
         const int c = span.edge_column(tid, V, seg, nseg);
         if (c >= 0) cp_async4(smem_u32(&ctl->edge[tid]), row_ptr + c);
@@ -1248,10 +1250,9 @@ int launch_select(cudaLaunchConfig_t& cfg, const StreamArgs& a, const RowDesc* r
     cfg.dynamicSmemBytes = Geometry<T>::smem_bytes(a.nseg, a.kmax, seg_cols);
     if (cfg.dynamicSmemBytes > (size_t)kSelectSmemMax) return (int)cudaErrorInvalidValue;
     if (a.kmax <= 64) {   // the keys that the warps of a row hand over have to fit (they do in every layout that plan_select gives)
-        const int cells = (a.n_vocab > 3 ? a.n_vocab - 3 : 0) / 4, sources = a.nseg * warps_with_data((cells + a.nseg - 1) / a.nseg, T / 32);
-        int most = 1;
-        while (most < 8 && 5 * most * sources < 8 * a.kmax) most *= 2;
-        if (most * (T / 32) * a.nseg > Geometry<T>::key_words(a.nseg)) return (int)cudaErrorInvalidValue;
+        // (a row has at least so many whole cells, and more cells or a smaller k mean no more keys)
+        const int cells = (a.n_vocab > 3 ? a.n_vocab - 3 : 0) / 4;
+        if (keys_per_warp(cells, a.nseg, T / 32, a.kmax) * (T / 32) * a.nseg > Geometry<T>::key_words(a.nseg)) return (int)cudaErrorInvalidValue;
     }
     SelectArgs<NDESC> args;
     args.a = a;
