@@ -524,7 +524,7 @@ def main():
     batch = eng.prepare_batch(sids, hists, VOCAB)
     kernels_per_step = batch.kernels_per_launch
 
-    # ---- the timed steps: a train of launches on one stream, no overlap between them
+    # ---- the timed steps: a train of launches on one stream: none reads or writes before the one before it is complete
     eng.set_launch_overlap(0)
     for i in range(args.warmup):
         batch.launch(bufs[i % n_buf].data_ptr())
@@ -654,7 +654,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": NCU_TRAFFIC_BYTES,
                          "peak_source": peak_src, "algorithmic_bytes_per_launch": bytes_launch, "frac_of_nominal_8000": achieved / 8000.0,
                          "kernel": "stream_select_kernel", "launch_us": ms_step * 1e3,
-                         "note": "achieved = algorithmic bytes / duration of one launch in the timed train (no overlap between launches)"},
+                         "note": "achieved = algorithmic bytes / duration of one launch in the timed train (a launch reads and writes nothing before the one before is complete; only placing its CTAs overlaps that one's end)"},
             "hidden_launch_latency_train": {"step_us": ms_hidden * 1e3, "rows_per_s": world * ROWS / (ms_hidden * 1e-3),
                                             "achieved_gb_s": bytes_launch / (ms_hidden * 1e-3) / 1e9, "frac": bytes_launch / (ms_hidden * 1e-3) / 1e9 / peak,
                                             "note": "fsb_set_launch_overlap(2): every CTA waits for the previous launch to complete before its first "

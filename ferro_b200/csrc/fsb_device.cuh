@@ -71,7 +71,7 @@ __device__ __forceinline__ void softcap_bounds(float thr, float cap, float& admi
 // `admit` alone, for a bound that will be refined: up to four caps from zero the softcap's slope is at least 1 - tanh(4)^2 = 0.0013, so what
 // lies 0.005 caps further down is 6.7e-6 caps below after it - more than the margin of 2^-20 caps and three roundings of 2^-22 - and
 // so below whatever a higher bound makes `seen`.  (All warps work out softcap_bounds alike, 1000 cycles of 32 warps' issue slots at every
-// refresh: 64 x 262144 23.4 -> 21.8 us.)
+// refresh: 1.6 us of a launch of 64 x 262144.)
 __device__ __forceinline__ void softcap_admit(float thr, float cap, float& admit, float& seen) {
     if (fabsf(thr) <= 4.0f * cap) admit = fmaxf(thr - 0.005f * cap, -FLT_MAX);
     else softcap_bounds(thr, cap, admit, seen);
@@ -280,7 +280,7 @@ static __device__ __noinline__ int select_list_topk(u64* list, int n, int k, u64
 // 64 more entries) and calls emit(rank, composite) once for each that ranks below k.
 //  n <= 128: by counting.  Four lanes count for an entry, or for two of them, each a quarter of the list, two entries per 16-byte
 //    broadcast read and no dependency between the reads (the quarters are interleaved: no bank conflicts); no atomics, one barrier.
-//    The list is padded to 64 or 128 entries, so that all reads are under way at once (64: 900 -> 670 cycles).
+//    The list is padded to 64 or 128 entries, so that all reads are under way at once (64: 670 cycles, 900 without).
 //  n <= kRankCap: in runs of 32 that the warps sort across their lanes; an entry's rank is its place in its run plus the
 //    larger entries of the other runs, by binary searches that do not depend on one another.
 //  longer lists are first cut down to k by bisection (`tmp`: scratch for k composites).
@@ -450,7 +450,7 @@ static __device__ __noinline__ int exact_cuts(double* x, double* e, int kk, doub
 // number, and that sum differs from S[i] / S by less than (2 * 256 + 5) * 2^-53 of it, the rounding of three chains of at most
 // 256 terms.  A comparison that S[i] decides by more than 1e-12 - seventeen times that - comes out the same, so the second
 // chain and the divisions run only where one is closer (equal logits with a cut between them), or where the probabilities are
-// recorded.  Per launch, us: 24 x 100003, k = 50 18.6 -> 17.5; 64 x 262144, k = 64 26.9 -> 25.7; 512 x 65536, k = 200 94.8 -> 90.6.
+// recorded: they would take 1.1 us of a launch of 24 x 100003, k = 50, 1.2 of 64 x 262144, k = 64, and 4.2 of 512 x 65536, k = 200.
 __device__ __forceinline__ void row_epilogue(const u64* srt, int kk, const RowTail r, double* work, SharedCtl* ctl, const TailOut o) {
     const int tid = threadIdx.x, lane = tid & 31;
     double* e = work;

@@ -24,9 +24,8 @@
 // a logit takes 19 fp64 operations, a conversion each way and some 40 others.  512 threads with 128 registers: with 1024 and 64 the
 // passes spilled, and what all warps compute alike was issued eight times per scheduler instead of four.  What one warp can compute for
 // all is left to one, and CTAs hand values to one another by counted stores (inbox_put): the cluster's barrier and its fences take 1 us.
-// us by time stamps, before -> after, 16 x 131072 in clusters of six, top-p 0.95: slice 5.8 -> 2.3, extremes 1.3 -> 0.6, weights and cumulative sums
-// 13.2 -> 15.3 (exact now, and the plan of what to look at), the rest 29 -> 7 (one look at the slice instead of two or three); 8 x 65536 in clusters of
-// eight: 2.7 -> 1.6, 1.3 -> 0.6, 8.1 -> 8.5, 11 -> 5.
+// us by time stamps, 16 x 131072 in clusters of six, top-p 0.95: slice 2.3, extremes 0.6, weights, cumulative sums and the plan of what to look at
+// 15.3, the rest 7 (29 where every crossing is resolved with a look at the slice of its own); 8 x 65536 in clusters of eight: 1.6, 0.6, 8.5, 5 (11).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -678,7 +677,7 @@ __device__ __forceinline__ int send_ranges(const RowCtx& rc, FullShared* sh, uns
 }
 
 // What the first CTA does with the lists that send_bins left there takes T threads: 256 of them, one candidate each, if
-// there are at most kShort (eight warps get through the barriers faster than thirty-two), else all.
+// there are at most kShort (eight warps get through the barriers faster than sixteen), else all.
 template <int T>
 __device__ __forceinline__ void list_sync() { block_sync<T, T == kFullThreads ? 0 : 1>(); }
 
@@ -1440,7 +1439,7 @@ __global__ void __launch_bounds__(kFullThreads, 1) full_row_kernel(const FullArg
         par ^= 1;
         cluster_sync_all();   // (the next use of x_small)
     }
-    // what follows from it, by one warp: thirty-two of them would issue the same instructions eight times per scheduler
+    // what follows from it, by one warp: sixteen of them would issue the same instructions four times per scheduler
     if (tid < 32) {
         RowPlan& pl = sh->plan;   // (all lanes store the same)
         const double total = __dmul_rn(u128_to_double(S), 2.168404344971008868014905601739883422851562500e-19);   // * 2^-62

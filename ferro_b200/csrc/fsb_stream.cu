@@ -38,9 +38,8 @@ namespace {
 // latency is its instruction count: a warp alone issues a dependent instruction every four to five cycles, and 32 warps that
 // all do the same take eight times their share of a scheduler, so steps after the stream are left to one warp or eight, and
 // what several CTAs need of one another goes by counted stores (inbox_put) instead of the cluster's barrier and its fences.
-// us per launch with launches chained (form 2), before -> after the final bound became the row's: 1 x 65536, k = 40 10.2 -> 7.9,
-// 32 x 131072, k = 40 14.4 -> 11.2, 72 x 131072, k = 50 21.0 -> 16.9, 64 x 262144, k = 64 23.3 -> 20.6, 512 x 32768, k = 40
-// 25.5 -> 24.5.
+// us per launch with launches chained (form 2): 1 x 65536, k = 40 7.9, 32 x 131072, k = 40 11.2, 72 x 131072, k = 50 16.9, 64 x 262144, k = 64
+// 20.6, 512 x 32768, k = 40 24.5; with a bound per segment and the cluster's barrier 2.3, 3.2, 4.1, 2.7 and 1.0 more.
 // The exact path (exact_select) makes no assumption: a radix selection over the transformed segment that reads it again
 // (from L2) per digit.  It runs when hundreds of equal logits reach the final bound.
 // Waits for another CTA end after a second or so at the latest.  A CTA whose wait has run out reports the row (kStatusLate) and uses nothing of
