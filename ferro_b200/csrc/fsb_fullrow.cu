@@ -46,6 +46,7 @@ constexpr int kMostListed = 768;                // candidates that are worth a l
 constexpr float kBinned = 19.4f;                // the bins cover this many temperatures below the maximum (weights down to 2^-28), the last one all the rest
 constexpr int kSendCap = 512;                   // candidates a CTA can hand to the first one
 constexpr int kShort = 256;                     // lists of up to this many candidates are ordered by counting
+constexpr int kAhead = 4;                       // logits that a thread looks at together in a descent
 constexpr int kStripes = 8;                     // copies of the level histogram (by warp): fewer warps hit one word at once
 constexpr int kLimbs = 4;                       // a weight is added to a histogram as four 16-bit limbs (32-bit native atomics)
 
@@ -205,12 +206,27 @@ struct RowCtx {
     const double* table;      // 2^(j / 64)
     u64 floor_c;              // candidates are those at or above this composite (0: all)
     float bin_scale;          // bins per logit
-    __device__ __forceinline__ float at(int i) const {   // logit i of the slice as the sampler sees it
-        if (vals) return vals[i];
-        float x = row[lo + i];
+    __device__ __forceinline__ float seen(float x, int i) const {   // what the sampler sees of logit i of the slice
         if (cap != 0.0f) x = __fmul_rn(cap, tanhf(__fdiv_rn(x, cap)));
         if (bitmap && ((bitmap[i >> 5] >> (i & 31)) & 1u)) x = x > 0.0f ? __fdiv_rn(x, pen) : __fmul_rn(x, pen);
         return x;
+    }
+    __device__ __forceinline__ float at(int i) const { return vals ? vals[i] : seen(row[lo + i], i); }
+    // Logits i, i + kFullThreads, ... of the slice, kAhead of them; what lies past its end is NaN.  A descent's pass is bound by latency - of
+    // reads from L2, where the row is not in shared memory, and of the weights' chains of fp64 operations - with 16 warps per SM to hide it:
+    // four reads and four weights at a time.  us, one logit at a time / four reads, weights one by one / both / eight reads: 4 x 300000 358, 329,
+    // 307, 323; 4 x 900000 1001, 908, 845, 892; 8 x 65536, k = 3000 52.1, 52.4, 46.6, 48.8.  With the next four on their way, too, 343.
+    __device__ __forceinline__ void ahead(int i, float (&x)[kAhead]) const {
+        const float nan = __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int at = i + q * kFullThreads;
+            x[q] = at >= n ? nan : vals ? vals[at] : row[lo + at];
+        }
+        if (vals) return;
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q)
+            if (i + q * kFullThreads < n) x[q] = seen(x[q], i + q * kFullThreads);
     }
     // (the up to three columns before the row's first 16-byte boundary come last in the first slice)
     __device__ __forceinline__ u64 comp(float x, int i) const { return make_comp(x, (i < main ? lo + i : i - main) + id_base); }
@@ -234,8 +250,8 @@ struct RowCtx {
         const u64 w = __double2ull_rn(__dmul_rn(e, 4611686018427387904.0));
         return Weight{(unsigned)(w >> 31), (int)(w & 0x7FFFFFFFull)};
     }
-    __device__ __forceinline__ Weight weight(float x) const {
-        if (odd) return odd_weight(x);
+    __device__ __forceinline__ Weight weight(float x) const { return odd ? odd_weight(x) : finite_weight(x); }
+    __device__ __forceinline__ Weight finite_weight(float x) const {   // (of a row that is not odd)
         const double y = scaled(fmaxf(__fsub_rn(x, mx), cut));
         const double magic = 6755399441055744.0;   // 1.5 * 2^52
         const double t = __fma_rn(y, 92.33248261689366, magic);   // 64 / ln 2
@@ -348,14 +364,19 @@ __device__ __forceinline__ void level_reduce_and_walk(FullShared* sh, int par, U
     }
     cluster_sync_all();
     if (tid < 256) {
+        u64 l[C], h[C];
+        unsigned c[C];
 #pragma unroll
         for (unsigned r = 0; r < (unsigned)C; ++r) {
-            const u64 l = ld_cluster_u64(map_to_rank(&sh->x_lo[par][tid], r));
-            const u64 h = ld_cluster_u64(map_to_rank(&sh->x_hi[par][tid], r));
-            const unsigned c = ld_cluster_u32(map_to_rank(&sh->x_cnt[par][tid], r));
-            lo += l;
-            hi += h + (lo < l ? 1ull : 0ull);
-            cnt += c;
+            l[r] = ld_cluster_u64(map_to_rank(&sh->x_lo[par][tid], r));
+            h[r] = ld_cluster_u64(map_to_rank(&sh->x_hi[par][tid], r));
+            c[r] = ld_cluster_u32(map_to_rank(&sh->x_cnt[par][tid], r));
+        }
+#pragma unroll
+        for (int r = 0; r < C; ++r) {
+            lo += l[r];
+            hi += h[r] + (lo < l[r] ? 1ull : 0ull);
+            cnt += c[r];
         }
     }
     if (by_count) {   // the "weight" of a digit is its number of candidates
@@ -443,24 +464,32 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx rc, FullShared* sh
             for (int i = tid; i < (int)((stripe_mask + 1u) * sizeof(sh->h[0]) / sizeof(uint4)); i += kFullThreads)
                 reinterpret_cast<uint4*>(&sh->h[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
-            const int n_iter = (rc.n + kFullThreads - 1) / kFullThreads;
-            for (int it = 0; it < n_iter; ++it) {
-                const int i = it * kFullThreads + tid;
-                bool active = false;
-                int digit = 0;
-                u64 wgt = 0ull;
-                if (i < rc.n) {
-                    const float x = rc.at(i);
-                    if (x == x) {   // NaNs take no part
-                        const u64 c = rc.comp(x, i);
-                        if (c >= floor_c && (c & mask) == pfx) {
-                            active = true;
-                            digit = (int)((unsigned)(c >> lo) & dmask);
-                            if (!by_count) wgt = rc.weight(x).value();
-                        }
-                    }
+            for (int i0 = tid; i0 - (tid & 31) < rc.n; i0 += kAhead * kFullThreads) {   // (whole warps)
+                float x[kAhead];
+                rc.ahead(i0, x);
+                int digit[kAhead];   // -1: takes no part
+                bool some = false;
+#pragma unroll
+                for (int q = 0; q < kAhead; ++q) {
+                    const u64 c = rc.comp(x[q], i0 + q * kFullThreads);
+                    const bool in = x[q] == x[q] && c >= floor_c && (c & mask) == pfx;
+                    digit[q] = in ? (int)((unsigned)(c >> lo) & dmask) : -1;
+                    some = some || in;
                 }
-                hist_add(sh, active, digit, wgt, !by_count, stripe_mask);
+                if (!__any_sync(0xffffffffu, some)) continue;
+                u64 w[kAhead];
+                if (by_count) {
+#pragma unroll
+                    for (int q = 0; q < kAhead; ++q) w[q] = 0ull;
+                } else if (rc.odd) {
+#pragma unroll
+                    for (int q = 0; q < kAhead; ++q) w[q] = rc.odd_weight(x[q]).value();
+                } else {   // a weight is a chain of dependent fp64 operations: several at once
+#pragma unroll
+                    for (int q = 0; q < kAhead; ++q) w[q] = rc.finite_weight(x[q]).value();
+                }
+#pragma unroll
+                for (int q = 0; q < kAhead; ++q) hist_add(sh, digit[q] >= 0, digit[q], w[q], !by_count, stripe_mask);
             }
             __syncthreads();
         }
@@ -486,11 +515,13 @@ __device__ __noinline__ Crossing cluster_descent(const RowCtx rc, FullShared* sh
     if (hb >= 0) {
         // the single candidate that matches the prefix, wherever it lies: its owner finds it, the cluster takes the maximum
         u64 mine = 0ull;
-        for (int i = tid; i < rc.n; i += kFullThreads) {
-            const float x = rc.at(i);
-            if (x == x) {
-                const u64 c = rc.comp(x, i);
-                if (c >= floor_c && (c & mask) == pfx) mine = c;
+        for (int i0 = tid; i0 < rc.n; i0 += kAhead * kFullThreads) {
+            float x[kAhead];
+            rc.ahead(i0, x);
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q) {
+                const u64 c = rc.comp(x[q], i0 + q * kFullThreads);
+                if (x[q] == x[q] && c >= floor_c && (c & mask) == pfx) mine = c;
             }
         }
         // exactly one thread of the cluster holds it: that thread tells every CTA, one barrier makes it visible
@@ -571,7 +602,11 @@ __device__ __forceinline__ void load4(const RowCtx& rc, int i, float (&x)[4]) {
         return;
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) x[e] = i + e < rc.n ? rc.at(i + e) : __int_as_float(0x7fc00000);
+    for (int e = 0; e < 4; ++e) x[e] = i + e >= rc.n ? __int_as_float(0x7fc00000) : rc.vals ? rc.vals[i + e] : rc.row[rc.lo + i + e];
+    if (rc.vals) return;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (i + e < rc.n) x[e] = rc.seen(x[e], i + e);
 }
 
 // Hands this CTA's candidates of bins [b_lo, b_hi] to the first CTA of the cluster, and counts its candidates of the bins before

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 CASES = [  # rows, logits, row stride beyond them, softcap
     (12, 1000, 0, 0.0), (12, 4099, 1, 0.0), (16, 20011, 0, 0.0), (15, 32768, 4, 0.0), (16, 65536, 0, 0.0), (23, 65541, 3, 0.0),
-    (14, 131072, 0, 0.0), (9, 262144, 0, 0.0), (6, 270001, 0, 0.0), (12, 30000, 0, 30.0), (12, 30001, 2, 30.0),
+    (14, 131072, 0, 0.0), (9, 262144, 0, 0.0), (6, 270001, 0, 0.0), (12, 30000, 0, 30.0), (12, 30001, 2, 30.0), (8, 266003, 2, 30.0),
 ]
 
 
